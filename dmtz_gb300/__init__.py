@@ -346,7 +346,7 @@ class Context:
         return a.value, b.value
 
     def autotune(self, f, g, dims=None):
-        """Time the gradient sweep for every brick shape / blocks-per-SM choice on
+        """Time the brick gradient kernel for every brick shape / blocks-per-SM choice on
         (f, g); keep the fastest in this context.  Returns (shape, blocks_per_sm, ms)."""
         dims = _dims_of(np.asarray(f), dims)
         ff, gg = _flat(f), _flat(g)
@@ -403,7 +403,7 @@ class Context:
         return [int(x) for x in c]
 
     def profile_sweep(self, f_ptr: int, g_ptr: int, dims, reps=10, on_device=True):
-        """Mean per-launch ms of the six gradient-sweep kernels and of the whole sweep."""
+        """Mean ms of one field's whole gradient in entries 0 and 6 (one kernel; the others are 0)."""
         ms = np.zeros(7, np.float64)
         self._check(self._L.dmtz_profile_sweep(self._h, *dims, _vp(f_ptr), _vp(g_ptr), int(bool(on_device)),
                                                int(reps), ms))

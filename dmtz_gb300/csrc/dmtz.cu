@@ -2,13 +2,13 @@
 //
 // Data layout in HBM, per field (original f, decompressed g), one entry per
 // anchor vertex, structure of arrays:
-//   key u64 | low u16 | pv u8 | ea2 u32 | fp3 u16 | fa3 u32 | eup u32 | fup u32 | crit u32
+//   pv u8 | eup u32 | fup u32 | crit u32 | tcode u32
 // plus, shared: f, g (float64), delta_counter (int32), request bits (1 bit per
 // vertex), the request list and the four mismatch lists (cell ids, int64).
 //
 // One correction round (main_3d.cu:6789-6921) is: fix rules on the mismatch
-// lists -> request bits/list; apply (bounded update of g); five pairing passes
-// on g; criticality + mismatch compaction.  Counters live on the device; the
+// lists -> request bits/list; apply (bounded update of g); the gradient of g
+// around the requests; mismatch compaction.  Counters live on the device; the
 // host reads four words per round (or none, in the CUDA-graph loop).
 #include <cuda_runtime.h>
 
@@ -26,8 +26,7 @@
 #include "../../include/dmtz.h"
 #include "cnn.cuh"
 #include "dmtz_common.cuh"
-#include "pairing.cuh"
-#include "pairing_fast.cuh"
+#include "gradient.cuh"
 #include "rules.cuh"
 
 using namespace dmtz;
@@ -152,36 +151,23 @@ __global__ void k_list_back(Lists T, Lists L) {
     if (tid < 4) L.n[tid] = T.n[tid];
 }
 
-// Dirty bricks, per pass.  The gradient state of an anchor depends on values
-// at most r_p anchors away in pass p: r = 1 (vertex pass), 2 (edge pass),
-// 3 (first triangle pass, -3..2), 3 (second edge pass), 4 (second triangle
-// pass), 5 (criticality, -5..4).  For every changed vertex, each brick within
-// 5 anchors gets bit r-1 for every r >= its distance (the largest per-axis gap
-// between the vertex and the brick's anchors); pass p re-pairs the bricks with
-// bit r_p - 1.  Flags are bytes packed four to a word (atomicOr on the word).
-constexpr int kRadii = 5;
-__global__ void k_mark_dirty(Grid g, int nbx, int nby, int nbz, int sx, int sy, int sz, const i64 *verts,
-                             const unsigned long long *nverts, uint32_t *flags) {
+// Dirty bricks.  A cell's pairing depends on the star of its highest vertex,
+// so a changed value reaches the cells whose highest vertex is the changed one
+// or a neighbour of it: anchors 2 below to 1 above per axis.  Every brick with
+// such an anchor is marked (one byte per brick; writers all store 1).
+constexpr int kReachLow = 2, kReachHigh = 1;
+__global__ void k_mark_dirty(Grid g, int nbx, int nby, int sx, int sy, int sz, const i64 *verts,
+                             const unsigned long long *nverts, uint8_t *flags) {
     const i64 n = (i64)*nverts;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
         int x, y, z;
         decode_v(g, verts[i], x, y, z);
-        const int x0 = max(x - kRadii, 0) / sx, x1 = min(x + kRadii, g.W - 1) / sx;
-        const int y0 = max(y - kRadii, 0) / sy, y1 = min(y + kRadii, g.H - 1) / sy;
-        const int z0 = max(z - kRadii, 0) / sz, z1 = min(z + kRadii, g.D - 1) / sz;
-        for (int bz = z0; bz <= z1; bz++) {
-            const int dz = max(0, max(bz * sz - z, z - (bz * sz + sz - 1)));
-            for (int by = y0; by <= y1; by++) {
-                const int dy = max(0, max(by * sy - y, y - (by * sy + sy - 1)));
-                for (int bx = x0; bx <= x1; bx++) {
-                    const int dx = max(0, max(bx * sx - x, x - (bx * sx + sx - 1)));
-                    const int d = max(dx, max(dy, dz));  // <= kRadii by the loop bounds
-                    const uint32_t mask = 0x1Fu & ~((1u << max(d - 1, 0)) - 1u);
-                    const i64 b = bx + (i64)nbx * (by + (i64)nby * bz);
-                    atomicOr(&flags[b >> 2], mask << (8 * (b & 3)));
-                }
-            }
-        }
+        const int x0 = max(x - kReachLow, 0) / sx, x1 = min(x + kReachHigh, g.W - 1) / sx;
+        const int y0 = max(y - kReachLow, 0) / sy, y1 = min(y + kReachHigh, g.H - 1) / sy;
+        const int z0 = max(z - kReachLow, 0) / sz, z1 = min(z + kReachHigh, g.D - 1) / sz;
+        for (int bz = z0; bz <= z1; bz++)
+            for (int by = y0; by <= y1; by++)
+                for (int bx = x0; bx <= x1; bx++) flags[bx + (i64)nbx * (by + (i64)nby * bz)] = 1;
     }
 }
 // Walk-cache tiles: 16^3 anchors.  Every brick the criticality pass re-pairs
@@ -201,23 +187,19 @@ __global__ void k_mark_tiles(const uint32_t *list, const unsigned long long *n, 
                 for (int tx = x0; tx <= x1; tx++) dirty[tx + (i64)ntx * (ty + (i64)nty * tz)] = 1;
     }
 }
-// one compacted brick list per radius (list r-1 holds the bricks with bit
-// r-1), and the flags cleared for the next round
-__global__ void k_compact_bricks(int nbx, int nby, int nbz, uint32_t *flags, uint32_t *lists, i64 stride,
-                                 unsigned long long *n) {
+// the marked bricks as a list, and the marks cleared for the next round (four
+// marks to a word)
+__global__ void k_compact_bricks(int nbx, int nby, int nbz, uint32_t *flags, uint32_t *list, unsigned long long *n) {
     const i64 nb = (i64)nbx * nby * nbz;
     for (i64 w = (i64)blockIdx.x * blockDim.x + threadIdx.x; w < (nb + 3) / 4; w += (i64)gridDim.x * blockDim.x) {
         const uint32_t word = flags[w];
         if (!word) continue;
         flags[w] = 0;
         for (int q = 0; q < 4; q++) {
-            const uint32_t m = (word >> (8 * q)) & 0xFFu;
-            if (!m) continue;
+            if (!((word >> (8 * q)) & 0xFFu)) continue;
             const i64 b = 4 * w + q;
             const int bx = (int)(b % nbx), by = (int)((b / nbx) % nby), bz = (int)(b / ((i64)nbx * nby));
-            const uint32_t code = (uint32_t)bx | ((uint32_t)by << 11) | ((uint32_t)bz << 22);
-            for (int r = 0; r < kRadii; r++)
-                if (m & (1u << r)) lists[r * stride + (i64)atomicAdd(&n[r], 1ull)] = code;
+            list[agg_slot(n)] = (uint32_t)bx | ((uint32_t)by << 11) | ((uint32_t)bz << 22);
         }
     }
 }
@@ -1511,12 +1493,7 @@ __global__ void k_propose(i64 V, const double *f, double *gv, const float *o, co
 }
 
 struct DevField {
-    uint64_t *key = nullptr;
-    uint16_t *low = nullptr;
     uint8_t *pv = nullptr;
-    uint32_t *ea2 = nullptr;
-    uint16_t *fp3 = nullptr;
-    uint32_t *fa3 = nullptr;
     uint32_t *eup = nullptr;
     uint32_t *fup = nullptr;
     uint32_t *crit = nullptr;
@@ -1550,13 +1527,13 @@ struct dmtz_ctx {
     i64 capDST = 0;
     i64 capAS = 0, capDS = 0, capSad2 = 0;
     uint8_t *succ = nullptr;  // original ascending-path successor of each tetrahedron
-    uint32_t *brick_flags = nullptr;  // per brick (a byte each, four to a word): radius bits of the next sweep
+    uint32_t *brick_flags = nullptr;  // per brick (a byte each, four to a word): in the next repair
     uint8_t *brick_fresh = nullptr;   // per brick: re-paired by the current round's criticality pass
     int inc_scan = 0;                 // repairs rebuild the mismatch lists incrementally (see k_list_keep)
     int strict_ds = 0;                // descending separatrix checks walk whole paths (k_ds_strict)
     i64 *list_tmp[4] = {nullptr, nullptr, nullptr, nullptr};  // rebuilt mismatch lists, capL entries each
-    uint32_t *brick_list = nullptr;   // compacted lists per radius, capB entries each
-    unsigned long long *brick_n = nullptr;  // their lengths
+    uint32_t *brick_list = nullptr;   // the repair's bricks, capB entries
+    unsigned long long *brick_n = nullptr;  // their number
     i64 *sad2 = nullptr;      // original 2-saddle triangles
     i64 *sad1 = nullptr;      // original 1-saddle edges (strict descending checks only)
     i64 capSad1 = 0;
@@ -1576,7 +1553,7 @@ struct dmtz_ctx {
     i64 capWS = 0;
     unsigned long long *counters = nullptr;  // [0..3] cp lists, [4] requests, [5,6] paths, [7] progress,
                                              // [8,9] min/max keys, [10] original 2-saddles, [12] edited
-                                             // vertices, [13,14] saddle counts, [15] surface anchors,
+                                             // vertices, [13,14] saddle counts,
                                              // [16] wall records, [17,18] deferred wall searches,
                                              // [20..23] rebuilt mismatch lists, [24] descending
                                              // records rebuildable, [25] their last count,
@@ -1589,9 +1566,7 @@ struct dmtz_ctx {
     std::vector<dmtz_ctx *> pool;  // worker contexts of dmtz_correct_batch
     uint8_t *mm = nullptr;         // mismatch bytes of the learned proposal's features
     i64 capMM = 0;
-    i64 *bnd = nullptr;            // surface anchors of the grid bndW x bndH x bndD (full sweeps)
-    i64 bnd_n = 0, bnd_cap = 0;
-    int bndW = 0, bndH = 0, bndD = 0;
+    int march_blocks = 0;          // blocks of k_grad_march the device holds at once (0: not asked yet)
     void *loopctl = nullptr;       // device copy of the graph loop's control block (kept: a
                                    // cudaFree per call would synchronise the whole device)
 };
@@ -1614,8 +1589,7 @@ cudaError_t dalloc(T **p, i64 n) {
 }
 
 void free_field(DevField &d) {
-    cudaFree(d.key); cudaFree(d.low); cudaFree(d.pv); cudaFree(d.ea2); cudaFree(d.fp3);
-    cudaFree(d.fa3); cudaFree(d.eup); cudaFree(d.fup); cudaFree(d.crit); cudaFree(d.tcode);
+    cudaFree(d.pv); cudaFree(d.eup); cudaFree(d.fup); cudaFree(d.crit); cudaFree(d.tcode);
     d = DevField();
 }
 void free_all(dmtz_ctx *c) {
@@ -1655,9 +1629,7 @@ void free_all(dmtz_ctx *c) {
 }
 
 dmtz_status alloc_field(dmtz_ctx *ctx, DevField &d, i64 V) {
-    CK(dalloc(&d.key, V)); CK(dalloc(&d.low, V)); CK(dalloc(&d.pv, V)); CK(dalloc(&d.ea2, V));
-    CK(dalloc(&d.fp3, V)); CK(dalloc(&d.fa3, V)); CK(dalloc(&d.eup, V)); CK(dalloc(&d.fup, V));
-    CK(dalloc(&d.crit, V)); CK(dalloc(&d.tcode, V));
+    CK(dalloc(&d.pv, V)); CK(dalloc(&d.eup, V)); CK(dalloc(&d.fup, V)); CK(dalloc(&d.crit, V)); CK(dalloc(&d.tcode, V));
     return DMTZ_OK;
 }
 
@@ -1700,7 +1672,7 @@ dmtz_status ensure(dmtz_ctx *ctx, const Grid &g) {
     CK(cudaMemset(ctx->reqbits, 0, sizeof(uint32_t) * (size_t)((V + 31) / 32 + 1)));
     CK(dalloc(&ctx->reqlist, V));
     CK(dalloc(&ctx->succ, 8 * V));
-    CK(dalloc(&ctx->brick_flags, (nbr + 3) / 4)); CK(dalloc(&ctx->brick_list, kRadii * nbr));
+    CK(dalloc(&ctx->brick_flags, (nbr + 3) / 4)); CK(dalloc(&ctx->brick_list, nbr));
     CK(dalloc(&ctx->brick_fresh, nbr));
     CK(dalloc(&ctx->brick_n, 8));
     CK(cudaMemset(ctx->brick_flags, 0, sizeof(uint32_t) * (size_t)((nbr + 3) / 4)));
@@ -1727,14 +1699,12 @@ dmtz_status grow_list(dmtz_ctx *ctx, const Grid &g, int k, i64 need) {
 
 FieldState view(const DevField &d, const double *val) {
     FieldState s;
-    s.val = val; s.key = d.key; s.low = d.low; s.pv = d.pv; s.ea2 = d.ea2; s.fp3 = d.fp3;
-    s.fa3 = d.fa3; s.eup = d.eup; s.fup = d.fup; s.crit = d.crit; s.tcode = d.tcode;
+    s.val = val; s.pv = d.pv; s.eup = d.eup; s.fup = d.fup; s.crit = d.crit; s.tcode = d.tcode;
     return s;
 }
 
 unsigned persistent_grid();
 
-// five passes + criticality (and mismatch lists when crit_o is given)
 i64 bricks_of(const Grid &g, int shape, int &nbx, int &nby, int &nbz) {
     nbx = (g.W + DMTZ_SHAPES[shape][0] - 1) / DMTZ_SHAPES[shape][0];
     nby = (g.H + DMTZ_SHAPES[shape][1] - 1) / DMTZ_SHAPES[shape][1];
@@ -1748,76 +1718,20 @@ bool shape_fits(const Grid &g, int shape) {
     return nbx <= 2048 && nby <= 2048 && nbz <= 1024;
 }
 
-unsigned sweep_grid(const dmtz_ctx *ctx, i64 nb) {
-    const unsigned cap = (unsigned)(persistent_grid() / 8) * (unsigned)ctx->tune_bps;
+// blocks of k_grad_bricks: its blocks hold 384 threads or more, so a quarter
+// of tune_bps (a count for blocks of 128) fills the SMs twice over
+unsigned brick_grid(const dmtz_ctx *ctx, i64 nb) {
+    const unsigned cap = (unsigned)(persistent_grid() / 8) * (unsigned)std::max(1, ctx->tune_bps / 4);
     return (unsigned)std::max<i64>(1, std::min<i64>(nb, cap));
 }
 
-// the five pairing passes and the criticality pass, each over its brick set
-void sweep_passes(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const BrickList bl[6], i64 nb_max) {
-    const unsigned gr = sweep_grid(ctx, nb_max);
-    cudaStream_t st = ctx->stream;
-    launch_pass<PASS_VERTEX>(g, s, bl[0], gr, st);
-    launch_pass<PASS_E2>(g, s, bl[1], gr, st);
-    launch_pass<PASS_F3>(g, s, bl[2], gr, st);
-    launch_pass<PASS_E4>(g, s, bl[3], gr, st);
-    launch_pass<PASS_F5>(g, s, bl[4], gr, st);
-    launch_pass<PASS_CRIT>(g, s, bl[5], gr, st);
-    ctx->launches += 6;
-}
-
-// the list of the grid's surface anchors, built once per grid shape
-bool surface_list(dmtz_ctx *ctx, const Grid &g) {
-    if (ctx->bnd && ctx->bndW == g.W && ctx->bndH == g.H && ctx->bndD == g.D) return true;
-    const i64 need = std::min<i64>(g.V, 2 * ((i64)g.W * g.H + (i64)g.W * g.D + (i64)g.H * g.D));
-    if (need > ctx->bnd_cap) {
-        cudaFree(ctx->bnd);
-        ctx->bnd = nullptr;
-        ctx->bnd_cap = 0;
-        if (dalloc(&ctx->bnd, need) != cudaSuccess) {
-            cudaGetLastError();
-            ctx->bnd = nullptr;
-            return false;
-        }
-        ctx->bnd_cap = need;
+// the gradient of a set of bricks
+void grad_bricks(const Grid &g, const FieldState &s, const BrickList &bl, unsigned grid, cudaStream_t st) {
+    switch (bl.shape) {
+    case 1: k_grad_bricks<16, 4, 2><<<grid, brick_threads<16, 4, 2>(), 0, st>>>(g, s, bl); break;
+    case 2: k_grad_bricks<32, 2, 2><<<grid, brick_threads<32, 2, 2>(), 0, st>>>(g, s, bl); break;
+    default: k_grad_bricks<8, 4, 4><<<grid, brick_threads<8, 4, 4>(), 0, st>>>(g, s, bl); break;
     }
-    cudaMemsetAsync(ctx->counters + 15, 0, sizeof(unsigned long long), ctx->stream);
-    k_bnd_list<<<grid_for(g.V), kBlock, 0, ctx->stream>>>(g, ctx->bnd, ctx->counters + 15);
-    unsigned long long n = 0;
-    cudaMemcpyAsync(&n, ctx->counters + 15, sizeof(n), cudaMemcpyDeviceToHost, ctx->stream);
-    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;
-    ctx->bnd_n = (i64)n;
-    ctx->bndW = g.W;
-    ctx->bndH = g.H;
-    ctx->bndD = g.D;
-    return true;
-}
-
-// the five pairing passes and the criticality pass over a set of bricks; a
-// full sweep runs the grid's surface anchors separately, in dense warps
-void sweep(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const BrickList &bl, i64 nb_max) {
-    if (bl.list == nullptr && surface_list(ctx, g)) {
-        const unsigned gr = sweep_grid(ctx, nb_max);
-        cudaStream_t st = ctx->stream;
-        const i64 *b = ctx->bnd;
-        const i64 nbd = ctx->bnd_n;
-        launch_pass<PASS_VERTEX>(g, s, bl, gr, st, 1);
-        launch_bnd<PASS_VERTEX>(g, s, b, nbd, st);
-        launch_pass<PASS_E2>(g, s, bl, gr, st, 1);
-        launch_bnd<PASS_E2>(g, s, b, nbd, st);
-        launch_pass<PASS_F3>(g, s, bl, gr, st, 1);
-        launch_bnd<PASS_F3>(g, s, b, nbd, st);
-        launch_pass<PASS_E4>(g, s, bl, gr, st, 1);
-        launch_bnd<PASS_E4>(g, s, b, nbd, st);
-        launch_pass<PASS_F5>(g, s, bl, gr, st, 1);
-        launch_bnd<PASS_F5>(g, s, b, nbd, st);
-        launch_pass<PASS_CRIT>(g, s, bl, gr, st, 1);
-        launch_bnd<PASS_CRIT>(g, s, b, nbd, st);
-        ctx->launches += 12;
-        return;
-    }
-    const BrickList per_pass[6] = {bl, bl, bl, bl, bl, bl};
-    sweep_passes(ctx, g, s, per_pass, nb_max);
 }
 
 BrickList all_bricks(const Grid &g, int shape, i64 &nb) {
@@ -1829,6 +1743,50 @@ BrickList all_bricks(const Grid &g, int shape, i64 &nb) {
     bl.dbx = make_fdiv((unsigned long long)bl.nbx);
     bl.dby = make_fdiv((unsigned long long)bl.nby);
     return bl;
+}
+
+// The gradient of the whole grid.  Grids whose bricks fit the GPU in one round
+// (three blocks of k_grad_bricks per SM) take one latency of that kernel: 16^3
+// 6.2 us, against 14.4 us for the march's five pipeline steps; larger ones
+// march (64^3: 25 us, 30 us in bricks; 256^3: 862 us, 1634 us in bricks).
+// Tiles of 32 x 16 columns and one block of 640 threads per SM: with two
+// blocks and 48 registers 935 us at 256^3 and 51 us instead of 43 us at 97 x 61 x
+// 75; 32 x 8 with three blocks 874 and 51 us; 64 x 8 1035 and 58 us.
+constexpr int kMarchX = 32, kMarchY = 16, kMarchBlocks = 1;
+void grad_full(dmtz_ctx *ctx, const Grid &g, const FieldState &s) {
+    {
+        i64 nb;
+        const BrickList bl = all_bricks(g, ctx->tune_shape, nb);
+        if (nb <= (i64)(persistent_grid() / 8) * 3) {
+            grad_bricks(g, s, bl, (unsigned)nb, ctx->stream);
+            ctx->launches++;
+            return;
+        }
+    }
+    using M = March<kMarchX, kMarchY>;
+    auto kern = k_grad_march<kMarchX, kMarchY, kMarchBlocks>;
+    if (!ctx->march_blocks) {
+        int per_sm = 0;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, M::NT, M::smem);
+        ctx->march_blocks = std::max(1, per_sm) * (int)(persistent_grid() / 8);
+    }
+    const int ntx = (g.W + kMarchX - 1) / kMarchX, nty = (g.H + kMarchY - 1) / kMarchY;
+    const i64 tiles = (i64)ntx * nty;
+    // planes per block: the fewest steps over all waves (a block's pipeline
+    // takes four steps more than it has planes)
+    int chunk = 1;
+    i64 best = -1;
+    for (int c = 1; c <= g.D; c++) {
+        const i64 waves = (tiles * ((g.D + c - 1) / c) + ctx->march_blocks - 1) / ctx->march_blocks, cost = waves * (c + 4);
+        if (best < 0 || cost < best) {
+            best = cost;
+            chunk = c;
+        }
+    }
+    const i64 blocks = tiles * ((g.D + chunk - 1) / chunk);
+    kern<<<(unsigned)blocks, M::NT, M::smem, ctx->stream>>>(g, s, ntx, nty, chunk);
+    ctx->launches++;
 }
 
 // mismatch lists of the decompressed gradient against crit_o
@@ -1846,9 +1804,7 @@ void scan_mismatch(dmtz_ctx *ctx, const Grid &g, const uint32_t *crit_d, const u
 
 // full gradient of one field (and its mismatch lists when crit_o is given)
 void run_pairing(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32_t *crit_o, int want_saddles) {
-    i64 nb;
-    const BrickList bl = all_bricks(g, ctx->tune_shape, nb);
-    sweep(ctx, g, s, bl, nb);
+    grad_full(ctx, g, s);
     if (crit_o) scan_mismatch(ctx, g, s.crit, crit_o, want_saddles);
 }
 
@@ -1857,39 +1813,30 @@ void run_pairing(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32
 void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32_t *crit_o, int want_saddles) {
     int nbx, nby, nbz;
     const int shape = ctx->tune_shape;
-    const i64 nb = bricks_of(g, shape, nbx, nby, nbz);
+    i64 nb = bricks_of(g, shape, nbx, nby, nbz);
     cudaStream_t st = ctx->stream;
-    cudaMemsetAsync(ctx->brick_n, 0, kRadii * sizeof(unsigned long long), st);
-    k_mark_dirty<<<persistent_grid(), kBlock, 0, st>>>(g, nbx, nby, nbz, DMTZ_SHAPES[shape][0], DMTZ_SHAPES[shape][1],
+    cudaMemsetAsync(ctx->brick_n, 0, sizeof(unsigned long long), st);
+    k_mark_dirty<<<persistent_grid(), kBlock, 0, st>>>(g, nbx, nby, DMTZ_SHAPES[shape][0], DMTZ_SHAPES[shape][1],
                                                         DMTZ_SHAPES[shape][2], ctx->reqlist, ctx->counters + 4,
-                                                        ctx->brick_flags);
-    k_compact_bricks<<<persistent_grid(), kBlock, 0, st>>>(nbx, nby, nbz, ctx->brick_flags, ctx->brick_list,
-                                                            ctx->capB, ctx->brick_n);
+                                                        reinterpret_cast<uint8_t *>(ctx->brick_flags));
+    k_compact_bricks<<<persistent_grid(), kBlock, 0, st>>>(nbx, nby, nbz, ctx->brick_flags, ctx->brick_list, ctx->brick_n);
     ctx->launches += 2;
-    const uint32_t *r5 = ctx->brick_list + (i64)(kRadii - 1) * ctx->capB;
-    const unsigned long long *r5n = ctx->brick_n + (kRadii - 1);
     if (ctx->inc_scan) {
         cudaMemsetAsync(ctx->brick_fresh, 0, (size_t)nb, st);
-        k_mark_fresh<<<persistent_grid(), kBlock, 0, st>>>(r5, r5n, ctx->brick_fresh, nbx, nby);
+        k_mark_fresh<<<persistent_grid(), kBlock, 0, st>>>(ctx->brick_list, ctx->brick_n, ctx->brick_fresh, nbx, nby);
         ctx->launches++;
     }
-    if (ctx->tile_dirty && ctx->ntx > 0) {  // the criticality pass's bricks cover every anchor re-paired
-        k_mark_tiles<<<persistent_grid(), kBlock, 0, st>>>(r5, r5n, DMTZ_SHAPES[shape][0],
+    if (ctx->tile_dirty && ctx->ntx > 0) {
+        k_mark_tiles<<<persistent_grid(), kBlock, 0, st>>>(ctx->brick_list, ctx->brick_n, DMTZ_SHAPES[shape][0],
                                                             DMTZ_SHAPES[shape][1], DMTZ_SHAPES[shape][2], ctx->ntx,
                                                             ctx->nty, ctx->ntz, ctx->tile_dirty);
         ctx->launches++;
     }
-    static const int radius[6] = {1, 2, 3, 3, 4, 5};  // per pass
-    BrickList bl[6];
-    for (int p = 0; p < 6; p++) {
-        bl[p].list = ctx->brick_list + (i64)(radius[p] - 1) * ctx->capB;
-        bl[p].n = ctx->brick_n + (radius[p] - 1);
-        bl[p].nbx = nbx; bl[p].nby = nby; bl[p].nbz = nbz;
-        bl[p].dbx = make_fdiv((unsigned long long)nbx);
-        bl[p].dby = make_fdiv((unsigned long long)nby);
-        bl[p].shape = shape;
-    }
-    sweep_passes(ctx, g, s, bl, nb);
+    BrickList bl = all_bricks(g, shape, nb);
+    bl.list = ctx->brick_list;
+    bl.n = ctx->brick_n;
+    grad_bricks(g, s, bl, brick_grid(ctx, nb), st);
+    ctx->launches++;
     if (!ctx->inc_scan) {
         scan_mismatch(ctx, g, s.crit, crit_o, want_saddles);
         return;
@@ -1906,7 +1853,7 @@ void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint3
     const unsigned pg = persistent_grid();
     cudaMemsetAsync(ctx->counters + 20, 0, 4 * sizeof(unsigned long long), st);
     k_list_keep<<<pg, kBlock, 0, st>>>(g, L, T, ctx->brick_fresh, sx, sy, sz, nbx, nby);
-    k_scan_fresh<<<pg, kBlock, 0, st>>>(g, s.crit, crit_o, T, r5, r5n, sx, sy, sz, want_saddles);
+    k_scan_fresh<<<pg, kBlock, 0, st>>>(g, s.crit, crit_o, T, ctx->brick_list, ctx->brick_n, sx, sy, sz, want_saddles);
     k_list_back<<<pg, kBlock, 0, st>>>(T, L);
     ctx->launches += 3;
 }
@@ -2437,7 +2384,6 @@ void dmtz_ctx_destroy(dmtz_ctx *ctx) {
     cudaSetDevice(ctx->device);
     free_all(ctx);
     cudaFree(ctx->mm);
-    cudaFree(ctx->bnd);
     cudaFree(ctx->loopctl);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->side) cudaStreamDestroy(ctx->side);
@@ -3107,8 +3053,8 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             // kernels per body run: switch + control, plus each state's own
             const int64_t det = detect_kernels(ctx, conn);  // separatrix detection kernels
             // a fix round: fix + update, then the repair (dirty marks, compaction,
-            // fresh and tile marks, six passes, the list rebuild)
-            const int64_t rnd = 2 + 2 + (ctx->inc_scan ? 1 : 0) + (ctx->tile_dirty ? 1 : 0) + 6 + (ctx->inc_scan ? 3 : 1);
+            // fresh and tile marks, the gradient, the list rebuild)
+            const int64_t rnd = 2 + 2 + (ctx->inc_scan ? 1 : 0) + (ctx->tile_dirty ? 1 : 0) + 1 + (ctx->inc_scan ? 3 : 1);
             const int64_t rnd_cp = rnd - 1 + (ps == 1 ? 5 : 3);  // the fix round's two forms (launch_fix_cp)
             ctx->launches += 2 * (fin.runs[0] + fin.runs[1] + fin.runs[2] + fin.runs[3]) + rnd_cp * fin.runs[LS_CP] +
                              (rnd + det) * fin.runs[LS_PDF] + det * fin.runs[LS_PCHECK] + rnd * fin.runs[LS_PFIX];
@@ -3508,11 +3454,14 @@ dmtz_status dmtz_autotune(dmtz_ctx *ctx, int W, int H, int D, const double *orig
         for (int bi = 0; bi < 4; bi++) {
             ctx->tune_shape = sh;
             ctx->tune_bps = bps_opts[bi];
-            run_pairing(ctx, g, Qs, nullptr, 1);  // warm
+            i64 nb;
+            const BrickList bl = all_bricks(g, sh, nb);
+            const unsigned gr = brick_grid(ctx, nb);
+            grad_bricks(g, Qs, bl, gr, st);  // warm
             float t_min = 1e30f;
             for (int r = 0; r < 3; r++) {
                 CK(cudaEventRecord(e0, st));
-                run_pairing(ctx, g, Qs, nullptr, 1);
+                grad_bricks(g, Qs, bl, gr, st);
                 CK(cudaEventRecord(e1, st));
                 CK(cudaEventSynchronize(e1));
                 float t = 0;
@@ -3630,50 +3579,17 @@ dmtz_status dmtz_profile_sweep(dmtz_ctx *ctx, int W, int H, int D, const double 
     const FieldState Ps = view(ctx->P, ctx->f), Qs = view(ctx->Q, ctx->g);
     run_pairing(ctx, g, Ps, nullptr, 1);
     run_pairing(ctx, g, Qs, ctx->P.crit, 1);  // warm-up
-    cudaEvent_t ev[7];
+    cudaEvent_t ev[2];
     for (auto &e : ev) CK(cudaEventCreate(&e));
-    double acc[6] = {0, 0, 0, 0, 0, 0};
+    CK(cudaEventRecord(ev[0], st));
+    for (int r = 0; r < reps; r++) grad_full(ctx, g, Qs);
+    CK(cudaEventRecord(ev[1], st));
+    CK(cudaEventSynchronize(ev[1]));
     float total = 0;
-    i64 nb;
-    const BrickList bl = all_bricks(g, ctx->tune_shape, nb);
-    const unsigned gr = sweep_grid(ctx, nb);
-    // as a full sweep runs them: each pass's brick kernel, then its surface anchors
-    const int sk = surface_list(ctx, g) ? 1 : 0;
-    const i64 *bd = ctx->bnd;
-    const i64 nbd = sk ? ctx->bnd_n : 0;
-    for (int r = 0; r < reps; r++) {
-        CK(cudaEventRecord(ev[0], st));
-        launch_pass<PASS_VERTEX>(g, Qs, bl, gr, st, sk);
-        launch_bnd<PASS_VERTEX>(g, Qs, bd, nbd, st);
-        CK(cudaEventRecord(ev[1], st));
-        launch_pass<PASS_E2>(g, Qs, bl, gr, st, sk);
-        launch_bnd<PASS_E2>(g, Qs, bd, nbd, st);
-        CK(cudaEventRecord(ev[2], st));
-        launch_pass<PASS_F3>(g, Qs, bl, gr, st, sk);
-        launch_bnd<PASS_F3>(g, Qs, bd, nbd, st);
-        CK(cudaEventRecord(ev[3], st));
-        launch_pass<PASS_E4>(g, Qs, bl, gr, st, sk);
-        launch_bnd<PASS_E4>(g, Qs, bd, nbd, st);
-        CK(cudaEventRecord(ev[4], st));
-        launch_pass<PASS_F5>(g, Qs, bl, gr, st, sk);
-        launch_bnd<PASS_F5>(g, Qs, bd, nbd, st);
-        CK(cudaEventRecord(ev[5], st));
-        launch_pass<PASS_CRIT>(g, Qs, bl, gr, st, sk);
-        launch_bnd<PASS_CRIT>(g, Qs, bd, nbd, st);
-        CK(cudaEventRecord(ev[6], st));
-        CK(cudaEventSynchronize(ev[6]));
-        for (int k = 0; k < 6; k++) {
-            float t = 0;
-            cudaEventElapsedTime(&t, ev[k], ev[k + 1]);
-            acc[k] += t;
-        }
-        float t = 0;
-        cudaEventElapsedTime(&t, ev[0], ev[6]);
-        total += t;
-    }
+    cudaEventElapsedTime(&total, ev[0], ev[1]);
     for (auto &e : ev) cudaEventDestroy(e);
-    for (int k = 0; k < 6; k++) ms[k] = acc[k] / reps;
-    ms[6] = total / reps;
+    for (int k = 0; k < 7; k++) ms[k] = 0;
+    ms[0] = ms[6] = total / reps;  // one kernel does every pass
     CK(cudaGetLastError());
     return DMTZ_OK;
 }
@@ -3689,13 +3605,8 @@ namespace {
 // starting on a 256-byte boundary
 constexpr i64 kNaV = DMTZ_NOALLOC_MAX_VERTICES;
 constexpr i64 na_round(i64 b) { return (b + 255) / 256 * 256; }
-constexpr i64 kNaKey = 0;
-constexpr i64 kNaLow = kNaKey + na_round(kNaV * 8);
-constexpr i64 kNaPv = kNaLow + na_round(kNaV * 2);
-constexpr i64 kNaEa2 = kNaPv + na_round(kNaV * 1);
-constexpr i64 kNaFp3 = kNaEa2 + na_round(kNaV * 4);
-constexpr i64 kNaFa3 = kNaFp3 + na_round(kNaV * 2);
-constexpr i64 kNaEup = kNaFa3 + na_round(kNaV * 4);
+constexpr i64 kNaPv = 0;
+constexpr i64 kNaEup = kNaPv + na_round(kNaV * 1);
 constexpr i64 kNaFup = kNaEup + na_round(kNaV * 4);
 // no criticality array: the export reads the pairing state alone
 constexpr i64 kNaBytes = kNaFup + na_round(kNaV * 4);
@@ -3742,12 +3653,7 @@ extern "C" dmtz_status dmtz_extract_noalloc(int W, int H, int D, const double *d
     if (noalloc_scratch(dev, &base) != cudaSuccess) return DMTZ_ERR_CUDA;
     FieldState s;
     s.val = data;
-    s.key = (uint64_t *)(base + kNaKey);
-    s.low = (uint16_t *)(base + kNaLow);
     s.pv = (uint8_t *)(base + kNaPv);
-    s.ea2 = (uint32_t *)(base + kNaEa2);
-    s.fp3 = (uint16_t *)(base + kNaFp3);
-    s.fa3 = (uint32_t *)(base + kNaFa3);
     s.eup = (uint32_t *)(base + kNaEup);
     s.fup = (uint32_t *)(base + kNaFup);
     s.crit = nullptr;
@@ -3755,12 +3661,7 @@ extern "C" dmtz_status dmtz_extract_noalloc(int W, int H, int D, const double *d
     cudaStream_t st = (cudaStream_t)stream;
     i64 nb;
     const BrickList bl = all_bricks(g, 0, nb);
-    const unsigned gb = (unsigned)std::max<i64>(1, std::min<i64>(nb, (i64)persistent_grid() * 2));
-    launch_pass<PASS_VERTEX>(g, s, bl, gb, st);
-    launch_pass<PASS_E2>(g, s, bl, gb, st);
-    launch_pass<PASS_F3>(g, s, bl, gb, st);
-    launch_pass<PASS_E4>(g, s, bl, gb, st);
-    launch_pass<PASS_F5>(g, s, bl, gb, st);
+    grad_bricks(g, s, bl, (unsigned)std::max<i64>(1, std::min<i64>(nb, persistent_grid())), st);
     k_export<<<grid_for(g.V), kBlock, 0, st>>>(g, s, PV, PE, PF, PT);
     return cudaGetLastError() == cudaSuccess ? DMTZ_OK : DMTZ_ERR_CUDA;
 }

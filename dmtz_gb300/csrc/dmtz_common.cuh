@@ -63,12 +63,6 @@ struct Grid {
     i64 bxy, byz, bxz;  // first ids of yz-plane, xz-plane, interior triangles
     i64 doff[14];  // linear offset of each stencil direction
     i64 coff[8];   // linear offset of each cube corner
-    // 32-bit copies for grids of fewer than 2^31 vertices (small != 0): the
-    // interior fast path indexes with 32-bit integers there
-    int small;
-    int WHi;
-    int doff32[14];
-    int coff32[8];
     // divisors of the id decodes: W, H, W-1, H-1, D-1, and the plane sizes
     // (W-1)H, W(H-1), W(D-1), (H-1)(D-1), (W-1)(D-1), (W-1)(H-1)
     FDiv dW, dH, dW1, dH1, dD1, dW1H, dWH1, dWD1, dH1D1, dW1D1, dW1H1;
@@ -95,10 +89,6 @@ static inline Grid make_grid(int W, int H, int D) {
                                     {-1, 0, 1}, {1, 0, -1}, {-1, 1, 1}, {1, -1, -1}};
     for (int i = 0; i < 14; i++) g.doff[i] = dirs[i][0] + dirs[i][1] * w + dirs[i][2] * w * h;
     for (int c8 = 0; c8 < 8; c8++) g.coff[c8] = (c8 & 1) + ((c8 >> 1) & 1) * w + ((c8 >> 2) & 1) * w * h;
-    g.small = g.V < (1LL << 31) ? 1 : 0;
-    g.WHi = g.small ? (int)g.WH : 0;
-    for (int i = 0; i < 14; i++) g.doff32[i] = g.small ? (int)g.doff[i] : 0;
-    for (int c8 = 0; c8 < 8; c8++) g.coff32[c8] = g.small ? (int)g.coff[c8] : 0;
     g.dW = make_fdiv(w); g.dH = make_fdiv(h); g.dW1 = make_fdiv(w - 1); g.dH1 = make_fdiv(h - 1);
     g.dD1 = make_fdiv(d - 1); g.dW1H = make_fdiv((w - 1) * h); g.dWH1 = make_fdiv(w * (h - 1));
     g.dWD1 = make_fdiv(w * (d - 1)); g.dH1D1 = make_fdiv((h - 1) * (d - 1)); g.dW1D1 = make_fdiv((w - 1) * (d - 1));
@@ -249,14 +239,9 @@ __device__ __forceinline__ int fup_get(uint32_t w, int s) { return (w >> (2 * s)
 // Per-field device state (structure of arrays, one entry per anchor vertex)
 struct FieldState {
     const double *val;   // field values (f or g)
-    uint64_t *key;       // okey(val)
-    uint16_t *low;       // bit i: neighbour i exists and is below this vertex
     uint8_t *pv;
-    uint32_t *ea2;       // edge pass a2=0 result
-    uint16_t *fp3;       // triangles paired after the first triangle pass
-    uint32_t *fa3;       // triangle pass a2=0 result
-    uint32_t *eup;       // final edge -> triangle
-    uint32_t *fup;       // final triangle -> tetrahedron
+    uint32_t *eup;       // edge -> triangle
+    uint32_t *fup;       // triangle -> tetrahedron
     uint32_t *crit;      // bit 0 vertex, 1..7 edges, 8..19 triangles, 20..25 tetrahedra
     uint32_t *tcode;     // 6 x 3 bits: which facet (TOPO_TET_FACE order) each tetrahedron
                          // is paired with, 7 = unpaired or absent (may be null)

@@ -260,10 +260,12 @@ typedef struct {
 dmtz_status dmtz_correct_batch(dmtz_ctx *ctx, int n, const dmtz_instance *inst, const dmtz_opts *opts,
                                dmtz_report *reports, dmtz_status *status, int workers);
 
-/* Brick shape (0: 8x4x4, 1: 16x4x2, 2: 32x2x2 anchors) and blocks per SM of
- * the gradient sweeps.  Results do not depend on them, only speed.
- * dmtz_autotune times a full sweep of `decp` for every shape and 8, 16, 32, 64
- * blocks per SM, keeps the fastest in the context and returns it in best[2]. */
+/* Brick shape (0: 8x4x4, 1: 16x4x2, 2: 32x2x2 anchors) and blocks per SM
+ * (counted for blocks of 128 threads) of the gradient kernel that re-pairs
+ * bricks after an update.  Results do not depend on them, only speed.
+ * dmtz_autotune times that kernel over every brick of `decp` for every shape
+ * and 8, 16, 32, 64 blocks per SM, keeps the fastest in the context and returns
+ * it in best[2]. */
 dmtz_status dmtz_set_tuning(dmtz_ctx *ctx, int shape, int blocks_per_sm);
 /* Memory of the mismatch lists (critical cells that differ between the two
  * gradients).  Each of the four lists starts with room for `fraction` of the
@@ -279,11 +281,10 @@ dmtz_status dmtz_get_tuning(const dmtz_ctx *ctx, int *shape, int *blocks_per_sm)
 dmtz_status dmtz_autotune(dmtz_ctx *ctx, int W, int H, int D, const double *orig, const double *decp, int on_device,
                           int best[2], double *best_ms);
 
-/* Timing of the gradient sweep that every correction round runs (the five
- * pairing passes of main_3d.cu:6864-6874 plus the critical-cell comparison
- * of :6903-6909), `reps` times on the context's stream between CUDA events.
- * ms[0..5] = mean per-launch time of the vertex, edge, triangle, edge,
- * triangle and criticality kernels; ms[6] = mean time of one whole sweep.
+/* Timing of one field's whole gradient (the five pairing passes of
+ * main_3d.cu:6864-6874 plus the criticality of every cell, one kernel), `reps`
+ * times on the context's stream between CUDA events.  ms[0] and ms[6] = mean
+ * time of one gradient; ms[1..5] = 0 (the passes have no kernels of their own).
  * No counterpart call in the reference (measurement only). */
 dmtz_status dmtz_profile_sweep(dmtz_ctx *ctx, int W, int H, int D, const double *orig, const double *decp,
                                int on_device, int reps, double ms[7]);
@@ -381,7 +382,7 @@ dmtz_status dmtz_correct_learned(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int
  *
  * Scratch: the per-vertex gradient state lives in one fixed device array
  * inside the library, sized for at most DMTZ_NOALLOC_MAX_VERTICES vertices
- * (64^3; about 7.6 MB that every GPU which loads the library keeps until the
+ * (64^3; about 2.4 MB that every GPU which loads the library keeps until the
  * process exits).  Larger grids return DMTZ_ERR_TOO_LARGE.  The first call on
  * a device looks up that array's device address (cudaGetSymbolAddress), so
  * make that first call before any stream capture.  The address is kept for
