@@ -38,15 +38,23 @@ static inline unsigned grid_for(i64 n) { return (unsigned)std::max<i64>(1, (n + 
 
 // --------------------------------------------------------------- mismatch compaction
 struct Lists {
-    i64 *l[4];                  // min, 1-saddle, 2-saddle, max (reference cell ids)
+    i64 *l[4];                  // min, 1-saddle, 2-saddle, max (cell codes, see rules.cuh)
     unsigned long long *n;      // 4 counters
     i64 cap[4];                 // capacities; a counter above its capacity = overflow,
                                 // the host grows the list and scans again
 };
 
-__device__ __forceinline__ void push_list(const Lists &L, int k, i64 id) {
+__device__ __forceinline__ void push_list(const Lists &L, int k, i64 code) {
     const unsigned long long at = agg_slot(&L.n[k]);
-    if ((i64)at < L.cap[k]) L.l[k][at] = id;
+    if ((i64)at < L.cap[k]) L.l[k][at] = code;
+}
+// the mismatched cells d (bits of FieldState::crit) of anchor v
+__device__ __forceinline__ void push_cells(const Lists &L, i64 v, uint32_t d) {
+    while (d) {
+        const int b = __ffs(d) - 1;
+        d &= d - 1;
+        push_list(L, b == 0 ? 0 : b < 8 ? 1 : b < 20 ? 2 : 3, cell_code(v, b));
+    }
 }
 
 // mismatch between the decompressed and the original critical cells
@@ -56,17 +64,7 @@ __global__ void k_mismatch_scan(Grid g, const uint32_t *crit_d, const uint32_t *
     for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += (i64)gridDim.x * blockDim.x) {
         uint32_t d = crit_d[v] ^ crit_o[v];
         if (!want_saddles) d &= 1u | (0x3Fu << 20);
-        if (!d) continue;
-        int x, y, z;
-        decode_v(g, v, x, y, z);
-        while (d) {
-            const int b = __ffs(d) - 1;
-            d &= d - 1;
-            if (b == 0) push_list(L, 0, v);
-            else if (b < 8) push_list(L, 1, edge_ref(g, x, y, z, b - 1));
-            else if (b < 20) push_list(L, 2, face_ref(g, x, y, z, b - 8));
-            else push_list(L, 3, tet_ref(g, x, y, z, b - 20));
-        }
+        push_cells(L, v, d);
     }
 }
 
@@ -88,27 +86,25 @@ __global__ void k_list_keep(Grid g, Lists L, Lists T, const uint8_t *fresh, int 
     const i64 n0 = min((i64)L.n[0], L.cap[0]), n1 = min((i64)L.n[1], L.cap[1]), n2 = min((i64)L.n[2], L.cap[2]),
               n3 = min((i64)L.n[3], L.cap[3]);
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n0 + n1 + n2 + n3; i += (i64)gridDim.x * blockDim.x) {
-        int k, x, y, z, sl;
-        i64 id;
+        int k;
+        i64 code;
         if (i < n0) {
             k = 0;
-            id = L.l[0][i];
-            decode_v(g, id, x, y, z);
+            code = L.l[0][i];
         } else if (i < n0 + n1) {
             k = 1;
-            id = L.l[1][i - n0];
-            edge_unref(g, id, x, y, z, sl);
+            code = L.l[1][i - n0];
         } else if (i < n0 + n1 + n2) {
             k = 2;
-            id = L.l[2][i - n0 - n1];
-            face_unref(g, id, x, y, z, sl);
+            code = L.l[2][i - n0 - n1];
         } else {
             k = 3;
-            id = L.l[3][i - n0 - n1 - n2];
-            tet_unref(g, id, x, y, z, sl);
+            code = L.l[3][i - n0 - n1 - n2];
         }
+        int x, y, z;
+        decode_v(g, code >> 5, x, y, z);
         if (fresh[x / sx + (i64)nbx * (y / sy + (i64)nby * (z / sz))]) continue;
-        push_list(T, k, id);
+        push_list(T, k, code);
     }
 }
 // the anchors of the fresh bricks (one block per listed brick step)
@@ -125,14 +121,7 @@ __global__ void k_scan_fresh(Grid g, const uint32_t *crit_d, const uint32_t *cri
             const i64 v = x + (i64)y * g.W + (i64)z * g.WH;
             uint32_t d = crit_d[v] ^ crit_o[v];
             if (!want_saddles) d &= 1u | (0x3Fu << 20);
-            while (d) {
-                const int bit = __ffs(d) - 1;
-                d &= d - 1;
-                if (bit == 0) push_list(T, 0, v);
-                else if (bit < 8) push_list(T, 1, edge_ref(g, x, y, z, bit - 1));
-                else if (bit < 20) push_list(T, 2, face_ref(g, x, y, z, bit - 8));
-                else push_list(T, 3, tet_ref(g, x, y, z, bit - 20));
-            }
+            push_cells(T, v, d);
         }
     }
 }
@@ -271,62 +260,37 @@ struct CpLists {
 
 // fix_minimum, [fix_saddle, fix_2saddle], fix_maximum over the current lists
 // (the host never runs this on an overflowed list; the clamp only keeps
-// every read inside the allocation).  Two forms, chosen on the device from
-// the list lengths, so that a graph can hold both: when every listed cell
-// fits one pass of the grid (`pass` threads), k_fix_cp gives each thread one
-// cell of the concatenated lists and the four rules' latency chains overlap;
-// longer lists (the first rounds of noisy fields: millions of cells) go to
-// one kernel per cell type, k_fix_cp_t, whose code holds one rule tree: in one
-// kernel the four case trees thrashed the instruction cache (a few active
-// lanes per warp, warps stalled on instruction fetch).  The rules only set
-// request bits, so neither form changes the result.
-__device__ __forceinline__ void cp_counts(const CpLists &L, int preserve_saddles, i64 n[4]) {
-    n[0] = min((i64)L.n[0], L.cap[0]);
-    n[1] = preserve_saddles ? min((i64)L.n[1], L.cap[1]) : 0;
-    n[2] = preserve_saddles ? min((i64)L.n[2], L.cap[2]) : 0;
-    n[3] = min((i64)L.n[3], L.cap[3]);
-}
-__global__ void k_fix_cp(RuleCtx c, CpLists L, int preserve_saddles, i64 pass) {
-    i64 n[4];
-    cp_counts(L, preserve_saddles, n);
-    if (n[0] + n[1] + n[2] + n[3] > pass) return;  // the per-type kernels take it
-    i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n[0]) { rule_min(c, L.l[0][i]); return; }
-    i -= n[0];
-    if (i < n[1]) { rule_saddle(c, L.l[1][i]); return; }
-    i -= n[1];
-    if (i < n[2]) { rule_2saddle(c, L.l[2][i]); return; }
-    i -= n[2];
-    if (i < n[3]) rule_max(c, L.l[3][i]);
-}
-template <int T>
-__global__ void k_fix_cp_t(RuleCtx c, CpLists L, int preserve_saddles, i64 pass) {
-    i64 n[4];
-    cp_counts(L, preserve_saddles, n);
-    if (n[0] + n[1] + n[2] + n[3] <= pass) return;  // k_fix_cp took it
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n[T]; i += (i64)gridDim.x * blockDim.x) {
-        if (T == 0) rule_min(c, L.l[0][i]);
-        else if (T == 1) rule_saddle(c, L.l[1][i]);
-        else if (T == 2) rule_2saddle(c, L.l[2][i]);
-        else rule_max(c, L.l[3][i]);
+// every read inside the allocation).  The four lists are taken one behind the
+// other, each padded to whole warps, so that a warp runs one rule: short
+// lists run side by side in different warps, and in long ones (the first
+// rounds of noisy fields: millions of cells) all warps of the GPU are in the
+// same rule's code.  The rules only set request bits, so the order does not
+// matter.
+__global__ void __launch_bounds__(kBlock) k_fix_cp(const __grid_constant__ RuleCtx c, CpLists L, int preserve_saddles) {
+    __shared__ RuleTab tab;
+    const i64 n0 = min((i64)L.n[0], L.cap[0]), n1 = preserve_saddles ? min((i64)L.n[1], L.cap[1]) : 0,
+              n2 = preserve_saddles ? min((i64)L.n[2], L.cap[2]) : 0, n3 = min((i64)L.n[3], L.cap[3]);
+    const i64 e0 = (n0 + 31) & ~31ll, e1 = e0 + ((n1 + 31) & ~31ll), e2 = e1 + ((n2 + 31) & ~31ll), e3 = e2 + n3;
+    i64 i = (i64)blockIdx.x * blockDim.x;
+    if (i >= e3) return;
+    load_rule_tab(tab);
+    const Rules R{c, tab};
+    for (i += threadIdx.x; i < e3; i += (i64)gridDim.x * blockDim.x) {
+        if (i < e0) {
+            if (i < n0) rule_min(R, L.l[0][i]);
+        } else if (i < e1) {
+            if (i - e0 < n1) rule_saddle(R, L.l[1][i - e0]);
+        } else if (i < e2) {
+            if (i - e1 < n2) rule_2saddle(R, L.l[2][i - e1]);
+        } else {
+            rule_max(R, L.l[3][i - e2]);
+        }
     }
-}
-// the critical-point fix round; returns the number of kernels launched
-inline int launch_fix_cp(const RuleCtx &rc, const CpLists &L, int ps, unsigned grid, cudaStream_t st) {
-    const i64 pass = (i64)grid * kBlock;
-    k_fix_cp<<<grid, kBlock, 0, st>>>(rc, L, ps, pass);
-    k_fix_cp_t<0><<<grid, kBlock, 0, st>>>(rc, L, ps, pass);
-    if (ps) {
-        k_fix_cp_t<1><<<grid, kBlock, 0, st>>>(rc, L, ps, pass);
-        k_fix_cp_t<2><<<grid, kBlock, 0, st>>>(rc, L, ps, pass);
-    }
-    k_fix_cp_t<3><<<grid, kBlock, 0, st>>>(rc, L, ps, pass);
-    return ps ? 5 : 3;
 }
 
 // separatrix records
 struct PathRec {
-    i64 *as_tet, *as_cur, *ds_edge, *ds_vert;
+    i64 *as_tet, *as_cur, *ds_edge, *ds_vert;  // cell codes; ds_vert: the vertex (-1: none)
     unsigned long long *n;  // [0] ascending, [1] descending
     i64 cap_as, cap_ds;     // at most one record per original 2-saddle / 1-saddle
 };
@@ -538,7 +502,7 @@ __device__ __forceinline__ void wall_defer(i64 *list, unsigned long long *n, i64
 }
 // first tier: every original 2-saddle (sad2 codes anchor * 12 + slot), stack
 // and cache in per-thread local memory
-__global__ void k_wall_t1(RuleCtx c, const i64 *sad2, const unsigned long long *nsad, i64 capsad, WallRec W,
+__global__ void k_wall_t1(const __grid_constant__ RuleCtx c, const i64 *sad2, const unsigned long long *nsad, i64 capsad, WallRec W,
                           i64 *next, unsigned long long *nnext, i64 capnext) {
     const i64 n = min((i64)*nsad, capsad);
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
@@ -557,7 +521,7 @@ __global__ void k_wall_t1(RuleCtx c, const i64 *sad2, const unsigned long long *
 }
 // a larger tier for list[first, first + count): one thread per 2-saddle face,
 // its stack and cache in scratch (stack_cap + 2^cache_bits entries each)
-__global__ void k_wall_tn(RuleCtx c, const i64 *list, i64 first, i64 count, WallRec W, i64 *next,
+__global__ void k_wall_tn(const __grid_constant__ RuleCtx c, const i64 *list, i64 first, i64 count, WallRec W, i64 *next,
                           unsigned long long *nnext, i64 capnext, i64 *scratch, int stack_cap, int cache_bits,
                           long long pop_cap) {
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (i64)gridDim.x * blockDim.x) {
@@ -571,7 +535,7 @@ __global__ void k_wall_tn(RuleCtx c, const i64 *list, i64 first, i64 count, Wall
         else if (r == 2) wall_defer(next, nnext, capnext, sf);
     }
 }
-__global__ void k_fix_wall(RuleCtx c, WallRec W) {
+__global__ void k_fix_wall(const __grid_constant__ RuleCtx c, WallRec W) {
     const i64 n = min((i64)*W.n, W.cap);
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x)
         rule_ds_wall(c, W.edge[i]);
@@ -629,7 +593,7 @@ __device__ bool first_diff(const Grid &g, const uint32_t *tcP, const uint32_t *t
         const int p = (tcP[ci] >> (3 * s)) & 7;
         if (p == 7) return false;
         if (p != (int)((tcQ[ci] >> (3 * s)) & 7)) {
-            cur = tet_ref(g, x, y, z, s);
+            cur = tet_code(ci, s);
             return true;
         }
         const int s8 = succ[ci * 8 + s];
@@ -650,13 +614,10 @@ __device__ bool first_diff(const Grid &g, const uint32_t *tcP, const uint32_t *t
 // the higher id, first) against the original ones; the first endpoint whose
 // minimum differs records (edge, trouble maker), the trouble maker carried
 // over from v1's walk into v2's as in the reference.
-__global__ void k_conn_ds(RuleCtx c, PathRec R, i64 cap) {
+__global__ void k_conn_ds(const __grid_constant__ RuleCtx c, PathRec R, i64 cap) {
     const Grid &g = c.g;
     for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += (i64)gridDim.x * blockDim.x) {
         uint32_t m = (c.P.crit[v] >> 1) & 0x7Fu;
-        if (!m) continue;
-        int x, y, z;
-        decode_v(g, v, x, y, z);
         while (m) {
             const int k = __ffs(m) - 1;
             m &= m - 1;
@@ -668,7 +629,7 @@ __global__ void k_conn_ds(RuleCtx c, PathRec R, i64 cap) {
                 if (eq != ep) {
                     const unsigned long long at = atomicAdd(&R.n[1], 1ull);
                     if ((i64)at < R.cap_ds) {
-                        R.ds_edge[at] = edge_ref(g, x, y, z, k);
+                        R.ds_edge[at] = edge_code(v, k);
                         R.ds_vert[at] = trouble;
                     }
                     break;
@@ -707,7 +668,7 @@ __global__ void k_conn_as(Grid g, const uint32_t *critP, const uint32_t *critQ, 
                 if (first_diff(g, tcP, tcQ, succ, cx, cy, cz, cs, cap, err, cur)) {
                     const unsigned long long at = atomicAdd(&R.n[0], 1ull);
                     if ((i64)at < R.cap_as) {
-                        R.as_tet[at] = tet_ref(g, cx, cy, cz, cs);
+                        R.as_tet[at] = tet_code(cx + (i64)cy * g.W + (i64)cz * g.WH, cs);
                         R.as_cur[at] = cur;
                     }
                     break;
@@ -878,7 +839,7 @@ __global__ void k_path_as_walk(Grid g, const i64 *sad2, const unsigned long long
             if (p == 7) {
                 r = -1;
             } else if (p != (int)((wq >> (3 * s)) & 7)) {
-                r = tet_ref(g, x, y, z, s);
+                r = tet_code(ci, s);
             } else if (s8 == 255) {
                 r = -1;
             } else if (++steps > cap) {
@@ -914,12 +875,10 @@ __global__ void k_path_as_pick(Grid g, const i64 *sad2, const unsigned long long
         const i64 code = sad2[i];
         const i64 v = code / 12;
         const int sl = (int)(code % 12);
-        int x, y, z;
-        decode_v(g, v, x, y, z);
         const signed char *tc = TOPO_FACE_COF[sl][j];
         const unsigned long long at = atomicAdd(&R.n[0], 1ull);
         if ((i64)at < R.cap_as) {
-            R.as_tet[at] = tet_ref(g, x + tc[0], y + tc[1], z + tc[2], tc[3]);
+            R.as_tet[at] = tet_code(v + tc[0] + tc[1] * (i64)g.W + tc[2] * g.WH, tc[3]);
             R.as_cur[at] = res[2 * i + j];
         }
     }
@@ -947,8 +906,8 @@ __global__ void k_ds_keep(Grid g, PathRec R, const unsigned long long *old_n, co
     const i64 n = min((i64)*old_n, R.cap_ds);
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
         const i64 e = R.ds_edge[i];
-        int x, y, z, k;
-        edge_unref(g, e, x, y, z, k);
+        int x, y, z;
+        decode_v(g, e >> 5, x, y, z);
         if (ds_anchor_dirty(g, T, x, y, z)) continue;
         const unsigned long long at = agg_slot(tn);
         if ((i64)at < tcap) {
@@ -957,7 +916,7 @@ __global__ void k_ds_keep(Grid g, PathRec R, const unsigned long long *old_n, co
         }
     }
 }
-__global__ void k_ds_tiles(RuleCtx c, const unsigned long long *valid, i64 *te, i64 *tv, unsigned long long *tn,
+__global__ void k_ds_tiles(const __grid_constant__ RuleCtx c, const unsigned long long *valid, i64 *te, i64 *tv, unsigned long long *tn,
                            i64 tcap, TileSat T) {
     const Grid &g = c.g;
     const bool all = *valid == 0;
@@ -987,7 +946,7 @@ __global__ void k_ds_tiles(RuleCtx c, const unsigned long long *valid, i64 *te, 
                         if (po != c.Q.pv[e]) {
                             const unsigned long long at = agg_slot(tn);
                             if ((i64)at < tcap) {
-                                te[at] = edge_ref(g, x, y, z, k);
+                                te[at] = edge_code(v, k);
                                 tv[at] = e;
                             }
                             break;
@@ -1034,7 +993,7 @@ __device__ __forceinline__ i64 dir_offset(const Grid &g, int d) {
 // second's, and idle lanes take new items from chunks of 64 handed out by a
 // ticket (*ticket, zero at launch): walks are long and uneven, and a lane that
 // finished does not wait for the warp's longest walk.
-__global__ void k_ds_strict(RuleCtx c, PathRec R, const i64 *sad1, const unsigned long long *nsad1, i64 step_cap,
+__global__ void k_ds_strict(const __grid_constant__ RuleCtx c, PathRec R, const i64 *sad1, const unsigned long long *nsad1, i64 step_cap,
                             unsigned long long *ticket) {
     const Grid &g = c.g;
     constexpr i64 kChunk = 64;
@@ -1065,12 +1024,10 @@ __global__ void k_ds_strict(RuleCtx c, PathRec R, const i64 *sad1, const unsigne
                 } else if (my < end) {
                     const i64 code = sad1[my], a = code / 7;
                     const int k = (int)(code - 7 * a);
-                    int x, y, z;
-                    decode_v(g, a, x, y, z);
                     const int ends = (int)((kEnds >> (6 * k)) & 63u), c0 = ends & 7, c1 = ends >> 3;
                     u = a + (c0 & 1) + ((c0 >> 1) & 1) * (i64)g.W + (c0 >> 2) * g.WH;
                     second = a + (c1 & 1) + ((c1 >> 1) & 1) * (i64)g.W + (c1 >> 2) * g.WH;
-                    edge = edge_ref(g, x, y, z, k);
+                    edge = edge_code(a, k);
                     item = my;
                     first = true;
                     steps = 0;
@@ -1106,11 +1063,16 @@ __global__ void k_ds_strict(RuleCtx c, PathRec R, const i64 *sad1, const unsigne
     }
 }
 
-__global__ void k_fix_path(RuleCtx c, PathRec R) {
-    const i64 na = min((i64)R.n[0], R.cap_as), nd = min((i64)R.n[1], R.cap_ds);
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < na + nd; i += (i64)gridDim.x * blockDim.x) {
-        if (i < na) rule_as_path(c, R.as_cur[i]);
-        else rule_ds_path(c, R.ds_vert[i - na]);
+__global__ void __launch_bounds__(kBlock) k_fix_path(const __grid_constant__ RuleCtx c, PathRec P) {
+    __shared__ RuleTab tab;
+    const i64 na = min((i64)P.n[0], P.cap_as), nd = min((i64)P.n[1], P.cap_ds), ea = (na + 31) & ~31ll;
+    i64 i = (i64)blockIdx.x * blockDim.x;
+    if (i >= ea + nd) return;
+    load_rule_tab(tab);
+    const Rules R{c, tab};
+    for (i += threadIdx.x; i < ea + nd; i += (i64)gridDim.x * blockDim.x) {
+        if (i < na) rule_as_path(R, P.as_cur[i]);
+        else if (i >= ea) rule_ds_path(R, P.ds_vert[i - ea]);
     }
 }
 
@@ -1119,7 +1081,7 @@ __global__ void k_fix_path(RuleCtx c, PathRec R) {
 // The delta is what the reference's buffer holds: get_delta(v), with the
 // buffer's "no request" sentinel -2000*range (a request whose delta is not
 // above the sentinel leaves the buffer unchanged under edit_type 0).
-__global__ void k_apply(RuleCtx c, double range, int preserve_type, int update, uint8_t *changed, double *delta_out) {
+__global__ void k_apply(const __grid_constant__ RuleCtx c, double range, int preserve_type, int update, uint8_t *changed, double *delta_out) {
     const i64 n = (i64)*c.reqn;
     const double sentinel = -2000.0 * range;
     const double tiny = 1e-15 * range;
@@ -1170,30 +1132,32 @@ constexpr uint8_t kSnapSeed = 2, kSnapGrow = 4;
 __device__ __forceinline__ void seed_vertex(const Grid &g, uint8_t *m, i64 v) {
     if (v >= 0 && v < g.V) m[v] = (uint8_t)(m[v] | kSnapSeed);
 }
+// the vertices of a listed cell
+__device__ __forceinline__ void seed_cell(const Grid &g, i64 code, uint8_t *m) {
+    const i64 v = code >> 5;
+    const int b = (int)(code & 31);
+    if (b == 0) {
+        seed_vertex(g, m, v);
+    } else if (b < 8) {
+        for (int j = 0; j < 2; j++) seed_vertex(g, m, v + g.coff[TOPO_EDGE_V[b - 1][j]]);
+    } else if (b < 20) {
+        for (int j = 0; j < 3; j++) seed_vertex(g, m, v + g.coff[TOPO_FACE_V[b - 8][j]]);
+    } else {
+        for (int j = 0; j < 4; j++) seed_vertex(g, m, v + g.coff[TOPO_TET_V[b - 20][j]]);
+    }
+}
 __global__ void k_seed_cells(Grid g, CpLists L, uint8_t *m) {
     const i64 n0 = min((i64)L.n[0], L.cap[0]), n1 = min((i64)L.n[1], L.cap[1]), n2 = min((i64)L.n[2], L.cap[2]),
               n3 = min((i64)L.n[3], L.cap[3]);
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n0 + n1 + n2 + n3; i += (i64)gridDim.x * blockDim.x) {
-        i64 vs[4] = {-1, -1, -1, -1};
-        if (i < n0) {
-            vs[0] = L.l[0][i];
-        } else if (i < n0 + n1) {
-            edge_verts(g, L.l[1][i - n0], vs[0], vs[1]);
-        } else if (i < n0 + n1 + n2) {
-            tri_verts(g, L.l[2][i - n0 - n1], vs[0], vs[1], vs[2]);
-        } else {
-            tet_verts(g, L.l[3][i - n0 - n1 - n2], vs[0], vs[1], vs[2], vs[3]);
-        }
-        for (int k = 0; k < 4; k++) seed_vertex(g, m, vs[k]);
-    }
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n0 + n1 + n2 + n3; i += (i64)gridDim.x * blockDim.x)
+        seed_cell(g, i < n0 ? L.l[0][i] : i < n0 + n1 ? L.l[1][i - n0] : i < n0 + n1 + n2 ? L.l[2][i - n0 - n1]
+                                                                                       : L.l[3][i - n0 - n1 - n2], m);
 }
 __global__ void k_seed_paths(Grid g, PathRec R, uint8_t *m) {
     const i64 na = min((i64)R.n[0], R.cap_as), nd = min((i64)R.n[1], R.cap_ds);
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < na + nd; i += (i64)gridDim.x * blockDim.x) {
-        i64 vs[4] = {-1, -1, -1, -1};
-        if (i < na) tet_verts(g, R.as_cur[i], vs[0], vs[1], vs[2], vs[3]);
-        else vs[0] = R.ds_vert[i - na];
-        for (int k = 0; k < 4; k++) seed_vertex(g, m, vs[k]);
+        if (i < na) seed_cell(g, R.as_cur[i], m);
+        else seed_vertex(g, m, R.ds_vert[i - na]);
     }
 }
 __global__ void k_seed_walls(Grid g, WallRec W, uint8_t *m) {
@@ -1231,7 +1195,7 @@ __global__ void k_dilate_axis(Grid g, uint8_t *m, int axis, int radius) {
         }
     }
 }
-__global__ void k_snap_mask(RuleCtx c, uint8_t *m) {
+__global__ void k_snap_mask(const __grid_constant__ RuleCtx c, uint8_t *m) {
     double *gv = const_cast<double *>(c.gv);
     for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < c.g.V; v += (i64)gridDim.x * blockDim.x) {
         const uint8_t b = m[v];
@@ -2455,6 +2419,7 @@ dmtz_status dmtz_mismatch(dmtz_ctx *ctx, int W, int H, int D, const double *orig
         if (!outs[k] || !hc[k]) continue;
         std::vector<i64> tmp(hc[k]);
         CK(cudaMemcpy(tmp.data(), ctx->lists[k], sizeof(i64) * hc[k], cudaMemcpyDeviceToHost));
+        for (i64 &q : tmp) q = code_ref(g, q);
         std::sort(tmp.begin(), tmp.end());
         for (size_t i = 0; i < tmp.size(); i++) outs[k][i] = (int32_t)tmp[i];
     }
@@ -2484,7 +2449,7 @@ dmtz_status dmtz_fix_round(dmtz_ctx *ctx, int W, int H, int D, const double *ori
     CK(cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), ctx->stream));
     CK(cudaMemsetAsync(ctx->errword, 0, sizeof(int), ctx->stream));
     RuleCtx rc = rule_ctx(ctx, g, bound, edit_type);
-    launch_fix_cp(rc, cp_lists(ctx), preserve_saddles, persistent_grid(), ctx->stream);
+    k_fix_cp<<<persistent_grid(), kBlock, 0, ctx->stream>>>(rc, cp_lists(ctx), preserve_saddles);
     double *dd = nullptr;
     CK(dalloc(&dd, g.V));
     const double sentinel = -2000.0 * range;
@@ -2548,13 +2513,14 @@ static dmtz_status path_detect_impl(dmtz_ctx *ctx, int W, int H, int D, const do
     }
     counts[0] = (int64_t)hc[0];
     counts[1] = (int64_t)hc[1];
-    auto fetch = [&](i64 *da, i64 *db, unsigned long long n, int32_t *oa, int32_t *ob) -> dmtz_status {
+    // codes to reference ids (the second column of the descending records holds vertices)
+    auto fetch = [&](i64 *da, i64 *db, unsigned long long n, int32_t *oa, int32_t *ob, bool vert) -> dmtz_status {
         if (!n || !oa) return DMTZ_OK;
         std::vector<i64> a(n), b(n);
         CK(cudaMemcpy(a.data(), da, sizeof(i64) * n, cudaMemcpyDeviceToHost));
         CK(cudaMemcpy(b.data(), db, sizeof(i64) * n, cudaMemcpyDeviceToHost));
         std::vector<std::pair<i64, i64>> p(n);
-        for (size_t i = 0; i < n; i++) p[i] = {a[i], b[i]};
+        for (size_t i = 0; i < n; i++) p[i] = {code_ref(g, a[i]), vert ? b[i] : code_ref(g, b[i])};
         std::sort(p.begin(), p.end());
         for (size_t i = 0; i < n; i++) {
             oa[i] = (int32_t)p[i].first;
@@ -2562,8 +2528,8 @@ static dmtz_status path_detect_impl(dmtz_ctx *ctx, int W, int H, int D, const do
         }
         return DMTZ_OK;
     };
-    if ((s = fetch(ctx->as_tet, ctx->as_cur, hc[0], as_tet, as_cur)) != DMTZ_OK) return s;
-    if ((s = fetch(ctx->ds_edge, ctx->ds_vert, hc[1], ds_edge, ds_vert)) != DMTZ_OK) return s;
+    if ((s = fetch(ctx->as_tet, ctx->as_cur, hc[0], as_tet, as_cur, false)) != DMTZ_OK) return s;
+    if ((s = fetch(ctx->ds_edge, ctx->ds_vert, hc[1], ds_edge, ds_vert, true)) != DMTZ_OK) return s;
     if (err & ERR_WALK) return fail(ctx, DMTZ_ERR_CYCLE, "a path walk exceeded its step cap");
     if (err & ERR_OOB) return fail(ctx, DMTZ_ERR_OOB, "a path rule indexed out of range");
     return DMTZ_OK;
@@ -2795,7 +2761,7 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
             if (state != LS_PCHECK) {
                 cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), st);
                 cudaMemsetAsync(ctx->counters + 7, 0, sizeof(unsigned long long), st);
-                if (state == LS_CP) launch_fix_cp(rc, L, ps, pgrid, st);
+                if (state == LS_CP) k_fix_cp<<<pgrid, kBlock, 0, st>>>(rc, L, ps);
                 else k_fix_path<<<pgrid, kBlock, 0, st>>>(rc, PR);
                 k_apply<<<pgrid, kBlock, 0, st>>>(rc, range, pt, 1, ctx->changed, nullptr);
                 repair_dirty(ctx, g, Qs, ctx->P.crit, state == LS_CP ? (ps == 1) : 1);
@@ -3055,8 +3021,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             // a fix round: fix + update, then the repair (dirty marks, compaction,
             // fresh and tile marks, the gradient, the list rebuild)
             const int64_t rnd = 2 + 2 + (ctx->inc_scan ? 1 : 0) + (ctx->tile_dirty ? 1 : 0) + 1 + (ctx->inc_scan ? 3 : 1);
-            const int64_t rnd_cp = rnd - 1 + (ps == 1 ? 5 : 3);  // the fix round's two forms (launch_fix_cp)
-            ctx->launches += 2 * (fin.runs[0] + fin.runs[1] + fin.runs[2] + fin.runs[3]) + rnd_cp * fin.runs[LS_CP] +
+            ctx->launches += 2 * (fin.runs[0] + fin.runs[1] + fin.runs[2] + fin.runs[3]) + rnd * fin.runs[LS_CP] +
                              (rnd + det) * fin.runs[LS_PDF] + det * fin.runs[LS_PCHECK] + rnd * fin.runs[LS_PFIX];
         }
         R.outer_iterations = fin.outer;
@@ -3084,12 +3049,12 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             CK(cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), st));
             CK(cudaMemsetAsync(ctx->counters + 7, 0, sizeof(unsigned long long), st));
             pt_.begin(PH_FIXCP);
-            const int nfix = launch_fix_cp(rc, cp_lists(ctx), ps, pgrid, st);
+            k_fix_cp<<<pgrid, kBlock, 0, st>>>(rc, cp_lists(ctx), ps);
             pt_.end();
             pt_.begin(PH_APPLY);
             k_apply<<<pgrid, kBlock, 0, st>>>(rc, range, pt, 1, ctx->changed, nullptr);
             pt_.end();
-            ctx->launches += nfix + 1;
+            ctx->launches += 2;
             pt_.begin(PH_PAIR);
             repair_dirty(ctx, g, Qs, ctx->P.crit, ps == 1);
             pt_.end();

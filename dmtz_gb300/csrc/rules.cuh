@@ -4,9 +4,24 @@
 // :3039-3983, fix_maximum :3985-4303, fix_as_vpath :5135-5244, fix_ds_vpath
 // :5246-5295) are a case analysis over the reference's union-valued pairing
 // arrays.  They are restated here branch for branch, including the
-// reference's quirks (shadowed variables, if/if chains, ids of one dimension
-// read as another), on top of accessors that rebuild paired_vertices /
-// _edges / _faces / _tetrahedras values from the packed gradient.
+// reference's quirks.
+//
+// Cells are codes: anchor vertex * 32 + the cell's bit of FieldState::crit (0
+// the vertex, 1..7 edges, 8..19 triangles, 20..25 tetrahedra), so a cell's
+// vertices, its partner and the partner's kind come from the anchor's words
+// and small tables in shared memory.  The reference tells the kinds apart by
+// comparing ids of one dimension with the counts of another and testing the
+// back pointer; for a consistent gradient that test succeeds for the partner's
+// own kind only, so asking for the kind is the same.  Where a rule's result depends on an
+// id's number (an id read as another dimension's), the number is computed and decoded
+// as the reference does (tet_verts and so on, "literal" below).
+//
+// A chain of dependent loads with little arithmetic: bound by latency.  With
+// cells as reference ids, every accessor decoded ids by 64-bit divisions (some
+// hundred instructions each, fetched cold in every launch) and the rule context was copied
+// to each thread's stack for the accessors that were called: a critical-point
+// round took 82 us on average on a noisy 97 x 61 x 75 field and 78 us at 16^3,
+// now 20 and 22 us (cold caches); 134 -> 54 us at 256^3.
 //
 // A rule "lowers" a vertex: it asks for d_deltaBuffer[v] = get_delta(v).
 // get_delta depends only on v's own value and counter, which no rule
@@ -17,16 +32,13 @@
 // Any index the reference would read or write outside its allocation is not
 // performed; it sets bit 0 of the error word instead.
 #pragma once
-#include "dmtz_common.cuh"
+#include "gradient.cuh"
 
 namespace dmtz {
 
 enum { ERR_OOB = 1, ERR_WALK = 2 };
 
-// The fix rules are long, branchy code run by few lanes of a warp at a time;
-// with their id and pairing accessors inlined at every call site the fix
-// kernel outgrew the instruction cache (ncu: warps stalled on instruction
-// fetch).  The accessors are therefore compiled once and called.
+// code of rarely taken paths and of the wall searches, compiled once and called
 #define DMTZ_SHARED_CODE __noinline__
 
 struct RuleCtx {
@@ -218,23 +230,6 @@ __device__ DMTZ_SHARED_CODE i64 pf_ref(const RuleCtx &c, const FieldState &s, i6
     }
     return -1;
 }
-// paired_tetrahedras[t]
-__device__ DMTZ_SHARED_CODE i64 pt_ref(const RuleCtx &c, const FieldState &s, i64 t) {
-    if (t < 0 || t >= c.g.T) {
-        atomicOr(c.err, ERR_OOB);
-        return -1;
-    }
-    int x, y, z, sl;
-    tet_unref(c.g, t, x, y, z, sl);
-    const i64 a = x + (i64)y * c.g.W + (i64)z * c.g.WH;
-    for (int j = 0; j < 4; j++) {
-        const signed char *tf = TOPO_TET_FACE[sl][j];
-        const i64 fa = a + tf[0] + (i64)tf[1] * c.g.W + (i64)tf[2] * c.g.WH;
-        if (fup_get(s.fup[fa], tf[3]) == tf[4] + 1) return face_ref(c.g, x + tf[0], y + tf[1], z + tf[2], tf[3]);
-    }
-    return -1;
-}
-
 // --------------------------------------------------------------- values, order, requests
 __device__ __forceinline__ double fval(const RuleCtx &c, i64 v) {
     if (v < 0 || v >= c.g.V) {
@@ -266,7 +261,7 @@ __device__ __forceinline__ double get_delta(const RuleCtx &c, i64 v) {
         return 0.0;
     }
     if (c.edit_type == 1) return -ldexp(1.0, -c.cnt[v]) * c.bound;
-    return __ddiv_rn(__dsub_rn(__dsub_rn(c.f[v], c.bound), c.gv[v]), 2.0);
+    return __dmul_rn(__dsub_rn(__dsub_rn(c.f[v], c.bound), c.gv[v]), 0.5);  // x / 2, rounded the same
 }
 // "lower v": the reference's swap(v, get_delta(v))
 __device__ __forceinline__ void lower(const RuleCtx &c, i64 v) {
@@ -294,14 +289,6 @@ __device__ __forceinline__ i64 fourth_of(i64 a, i64 b, i64 cc, i64 d, i64 v1, i6
     else if (cc != v1 && cc != v2 && cc != v3) v4 = cc;
     return v4;
 }
-__device__ __forceinline__ bool adjacent(const Grid &g, i64 a, i64 b, int &d) {
-    int ax, ay, az, bx, by, bz;
-    decode_v(g, a, ax, ay, az);
-    decode_v(g, b, bx, by, bz);
-    d = dir_of(bx - ax, by - ay, bz - az);
-    return d >= 0;
-}
-
 // argmin over the common neighbours n of (v1, v2) with exactly one of v1, v2
 // above n in the ORIGINAL field (the rescan of fix_saddle, main_3d.cu:2942-3015)
 __device__ DMTZ_SHARED_CODE i64 rescan_edge(const RuleCtx &c, i64 v1, i64 v2) {
@@ -357,377 +344,438 @@ __device__ DMTZ_SHARED_CODE i64 smallest_vertex(const RuleCtx &c, i64 v1, i64 v2
     return found ? bid : -1;
 }
 
-// --------------------------------------------------------------- A8 fix_minimum
-__device__ inline void rule_min(const RuleCtx &c, i64 id) {
-    const i64 pv = pv_ref(c, c.P, id);
-    if (pv != -1) {
-        i64 vertex, v2;
-        edge_verts(c.g, pv, vertex, v2);
-        if (vertex != id) v2 = vertex;
-        lower(c, v2);
-    } else {
-        lower(c, id);
+// --------------------------------------------------------------- cells as codes
+// Tables of the code arithmetic.  Offsets are (dx+1) | (dy+1) << 2 | (dz+1) <<
+// 4 (six bits), corners dx + 2 dy + 4 dz (three bits).
+struct RuleTab {
+    uint16_t edge[7];     // corners, higher id first: 3 bits each
+    uint16_t face[12];    // three corners
+    uint16_t tet[6];      // four corners
+    uint16_t ecof[42];    // [family * 6 + i]: coface i: offset | slot << 6
+    uint16_t fcof[24];    // [slot * 2 + i]: coface i: offset | slot << 6
+    uint16_t fedge[36];   // [slot * 3 + j]: edge opposite corner j: offset | family << 6 | (coface index + 1) << 9
+    uint16_t tface[24];   // [slot * 4 + j]: facet opposite corner j: offset | slot << 6
+};
+constexpr uint16_t tab_off(int x, int y, int z) { return (uint16_t)((x + 1) | ((y + 1) << 2) | ((z + 1) << 4)); }
+constexpr RuleTab make_rule_tab() {
+    RuleTab t = {};
+    for (int k = 0; k < 7; k++) {
+        t.edge[k] = (uint16_t)(cxt::TOPO_EDGE_V[k][0] | (cxt::TOPO_EDGE_V[k][1] << 3));
+        for (int i = 0; i < cxt::TOPO_EDGE_NCOF[k]; i++) {
+            const signed char *f = cxt::TOPO_EDGE_COF[k][i];
+            t.ecof[k * 6 + i] = (uint16_t)(tab_off(f[0], f[1], f[2]) | (f[3] << 6));
+        }
     }
+    for (int s = 0; s < 12; s++) {
+        for (int j = 0; j < 3; j++) {
+            const signed char *e = cxt::TOPO_FACE_EDGE[s][j];
+            t.face[s] |= (uint16_t)(cxt::TOPO_FACE_V[s][j] << (3 * j));
+            t.fedge[s * 3 + j] = (uint16_t)(tab_off(e[0], e[1], e[2]) | (e[3] << 6) | ((e[4] + 1) << 9));
+        }
+        for (int i = 0; i < 2; i++) {
+            const signed char *f = cxt::TOPO_FACE_COF[s][i];
+            t.fcof[s * 2 + i] = (uint16_t)(tab_off(f[0], f[1], f[2]) | (f[3] << 6));
+        }
+    }
+    for (int q = 0; q < 6; q++)
+        for (int j = 0; j < 4; j++) {
+            const signed char *f = cxt::TOPO_TET_FACE[q][j];
+            t.tet[q] |= (uint16_t)(cxt::TOPO_TET_V[q][j] << (3 * j));
+            t.tface[q * 4 + j] = (uint16_t)(tab_off(f[0], f[1], f[2]) | (f[3] << 6));
+        }
+    return t;
+}
+static __device__ const RuleTab kRuleTab = make_rule_tab();
+// the tables into shared memory (every thread of the block calls this)
+__device__ __forceinline__ void load_rule_tab(RuleTab &t) {
+    const uint16_t *src = reinterpret_cast<const uint16_t *>(&kRuleTab);
+    uint16_t *dst = reinterpret_cast<uint16_t *>(&t);
+    for (int i = threadIdx.x; i < (int)(sizeof(RuleTab) / 2); i += blockDim.x) dst[i] = src[i];
+    __syncthreads();
+}
+
+enum { KIND_VERTEX = 0, KIND_EDGE, KIND_FACE, KIND_TET };
+__host__ __device__ __forceinline__ i64 cell_code(i64 anchor, int bit) { return anchor * 32 + bit; }
+__host__ __device__ __forceinline__ i64 edge_code(i64 anchor, int k) { return anchor * 32 + 1 + k; }
+__host__ __device__ __forceinline__ i64 face_code(i64 anchor, int s) { return anchor * 32 + 8 + s; }
+__host__ __device__ __forceinline__ i64 tet_code(i64 anchor, int t) { return anchor * 32 + 20 + t; }
+__host__ __device__ __forceinline__ int cell_kind(i64 code) {
+    const int b = (int)(code & 31);
+    return b == 0 ? KIND_VERTEX : b < 8 ? KIND_EDGE : b < 20 ? KIND_FACE : KIND_TET;
+}
+// reference id of a cell
+__host__ __device__ __forceinline__ i64 code_ref(const Grid &g, i64 code) {
+    const i64 v = code >> 5;
+    const int b = (int)(code & 31);
+#ifdef __CUDA_ARCH__
+    int x, y, z;
+    decode_v(g, v, x, y, z);
+#else
+    const i64 x = v % g.W, y = (v / g.W) % g.H, z = v / g.WH;
+#endif
+    return b == 0 ? v : b < 8 ? edge_ref(g, x, y, z, b - 1) : b < 20 ? face_ref(g, x, y, z, b - 8) : tet_ref(g, x, y, z, b - 20);
+}
+
+struct Rules {
+    const RuleCtx &c;
+    const RuleTab &t;
+    __device__ __forceinline__ i64 moved(i64 a, unsigned off) const {
+        return a + ((int)(off & 3u) - 1) + ((int)((off >> 2) & 3u) - 1) * (i64)c.g.W + ((int)((off >> 4) & 3u) - 1) * c.g.WH;
+    }
+    __device__ __forceinline__ i64 corner(i64 a, unsigned c3) const {
+        return a + (c3 & 1u) + ((c3 >> 1) & 1u) * (i64)c.g.W + ((c3 >> 2) & 1u) * c.g.WH;
+    }
+    // vertices, highest id first
+    __device__ __forceinline__ void verts(i64 code, i64 &v1, i64 &v2) const {
+        const unsigned m = t.edge[(code & 31) - 1];
+        v1 = corner(code >> 5, m);
+        v2 = corner(code >> 5, m >> 3);
+    }
+    __device__ __forceinline__ void verts(i64 code, i64 &v1, i64 &v2, i64 &v3) const {
+        const unsigned m = t.face[(code & 31) - 8];
+        v1 = corner(code >> 5, m);
+        v2 = corner(code >> 5, m >> 3);
+        v3 = corner(code >> 5, m >> 6);
+    }
+    __device__ __forceinline__ void verts(i64 code, i64 &v1, i64 &v2, i64 &v3, i64 &v4) const {
+        const unsigned m = t.tet[(code & 31) - 20];
+        v1 = corner(code >> 5, m);
+        v2 = corner(code >> 5, m >> 3);
+        v3 = corner(code >> 5, m >> 6);
+        v4 = corner(code >> 5, m >> 9);
+    }
+    __device__ __forceinline__ i64 third(i64 face, i64 v1, i64 v2) const {
+        i64 a, b, d;
+        verts(face, a, b, d);
+        return third_of(a, b, d, v1, v2);
+    }
+    __device__ __forceinline__ i64 fourth(i64 tet, i64 v1, i64 v2, i64 v3) const {
+        i64 a, b, d, e;
+        verts(tet, a, b, d, e);
+        return fourth_of(a, b, d, e, v1, v2, v3);
+    }
+    // the other end of vertex v's paired edge, or -1
+    __device__ __forceinline__ i64 below(const FieldState &s, i64 v) const {
+        const int d = s.pv[v];
+        return d == 15 ? -1 : v + c.g.doff[d];
+    }
+    // partners (code, or -1 for a critical cell)
+    __device__ __forceinline__ i64 edge_partner(const FieldState &s, i64 e) const {
+        const i64 a = e >> 5;
+        const int k = (int)(e & 31) - 1, up = eup_get(s.eup[a], k);
+        if (up) {
+            const unsigned f = t.ecof[k * 6 + up - 1];
+            return face_code(moved(a, f), (int)(f >> 6));
+        }
+        i64 p, q;
+        verts(e, p, q);
+        const int dp = s.pv[p], dq = s.pv[q];
+        if (dp != 15 && p + c.g.doff[dp] == q) return cell_code(p, 0);
+        if (dq != 15 && q + c.g.doff[dq] == p) return cell_code(q, 0);
+        return -1;
+    }
+    __device__ __forceinline__ i64 face_partner(const FieldState &s, i64 f) const {
+        const i64 a = f >> 5;
+        const int sl = (int)(f & 31) - 8, up = fup_get(s.fup[a], sl);
+        if (up) {
+            const unsigned q = t.fcof[sl * 2 + up - 1];
+            return tet_code(moved(a, q), (int)(q >> 6));
+        }
+        i64 r = -1;
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const unsigned e = t.fedge[sl * 3 + j];
+            const i64 ea = moved(a, e);
+            const int k = (int)((e >> 6) & 7u);
+            if (eup_get(s.eup[ea], k) == (int)(e >> 9)) r = edge_code(ea, k);
+        }
+        return r;
+    }
+    __device__ __forceinline__ i64 tet_partner(const FieldState &s, i64 q) const {
+        const i64 a = q >> 5;
+        const int ts = (int)(q & 31) - 20, j = (int)((s.tcode[a] >> (3 * ts)) & 7u);
+        if (j == 7) return -1;
+        const unsigned f = t.tface[ts * 4 + j];
+        return face_code(moved(a, f), (int)(f >> 6));
+    }
+};
+
+// --------------------------------------------------------------- A8 fix_minimum
+__device__ __forceinline__ void rule_min(const Rules &R, i64 v) {
+    const i64 w = R.below(R.c.P, v >> 5);
+    lower(R.c, w >= 0 ? w : v >> 5);
 }
 
 // --------------------------------------------------------------- A9 fix_saddle
-__device__ inline void rule_saddle(const RuleCtx &c, i64 id) {
-    const Grid &G = c.g;
-    i64 edge = id;
-    const i64 pe = pe_ref(c, c.P, id);
-    if (pe != -1) {
-        if (pe < G.V && pe >= 0 && pv_ref(c, c.P, pe) == id) {
-            i64 v1, v2;
-            edge_verts(G, edge, v1, v2);
-            if (v2 != pe) v1 = pe;
-            else { v2 = v1; v1 = pe; }
-            const i64 q = pv_ref(c, c.Q, v1);
-            if (q == -1 || q < 0 || q >= G.E) return;
-            i64 fv1, fv2;
-            edge_verts(G, q, fv1, fv2);
-            const i64 false_v2 = v1 == fv1 ? fv2 : fv1;
-            const double a = gval(c, v2), b = gval(c, false_v2);
-            if (a > b || (a == b && v2 > false_v2)) lower(c, v2);
-        } else if (pe < G.F && pe >= 0 && pf_ref(c, c.P, pe) == id) {
-            const i64 face = pe;
-            i64 v1, v2, a, b, v3;
-            edge_verts(G, edge, v1, v2);
-            tri_verts(G, face, a, b, v3);
-            v3 = third_of(a, b, v3, v1, v2);
-            const i64 osv1 = !above_g(c, v1, v3) ? v3 : v1;
-            const i64 osv1_1 = !above_g(c, v2, v3) ? v3 : v2;
-            const bool v1_edge = above_g(c, v1, v3), v2_edge = above_g(c, v2, v3);
-            bool o_v1_edge = above_f(c, v1, v3), o_v2_edge = above_f(c, v2, v3);
-            if (v1_edge && v2_edge) {
-                lower(c, v3);
-            } else if (o_v1_edge && o_v2_edge) {
-                lower(c, v3);
-            } else {
-                const i64 pe2 = pe_ref(c, c.P, id);
-                i64 qf = -1;
-                bool cond = pe2 != -1 && pe2 < G.F && pe2 >= 0;
-                if (cond) {
-                    qf = pf_ref(c, c.Q, pe2);
-                    cond = qf != -1 && pe_ref(c, c.Q, qf) == pe2;
-                }
-                if (cond) {
-                    const i64 false_edge = qf;
-                    edge = false_edge;
-                    i64 a1, b1;
-                    edge_verts(G, false_edge, a1, b1);
-                    const i64 false_v = (a1 != v1 && a1 != v2) ? a1 : b1;
-                    const double diff = get_delta(c, false_v);
-                    i64 w1, w2, p, q, w3;
-                    edge_verts(G, edge, w1, w2);
-                    tri_verts(G, face, p, q, w3);
-                    w3 = third_of(p, q, w3, w1, w2);
-                    o_v1_edge = above_f(c, w2, w3);
-                    o_v2_edge = above_f(c, w1, w3);
-                    bool take = o_v1_edge && o_v2_edge;
-                    i64 pfe = -1;
-                    if (take) {
-                        pfe = pe_ref(c, c.P, false_edge);
-                        take = pfe != -1 && pf_ref(c, c.P, pfe) == false_edge;
-                    }
-                    if (take) {
-                        i64 r, s2, u3;
-                        tri_verts(G, pfe, r, s2, u3);
-                        u3 = third_of(r, s2, u3, w1, w2);
-                        lower(c, u3);
-                    } else if (fabs(diff) > 0) {
-                        lower(c, false_v);
-                    }
-                } else {
-                    if (o_v1_edge && !v1_edge) lower(c, osv1);
-                    else lower(c, osv1_1);
-                }
-            }
+__device__ __forceinline__ void rule_saddle(const Rules &R, i64 id) {
+    const RuleCtx &c = R.c;
+    i64 v1, v2;
+    R.verts(id, v1, v2);
+    const i64 pe = R.edge_partner(c.P, id);
+    if (pe != -1 && cell_kind(pe) == KIND_VERTEX) {
+        if (v2 == pe >> 5) v2 = v1;
+        v1 = pe >> 5;
+        const i64 false_v2 = R.below(c.Q, v1);
+        if (false_v2 < 0) return;
+        const double a = gval(c, v2), b = gval(c, false_v2);
+        if (a > b || (a == b && v2 > false_v2)) lower(c, v2);
+        return;
+    }
+    const i64 qe = pe == -1 ? R.edge_partner(c.Q, id) : -1;
+    if (pe == -1 && (qe == -1 || cell_kind(qe) == KIND_VERTEX)) {
+        if (qe != -1) lower(c, qe >> 5);
+        return;
+    }
+    const i64 face = pe != -1 ? pe : qe;
+    const i64 v3 = R.third(face, v1, v2);
+    const bool g1 = above_g(c, v1, v3), g2 = above_g(c, v2, v3), f1 = above_f(c, v1, v3), f2 = above_f(c, v2, v3);
+    if (pe != -1) {  // originally paired with this face
+        if ((g1 && g2) || (f1 && f2)) {
+            lower(c, v3);
+            return;
         }
-    } else {
-        const i64 qe = pe_ref(c, c.Q, id);
-        if (qe != -1 && qe < G.V && qe >= 0 && pv_ref(c, c.Q, qe) == id) {
-            lower(c, qe);
-        } else if (qe != -1 && qe < G.F && qe >= 0 && pf_ref(c, c.Q, qe) == id) {
-            i64 v1, v2, a, b, v3;
-            edge_verts(G, edge, v1, v2);
-            tri_verts(G, qe, a, b, v3);
-            v3 = third_of(a, b, v3, v1, v2);
-            const bool v1_edge = above_g(c, v2, v3), v2_edge = above_g(c, v1, v3);
-            const bool or_v1_edge = above_f(c, v2, v3), or_v2_edge = above_f(c, v1, v3);
-            if (v1_edge == v2_edge) {
-                if (v1_edge != or_v1_edge) lower(c, v2);
-                if (v2_edge != or_v2_edge) lower(c, v1);
-            } else {
-                // paired_edges[id] is -1 on this branch; the reference's
-                // "paired with a vertex" sub-case cannot occur
-                const i64 m = rescan_edge(c, v1, v2);
-                if (m != -1) {
-                    lower(c, m);
-                } else {
-                    lower(c, v1);
-                    lower(c, v2);
+        const i64 qf = R.face_partner(c.Q, face);
+        if (qf != -1 && cell_kind(qf) == KIND_EDGE) {
+            i64 w1, w2;
+            R.verts(qf, w1, w2);
+            const i64 false_v = (w1 != v1 && w1 != v2) ? w1 : w2;
+            const i64 w3 = R.third(face, w1, w2);
+            if (above_f(c, w2, w3) && above_f(c, w1, w3)) {
+                const i64 pfe = R.edge_partner(c.P, qf);
+                if (pfe != -1 && cell_kind(pfe) == KIND_FACE) {
+                    lower(c, R.third(pfe, w1, w2));
+                    return;
                 }
             }
+            if (fabs(get_delta(c, false_v)) > 0) lower(c, false_v);
+        } else if (f1 && !g1) {
+            lower(c, g1 ? v1 : v3);
+        } else {
+            lower(c, g2 ? v2 : v3);
+        }
+        return;
+    }
+    // originally critical, now paired with this face
+    if (g1 == g2) {
+        if (g2 != f2) lower(c, v2);
+        if (g1 != f1) lower(c, v1);
+    } else {
+        const i64 m = rescan_edge(c, v1, v2);
+        if (m != -1) {
+            lower(c, m);
+        } else {
+            lower(c, v1);
+            lower(c, v2);
         }
     }
 }
 
 // --------------------------------------------------------------- A10 fix_2saddle
-__device__ inline void rule_2saddle(const RuleCtx &c, i64 id) {
+__device__ __forceinline__ void rule_2saddle(const Rules &R, i64 id) {
+    const RuleCtx &c = R.c;
     const Grid &G = c.g;
-    const i64 pf = pf_ref(c, c.P, id);
-    if (pf != -1) {
-        if (pf < G.E && pf >= 0 && pe_ref(c, c.P, pf) == id) {
-            const i64 edge = pf;
-            i64 v1, v2, a, b, v3;
-            edge_verts(G, edge, v1, v2);
-            tri_verts(G, id, a, b, v3);
-            v3 = third_of(a, b, v3, v1, v2);
-            bool v1_edge = above_g(c, v2, v3), v2_edge = above_g(c, v1, v3);
-            bool o_v1_edge = above_f(c, v2, v3), o_v2_edge = above_f(c, v1, v3);
-            if (v1_edge && v2_edge) {
-                const i64 f_id = pe_ref(c, c.P, edge);
-                if (f_id == -1 || pf_ref(c, c.P, f_id) != edge) return;
-                i64 p, q, w3;
-                tri_verts(G, f_id, p, q, w3);
-                w3 = third_of(p, q, w3, v1, v2);
-                lower(c, w3);
-            } else if (o_v1_edge != o_v2_edge && v1_edge != v2_edge) {
-                const i64 f_id = pe_ref(c, c.Q, edge);
-                if (f_id == -1 || pf_ref(c, c.Q, f_id) != edge) {
-                    lower(c, v3);
-                } else if (f_id < G.F && f_id >= 0) {
-                    i64 p, q, v3_1;
-                    tri_verts(G, f_id, p, q, v3_1);
-                    v3_1 = third_of(p, q, v3_1, v1, v2);
-                    v1_edge = above_g(c, v2, v3_1);
-                    v2_edge = above_g(c, v1, v3_1);
-                    o_v1_edge = above_f(c, v2, v3_1);
-                    o_v2_edge = above_f(c, v1, v3_1);
-                    if (v1_edge && v2_edge && ((!o_v1_edge && o_v2_edge) || (o_v1_edge && !o_v2_edge))) {
-                        if (!o_v1_edge) lower(c, v2);
-                        else lower(c, v1);
-                    } else {
-                        lower(c, v3);
-                    }
-                }
-            } else if (!above_g(c, v1, v3) || !above_g(c, v2, v3)) {
-                lower(c, v3);
+    const i64 pf = R.face_partner(c.P, id);
+    if (pf != -1 && cell_kind(pf) == KIND_EDGE) {
+        i64 v1, v2;
+        R.verts(pf, v1, v2);
+        const i64 v3 = R.third(id, v1, v2);
+        const bool g1 = above_g(c, v2, v3), g2 = above_g(c, v1, v3), f1 = above_f(c, v2, v3), f2 = above_f(c, v1, v3);
+        if (g1 && g2) {  // the edge's original face is this one
+            lower(c, v3);
+        } else if (f1 != f2 && g1 != g2) {
+            const i64 ff = R.edge_partner(c.Q, pf);
+            i64 w = v3;
+            if (ff != -1 && cell_kind(ff) == KIND_FACE) {
+                const i64 u = R.third(ff, v1, v2);
+                const bool h1 = above_f(c, v2, u), h2 = above_f(c, v1, u);
+                if (above_g(c, v2, u) && above_g(c, v1, u) && h1 != h2) w = !h1 ? v2 : v1;
             }
-        } else if (pf < G.T && pf >= 0 && pt_ref(c, c.P, pf) == id) {
-            const i64 tet = pf;
-            i64 v1, v2, v3, a, b, cc, v4;
-            tri_verts(G, id, v1, v2, v3);
-            tet_verts(G, tet, a, b, cc, v4);
-            v4 = fourth_of(a, b, cc, v4, v1, v2, v3);
-            const bool or1 = above_f(c, v3, v4), or2 = above_f(c, v2, v4), or3 = above_f(c, v1, v4);
-            if (!or1 || !or2 || !or3) {
-                const i64 pff = pt_ref(c, c.Q, tet);
-                if (pff != -1) {
-                    i64 v1_1, v2_1, v3_1;
-                    tri_verts(G, pff, v1_1, v2_1, v3_1);
-                    const bool f1 = above_g(c, v3_1, v4), f2 = above_g(c, v2_1, v4), f3 = above_g(c, v1_1, v4);
-                    const bool o1 = above_f(c, v3_1, v4), o2 = above_f(c, v2_1, v4), o3 = above_f(c, v1_1, v4);
-                    if ((!f1 || !f2 || !f3) && (!o1 || !o2 || !o3)) {
-                        const i64 id2 = pf_ref(c, c.P, pff);
-                        if (id2 >= 0 && id2 < G.E && pe_ref(c, c.P, id2) == pff) {
-                            i64 w1, w2;
-                            edge_verts(G, id2, w1, w2);
-                            i64 w3 = v3_1;
-                            if (v1_1 != w1 && w2 != v1_1) w3 = v1_1;
-                            else if (v2_1 != w1 && v2_1 != w2) w3 = v2_1;
-                            lower(c, w3);
-                        } else if (id2 >= 0 && id2 < G.T && pt_ref(c, c.P, id2) == pff) {
-                            i64 t1, t2, t3, t4;
-                            tet_verts(G, id2, t1, t2, t3, t4);
-                            if (t1 != v1_1 && t1 != v2_1 && t1 != v3_1) t4 = v1_1;
-                            else if (t2 != v1_1 && t2 != v2_1 && t2 != v3_1) t4 = v2_1;
-                            else if (t3 != v1_1 && t3 != v2_1 && t3 != v3_1) t4 = v3_1;
-                            (void)get_delta(c, t4);
-                            lower(c, t1);
-                            lower(c, t2);
-                            lower(c, t3);
-                            lower(c, t4);
-                        }
-                    } else {
-                        lower(c, v1_1);
-                        lower(c, v2_1);
-                        lower(c, v3_1);
-                    }
-                } else {
-                    lower(c, v4);
-                }
-            } else {
-                lower(c, v4);
-            }
+            lower(c, w);
+        } else if (!g1 || !g2) {
+            lower(c, v3);
         }
+        return;
+    }
+    if (pf != -1) {  // originally paired with a tetrahedron
+        i64 v1, v2, v3;
+        R.verts(id, v1, v2, v3);
+        const i64 v4 = R.fourth(pf, v1, v2, v3);
+        if (above_f(c, v3, v4) && above_f(c, v2, v4) && above_f(c, v1, v4)) {
+            lower(c, v4);
+            return;
+        }
+        const i64 pff = R.tet_partner(c.Q, pf);
+        if (pff == -1) {
+            lower(c, v4);
+            return;
+        }
+        i64 u1, u2, u3;
+        R.verts(pff, u1, u2, u3);
+        const bool ga = above_g(c, u3, v4) && above_g(c, u2, v4) && above_g(c, u1, v4);
+        const bool fa = above_f(c, u3, v4) && above_f(c, u2, v4) && above_f(c, u1, v4);
+        if (ga || fa) {
+            lower(c, u1);
+            lower(c, u2);
+            lower(c, u3);
+            return;
+        }
+        const i64 id2 = R.face_partner(c.P, pff);
+        if (id2 == -1) return;
+        if (cell_kind(id2) == KIND_EDGE) {
+            i64 w1, w2;
+            R.verts(id2, w1, w2);
+            lower(c, third_of(u1, u2, u3, w1, w2));
+        } else {
+            // as the reference has it: the fourth vertex is replaced by one of the
+            // face's when an earlier one is not on the face
+            i64 t1, t2, t3, t4;
+            R.verts(id2, t1, t2, t3, t4);
+            if (t1 != u1 && t1 != u2 && t1 != u3) t4 = u1;
+            else if (t2 != u1 && t2 != u2 && t2 != u3) t4 = u2;
+            else if (t3 != u1 && t3 != u2 && t3 != u3) t4 = u3;
+            lower(c, t1);
+            lower(c, t2);
+            lower(c, t3);
+            lower(c, t4);
+        }
+        return;
+    }
+    const i64 qf = R.face_partner(c.Q, id);
+    if (qf == -1) return;
+    if (cell_kind(qf) == KIND_EDGE) {
+        i64 v1, v2;
+        R.verts(qf, v1, v2);
+        const i64 tf = R.edge_partner(c.P, qf);
+        if (tf == -1) return;
+        if (cell_kind(tf) == KIND_FACE) {
+            lower(c, R.third(tf, v1, v2));
+        } else {
+            lower(c, v1);
+            lower(c, v2);
+        }
+        return;
+    }
+    i64 v1, v2, v3;
+    R.verts(id, v1, v2, v3);
+    const i64 v4 = R.fourth(qf, v1, v2, v3);
+    const bool g1 = above_g(c, v3, v4), g2 = above_g(c, v2, v4), g3 = above_g(c, v1, v4);
+    const bool f1 = above_f(c, v3, v4), f2 = above_f(c, v2, v4), f3 = above_f(c, v1, v4);
+    if (g1 && g2 && g3) {
+        if (!f1) lower(c, v3);
+        else if (!f2) lower(c, v2);
+        else if (!f3) lower(c, v1);
+        return;
+    }
+    // the reference compares this face id with the number of tetrahedra
+    const i64 true_cell = R.tet_partner(c.P, qf);
+    i64 m = -1;
+    if (!(true_cell != -1 && code_ref(G, true_cell) < G.T)) m = smallest_vertex(c, v1, v2, v3);
+    if (m != -1) {
+        lower(c, m);
     } else {
-        const i64 qf = pf_ref(c, c.Q, id);
-        if (qf != -1 && qf < G.E && qf >= 0 && pe_ref(c, c.Q, qf) == id) {
-            const i64 edge_id = qf;
-            i64 v1, v2;
-            edge_verts(G, edge_id, v1, v2);
-            const i64 sv1 = !above_g(c, v1, v2) ? v2 : v1;
-            const i64 sv2 = !above_g(c, v1, v2) ? v1 : v2;
-            const i64 true_face_id = pe_ref(c, c.P, edge_id);
-            if (true_face_id != -1 && pf_ref(c, c.P, true_face_id) == edge_id) {
-                i64 p, q, w3;
-                tri_verts(G, true_face_id, p, q, w3);
-                if (sv1 != p && sv2 != p) w3 = p;
-                if (sv1 != q && sv2 != q) w3 = q;
-                lower(c, w3);
-            } else if (true_face_id >= 0 && true_face_id < G.V && pv_ref(c, c.P, true_face_id) == edge_id) {
-                lower(c, sv1);
-                lower(c, sv2);
-            }
-        } else if (qf != -1 && qf < G.T && qf >= 0 && pt_ref(c, c.Q, qf) == id) {
-            const i64 tet = qf;
-            i64 v1, v2, v3, a, b, cc, v4;
-            tri_verts(G, id, v1, v2, v3);
-            tet_verts(G, tet, a, b, cc, v4);
-            v4 = fourth_of(a, b, cc, v4, v1, v2, v3);
-            const bool f1 = above_g(c, v3, v4), f2 = above_g(c, v2, v4), f3 = above_g(c, v1, v4);
-            const bool o1 = above_f(c, v3, v4), o2 = above_f(c, v2, v4), o3 = above_f(c, v1, v4);
-            if (f1 && f2 && f3) {
-                if (f1 != o1) lower(c, v3);
-                else if (f2 != o2) lower(c, v2);
-                else if (f3 != o3) lower(c, v1);
-            } else {
-                const i64 true_cell = pt_ref(c, c.P, tet);
-                if (true_cell >= 0 && true_cell < G.T) {
-                    lower(c, v1);
-                    lower(c, v2);
-                    lower(c, v3);
-                } else {
-                    const i64 m = smallest_vertex(c, v1, v2, v3);
-                    if (m != -1) {
-                        lower(c, m);
-                    } else {
-                        lower(c, v1);
-                        lower(c, v2);
-                        lower(c, v3);
-                    }
-                }
-            }
-        }
+        lower(c, v1);
+        lower(c, v2);
+        lower(c, v3);
     }
 }
 
 // --------------------------------------------------------------- A11 fix_maximum
-__device__ inline void rule_max(const RuleCtx &c, i64 id) {
-    const Grid &G = c.g;
-    const i64 pt = pt_ref(c, c.P, id);
-    if (pt != -1) {
-        const i64 face1 = pt;
-        i64 v1, v2, v3, a, b, cc, v4;
-        tri_verts(G, face1, v1, v2, v3);
-        tet_verts(G, id, a, b, cc, v4);
-        v4 = fourth_of(a, b, cc, v4, v1, v2, v3);
-        const bool o1 = above_f(c, v1, v4), o2 = above_f(c, v2, v4), o3 = above_f(c, v3, v4);
-        if (o1 && o2 && o3) {
-            lower(c, v4);
-        } else {
-            const i64 fc = pf_ref(c, c.Q, face1);
-            if (fc >= 0) {
-                if (fc < G.E && pe_ref(c, c.Q, fc) == face1) {
-                    i64 e1, e2;
-                    edge_verts(G, fc, e1, e2);
-                    lower(c, above_g(c, e1, e2) ? e1 : e2);
-                } else if (fc < G.T && pt_ref(c, c.Q, fc) == face1) {
-                    lower(c, v4);
-                }
-            }
-        }
-    } else {
-        const i64 face1 = pt_ref(c, c.Q, id);
-        i64 v1, v2, v3, a, b, cc, v4;
-        tri_verts(G, face1, v1, v2, v3);
-        tet_verts(G, id, a, b, cc, v4);
-        v4 = fourth_of(a, b, cc, v4, v1, v2, v3);
-        const bool f1 = above_g(c, v1, v4), f2 = above_g(c, v2, v4), f3 = above_g(c, v3, v4);
-        const bool o1 = above_f(c, v1, v4), o2 = above_f(c, v2, v4), o3 = above_f(c, v3, v4);
-        if (f1 && f2 && f3) {
-            if (!o1 && f1) lower(c, v1);
-            if (!o2 && f2) lower(c, v2);
-            if (!o3 && f3) lower(c, v3);
-            if (o1 && o2 && o3) {
-                const i64 it = pf_ref(c, c.P, face1);
-                if (it != -1) {
-                    // the reference reads this id as a tetrahedron whatever its kind
-                    if (it < 0 || it >= G.T) atomicOr(c.err, ERR_OOB);
-                    i64 p, q, r, w4;
-                    tet_verts(G, it, p, q, r, w4);
-                    w4 = fourth_of(p, q, r, w4, v1, v2, v3);
-                    lower(c, w4);
-                }
-            }
-        } else {
-            const i64 pid = pf_ref(c, c.P, face1);
-            if (pid != -1) {
-                if (pid >= 0 && pid < G.E && pe_ref(c, c.P, pid) == face1) {
-                    i64 e1, e2;
-                    edge_verts(G, pid, e1, e2);
-                    lower(c, e1);
-                    lower(c, e2);
-                } else {
-                    if (pid < 0 || pid >= G.T) atomicOr(c.err, ERR_OOB);
-                    i64 p, q, r, s2;
-                    tet_verts(G, pid, p, q, r, s2);
-                    lower(c, p);
-                    lower(c, q);
-                    lower(c, r);
-                    lower(c, s2);
-                }
-            } else {
-                if (!o1) lower(c, v1);
-                if (!o2) lower(c, v2);
-                if (!o3) lower(c, v3);
-            }
-        }
-    }
+// the reference reads an edge id as a tetrahedron's: its vertex that is none of v1, v2, v3
+__device__ DMTZ_SHARED_CODE i64 literal_fourth(const Grid &G, i64 id, i64 v1, i64 v2, i64 v3, int *err) {
+    if (id < 0 || id >= G.T) atomicOr(err, ERR_OOB);
+    i64 p, q, r, w;
+    tet_verts(G, id, p, q, r, w);
+    return fourth_of(p, q, r, w, v1, v2, v3);
 }
-
-// --------------------------------------------------------------- A12/A13 separatrix checks
-// cofaces of a triangle in get_cell_tetra order (main_3d.cu:4363-4430):
-// x = first existing coface, y = last existing (left as given when only one)
-__device__ inline int face_cofaces(const Grid &g, i64 t, i64 out[2]) {
-    int x, y, z, sl;
-    face_unref(g, t, x, y, z, sl);
-    int n = 0;
-    for (int j = 0; j < TOPO_FACE_NCOF[sl]; j++) {
-        const signed char *tc = TOPO_FACE_COF[sl][j];
-        if (!cell_ok(g, x + tc[0], y + tc[1], z + tc[2], 1, 1, 1)) continue;
-        out[n++] = tet_ref(g, x + tc[0], y + tc[1], z + tc[2], tc[3]);
+__device__ __forceinline__ void rule_max(const Rules &R, i64 id) {
+    const RuleCtx &c = R.c;
+    const i64 pt = R.tet_partner(c.P, id);
+    const i64 face = pt != -1 ? pt : R.tet_partner(c.Q, id);
+    if (face == -1) return;  // critical in both: not listed
+    i64 v1, v2, v3;
+    R.verts(face, v1, v2, v3);
+    const i64 v4 = R.fourth(id, v1, v2, v3);
+    const bool f1 = above_f(c, v1, v4), f2 = above_f(c, v2, v4), f3 = above_f(c, v3, v4);
+    if (pt != -1) {
+        if (f1 && f2 && f3) {
+            lower(c, v4);
+            return;
+        }
+        const i64 fc = R.face_partner(c.Q, face);
+        if (fc == -1) return;
+        i64 w = v4;
+        if (cell_kind(fc) == KIND_EDGE) {
+            i64 e1, e2;
+            R.verts(fc, e1, e2);
+            w = above_g(c, e1, e2) ? e1 : e2;
+        }
+        lower(c, w);
+        return;
     }
-    return n;
+    const bool g1 = above_g(c, v1, v4), g2 = above_g(c, v2, v4), g3 = above_g(c, v3, v4);
+    if (g1 && g2 && g3) {
+        if (!f1) lower(c, v1);
+        if (!f2) lower(c, v2);
+        if (!f3) lower(c, v3);
+        if (f1 && f2 && f3) {
+            const i64 it = R.face_partner(c.P, face);
+            if (it != -1)
+                lower(c, cell_kind(it) == KIND_TET ? R.fourth(it, v1, v2, v3)
+                                                   : literal_fourth(c.g, code_ref(c.g, it), v1, v2, v3, c.err));
+        }
+        return;
+    }
+    const i64 pid = R.face_partner(c.P, face);
+    if (pid == -1) {
+        if (!f1) lower(c, v1);
+        if (!f2) lower(c, v2);
+        if (!f3) lower(c, v3);
+    } else if (cell_kind(pid) == KIND_EDGE) {
+        i64 e1, e2;
+        R.verts(pid, e1, e2);
+        lower(c, e1);
+        lower(c, e2);
+    } else {
+        i64 p, q, r, w;
+        R.verts(pid, p, q, r, w);
+        lower(c, p);
+        lower(c, q);
+        lower(c, r);
+        lower(c, w);
+    }
 }
 
 // --------------------------------------------------------------- A15 fix_as_vpath (type 2)
-__device__ inline void rule_as_path(const RuleCtx &c, i64 t_idx) {
-    const Grid &G = c.g;
-    const i64 true_edge = pt_ref(c, c.P, t_idx);
-    const i64 false_edge = pt_ref(c, c.Q, t_idx);
-    const i64 pfe = pf_ref(c, c.P, false_edge);
-    if (pfe >= 0 && pfe < G.T && pt_ref(c, c.P, pfe) == false_edge) {
-        i64 v1, v2, v3, a, b, cc, d;
-        tri_verts(G, false_edge, v1, v2, v3);
-        tet_verts(G, pfe, a, b, cc, d);
-        lower(c, fourth_of(a, b, cc, d, v1, v2, v3));
+__device__ __forceinline__ void rule_as_path(const Rules &R, i64 tet) {
+    const RuleCtx &c = R.c;
+    const i64 tf = R.tet_partner(c.P, tet), ff = R.tet_partner(c.Q, tet);
+    i64 v1, v2, v3, a = -1, b = -1, tv3 = -1;
+    if (ff == -1) {  // the reference reads its arrays at -1 here
+        atomicOr(c.err, ERR_OOB);
+        tri_verts(c.g, -1, a, b, tv3);
     } else {
-        i64 v1, v2, v3, a, b, tv3;
-        tri_verts(G, true_edge, v1, v2, v3);
-        tri_verts(G, false_edge, a, b, tv3);
-        if (a != v1 && a != v2 && a != v3) tv3 = a;
-        else if (b != v1 && b != v2 && b != v3) tv3 = b;
-        lower(c, tv3);
+        R.verts(ff, a, b, tv3);
+        const i64 pfe = R.face_partner(c.P, ff);
+        if (pfe != -1 && cell_kind(pfe) == KIND_TET) {
+            lower(c, R.fourth(pfe, a, b, tv3));
+            return;
+        }
     }
+    if (tf == -1) tri_verts(c.g, -1, v1, v2, v3);
+    else R.verts(tf, v1, v2, v3);
+    lower(c, fourth_of(a, b, tv3, tv3, v1, v2, v3));
 }
 // A14 fix_ds_vpath (type 0)
-__device__ inline void rule_ds_path(const RuleCtx &c, i64 v_idx) {
-    const i64 tpe = pv_ref(c, c.P, v_idx);
+__device__ DMTZ_SHARED_CODE void literal_ds_path(const RuleCtx &c, i64 v) {
+    const i64 tpe = pv_ref(c, c.P, v);
     i64 v1, v2;
     edge_verts(c.g, tpe, v1, v2);
-    lower(c, v_idx == v1 ? v2 : v1);
+    lower(c, v == v1 ? v2 : v1);
+}
+__device__ __forceinline__ void rule_ds_path(const Rules &R, i64 v) {
+    const i64 w = v >= 0 && v < R.c.g.V ? R.below(R.c.P, v) : -1;
+    if (w >= 0) lower(R.c, w);
+    else literal_ds_path(R.c, v);  // no vertex (-1), or a critical one
 }
 
 // fix_ds_wall (main_3d.cu:5297-5413) for the wall record edge e: the edge's
