@@ -159,23 +159,6 @@ __global__ void k_mark_dirty(Grid g, int nbx, int nby, int sx, int sy, int sz, c
                 for (int bx = x0; bx <= x1; bx++) flags[bx + (i64)nbx * (by + (i64)nby * bz)] = 1;
     }
 }
-// Walk-cache tiles: 16^3 anchors.  Every brick the criticality pass re-pairs
-// marks the tiles it overlaps (a brick spans at most 3 tiles per axis).
-constexpr int kTile = 16, kTileShift = 4;
-__global__ void k_mark_tiles(const uint32_t *list, const unsigned long long *n, int sx, int sy, int sz, int ntx,
-                             int nty, int ntz, uint8_t *dirty) {
-    const i64 nb = (i64)*n;
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += (i64)gridDim.x * blockDim.x) {
-        const uint32_t e = list[i];
-        const int bx = e & 0x7FF, by = (e >> 11) & 0x7FF, bz = e >> 22;
-        const int x0 = (bx * sx) >> kTileShift, x1 = min((bx * sx + sx - 1) >> kTileShift, ntx - 1);
-        const int y0 = (by * sy) >> kTileShift, y1 = min((by * sy + sy - 1) >> kTileShift, nty - 1);
-        const int z0 = (bz * sz) >> kTileShift, z1 = min((bz * sz + sz - 1) >> kTileShift, ntz - 1);
-        for (int tz = z0; tz <= z1; tz++)
-            for (int ty = y0; ty <= y1; ty++)
-                for (int tx = x0; tx <= x1; tx++) dirty[tx + (i64)ntx * (ty + (i64)nty * tz)] = 1;
-    }
-}
 // the marked bricks as a list, and the marks cleared for the next round (four
 // marks to a word)
 __global__ void k_compact_bricks(int nbx, int nby, int nbz, uint32_t *flags, uint32_t *list, unsigned long long *n) {
@@ -295,62 +278,51 @@ struct PathRec {
     i64 cap_as, cap_ds;     // at most one record per original 2-saddle / 1-saddle
 };
 
-// Original ascending paths (is_false, main_3d.cu:4437-4497) step from a
-// tetrahedron through the facet it is paired with to that facet's other
-// coface (get_cell_tetra's other one; none = the path leaves the grid).  The
-// original gradient is fixed during a correction, so each tetrahedron's
-// successor is computed once and stored in one byte: the successor's anchor
-// offset ((dx+1) + 3(dy+1) + 9(dz+1), each in -1..1) times 6 plus its slot;
-// 255 = the path ends (a maximum, or a boundary facet).  The six bytes of an
-// anchor's tetrahedra share one 8-byte word (one coalesced store).  The
-// reference's back-pointer test on the way is always true for a consistent
-// gradient.
-__device__ __forceinline__ uint8_t asc_step(const Grid &g, int x, int y, int z, int ts, uint32_t tc) {
-    const int j = (tc >> (3 * ts)) & 7;
-    if (j == 7) return 255;
-    const signed char *tf = TOPO_TET_FACE[ts][j];
-    const int fs = tf[3], other = 1 - tf[4];
-    if (other >= TOPO_FACE_NCOF[fs]) return 255;
-    const signed char *oc = TOPO_FACE_COF[fs][other];
-    const int dx = tf[0] + oc[0], dy = tf[1] + oc[1], dz = tf[2] + oc[2];
-    if (!cell_ok(g, x + dx, y + dy, z + dz, 1, 1, 1)) return 255;
-    return (uint8_t)(((dx + 1) + 3 * (dy + 1) + 9 * (dz + 1)) * 6 + oc[3]);
-}
-// asc_step with the tetrahedron slot TS fixed at compile time: the facet and
-// coface tables become immediates (runtime-indexed table reads with different
-// indices across a warp are served one index at a time)
-template <int TS>
-__device__ __forceinline__ uint8_t asc_step_c(const Grid &g, int x, int y, int z, uint32_t tc) {
-    const int j = (tc >> (3 * TS)) & 7;
-    uint8_t out = 255;
-    DMTZ_FOR(4, J, {
-        constexpr int jj = decltype(J)::value;
-        constexpr int fs = cxt::TOPO_TET_FACE[TS][jj][3], other = 1 - cxt::TOPO_TET_FACE[TS][jj][4];
-        if constexpr (other < cxt::TOPO_FACE_NCOF[fs]) {
-            constexpr int dx = cxt::TOPO_TET_FACE[TS][jj][0] + cxt::TOPO_FACE_COF[fs][other][0],
-                          dy = cxt::TOPO_TET_FACE[TS][jj][1] + cxt::TOPO_FACE_COF[fs][other][1],
-                          dz = cxt::TOPO_TET_FACE[TS][jj][2] + cxt::TOPO_FACE_COF[fs][other][2],
-                          os = cxt::TOPO_FACE_COF[fs][other][3];
-            constexpr uint8_t code = (uint8_t)(((dx + 1) + 3 * (dy + 1) + 9 * (dz + 1)) * 6 + os);
-            if (j == jj) out = cell_ok(g, x + dx, y + dy, z + dz, 1, 1, 1) ? code : (uint8_t)255;
+// Ascending paths (is_false, main_3d.cu:4437-4497) step from a tetrahedron
+// through the facet it is paired with to that facet's other coface
+// (get_cell_tetra's other one; none = the path leaves the grid).  That coface
+// lies in the same cube or in the one across a face, so a step is one byte per
+// (slot, facet): direction (0 none, 1 +x, 2 -x, 3 +y, 4 -y, 5 +z, 6 -z) * 8 +
+// new slot.  The reference's back-pointer test on the way is always true for a
+// consistent gradient.
+struct AscTab {
+    uint8_t next[24];  // [slot * 4 + facet]
+};
+constexpr AscTab make_asc_tab() {
+    AscTab t = {};
+    for (int s = 0; s < 6; s++)
+        for (int j = 0; j < 4; j++) {
+            const signed char *f = cxt::TOPO_TET_FACE[s][j], *c = cxt::TOPO_FACE_COF[f[3]][1 - f[4]];
+            const int dx = f[0] + c[0], dy = f[1] + c[1], dz = f[2] + c[2];
+            const int o = dx ? (dx > 0 ? 1 : 2) : dy ? (dy > 0 ? 3 : 4) : dz ? (dz > 0 ? 5 : 6) : 0;
+            t.next[s * 4 + j] = (uint8_t)(o * 8 + c[3]);
         }
-    });
-    return out;
+    return t;
 }
-__global__ void k_path_succ(Grid g, const uint32_t *tcodeP, uint8_t *succ) {
-    i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= g.V) return;
-    int x, y, z;
-    decode_v(g, v, x, y, z);
-    const bool cube = cell_ok(g, x, y, z, 1, 1, 1);
-    const uint32_t tc = tcodeP[v];
-    uint64_t packed = 0xFFFF000000000000ull;
-    DMTZ_FOR(6, TS, {
-        constexpr int ts = decltype(TS)::value;
-        const uint8_t out = cube ? asc_step_c<ts>(g, x, y, z, tc) : (uint8_t)255;
-        packed |= (uint64_t)out << (8 * ts);
-    });
-    reinterpret_cast<uint64_t *>(succ)[v] = packed;
+constexpr bool asc_steps_are_axial() {
+    for (int s = 0; s < 6; s++)
+        for (int j = 0; j < 4; j++) {
+            const signed char *f = cxt::TOPO_TET_FACE[s][j], *c = cxt::TOPO_FACE_COF[f[3]][1 - f[4]];
+            const int dx = f[0] + c[0], dy = f[1] + c[1], dz = f[2] + c[2];
+            if (dx * dx + dy * dy + dz * dz > 1) return false;
+        }
+    return true;
+}
+static_assert(asc_steps_are_axial(), "a facet's cofaces lie in one cube or in two that share a face");
+static __device__ const AscTab kAscTab = make_asc_tab();
+// the table into shared memory (every thread of the block calls this)
+__device__ __forceinline__ void load_asc_tab(AscTab &t) {
+    if (threadIdx.x < 24) t.next[threadIdx.x] = kAscTab.next[threadIdx.x];
+    __syncthreads();
+}
+// one step from (x, y, z, s) with facet j (0..3); false: the path leaves the grid
+__device__ __forceinline__ bool asc_move(const Grid &g, const AscTab &t, int &x, int &y, int &z, int &s, int j) {
+    const int e = t.next[s * 4 + j], o = e >> 3;
+    x += (o == 1) - (o == 2);
+    y += (o == 3) - (o == 4);
+    z += (o == 5) - (o == 6);
+    s = e & 7;
+    return (unsigned)x < (unsigned)(g.W - 1) && (unsigned)y < (unsigned)(g.H - 1) && (unsigned)z < (unsigned)(g.D - 1);
 }
 
 // compact list of original critical cells of one dimension: criticality
@@ -567,17 +539,11 @@ __device__ i64 desc_end(const Grid &g, const uint8_t *pv, const uint8_t *pvo, i6
 // End of the ascending path from tetrahedron (x, y, z, s) under tet codes tc:
 // the maximum reached (reference id) or -1 when the path leaves the grid
 // (get_paired_id, main_3d.cu:4499-4537)
-__device__ i64 asc_end(const Grid &g, const uint32_t *tc, int x, int y, int z, int s, i64 cap, int *err) {
+__device__ i64 asc_end(const Grid &g, const AscTab &t, const uint32_t *tc, int x, int y, int z, int s, i64 cap, int *err) {
     for (i64 steps = 0;; steps++) {
-        const uint32_t code = tc[x + (i64)y * g.W + (i64)z * g.WH];
-        if (((code >> (3 * s)) & 7) == 7) return tet_ref(g, x, y, z, s);
-        const int s8 = asc_step(g, x, y, z, s, code);
-        if (s8 == 255) return -1;
-        const int d = s8 / 6;
-        s = s8 - 6 * d;
-        x += d % 3 - 1;
-        y += (d / 3) % 3 - 1;
-        z += d / 9 - 1;
+        const int j = (tc[x + (i64)y * g.W + (i64)z * g.WH] >> (3 * s)) & 7;
+        if (j == 7) return tet_ref(g, x, y, z, s);
+        if (!asc_move(g, t, x, y, z, s, j)) return -1;
         if (steps > cap) {
             atomicOr(err, ERR_WALK);
             return -1;
@@ -586,8 +552,8 @@ __device__ i64 asc_end(const Grid &g, const uint32_t *tc, int x, int y, int z, i
 }
 // is_false (main_3d.cu:4437-4497): along the original ascending path from the
 // tetrahedron, the first one whose decompressed pairing differs (into cur)
-__device__ bool first_diff(const Grid &g, const uint32_t *tcP, const uint32_t *tcQ, const uint8_t *succ, int x, int y,
-                           int z, int s, i64 cap, int *err, i64 &cur) {
+__device__ bool first_diff(const Grid &g, const AscTab &t, const uint32_t *tcP, const uint32_t *tcQ, int x, int y, int z,
+                           int s, i64 cap, int *err, i64 &cur) {
     for (i64 steps = 0;; steps++) {
         const i64 ci = x + (i64)y * g.W + (i64)z * g.WH;
         const int p = (tcP[ci] >> (3 * s)) & 7;
@@ -596,13 +562,7 @@ __device__ bool first_diff(const Grid &g, const uint32_t *tcP, const uint32_t *t
             cur = tet_code(ci, s);
             return true;
         }
-        const int s8 = succ[ci * 8 + s];
-        if (s8 == 255) return false;
-        const int d = s8 / 6;
-        s = s8 - 6 * d;
-        x += d % 3 - 1;
-        y += (d / 3) % 3 - 1;
-        z += d / 9 - 1;
+        if (!asc_move(g, t, x, y, z, s, p)) return false;
         if (steps > cap) {
             atomicOr(err, ERR_WALK);
             return false;
@@ -647,7 +607,9 @@ __global__ void k_conn_ds(const __grid_constant__ RuleCtx c, PathRec R, i64 cap)
 // direction loop's counter instead of the triangle (all triangles share 28
 // slots, written concurrently), so its own result depends on scheduling.
 __global__ void k_conn_as(Grid g, const uint32_t *critP, const uint32_t *critQ, const uint32_t *tcP,
-                          const uint32_t *tcQ, const uint8_t *succ, PathRec R, i64 cap, int *err) {
+                          const uint32_t *tcQ, PathRec R, i64 cap, int *err) {
+    __shared__ AscTab tab;
+    load_asc_tab(tab);
     for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += (i64)gridDim.x * blockDim.x) {
         uint32_t m = (critQ[v] >> 8) & 0xFFFu;
         if (!m) continue;
@@ -661,11 +623,11 @@ __global__ void k_conn_as(Grid g, const uint32_t *critP, const uint32_t *critQ, 
                 const signed char *tc = TOPO_FACE_COF[sl][j];
                 const int cx = x + tc[0], cy = y + tc[1], cz = z + tc[2], cs = tc[3];
                 if (!cell_ok(g, cx, cy, cz, 1, 1, 1)) continue;
-                const i64 eq = asc_end(g, tcQ, cx, cy, cz, cs, cap, err);
-                const i64 ep = ((mp >> sl) & 1u) ? asc_end(g, tcP, cx, cy, cz, cs, cap, err) : -1;
+                const i64 eq = asc_end(g, tab, tcQ, cx, cy, cz, cs, cap, err);
+                const i64 ep = ((mp >> sl) & 1u) ? asc_end(g, tab, tcP, cx, cy, cz, cs, cap, err) : -1;
                 if (eq == ep) continue;
                 i64 cur;
-                if (first_diff(g, tcP, tcQ, succ, cx, cy, cz, cs, cap, err, cur)) {
+                if (first_diff(g, tab, tcP, tcQ, cx, cy, cz, cs, cap, err, cur)) {
                     const unsigned long long at = atomicAdd(&R.n[0], 1ull);
                     if ((i64)at < R.cap_as) {
                         R.as_tet[at] = tet_code(cx + (i64)cy * g.W + (i64)cz * g.WH, cs);
@@ -676,59 +638,6 @@ __global__ void k_conn_as(Grid g, const uint32_t *critP, const uint32_t *critQ, 
             }
         }
     }
-}
-
-// 3-D prefix sum of the dirty tiles (sat = number of dirty tiles in the box
-// from the origin to the tile), one thread per line per axis; the x pass
-// also clears the dirty marks for the next detection
-__global__ void k_sat_x(uint8_t *dirty, uint32_t *sat, int ntx, int nty, int ntz) {
-    const i64 lines = (i64)nty * ntz;
-    for (i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x; t < lines; t += (i64)gridDim.x * blockDim.x) {
-        uint32_t run = 0;
-        for (int x = 0; x < ntx; x++) {
-            const i64 i = t * ntx + x;
-            run += dirty[i];
-            dirty[i] = 0;
-            sat[i] = run;
-        }
-    }
-}
-__global__ void k_sat_yz(uint32_t *sat, int ntx, int nty, int ntz, int axis) {
-    const i64 lines = axis == 1 ? (i64)ntx * ntz : (i64)ntx * nty;
-    const int n = axis == 1 ? nty : ntz;
-    const i64 step = axis == 1 ? (i64)ntx : (i64)ntx * nty;
-    for (i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x; t < lines; t += (i64)gridDim.x * blockDim.x) {
-        const i64 base = axis == 1 ? (t % ntx) + (t / ntx) * (i64)ntx * nty : t;
-        uint32_t run = 0;
-        for (int k = 0; k < n; k++) {
-            run += sat[base + k * step];
-            sat[base + k * step] = run;
-        }
-    }
-}
-// a walk's tile box: x0 x1 y0 y1 z0 z1 in 10-bit fields, bit 63 = known
-// (a box with x0 > x1 is empty: the walk reads nothing that can change)
-constexpr unsigned long long kBoxKnown = 1ull << 63;
-__device__ __forceinline__ unsigned long long box_pack(int x0, int x1, int y0, int y1, int z0, int z1) {
-    return kBoxKnown | (unsigned long long)x0 | ((unsigned long long)x1 << 10) | ((unsigned long long)y0 << 20) |
-           ((unsigned long long)y1 << 30) | ((unsigned long long)z0 << 40) | ((unsigned long long)z1 << 50);
-}
-struct TileSat {
-    const uint32_t *sat;
-    int ntx, nty, ntz;
-};
-__device__ __forceinline__ uint32_t sat_at(const TileSat &T, int x, int y, int z) {
-    if (x < 0 || y < 0 || z < 0) return 0u;
-    return T.sat[x + (i64)T.ntx * (y + (i64)T.nty * z)];
-}
-// dirty tiles in a known box (0 for an empty box)
-__device__ __forceinline__ uint32_t box_dirty(const TileSat &T, unsigned long long b) {
-    const int x0 = (int)(b & 1023), x1 = (int)((b >> 10) & 1023), y0 = (int)((b >> 20) & 1023),
-              y1 = (int)((b >> 30) & 1023), z0 = (int)((b >> 40) & 1023), z1 = (int)((b >> 50) & 1023);
-    if (x0 > x1) return 0u;
-    return sat_at(T, x1, y1, z1) - sat_at(T, x0 - 1, y1, z1) - sat_at(T, x1, y0 - 1, z1) - sat_at(T, x1, y1, z0 - 1) +
-           sat_at(T, x0 - 1, y0 - 1, z1) + sat_at(T, x0 - 1, y1, z0 - 1) + sat_at(T, x1, y0 - 1, z0 - 1) -
-           sat_at(T, x0 - 1, y0 - 1, z0 - 1);
 }
 
 // start tetrahedron (anchor offset, slot) of coface j of a triangle of slot
@@ -757,217 +666,396 @@ __device__ __forceinline__ void face_cof_start(int sl, int j, int &dx, int &dy, 
 static_assert(cxt::TOPO_FACE_NCOF[0] == 2 && cxt::TOPO_FACE_NCOF[5] == 2 && cxt::TOPO_FACE_NCOF[11] == 2,
               "every triangle slot has two cofaces");
 
+// --------------------------------------------------- geometry-mode separatrix checks
 // get_false_as_vpath (main_3d.cu:4540-4610) with is_false: for each original
 // 2-saddle triangle, its cofaces in search order; along each one's original
 // ascending path, the first tetrahedron whose decompressed pairing differs is
-// recorded, for the first coface that has one.  Done in two kernels for
-// parallelism: (2-saddle, coface) walks (res = the first differing
-// tetrahedron, -1 none, -2 no coface), then one thread per 2-saddle keeps the
-// first coface in search order that has one.  Walk lengths vary a lot, so a lane whose walk ends takes the next
-// walk of its warp's contiguous range of walks instead of idling until the
-// warp's longest walk ends (one step per loop turn; the warp refills its free
-// lanes together, without atomics).
+// recorded, for the first coface that has one.  get_false_ds_vpath
+// (:4837-4959): the reference's walk never advances past the first vertex
+// (dec_current_id stays at the start), so each 1-saddle endpoint's
+// steepest-descent pairing is compared once, v1 (higher id) first.
 //
-// Walk cache: a walk's result depends only on the decompressed pairing of the
-// tetrahedra it visited (up to its first differing one, or to its end), and
-// those sit at anchors inside the box of tiles the walk recorded.  A walk
-// whose box holds no tile re-paired since the last detection keeps its
-// result and is not walked again.
-// Walks are handed out in chunks of kWalkChunk by a ticket (*ticket, zero at
-// launch): a warp's idle lanes take the next walks of its chunk, then of the
-// next free chunk of the whole list, so warps that meet long walks do not hold
-// the kernel's end while others sit idle (one atomic per chunk, not per refill).
-__global__ void k_path_as_walk(Grid g, const i64 *sad2, const unsigned long long *nsad, const uint32_t *tcP,
-                               const uint32_t *tcQ, const uint8_t *succ, i64 *res, i64 cap, int *err,
-                               unsigned long long *wbox, TileSat T, unsigned long long *ticket) {
-    constexpr i64 kWalkChunk = 64;
-    const i64 n = 2 * (i64)*nsad;
-    const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
-    i64 pos = 0, end = 0;  // the warp's current chunk (the same in every lane)
-    i64 item = -1, steps = 0;
-    int x = 0, y = 0, z = 0, s = 0;
-    int bx0 = 0, bx1 = 0, by0 = 0, by1 = 0, bz0 = 0, bz1 = 0;  // tile box of the current walk
-    bool drained = false;
-    while (true) {
-        const unsigned want = __ballot_sync(full, item < 0 && !drained);
-        if (want) {
-            if (pos >= end) {  // the warp's chunk is used up: take the next one
-                unsigned long long b0 = 0;
-                if (lane == 0) b0 = atomicAdd(ticket, (unsigned long long)kWalkChunk);
-                pos = (i64)__shfl_sync(full, b0, 0);
-                end = min(n, pos + kWalkChunk);
-            }
-            const i64 my = pos + __popc(want & ((1u << lane) - 1u));
-            if (item < 0 && !drained) {
-                if (pos >= n) {
-                    drained = true;  // no walk is left anywhere
-                } else if (my < end) {
-                    const unsigned long long b = wbox[my];
-                    if (!(b & kBoxKnown) || box_dirty(T, b) != 0u) {
-                        item = my;
-                        steps = 0;
-                        const i64 code = sad2[my >> 1];
-                        const int j = (int)(my & 1);
-                        int vx, vy, vz, dx, dy, dz;
-                        decode_v(g, code / 12, vx, vy, vz);
-                        face_cof_start((int)(code % 12), j, dx, dy, dz, s);
-                        x = vx + dx;
-                        y = vy + dy;
-                        z = vz + dz;
-                        bx0 = bx1 = x >> kTileShift;
-                        by0 = by1 = y >> kTileShift;
-                        bz0 = bz1 = z >> kTileShift;
-                        const bool ok = cell_ok(g, x, y, z, 1, 1, 1);
-                        if (!ok) {  // no coface there: static, never walked again
-                            res[item] = -2;
-                            wbox[item] = box_pack(1, 0, 0, 0, 0, 0);
-                            item = -1;
-                        }
-                    }
-                }  // else: past this chunk's end, the next refill takes a new chunk
-            }
-            pos = min(pos + (i64)__popc(want), end);
-        }
-        if (__all_sync(full, item < 0 && drained)) break;
-        if (item >= 0) {  // one step of the walk
-            const i64 ci = x + (i64)y * g.W + (i64)z * g.WH;
-            const uint32_t wp = tcP[ci], wq = tcQ[ci];
-            const int s8 = succ[ci * 8 + s];
-            const int p = (wp >> (3 * s)) & 7;
-            i64 r = 0;
-            bool fin = true;
-            if (p == 7) {
-                r = -1;
-            } else if (p != (int)((wq >> (3 * s)) & 7)) {
-                r = tet_code(ci, s);
-            } else if (s8 == 255) {
-                r = -1;
-            } else if (++steps > cap) {
-                atomicOr(err, ERR_WALK);
-                r = -1;
-            } else {
-                const int d = s8 / 6;
-                s = s8 - 6 * d;
-                x += d % 3 - 1;
-                y += (d / 3) % 3 - 1;
-                z += d / 9 - 1;
-                bx0 = min(bx0, x >> kTileShift);
-                bx1 = max(bx1, x >> kTileShift);
-                by0 = min(by0, y >> kTileShift);
-                by1 = max(by1, y >> kTileShift);
-                bz0 = min(bz0, z >> kTileShift);
-                bz1 = max(bz1, z >> kTileShift);
-                fin = false;
-            }
-            if (fin) {
-                res[item] = r;
-                wbox[item] = box_pack(bx0, bx1, by0, by1, bz0, bz1);
-                item = -1;
-            }
-        }
-    }
+// The original paths never change during a correction.  They are traced once
+// (k_path_trace): every tetrahedron on one gets a bit beside its pairing code
+// (bit 18 + slot of the original tcode word), and every 2-saddle the box of
+// bricks its paths visit.  A path is false only if a marked tetrahedron's
+// pairing differs.  Per brick, two flags say whether it holds such a
+// tetrahedron (as), or an original 1-saddle with a differing endpoint (ds);
+// k_path_flags sets them once and the gradient kernel refreshes them for the
+// bricks it re-pairs (a changed value reaches exactly their anchors).  A
+// detection then walks from the 2-saddles whose box holds a flagged brick and looks
+// at the 1-saddles of flagged bricks, and at nothing else.
+//
+// Bound by the reads of the boxes (8 bytes per 2-saddle) and by the latency
+// of the walks left over (dependent loads).  Before, every 2-saddle near
+// re-paired tiles of 16^3 anchors was walked to its path's end and every 1-saddle
+// there checked, in eight kernels with a prefix sum over the tiles: 180 -> 27
+// us per detection on a noisy 97 x 61 x 75 field (paths of some hundred
+// steps), 677 -> 164 us at 256^3 (cold caches).
+// a 2-saddle's box of bricks: x0 x1 (11 bits each), y0 y1 (11), z0 z1 (10); x0 > x1: empty
+__device__ __forceinline__ unsigned long long box_pack(int x0, int x1, int y0, int y1, int z0, int z1) {
+    return (unsigned long long)x0 | ((unsigned long long)x1 << 11) | ((unsigned long long)y0 << 22) |
+           ((unsigned long long)y1 << 33) | ((unsigned long long)z0 << 44) | ((unsigned long long)z1 << 54);
 }
-__global__ void k_path_as_pick(Grid g, const i64 *sad2, const unsigned long long *nsad, const i64 *res, PathRec R) {
-    const i64 n = (i64)*nsad;
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        const int j = res[2 * i] >= 0 ? 0 : (res[2 * i + 1] >= 0 ? 1 : -1);
-        if (j < 0) continue;
-        const i64 code = sad2[i];
-        const i64 v = code / 12;
-        const int sl = (int)(code % 12);
-        const signed char *tc = TOPO_FACE_COF[sl][j];
-        const unsigned long long at = atomicAdd(&R.n[0], 1ull);
-        if ((i64)at < R.cap_as) {
-            R.as_tet[at] = tet_code(v + tc[0] + tc[1] * (i64)g.W + tc[2] * g.WH, tc[3]);
-            R.as_cur[at] = res[2 * i + j];
+__device__ __forceinline__ unsigned long long box_union(unsigned long long a, unsigned long long b) {
+    const int ax0 = (int)(a & 2047), ax1 = (int)((a >> 11) & 2047), bx0 = (int)(b & 2047), bx1 = (int)((b >> 11) & 2047);
+    if (ax0 > ax1) return b;
+    if (bx0 > bx1) return a;
+    return box_pack(min(ax0, bx0), max(ax1, bx1), min((int)((a >> 22) & 2047), (int)((b >> 22) & 2047)),
+                    max((int)((a >> 33) & 2047), (int)((b >> 33) & 2047)), min((int)((a >> 44) & 1023), (int)((b >> 44) & 1023)),
+                    max((int)(a >> 54), (int)(b >> 54)));
+}
+// does the box hold a flagged brick?  Boxes of more than kBoxBricks bricks (a
+// straight path) count as holding one: looking would cost more than walking
+constexpr int kBoxBricks = 27;
+__device__ __forceinline__ bool box_flagged(const uint8_t *flags, int nbx, int nby, unsigned long long b) {
+    const int x0 = (int)(b & 2047), x1 = (int)((b >> 11) & 2047), y0 = (int)((b >> 22) & 2047), y1 = (int)((b >> 33) & 2047),
+              z0 = (int)((b >> 44) & 1023), z1 = (int)(b >> 54);
+    if (x0 > x1) return false;
+    if ((x1 - x0 + 1) * (y1 - y0 + 1) * (z1 - z0 + 1) > kBoxBricks) return true;
+    unsigned any = 0;
+    for (int z = z0; z <= z1; z++)
+        for (int y = y0; y <= y1; y++) {
+            const uint8_t *row = flags + (i64)nbx * (y + (i64)nby * z);
+            for (int x = x0; x <= x1; x++) any |= row[x];
+        }
+    return any != 0;
+}
+// Work items handed out to warps in chunks (a multiple of 32): a warp's first
+// chunk is its own index, further ones come from *ticket (zero at launch), so
+// that warps that meet long walks do not hold the kernel's end.  Returns the
+// chunk's first item.
+__device__ __forceinline__ i64 next_chunk(bool &first, i64 chunk, unsigned long long *ticket) {
+    const i64 warps = (i64)gridDim.x * (blockDim.x / 32);
+    i64 c;
+    if (first) {
+        c = (i64)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+        first = false;
+    } else {
+        unsigned long long t = 0;
+        if ((threadIdx.x & 31) == 0) t = atomicAdd(ticket, 1ull);
+        c = warps + (i64)__shfl_sync(0xffffffffu, t, 0);
+    }
+    return c * chunk;
+}
+// chunk size that gives every warp of the grid about eight chunks
+__device__ __forceinline__ i64 chunk_size(i64 n, i64 most) {
+    const i64 c = (n / ((i64)gridDim.x * (blockDim.x / 32) * 8) + 31) / 32 * 32;
+    return c < 32 ? 32 : (c > most ? most : c);
+}
+
+// Paths of more than kSegment steps are cut into segments, each an item of its
+// own (start, box, slot of its 2-saddle among the ones with such paths, order:
+// coface << 25 | index along the path): a detection's longest chain of dependent
+// loads is then one segment's, and a long path is looked at only where its bricks are flagged.
+constexpr int kSegment = 16;
+struct Segment {
+    unsigned long long box;
+    i64 start;  // tetrahedron code
+    uint32_t slot, order;
+};
+struct LongPaths {
+    Segment *seg;
+    i64 *sad;                 // per slot: the 2-saddle (anchor * 12 + triangle slot)
+    unsigned long long *res;  // per slot: lowest (order << 38 | code) found, ~0: none
+    unsigned long long *n;    // [0] segments, [1] slots
+    i64 cap_seg, cap_slot;
+};
+// One lane per 2-saddle, both cofaces one after the other; a lane that is done
+// takes the chunk's next 2-saddle.
+__global__ void __launch_bounds__(kBlock) k_path_trace(Grid g, const i64 *sad2, const unsigned long long *nsad, uint32_t *tcP,
+                                                      unsigned long long *box, LongPaths L, int shx, int shy, int shz,
+                                                      i64 cap, int *err, unsigned long long *ticket) {
+    __shared__ AscTab tab;
+    load_asc_tab(tab);
+    const i64 n = (i64)*nsad, chunk = chunk_size(n, 256);
+    const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
+    constexpr unsigned long long kEmpty = 1ull;  // x0 = 1 > x1 = 0
+    bool first = true;
+    for (i64 base = next_chunk(first, chunk, ticket); base < n; base = next_chunk(first, chunk, ticket)) {
+        const i64 end = min(n, base + chunk);
+        i64 pos = base, item = -1, steps = 0, code = 0, start = 0, start0 = 0;
+        int x = 0, y = 0, z = 0, s = 0, j = 0;
+        int bx0 = 0, bx1 = 0, by0 = 0, by1 = 0, bz0 = 0, bz1 = 0;  // box of the current segment
+        unsigned long long box0 = kEmpty;                            // box of a short first path
+        i64 slot = -1;
+        unsigned segs = 0;
+        bool on = false;  // on a path
+        auto reset_box = [&]() { bx0 = 2047, bx1 = 0, by0 = 2047, by1 = 0, bz0 = 1023, bz1 = 0; };
+        auto push = [&](unsigned long long b, i64 from, unsigned order) {
+            const unsigned long long at = agg_slot(&L.n[0]);
+            if ((i64)at < L.cap_seg) L.seg[at] = Segment{b, from, (uint32_t)slot, order};
+        };
+        while (true) {
+            const unsigned want = __ballot_sync(full, item < 0);
+            if (want) {
+                const i64 my = pos + __popc(want & ((1u << lane) - 1u));
+                if (item < 0 && my < end) {
+                    item = my;
+                    code = sad2[my];
+                    j = 0;
+                    on = false;
+                    slot = -1;
+                    reset_box();
+                }
+                pos = min(end, pos + (i64)__popc(want));
+            }
+            if (__all_sync(full, item < 0)) break;
+            if (item < 0) continue;
+            if (!on) {
+                if (j == 2) {
+                    box[item] = slot >= 0 ? kEmpty : box_union(box0, box_pack(bx0, bx1, by0, by1, bz0, bz1));
+                    item = -1;
+                    continue;
+                }
+                box0 = j == 1 ? box_pack(bx0, bx1, by0, by1, bz0, bz1) : kEmpty;
+                start0 = start;
+                reset_box();
+                int vx, vy, vz, dx, dy, dz;
+                decode_v(g, code / 12, vx, vy, vz);
+                face_cof_start((int)(code % 12), j, dx, dy, dz, s);
+                x = vx + dx;
+                y = vy + dy;
+                z = vz + dz;
+                j++;
+                steps = 0;
+                segs = 0;
+                start = tet_code(x + (i64)y * g.W + (i64)z * g.WH, s);
+                on = cell_ok(g, x, y, z, 1, 1, 1);
+                if (!on) continue;
+            }
+            const i64 ci = x + (i64)y * g.W + (i64)z * g.WH;
+            const uint32_t w = tcP[ci];
+            const int p = (int)((w >> (3 * s)) & 7u);
+            if (p != 7) {
+                const uint32_t mark = 1u << (18 + s);
+                if (!(w & mark)) atomicOr(&tcP[ci], mark);
+                bx0 = min(bx0, x >> shx);
+                bx1 = max(bx1, x >> shx);
+                by0 = min(by0, y >> shy);
+                by1 = max(by1, y >> shy);
+                bz0 = min(bz0, z >> shz);
+                bz1 = max(bz1, z >> shz);
+                on = asc_move(g, tab, x, y, z, s, p);
+                if (++steps > cap) {
+                    atomicOr(err, ERR_WALK);
+                    on = false;
+                }
+            } else {
+                on = false;
+            }
+            const bool cut = on && steps % kSegment == 0;
+            if (cut && slot < 0) {  // a long path: both cofaces' paths go to the segments
+                slot = (i64)agg_slot(&L.n[1]);
+                if (slot < L.cap_slot) {
+                    L.sad[slot] = code;
+                    L.res[slot] = ~0ull;
+                }
+                if (j == 2) push(box0, start0, 0u);
+            }
+            if (cut || (!on && slot >= 0)) {
+                push(box_pack(bx0, bx1, by0, by1, bz0, bz1), start, ((unsigned)(j - 1) << 25) | segs);
+                segs++;
+                start = tet_code(x + (i64)y * g.W + (i64)z * g.WH, s);
+                reset_box();
+            }
         }
     }
 }
 
-// get_false_ds_vpath (main_3d.cu:4837-4959): the reference's walk never
-// advances past the first vertex (dec_current_id stays at the start), so each
-// endpoint's steepest-descent pairing is compared once, v1 (higher id) first.
-//
-// Incremental descending checks.  A 1-saddle's record depends on the
-// decompressed pairing at its endpoints (its anchor, or the anchor + 1 along
-// some axes).  Per anchor, C = "the tile box from the anchor's tile to the
-// tile of anchor + (1,1,1) holds a tile re-paired since the last detection".
-// Records of anchors with C false are kept; the anchors with C true are
-// checked again (in the tiles whose box from the tile to tile + (1,1,1) is
-// dirty); the first detection after the set-up checks every anchor.
-__device__ __forceinline__ bool ds_anchor_dirty(const Grid &g, const TileSat &T, int x, int y, int z) {
-    return box_dirty(T, box_pack(x >> kTileShift, min(x + 1, g.W - 1) >> kTileShift, y >> kTileShift,
-                                 min(y + 1, g.H - 1) >> kTileShift, z >> kTileShift,
-                                 min(z + 1, g.D - 1) >> kTileShift)) != 0u;
+// an original 1-saddle's first differing endpoint (or -1)
+template <int K>
+__device__ __forceinline__ i64 ds_differs(const Grid &g, const uint8_t *pvP, const uint8_t *pvQ, i64 v) {
+    constexpr int c0 = cxt::TOPO_EDGE_V[K][0], c1 = cxt::TOPO_EDGE_V[K][1];
+    const i64 a = v + cxt::ccx(c0) + cxt::ccy(c0) * (i64)g.W + cxt::ccz(c0) * g.WH,
+              b = v + cxt::ccx(c1) + cxt::ccy(c1) * (i64)g.W + cxt::ccz(c1) * g.WH;
+    const int pa = pvP[a], pb = pvP[b];
+    if (pa != 15 && pa != pvQ[a]) return a;
+    if (pb != 15 && pb != pvQ[b]) return b;
+    return -1;
 }
-__global__ void k_ds_keep(Grid g, PathRec R, const unsigned long long *old_n, const unsigned long long *valid, i64 *te,
-                          i64 *tv, unsigned long long *tn, i64 tcap, TileSat T) {
-    if (!*valid) return;
-    const i64 n = min((i64)*old_n, R.cap_ds);
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        const i64 e = R.ds_edge[i];
-        int x, y, z;
-        decode_v(g, e >> 5, x, y, z);
-        if (ds_anchor_dirty(g, T, x, y, z)) continue;
-        const unsigned long long at = agg_slot(tn);
-        if ((i64)at < tcap) {
-            te[at] = e;
-            tv[at] = R.ds_vert[i];
-        }
-    }
-}
-__global__ void k_ds_tiles(const __grid_constant__ RuleCtx c, const unsigned long long *valid, i64 *te, i64 *tv, unsigned long long *tn,
-                           i64 tcap, TileSat T) {
-    const Grid &g = c.g;
-    const bool all = *valid == 0;
-    const i64 nt = (i64)T.ntx * T.nty * T.ntz;
-    for (i64 t = blockIdx.x; t < nt; t += gridDim.x) {
-        const int tx = (int)(t % T.ntx), ty = (int)((t / T.ntx) % T.nty), tz = (int)(t / ((i64)T.ntx * T.nty));
-        if (!all && box_dirty(T, box_pack(tx, min(tx + 1, T.ntx - 1), ty, min(ty + 1, T.nty - 1), tz,
-                                          min(tz + 1, T.ntz - 1))) == 0u)
-            continue;  // the same for every thread of the block
-        for (int a = threadIdx.x; a < kTile * kTile * kTile; a += blockDim.x) {
-            const int x = tx * kTile + a % kTile, y = ty * kTile + (a / kTile) % kTile, z = tz * kTile + a / (kTile * kTile);
-            if (x >= g.W || y >= g.H || z >= g.D) continue;
-            if (!all && !ds_anchor_dirty(g, T, x, y, z)) continue;
-            const i64 v = x + (i64)y * g.W + (i64)z * g.WH;
-            const uint32_t m = (c.P.crit[v] >> 1) & 0x7Fu;
-            if (!m) continue;
+// both flags of every brick (zero at launch)
+__global__ void k_path_flags(Grid g, PathFlags F, const uint32_t *tcQ, const uint8_t *pvQ, int nbx, int nby, int shx, int shy,
+                             int shz) {
+    for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += (i64)gridDim.x * blockDim.x) {
+        const uint32_t m = (F.critP[v] >> 1) & 0x7Fu;
+        bool ds = false;
+        if (m)
             DMTZ_FOR(7, K, {
                 constexpr int k = decltype(K)::value;
-                constexpr int c0 = cxt::TOPO_EDGE_V[k][0], c1 = cxt::TOPO_EDGE_V[k][1];
-                if ((m >> k) & 1u) {
-                    const i64 ends[2] = {v + cxt::ccx(c0) + cxt::ccy(c0) * (i64)g.W + cxt::ccz(c0) * g.WH,
-                                         v + cxt::ccx(c1) + cxt::ccy(c1) * (i64)g.W + cxt::ccz(c1) * g.WH};
-                    for (int j = 0; j < 2; j++) {
-                        const i64 e = ends[j];
-                        const int po = c.P.pv[e];
-                        if (po == 15) continue;
-                        if (po != c.Q.pv[e]) {
-                            const unsigned long long at = agg_slot(tn);
-                            if ((i64)at < tcap) {
-                                te[at] = edge_code(v, k);
-                                tv[at] = e;
-                            }
-                            break;
-                        }
-                    }
-                }
+                if ((m >> k) & 1u) ds |= ds_differs<k>(g, F.pvP, pvQ, v) >= 0;
             });
-        }
+        const bool as = tet_path_differs(F.tcP[v], tcQ[v]);
+        if (!as && !ds) continue;
+        int x, y, z;
+        decode_v(g, v, x, y, z);
+        const i64 b = (x >> shx) + (i64)nbx * ((y >> shy) + (i64)nby * (z >> shz));
+        if (as) F.as[b] = 1;
+        if (ds) F.ds[b] = 1;
     }
 }
-__global__ void k_ds_back(PathRec R, const i64 *te, const i64 *tv, const unsigned long long *tn,
-                          unsigned long long *valid) {
-    const i64 n = min((i64)*tn, R.cap_ds);
-    const i64 tid = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    for (i64 i = tid; i < n; i += (i64)gridDim.x * blockDim.x) {
-        R.ds_edge[i] = te[i];
-        R.ds_vert[i] = tv[i];
+
+// One detection: the first gridDim.x - ds_blocks blocks take the 2-saddles and
+// the segments of long paths, the others the bricks with a differing 1-saddle
+// endpoint (strict: none, k_ds_strict does those).
+constexpr int kQueue = 512;
+__global__ void __launch_bounds__(kBlock) k_path_detect(Grid g, PathFlags F, const i64 *sad2, const unsigned long long *nsad,
+                                                       const unsigned long long *box, const uint32_t *tcQ,
+                                                       const uint8_t *pvQ, LongPaths L, PathRec R,
+                                                       unsigned long long *ticket, int nbx, int nby, int nbz, int shape_x,
+                                                       int shape_y, int shape_z, int ds_blocks) {
+    const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const unsigned as_blocks = gridDim.x - (unsigned)ds_blocks;
+    if (blockIdx.x >= as_blocks) {
+        const i64 nb = (i64)nbx * nby * nbz;
+        const i64 w0 = (i64)(blockIdx.x - as_blocks) * (blockDim.x / 32) + warp, ws = (i64)ds_blocks * (blockDim.x / 32);
+        for (i64 b0 = w0 * 32; b0 < nb; b0 += ws * 32) {
+            unsigned m = __ballot_sync(full, b0 + lane < nb && F.ds[b0 + lane]);
+            for (; m; m &= m - 1) {
+                const i64 b = b0 + __ffs(m) - 1;
+                const int x0 = (int)(b % nbx) * shape_x, y0 = (int)((b / nbx) % nby) * shape_y,
+                          z0 = (int)(b / ((i64)nbx * nby)) * shape_z;
+                for (int t = lane; t < DMTZ_BRICK; t += 32) {
+                    const int x = x0 + t % shape_x, y = y0 + (t / shape_x) % shape_y, z = z0 + t / (shape_x * shape_y);
+                    if (x >= g.W || y >= g.H || z >= g.D) continue;
+                    const i64 v = x + (i64)y * g.W + (i64)z * g.WH;
+                    const uint32_t c = (F.critP[v] >> 1) & 0x7Fu;
+                    if (!c) continue;
+                    DMTZ_FOR(7, K, {
+                        constexpr int k = decltype(K)::value;
+                        if ((c >> k) & 1u) {
+                            const i64 e = ds_differs<k>(g, F.pvP, pvQ, v);
+                            if (e >= 0) {
+                                const unsigned long long at = agg_slot(&R.n[1]);
+                                if ((i64)at < R.cap_ds) {
+                                    R.ds_edge[at] = edge_code(v, k);
+                                    R.ds_vert[at] = e;
+                                }
+                            }
+                        }
+                    });
+                }
+            }
+        }
+        return;
     }
-    if (tid == 0) {
-        R.n[1] = *tn;
-        *valid = 1ull;
+    __shared__ uint16_t queue[kBlock / 32][kQueue];  // per warp: the chunk's items to walk
+    __shared__ AscTab tab;
+    load_asc_tab(tab);
+    const i64 n2 = (i64)*nsad, n = n2 + min((i64)L.n[0], L.cap_seg);  // 2-saddles, then segments
+    const i64 warps = (i64)as_blocks * (blockDim.x / 32);
+    i64 chunk = (n / (warps * 8) + 31) / 32 * 32;
+    chunk = chunk < 32 ? 32 : (chunk > kQueue ? kQueue : chunk);
+    bool own = true;
+    while (true) {
+        i64 c;
+        if (own) {
+            c = (i64)blockIdx.x * (blockDim.x / 32) + warp;
+            own = false;
+        } else {
+            unsigned long long t = 0;
+            if (lane == 0) t = atomicAdd(ticket, 1ull);
+            c = warps + (i64)__shfl_sync(full, t, 0);
+        }
+        const i64 base = c * chunk;
+        if (base >= n) return;
+        int cnt = 0;
+        for (int k = 0; k < (int)chunk; k += 32) {
+            const i64 i = base + k + lane;
+            const bool d = i < n && box_flagged(F.as, nbx, nby, i < n2 ? box[i] : L.seg[i - n2].box);
+            const unsigned m = __ballot_sync(full, d);
+            if (d) queue[warp][cnt + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(k + lane);
+            cnt += __popc(m);
+        }
+        __syncwarp();
+        // lanes whose walk ended take the next item of the queue.  A 2-saddle's
+        // paths (code >= 0) are at most kSegment steps each, and so is a segment (code = -1)
+        int pos = 0, item = -1, s = 0, j = 0, x = 0, y = 0, z = 0, steps = 0;
+        i64 code = 0, start = 0;
+        uint32_t slot = 0, order = 0;
+        bool on = false;
+        while (true) {
+            const unsigned want = __ballot_sync(full, item < 0);
+            if (want) {
+                const int my = pos + __popc(want & ((1u << lane) - 1u));
+                if (item < 0 && my < cnt) {
+                    item = queue[warp][my];
+                    steps = 0;
+                    if (base + item < n2) {
+                        code = sad2[base + item];
+                        j = 0;
+                        on = false;
+                    } else {
+                        const Segment q = L.seg[base + item - n2];
+                        code = -1;
+                        j = 2;
+                        on = true;
+                        slot = q.slot;
+                        order = q.order;
+                        decode_v(g, q.start >> 5, x, y, z);
+                        s = (int)(q.start & 31) - 20;
+                    }
+                }
+                pos = min(cnt, pos + __popc(want));
+            }
+            if (__all_sync(full, item < 0)) break;
+            if (item < 0) continue;
+            if (!on) {  // the next coface, or done
+                if (j == 2) {
+                    item = -1;
+                    continue;
+                }
+                int vx, vy, vz, dx, dy, dz;
+                decode_v(g, code / 12, vx, vy, vz);
+                face_cof_start((int)(code % 12), j, dx, dy, dz, s);
+                x = vx + dx;
+                y = vy + dy;
+                z = vz + dz;
+                j++;
+                steps = 0;
+                on = cell_ok(g, x, y, z, 1, 1, 1);
+                start = tet_code(x + (i64)y * g.W + (i64)z * g.WH, s);
+                if (!on) continue;
+            }
+            const i64 ci = x + (i64)y * g.W + (i64)z * g.WH;
+            const uint32_t wp = F.tcP[ci], wq = tcQ[ci];
+            const int p = (wp >> (3 * s)) & 7;
+            if (p == 7) {
+                on = false;
+            } else if (p != (int)((wq >> (3 * s)) & 7)) {
+                if (code >= 0) {
+                    const unsigned long long at = agg_slot(&R.n[0]);
+                    if ((i64)at < R.cap_as) {
+                        R.as_tet[at] = start;
+                        R.as_cur[at] = tet_code(ci, s);
+                    }
+                } else {
+                    atomicMin(&L.res[slot], ((unsigned long long)order << 38) | (unsigned long long)tet_code(ci, s));
+                }
+                item = -1;
+            } else {
+                on = asc_move(g, tab, x, y, z, s, p) && ++steps < kSegment;
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// the records of the 2-saddles with long paths, and their slots for the next detection
+__global__ void k_path_long(Grid g, LongPaths L, PathRec R) {
+    const i64 n = min((i64)L.n[1], L.cap_slot);
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
+        const unsigned long long r = L.res[i];
+        if (r == ~0ull) continue;
+        L.res[i] = ~0ull;
+        const i64 code = L.sad[i], v = code / 12;
+        int dx, dy, dz, s;
+        face_cof_start((int)(code % 12), (int)(r >> 63), dx, dy, dz, s);  // order's top bit: the coface
+        const unsigned long long at = agg_slot(&R.n[0]);
+        if ((i64)at < R.cap_as) {
+            R.as_tet[at] = tet_code(v + dx + dy * (i64)g.W + dz * g.WH, s);
+            R.as_cur[at] = (i64)(r & ((1ull << 38) - 1));
+        }
     }
 }
 
@@ -1257,7 +1345,9 @@ __global__ void k_desc_init(Grid g, const uint8_t *pv, i64 *lab) {
         lab[v] = d == 15 ? v : v + g.doff[d];
     }
 }
-__global__ void k_asc_init(Grid g, const uint32_t *tcode, const uint8_t *succ, i64 *lab) {
+__global__ void k_asc_init(Grid g, const uint32_t *tcode, i64 *lab) {
+    __shared__ AscTab tab;
+    load_asc_tab(tab);
     for (i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x; t < 6 * g.V; t += (i64)gridDim.x * blockDim.x) {
         const i64 v = t / 6;
         const int ts = (int)(t - 6 * v);
@@ -1267,18 +1357,14 @@ __global__ void k_asc_init(Grid g, const uint32_t *tcode, const uint8_t *succ, i
             lab[t] = -2;  // no such tetrahedron
             continue;
         }
-        if (((tcode[v] >> (3 * ts)) & 7) == 7) {
+        const int j = (tcode[v] >> (3 * ts)) & 7;
+        if (j == 7) {
             lab[t] = t;  // a maximum
             continue;
         }
-        const int s8 = succ[v * 8 + ts];
-        if (s8 == 255) {
-            lab[t] = -1;  // leaves through the boundary
-            continue;
-        }
-        const int d = s8 / 6;
-        const i64 nv = v + (d % 3 - 1) + (i64)((d / 3) % 3 - 1) * g.W + (i64)(d / 9 - 1) * g.WH;
-        lab[t] = nv * 6 + (s8 - 6 * d);
+        int s = ts;
+        const bool in = asc_move(g, tab, x, y, z, s, j);
+        lab[t] = in ? (x + (i64)y * g.W + (i64)z * g.WH) * 6 + s : -1;  // -1: leaves through the boundary
     }
 }
 __global__ void k_jump(i64 *lab, i64 n, int *changed) {
@@ -1487,10 +1573,7 @@ struct dmtz_ctx {
     double list_frac = 1.0 / 16;
     i64 list_min = 1 << 20;
     i64 *as_tet = nullptr, *as_cur = nullptr, *ds_edge = nullptr, *ds_vert = nullptr;
-    i64 *ds_tmp_edge = nullptr, *ds_tmp_vert = nullptr;  // descending records being rebuilt, capDST each
-    i64 capDST = 0;
     i64 capAS = 0, capDS = 0, capSad2 = 0;
-    uint8_t *succ = nullptr;  // original ascending-path successor of each tetrahedron
     uint32_t *brick_flags = nullptr;  // per brick (a byte each, four to a word): in the next repair
     uint8_t *brick_fresh = nullptr;   // per brick: re-paired by the current round's criticality pass
     int inc_scan = 0;                 // repairs rebuild the mismatch lists incrementally (see k_list_keep)
@@ -1501,15 +1584,16 @@ struct dmtz_ctx {
     i64 *sad2 = nullptr;      // original 2-saddle triangles
     i64 *sad1 = nullptr;      // original 1-saddle edges (strict descending checks only)
     i64 capSad1 = 0;
-    i64 *as_res = nullptr;    // per (2-saddle, coface) walk results, 2 x capSad2
-    // walk cache: per walk, the box of 16^3-anchor tiles its last walk visited
-    // (walk_box); per tile, whether the decompressed gradient was recomputed
-    // there since the last detection (tile_dirty) and its 3-D prefix sum
-    unsigned long long *walk_box = nullptr;
-    uint8_t *tile_dirty = nullptr;
-    uint32_t *tile_sat = nullptr;
-    i64 capWB = 0, capTile = 0;
-    int ntx = 0, nty = 0, ntz = 0;
+    // separatrix checks (see k_path_detect): the box of bricks of each 2-saddle's
+    // paths, and two flags per brick (path_keep: repairs refresh them)
+    unsigned long long *path_box = nullptr;
+    uint8_t *path_as = nullptr, *path_ds = nullptr;
+    i64 capPB = 0;
+    int path_keep = 0;
+    Segment *seg = nullptr;  // segments of long paths, capSeg; per 2-saddle with one: capSlot
+    i64 *seg_sad = nullptr;
+    unsigned long long *seg_res = nullptr;
+    i64 capSeg = 0, capSlot = 0;
     i64 *wall_sad = nullptr, *wall_edge = nullptr;  // wall records (preserve_connectors = 1), capWall each
     i64 *wall_next[2] = {nullptr, nullptr};          // 2-saddles handed to the next search tier
     i64 capWall = 0;
@@ -1519,9 +1603,10 @@ struct dmtz_ctx {
                                              // [8,9] min/max keys, [10] original 2-saddles, [12] edited
                                              // vertices, [13,14] saddle counts,
                                              // [16] wall records, [17,18] deferred wall searches,
-                                             // [20..23] rebuilt mismatch lists, [24] descending
-                                             // records rebuildable, [25] their last count,
-                                             // [26] rebuilt descending records
+                                             // [20..23] rebuilt mismatch lists, [25,26]
+                                             // path segments and their slots, [27] ticket of
+                                             // the separatrix walks, [28] original 1-saddles, [29]
+                                             // ticket of the strict descending walks
     int *errword = nullptr;
     uint8_t *changed = nullptr;
     int64_t launches = 0;  // kernels launched by the current call
@@ -1567,12 +1652,13 @@ void free_all(dmtz_ctx *c) {
     c->capAS = c->capDS = c->capSad2 = 0;
     cudaFree(c->as_tet); cudaFree(c->as_cur); cudaFree(c->ds_edge); cudaFree(c->ds_vert);
     cudaFree(c->counters); cudaFree(c->errword); cudaFree(c->changed);
-    cudaFree(c->succ); cudaFree(c->sad2); cudaFree(c->brick_flags); cudaFree(c->brick_list);
-    cudaFree(c->as_res);
-    c->as_res = nullptr;
-    cudaFree(c->walk_box); cudaFree(c->tile_dirty); cudaFree(c->tile_sat);
-    c->walk_box = nullptr; c->tile_dirty = nullptr; c->tile_sat = nullptr;
-    c->capWB = c->capTile = 0;
+    cudaFree(c->sad2); cudaFree(c->brick_flags); cudaFree(c->brick_list);
+    cudaFree(c->path_box); cudaFree(c->path_as); cudaFree(c->path_ds);
+    c->path_box = nullptr; c->path_as = c->path_ds = nullptr;
+    cudaFree(c->seg); cudaFree(c->seg_sad); cudaFree(c->seg_res);
+    c->seg = nullptr; c->seg_sad = nullptr; c->seg_res = nullptr;
+    c->capSeg = c->capSlot = 0;
+    c->capPB = 0;
     cudaFree(c->wall_sad); cudaFree(c->wall_edge); cudaFree(c->wall_next[0]); cudaFree(c->wall_next[1]);
     cudaFree(c->wall_scratch);
     c->wall_sad = c->wall_edge = c->wall_next[0] = c->wall_next[1] = c->wall_scratch = nullptr;
@@ -1582,12 +1668,9 @@ void free_all(dmtz_ctx *c) {
     cudaFree(c->sad1);
     c->sad1 = nullptr;
     c->capSad1 = 0;
-    c->succ = nullptr; c->sad2 = nullptr; c->brick_flags = nullptr; c->brick_list = nullptr;
+    c->sad2 = nullptr; c->brick_flags = nullptr; c->brick_list = nullptr;
     c->f = c->g = nullptr; c->cnt = nullptr; c->reqbits = nullptr; c->reqlist = nullptr;
     c->as_tet = c->as_cur = c->ds_edge = c->ds_vert = nullptr; c->counters = nullptr;
-    cudaFree(c->ds_tmp_edge); cudaFree(c->ds_tmp_vert);
-    c->ds_tmp_edge = c->ds_tmp_vert = nullptr;
-    c->capDST = 0;
     c->errword = nullptr; c->changed = nullptr;
     c->capV = c->capE = c->capF = c->capT = c->capB = 0;
 }
@@ -1635,9 +1718,9 @@ dmtz_status ensure(dmtz_ctx *ctx, const Grid &g) {
     CK(dalloc(&ctx->reqbits, (V + 31) / 32 + 1));
     CK(cudaMemset(ctx->reqbits, 0, sizeof(uint32_t) * (size_t)((V + 31) / 32 + 1)));
     CK(dalloc(&ctx->reqlist, V));
-    CK(dalloc(&ctx->succ, 8 * V));
     CK(dalloc(&ctx->brick_flags, (nbr + 3) / 4)); CK(dalloc(&ctx->brick_list, nbr));
     CK(dalloc(&ctx->brick_fresh, nbr));
+    CK(dalloc(&ctx->path_as, nbr)); CK(dalloc(&ctx->path_ds, nbr));
     CK(dalloc(&ctx->brick_n, 8));
     CK(cudaMemset(ctx->brick_flags, 0, sizeof(uint32_t) * (size_t)((nbr + 3) / 4)));
     ctx->capB = nbr;
@@ -1682,6 +1765,20 @@ bool shape_fits(const Grid &g, int shape) {
     return nbx <= 2048 && nby <= 2048 && nbz <= 1024;
 }
 
+PathFlags path_flags(const dmtz_ctx *ctx) {
+    return PathFlags{ctx->path_as, ctx->path_ds, ctx->P.tcode, ctx->P.crit, ctx->P.pv};
+}
+LongPaths long_paths(const dmtz_ctx *ctx) {
+    return LongPaths{ctx->seg, ctx->seg_sad, ctx->seg_res, ctx->counters + 25, ctx->capSeg, ctx->capSlot};
+}
+// log2 of the brick extents
+void shape_shifts(int shape, int sh[3]) {
+    for (int k = 0; k < 3; k++) {
+        sh[k] = 0;
+        while ((1 << sh[k]) < DMTZ_SHAPES[shape][k]) sh[k]++;
+    }
+}
+
 // blocks of k_grad_bricks: its blocks hold 384 threads or more, so a quarter
 // of tune_bps (a count for blocks of 128) fills the SMs twice over
 unsigned brick_grid(const dmtz_ctx *ctx, i64 nb) {
@@ -1690,11 +1787,12 @@ unsigned brick_grid(const dmtz_ctx *ctx, i64 nb) {
 }
 
 // the gradient of a set of bricks
-void grad_bricks(const Grid &g, const FieldState &s, const BrickList &bl, unsigned grid, cudaStream_t st) {
+void grad_bricks(const Grid &g, const FieldState &s, const BrickList &bl, unsigned grid, cudaStream_t st,
+                 const PathFlags &F = PathFlags{}) {
     switch (bl.shape) {
-    case 1: k_grad_bricks<16, 4, 2><<<grid, brick_threads<16, 4, 2>(), 0, st>>>(g, s, bl); break;
-    case 2: k_grad_bricks<32, 2, 2><<<grid, brick_threads<32, 2, 2>(), 0, st>>>(g, s, bl); break;
-    default: k_grad_bricks<8, 4, 4><<<grid, brick_threads<8, 4, 4>(), 0, st>>>(g, s, bl); break;
+    case 1: k_grad_bricks<16, 4, 2><<<grid, brick_threads<16, 4, 2>(), 0, st>>>(g, s, bl, F); break;
+    case 2: k_grad_bricks<32, 2, 2><<<grid, brick_threads<32, 2, 2>(), 0, st>>>(g, s, bl, F); break;
+    default: k_grad_bricks<8, 4, 4><<<grid, brick_threads<8, 4, 4>(), 0, st>>>(g, s, bl, F); break;
     }
 }
 
@@ -1790,16 +1888,10 @@ void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint3
         k_mark_fresh<<<persistent_grid(), kBlock, 0, st>>>(ctx->brick_list, ctx->brick_n, ctx->brick_fresh, nbx, nby);
         ctx->launches++;
     }
-    if (ctx->tile_dirty && ctx->ntx > 0) {
-        k_mark_tiles<<<persistent_grid(), kBlock, 0, st>>>(ctx->brick_list, ctx->brick_n, DMTZ_SHAPES[shape][0],
-                                                            DMTZ_SHAPES[shape][1], DMTZ_SHAPES[shape][2], ctx->ntx,
-                                                            ctx->nty, ctx->ntz, ctx->tile_dirty);
-        ctx->launches++;
-    }
     BrickList bl = all_bricks(g, shape, nb);
     bl.list = ctx->brick_list;
     bl.n = ctx->brick_n;
-    grad_bricks(g, s, bl, brick_grid(ctx, nb), st);
+    grad_bricks(g, s, bl, brick_grid(ctx, nb), st, ctx->path_keep ? path_flags(ctx) : PathFlags{});
     ctx->launches++;
     if (!ctx->inc_scan) {
         scan_mismatch(ctx, g, s.crit, crit_o, want_saddles);
@@ -1896,23 +1988,49 @@ PathRec path_rec(const dmtz_ctx *ctx) {
 // and record buffers sized by the original saddle counts (each original
 // 2-saddle gives at most one ascending record, each 1-saddle at most one
 // descending record)
-// the rebuild buffers of the descending records, as large as the records
-dmtz_status ensure_ds_tmp(dmtz_ctx *ctx) {
-    const i64 need = std::max<i64>(ctx->capDS, 1);
-    if (ctx->capDST >= need) return DMTZ_OK;
-    cudaFree(ctx->ds_tmp_edge);
-    cudaFree(ctx->ds_tmp_vert);
-    ctx->ds_tmp_edge = ctx->ds_tmp_vert = nullptr;
-    ctx->capDST = 0;
-    CK(dalloc(&ctx->ds_tmp_edge, need));
-    CK(dalloc(&ctx->ds_tmp_vert, need));
-    ctx->capDST = need;
-    return DMTZ_OK;
+// the original paths' marks, boxes and segments (after the 2-saddle list).
+// Room for the segments: what the last field needed, at first one per 16 vertices
+// and 2-saddle slot per 64; a trace that needs more is repeated.
+dmtz_status trace_paths(dmtz_ctx *ctx, const Grid &g) {
+    cudaStream_t st = ctx->stream;
+    i64 need_seg = std::max<i64>(g.V / 16, 1024), need_slot = std::max<i64>(g.V / 64, 256);
+    int sh[3];
+    shape_shifts(ctx->tune_shape, sh);
+    while (true) {
+        if (need_seg > ctx->capSeg) {
+            cudaFree(ctx->seg);
+            ctx->seg = nullptr;
+            ctx->capSeg = 0;
+            CK(dalloc(&ctx->seg, need_seg));
+            ctx->capSeg = need_seg;
+        }
+        if (need_slot > ctx->capSlot) {
+            cudaFree(ctx->seg_sad);
+            cudaFree(ctx->seg_res);
+            ctx->seg_sad = nullptr;
+            ctx->seg_res = nullptr;
+            ctx->capSlot = 0;
+            CK(dalloc(&ctx->seg_sad, need_slot));
+            CK(dalloc(&ctx->seg_res, need_slot));
+            ctx->capSlot = need_slot;
+        }
+        CK(cudaMemsetAsync(ctx->counters + 25, 0, 3 * sizeof(unsigned long long), st));  // segments, slots, ticket
+        k_path_trace<<<persistent_grid(), kBlock, 0, st>>>(g, ctx->sad2, ctx->counters + 10, ctx->P.tcode, ctx->path_box,
+                                                           long_paths(ctx), sh[0], sh[1], sh[2], g.T + 16, ctx->errword,
+                                                           ctx->counters + 27);
+        ctx->launches++;
+        unsigned long long n[2] = {0, 0};
+        CK(cudaMemcpyAsync(n, ctx->counters + 25, sizeof(n), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        CK(cudaGetLastError());
+        if ((i64)n[0] <= ctx->capSeg && (i64)n[1] <= ctx->capSlot) return DMTZ_OK;
+        need_seg = std::max<i64>(need_seg, (i64)n[0]);
+        need_slot = std::max<i64>(need_slot, (i64)n[1]);
+    }
 }
 
 dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g) {
     cudaStream_t st = ctx->stream;
-    dmtz_status s0;
     CK(cudaMemsetAsync(ctx->counters + 13, 0, 2 * sizeof(unsigned long long), st));
     k_count_saddles<<<persistent_grid(), kBlock, 0, st>>>(g.V, ctx->P.crit, ctx->counters + 13);
     unsigned long long n[2] = {0, 0};
@@ -1931,13 +2049,11 @@ dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g) {
         cudaFree(ctx->as_tet);
         cudaFree(ctx->as_cur);
         cudaFree(ctx->sad2);
-        cudaFree(ctx->as_res);
-        ctx->as_tet = ctx->as_cur = ctx->sad2 = ctx->as_res = nullptr;
+        ctx->as_tet = ctx->as_cur = ctx->sad2 = nullptr;
         ctx->capAS = ctx->capSad2 = 0;
         CK(dalloc(&ctx->as_tet, (i64)n[1]));
         CK(dalloc(&ctx->as_cur, (i64)n[1]));
         CK(dalloc(&ctx->sad2, (i64)n[1]));
-        CK(dalloc(&ctx->as_res, 2 * (i64)n[1]));
         ctx->capAS = ctx->capSad2 = (i64)n[1];
     }
     // buffers exist even when a count is 0 (kernels take their addresses)
@@ -1949,37 +2065,16 @@ dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g) {
         CK(dalloc(&ctx->as_tet, 1));
         CK(dalloc(&ctx->as_cur, 1));
         CK(dalloc(&ctx->sad2, 1));
-        CK(dalloc(&ctx->as_res, 2));
     }
-    if ((s0 = ensure_ds_tmp(ctx)) != DMTZ_OK) return s0;
-    CK(cudaMemsetAsync(ctx->counters + 24, 0, 3 * sizeof(unsigned long long), st));
-    // walk cache: every walk runs at the first detection
-    const i64 nw = std::max<i64>(2 * (i64)n[1], 2);
-    if (nw > ctx->capWB) {
-        cudaFree(ctx->walk_box);
-        ctx->walk_box = nullptr;
-        ctx->capWB = 0;
-        CK(dalloc(&ctx->walk_box, nw));
-        ctx->capWB = nw;
+    const i64 nbox = std::max<i64>((i64)n[1], 1);
+    if (nbox > ctx->capPB) {
+        cudaFree(ctx->path_box);
+        ctx->path_box = nullptr;
+        ctx->capPB = 0;
+        CK(dalloc(&ctx->path_box, nbox));
+        ctx->capPB = nbox;
     }
-    ctx->ntx = (g.W + kTile - 1) / kTile;
-    ctx->nty = (g.H + kTile - 1) / kTile;
-    ctx->ntz = (g.D + kTile - 1) / kTile;
-    const i64 nt = (i64)ctx->ntx * ctx->nty * ctx->ntz;
-    if (nt > ctx->capTile) {
-        cudaFree(ctx->tile_dirty);
-        cudaFree(ctx->tile_sat);
-        ctx->tile_dirty = nullptr;
-        ctx->tile_sat = nullptr;
-        ctx->capTile = 0;
-        CK(dalloc(&ctx->tile_dirty, nt));
-        CK(dalloc(&ctx->tile_sat, nt));
-        ctx->capTile = nt;
-    }
-    CK(cudaMemsetAsync(ctx->walk_box, 0, sizeof(unsigned long long) * (size_t)nw, st));
-    CK(cudaMemsetAsync(ctx->tile_dirty, 0, (size_t)nt, st));
     CK(cudaMemsetAsync(ctx->counters + 10, 0, sizeof(unsigned long long), st));
-    k_path_succ<<<grid_for(g.V), kBlock, 0, st>>>(g, ctx->P.tcode, ctx->succ);
     k_crit_list<8, 12><<<persistent_grid(), kBlock, 0, st>>>(g, ctx->P.crit, ctx->sad2, ctx->capSad2,
                                                              ctx->counters + 10);
     if (ctx->strict_ds) {  // the whole-path descending checks walk from the 1-saddle list
@@ -1996,7 +2091,21 @@ dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g) {
                                                                 ctx->counters + 28);
         ctx->launches++;
     }
-    ctx->launches += 3;
+    ctx->launches += 2;
+    return trace_paths(ctx, g);
+}
+
+// the bricks' path flags, from both gradients; repairs keep them from here on
+dmtz_status init_path_flags(dmtz_ctx *ctx, const Grid &g) {
+    int nbx, nby, nbz, sh[3];
+    const i64 nb = bricks_of(g, ctx->tune_shape, nbx, nby, nbz);
+    shape_shifts(ctx->tune_shape, sh);
+    CK(cudaMemsetAsync(ctx->path_as, 0, (size_t)nb, ctx->stream));
+    CK(cudaMemsetAsync(ctx->path_ds, 0, (size_t)nb, ctx->stream));
+    k_path_flags<<<persistent_grid(), kBlock, 0, ctx->stream>>>(g, path_flags(ctx), ctx->Q.tcode, ctx->Q.pv, nbx, nby, sh[0],
+                                                                sh[1], sh[2]);
+    ctx->launches++;
+    ctx->path_keep = 1;
     CK(cudaGetLastError());
     return DMTZ_OK;
 }
@@ -2006,45 +2115,31 @@ dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g) {
 // (also used while capturing the graph loop)
 void launch_detect(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const PathRec &R, unsigned grid, int conn) {
     cudaStream_t st = ctx->stream;
-    // the last detection's descending record count, for the incremental rebuild
-    cudaMemcpyAsync(ctx->counters + 25, ctx->counters + 6, sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st);
     cudaMemsetAsync(ctx->counters + 5, 0, 2 * sizeof(unsigned long long), st);
     if (conn) {
-        k_conn_as<<<grid, kBlock, 0, st>>>(g, ctx->P.crit, ctx->Q.crit, ctx->P.tcode, ctx->Q.tcode, ctx->succ, R,
+        k_conn_as<<<grid, kBlock, 0, st>>>(g, ctx->P.crit, ctx->Q.crit, ctx->P.tcode, ctx->Q.tcode, R,
                                            g.T + 16, ctx->errword);
         k_conn_ds<<<grid, kBlock, 0, st>>>(rc, R, g.V + 16);
     } else {
-        const int ntx = ctx->ntx, nty = ctx->nty, ntz = ctx->ntz;
-        k_sat_x<<<grid_for((i64)nty * ntz), kBlock, 0, st>>>(ctx->tile_dirty, ctx->tile_sat, ntx, nty, ntz);
-        k_sat_yz<<<grid_for((i64)ntx * ntz), kBlock, 0, st>>>(ctx->tile_sat, ntx, nty, ntz, 1);
-        k_sat_yz<<<grid_for((i64)ntx * nty), kBlock, 0, st>>>(ctx->tile_sat, ntx, nty, ntz, 2);
-        TileSat T;
-        T.sat = ctx->tile_sat;
-        T.ntx = ntx;
-        T.nty = nty;
-        T.ntz = ntz;
+        int nbx, nby, nbz;
+        const int shape = ctx->tune_shape, *sx = DMTZ_SHAPES[shape];
+        const i64 nb = bricks_of(g, shape, nbx, nby, nbz);
+        const int ds_blocks = ctx->strict_ds ? 0 : (int)std::min<i64>((nb + 255) / 256, grid / 8);
         cudaMemsetAsync(ctx->counters + 27, 0, sizeof(unsigned long long), st);  // the walks' ticket
-        k_path_as_walk<<<grid, kBlock, 0, st>>>(g, ctx->sad2, ctx->counters + 10, ctx->P.tcode, ctx->Q.tcode,
-                                                ctx->succ, ctx->as_res, g.T + 16, ctx->errword, ctx->walk_box, T,
-                                                ctx->counters + 27);
-        k_path_as_pick<<<grid, kBlock, 0, st>>>(g, ctx->sad2, ctx->counters + 10, ctx->as_res, R);
+        k_path_detect<<<grid + (unsigned)ds_blocks, kBlock, 0, st>>>(g, path_flags(ctx), ctx->sad2, ctx->counters + 10,
+                                                                     ctx->path_box, ctx->Q.tcode, ctx->Q.pv, long_paths(ctx),
+                                                                     R, ctx->counters + 27, nbx, nby, nbz, sx[0], sx[1],
+                                                                     sx[2], ds_blocks);
+        k_path_long<<<grid / 8, kBlock, 0, st>>>(g, long_paths(ctx), R);
         if (ctx->strict_ds) {  // whole-path descending checks of every 1-saddle, into the records
             cudaMemsetAsync(ctx->counters + 29, 0, sizeof(unsigned long long), st);  // the walks' ticket
             k_ds_strict<<<grid, kBlock, 0, st>>>(rc, R, ctx->sad1, ctx->counters + 28, g.V + 16,
                                                  ctx->counters + 29);
-            return;
         }
-        cudaMemsetAsync(ctx->counters + 26, 0, sizeof(unsigned long long), st);
-        k_ds_keep<<<grid, kBlock, 0, st>>>(g, R, ctx->counters + 25, ctx->counters + 24, ctx->ds_tmp_edge,
-                                           ctx->ds_tmp_vert, ctx->counters + 26, ctx->capDST, T);
-        k_ds_tiles<<<grid, kBlock, 0, st>>>(rc, ctx->counters + 24, ctx->ds_tmp_edge, ctx->ds_tmp_vert,
-                                            ctx->counters + 26, ctx->capDST, T);
-        k_ds_back<<<grid, kBlock, 0, st>>>(R, ctx->ds_tmp_edge, ctx->ds_tmp_vert, ctx->counters + 26,
-                                           ctx->counters + 24);
     }
 }
 // kernels one detection launches
-int detect_kernels(const dmtz_ctx *ctx, int conn) { return conn ? 2 : (ctx->strict_ds ? 6 : 8); }
+int detect_kernels(const dmtz_ctx *ctx, int conn) { return conn ? 2 : (ctx->strict_ds ? 3 : 2); }
 void detect_paths(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const PathRec &R, unsigned grid, int conn = 0) {
     launch_detect(ctx, g, rc, R, grid, conn);
     ctx->launches += detect_kernels(ctx, conn);
@@ -2479,6 +2574,8 @@ static dmtz_status path_detect_impl(dmtz_ctx *ctx, int W, int H, int D, const do
     CK(cudaMemsetAsync(ctx->errword, 0, sizeof(int), ctx->stream));
     RuleCtx rc = rule_ctx(ctx, g, 0.0, 0);
     if ((s = prep_paths(ctx, g)) != DMTZ_OK) return s;
+    if ((s = init_path_flags(ctx, g)) != DMTZ_OK) return s;
+    ctx->path_keep = 0;
     unsigned long long hc[2];
     int err = 0;
     for (int attempt = 0; attempt < 2; attempt++) {
@@ -2506,9 +2603,6 @@ static dmtz_status path_detect_impl(dmtz_ctx *ctx, int W, int H, int D, const do
             CK(dalloc(&ctx->ds_edge, (i64)hc[1]));
             CK(dalloc(&ctx->ds_vert, (i64)hc[1]));
             ctx->capDS = (i64)hc[1];
-            if ((s = ensure_ds_tmp(ctx)) != DMTZ_OK) return s;
-            // records past the old capacity were not kept: the next detection scans everything
-            CK(cudaMemsetAsync(ctx->counters + 24, 0, sizeof(unsigned long long), ctx->stream));
         }
     }
     counts[0] = (int64_t)hc[0];
@@ -2890,6 +2984,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     if (!(rel_eps >= 0.0) || !std::isfinite(rel_eps)) return fail(ctx, DMTZ_ERR_ARG, "rel_eps must be finite and >= 0");
     const i64 max_rounds = opts->max_rounds > 0 ? opts->max_rounds : 100000;
     ctx->inc_scan = 0;  // full scans until the loop starts
+    ctx->path_keep = 0;
     ctx->strict_ds = (opts->strict_separatrices && !conn) ? 1 : 0;
     CK(cudaSetDevice(ctx->device));
     if ((s = ensure(ctx, g)) != DMTZ_OK) return s;
@@ -2932,6 +3027,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     run_pairing(ctx, g, Qs, ctx->P.crit, 1);
     k_fill_i32<<<grid_for(g.V), kBlock, 0, st>>>(ctx->cnt, 1, g.V);
     ctx->launches++;
+    if (pvp == 1 && !conn && (s = init_path_flags(ctx, g)) != DMTZ_OK) return s;
     pt_.end();
     unsigned long long hc[8];
     auto read_counts = [&]() -> dmtz_status {
@@ -3019,8 +3115,8 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             // kernels per body run: switch + control, plus each state's own
             const int64_t det = detect_kernels(ctx, conn);  // separatrix detection kernels
             // a fix round: fix + update, then the repair (dirty marks, compaction,
-            // fresh and tile marks, the gradient, the list rebuild)
-            const int64_t rnd = 2 + 2 + (ctx->inc_scan ? 1 : 0) + (ctx->tile_dirty ? 1 : 0) + 1 + (ctx->inc_scan ? 3 : 1);
+            // fresh marks, the gradient, the list rebuild)
+            const int64_t rnd = 2 + 2 + (ctx->inc_scan ? 1 : 0) + 1 + (ctx->inc_scan ? 3 : 1);
             ctx->launches += 2 * (fin.runs[0] + fin.runs[1] + fin.runs[2] + fin.runs[3]) + rnd * fin.runs[LS_CP] +
                              (rnd + det) * fin.runs[LS_PDF] + det * fin.runs[LS_PCHECK] + rnd * fin.runs[LS_PFIX];
         }
@@ -3254,7 +3350,6 @@ dmtz_status dmtz_labels(dmtz_ctx *ctx, int W, int H, int D, const double *data, 
     if ((s = ensure(ctx, g)) != DMTZ_OK) return s;
     if ((s = upload(ctx, ctx->f, data, g.V, on_device)) != DMTZ_OK) return s;
     run_pairing(ctx, g, view(ctx->P, ctx->f), nullptr, 1);
-    k_path_succ<<<grid_for(g.V), kBlock, 0, ctx->stream>>>(g, ctx->P.tcode, ctx->succ);
     i64 *dl = nullptr, *al = nullptr;
     int32_t *dout = nullptr, *aout = nullptr;
     CK(dalloc(&dl, g.V));
@@ -3263,7 +3358,7 @@ dmtz_status dmtz_labels(dmtz_ctx *ctx, int W, int H, int D, const double *data, 
     CK(dalloc(&aout, g.T));
     const unsigned pg = persistent_grid();
     k_desc_init<<<pg, kBlock, 0, ctx->stream>>>(g, ctx->P.pv, dl);
-    k_asc_init<<<pg, kBlock, 0, ctx->stream>>>(g, ctx->P.tcode, ctx->succ, al);
+    k_asc_init<<<pg, kBlock, 0, ctx->stream>>>(g, ctx->P.tcode, al);
     if ((s = jump_to_roots(ctx, dl, g.V)) == DMTZ_OK) s = jump_to_roots(ctx, al, 6 * g.V);
     if (s == DMTZ_OK) {
         k_desc_out<<<pg, kBlock, 0, ctx->stream>>>(g, dl, dout);
@@ -3294,23 +3389,20 @@ dmtz_status dmtz_separatrix_agreement(dmtz_ctx *ctx, int W, int H, int D, const 
     run_pairing(ctx, g, view(ctx->P, ctx->f), nullptr, 1);
     run_pairing(ctx, g, view(ctx->Q, ctx->g), nullptr, 1);
     i64 *dP = nullptr, *dQ = nullptr, *aP = nullptr, *aQ = nullptr;
-    uint8_t *succQ = nullptr;
     unsigned long long *cnt = nullptr;
     auto release = [&]() {
-        cudaFree(dP); cudaFree(dQ); cudaFree(aP); cudaFree(aQ); cudaFree(succQ); cudaFree(cnt);
+        cudaFree(dP); cudaFree(dQ); cudaFree(aP); cudaFree(aQ); cudaFree(cnt);
     };
     if (dalloc(&dP, g.V) != cudaSuccess || dalloc(&dQ, g.V) != cudaSuccess || dalloc(&aP, 6 * g.V) != cudaSuccess ||
-        dalloc(&aQ, 6 * g.V) != cudaSuccess || dalloc(&succQ, 8 * g.V) != cudaSuccess || dalloc(&cnt, 5) != cudaSuccess) {
+        dalloc(&aQ, 6 * g.V) != cudaSuccess || dalloc(&cnt, 5) != cudaSuccess) {
         release();
         return fail(ctx, DMTZ_ERR_CUDA, "cannot allocate label buffers");
     }
     const unsigned pg = persistent_grid();
-    k_path_succ<<<grid_for(g.V), kBlock, 0, st>>>(g, ctx->P.tcode, ctx->succ);
-    k_path_succ<<<grid_for(g.V), kBlock, 0, st>>>(g, ctx->Q.tcode, succQ);
     k_desc_init<<<pg, kBlock, 0, st>>>(g, ctx->P.pv, dP);
     k_desc_init<<<pg, kBlock, 0, st>>>(g, ctx->Q.pv, dQ);
-    k_asc_init<<<pg, kBlock, 0, st>>>(g, ctx->P.tcode, ctx->succ, aP);
-    k_asc_init<<<pg, kBlock, 0, st>>>(g, ctx->Q.tcode, succQ, aQ);
+    k_asc_init<<<pg, kBlock, 0, st>>>(g, ctx->P.tcode, aP);
+    k_asc_init<<<pg, kBlock, 0, st>>>(g, ctx->Q.tcode, aQ);
     s = jump_to_roots(ctx, dP, g.V);
     if (s == DMTZ_OK) s = jump_to_roots(ctx, dQ, g.V);
     if (s == DMTZ_OK) s = jump_to_roots(ctx, aP, 6 * g.V);

@@ -213,6 +213,7 @@ __host__ __device__ constexpr uint32_t ends_at(int hi, int c) {
         if (TOPO_EDGE_V[k][hi ? 0 : 1] == c) m |= 1u << k;
     return m;
 }
+__host__ __device__ constexpr uint32_t edges_at(int c) { return ends_at(0, c) | ends_at(1, c); }
 // cells that need the anchor's +x (bit 0), +y (1) or +z (2) neighbour
 __host__ __device__ constexpr uint32_t edges_over(int axis) {
     uint32_t m = 0;
@@ -422,6 +423,11 @@ __host__ __device__ __forceinline__ CellWords grad_stage2(const uint4 *w0, const
     return o;
 }
 
+// six bits to stride 3
+__host__ __device__ __forceinline__ uint32_t spread3(uint32_t b) {
+    const uint32_t g = (b & 7u) | ((b & 0x38u) << 6);
+    return (g | (g << 2) | (g << 4)) & 0x9249u;
+}
 // ------------------------------------------------------------------- stage 3
 // Outputs of one anchor (FieldState's eup, fup, crit, tcode).  c0: the cell words of the anchor's plane at the anchor,
 // cm: of the plane below; rows ROW apart.  last: bit per axis, the anchor is on
@@ -485,12 +491,8 @@ __host__ __device__ __forceinline__ AnchorOut grad_stage3(const CellWords *cm, c
     const uint32_t none = (~(r0 | r1 | r2 | r3) & 0x3Fu) | (~exT & 0x3Fu);
     o.crit = (a.pa >> 31) | ((exE & ~(upE | (a.pa >> 24))) << 1) | ((exF & ~(upF | (a.pb >> 12))) << 8) |
              ((none & exT) << 20);
-    // facet index of each tetrahedron, 7 = unpaired or absent: six bits to stride 3
-    auto spread = [](uint32_t b) {
-        const uint32_t g = (b & 7u) | ((b & 0x38u) << 6);
-        return (g | (g << 2) | (g << 4)) & 0x9249u;
-    };
-    o.tcode = spread(r1 | r3 | none) | (spread(r2 | r3 | none) << 1) | (spread(none) << 2);
+    // facet index of each tetrahedron, 7 = unpaired or absent
+    o.tcode = spread3(r1 | r3 | none) | (spread3(r2 | r3 | none) << 1) | (spread3(none) << 2);
     return o;
 }
 
@@ -530,6 +532,18 @@ __device__ __forceinline__ void brick_coords(const BrickList &bl, i64 b, int &bx
     }
 }
 
+// Separatrix flags of the bricks (see k_path_detect), refreshed with a brick's gradient.
+struct PathFlags {
+    uint8_t *as, *ds;            // per brick; nullptr: not kept
+    const uint32_t *tcP, *critP; // original tetrahedron codes with path bits (18 + slot), original criticality
+    const uint8_t *pvP;          // original steepest descent
+};
+// does a tetrahedron on an original path pair differently?
+__host__ __device__ __forceinline__ bool tet_path_differs(uint32_t tcP, uint32_t tcQ) {
+    const uint32_t x = tcP ^ tcQ, on = tcP >> 18;
+    return on && ((x | (x >> 1) | (x >> 2)) & 0x9249u & spread3(on));
+}
+
 // The gradient of the listed bricks, one block per brick step.  One thread per
 // stage-1 anchor (the brick and one layer around it: 360 of 384 threads for
 // 8 x 4 x 4), so each stage is one round; in the later stages the surplus
@@ -539,7 +553,8 @@ __host__ __device__ constexpr int brick_threads() {
     return ((SX + 2) * (SY + 2) * (SZ + 2) + 31) / 32 * 32;
 }
 template <int SX, int SY, int SZ>
-__global__ void __launch_bounds__((brick_threads<SX, SY, SZ>())) k_grad_bricks(Grid g, FieldState s, BrickList bl) {
+__global__ void __launch_bounds__((brick_threads<SX, SY, SZ>()), SX == 8 ? 3 : 2) k_grad_bricks(Grid g, FieldState s, BrickList bl,
+                                                                                        PathFlags F) {
     static_assert(SX * SY * SZ == DMTZ_BRICK, "a brick is 128 anchors");
     constexpr int NT = brick_threads<SX, SY, SZ>();
     constexpr int KX = SX + 4, KY = SY + 4, KZ = SZ + 4, NK = KX * KY * KZ;  // keys: two layers around
@@ -549,6 +564,8 @@ __global__ void __launch_bounds__((brick_threads<SX, SY, SZ>())) k_grad_bricks(G
     __shared__ uint4 sw[NW];
     __shared__ uint32_t sf[NW];
     __shared__ CellWords sc[NC];
+    __shared__ uint8_t sp[NW], sq[NW];  // steepest descent of this field and of the original one
+    __shared__ uint32_t flag;  // bit 0: as, bit 1: ds
     const int t = threadIdx.x;
     const int wx = t % WX, wy = (t / WX) % WY, wz = t / (WX * WY);
     const int cx = t % CX, cy = (t / CX) % CY, cz = t / (CX * CY);
@@ -563,18 +580,34 @@ __global__ void __launch_bounds__((brick_threads<SX, SY, SZ>())) k_grad_bricks(G
             const bool in = ux >= 0 && uy >= 0 && uz >= 0 && ux < g.W && uy < g.H && uz < g.D;
             sk[e] = in ? okey(s.val[ux + (i64)uy * g.W + (i64)uz * g.WH]) : kKeyAbsent;
         }
+        // what the path flags compare with, loaded with the keys
+        uint32_t tcP = 0, critP = 0;
+        if (F.as) {
+            const int x = x0 + wx - 1, y = y0 + wy - 1, z = z0 + wz - 1;
+            if (t < NW) {
+                const bool in = x >= 0 && y >= 0 && z >= 0 && x < g.W && y < g.H && z < g.D;
+                sq[t] = in ? F.pvP[x + (i64)y * g.W + (i64)z * g.WH] : (uint8_t)15;
+            }
+            if (t < DMTZ_BRICK && x0 + ox < g.W && y0 + oy < g.H && z0 + oz < g.D) {
+                const i64 v = (x0 + ox) + (i64)(y0 + oy) * g.W + (i64)(z0 + oz) * g.WH;
+                tcP = F.tcP[v];
+                critP = F.critP[v];
+            }
+        }
         __syncthreads();
         if (t < NW) {
             const uint64_t *k0 = sk + (wx + 1) + KX * ((wy + 1) + KY * (wz + 1));
             const StarWords w = grad_stage1<KX>(k0 - KX * KY, k0, k0 + KX * KY);
             sw[t] = make_uint4(w.x, w.y, w.z, w.w);
             sf[t] = w.w4;
+            sp[t] = (uint8_t)w.pv;
             const int x = x0 + wx - 1, y = y0 + wy - 1, z = z0 + wz - 1;
             if (wx >= 1 && wy >= 1 && wz >= 1 && wx <= SX && wy <= SY && wz <= SZ && x < g.W && y < g.H && z < g.D)
                 s.pv[x + (i64)y * g.W + (i64)z * g.WH] = (uint8_t)w.pv;
         }
         __syncthreads();
         if (t < NC) {
+            if (t == 0) flag = 0;
             const int i = cx + WX * (cy + WY * cz);
             sc[t] = grad_stage2<WX>(sw + i, sw + i + WX * WY, sf + i, sf + i + WX * WY);
         }
@@ -590,6 +623,27 @@ __global__ void __launch_bounds__((brick_threads<SX, SY, SZ>())) k_grad_bricks(G
                 s.fup[v] = o.fup;
                 if (s.crit) s.crit[v] = o.crit;
                 if (s.tcode) s.tcode[v] = o.tcode;
+                if (F.as) {
+                    // an original 1-saddle with an endpoint whose descent differs: the
+                    // anchor and the corners its edges reach
+                    const uint32_t m = (critP >> 1) & 0x7Fu;
+                    uint32_t differ = 0;  // bit per corner
+                    DMTZ_FOR(5, C, {
+                        constexpr int c = decltype(C)::value == 3 ? 4 : decltype(C)::value == 4 ? 6 : decltype(C)::value;
+                        const int i = (ox + 1 + cxt::ccx(c)) + WX * ((oy + 1 + cxt::ccy(c)) + WY * (oz + 1 + cxt::ccz(c)));
+                        if (sq[i] != 15 && sq[i] != sp[i]) differ |= cxt::edges_at(c);
+                    });
+                    const uint32_t f = (tet_path_differs(tcP, o.tcode) ? 1u : 0u) | ((m & differ) ? 2u : 0u);
+                    if (f) atomicOr(&flag, f);
+                }
+            }
+        }
+        if (F.as) {
+            __syncthreads();
+            if (t == 0) {
+                const i64 b = bx + (i64)bl.nbx * (by + (i64)bl.nby * bz);
+                F.as[b] = (uint8_t)(flag & 1u);
+                F.ds[b] = (uint8_t)(flag >> 1);
             }
         }
         // the next brick's keys may land now: stage 1 of this one is behind two
