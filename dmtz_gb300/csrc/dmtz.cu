@@ -37,107 +37,18 @@ static const int kBlock = 256;
 static inline unsigned grid_for(i64 n) { return (unsigned)std::max<i64>(1, (n + kBlock - 1) / kBlock); }
 
 // --------------------------------------------------------------- mismatch compaction
-struct Lists {
-    i64 *l[4];                  // min, 1-saddle, 2-saddle, max (cell codes, see rules.cuh)
-    unsigned long long *n;      // 4 counters
-    i64 cap[4];                 // capacities; a counter above its capacity = overflow,
-                                // the host grows the list and scans again
-};
-
-__device__ __forceinline__ void push_list(const Lists &L, int k, i64 code) {
-    const unsigned long long at = agg_slot(&L.n[k]);
-    if ((i64)at < L.cap[k]) L.l[k][at] = code;
-}
-// the mismatched cells d (bits of FieldState::crit) of anchor v
-__device__ __forceinline__ void push_cells(const Lists &L, i64 v, uint32_t d) {
-    while (d) {
-        const int b = __ffs(d) - 1;
-        d &= d - 1;
-        push_list(L, b == 0 ? 0 : b < 8 ? 1 : b < 20 ? 2 : 3, cell_code(v, b));
-    }
-}
-
 // mismatch between the decompressed and the original critical cells
 // (get_false_minimum / saddle / 2_saddle / maximum, main_3d.cu:2492-2550):
 // a scan of the two criticality masks, compacting mismatched cells' ids
-__global__ void k_mismatch_scan(Grid g, const uint32_t *crit_d, const uint32_t *crit_o, Lists L, int want_saddles) {
-    for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += (i64)gridDim.x * blockDim.x) {
-        uint32_t d = crit_d[v] ^ crit_o[v];
+__global__ void __launch_bounds__(kBlock) k_mismatch_scan(Grid g, const uint32_t *crit_d, const uint32_t *crit_o, Lists L,
+                                                         int want_saddles) {
+    const i64 step = (i64)gridDim.x * blockDim.x;
+    for (i64 b = (i64)blockIdx.x * blockDim.x; b < g.V; b += step) {  // the block's warps stay whole
+        const i64 v = b + threadIdx.x;
+        uint32_t d = v < g.V ? crit_d[v] ^ crit_o[v] : 0u;
         if (!want_saddles) d &= 1u | (0x3Fu << 20);
-        push_cells(L, v, d);
+        push_warp(L, v, d);
     }
-}
-
-// Incremental mismatch lists.  A cell's mismatch status changes only where
-// its anchor's criticality mask was recomputed, i.e. in the bricks of the
-// round's criticality pass (marked fresh).  The new lists are the old entries
-// outside fresh bricks plus a scan of the fresh bricks' anchors, built in T
-// and copied back.  Valid when every scan of the run uses the same saddle
-// flag and the old lists were complete (an overflow is followed by a full
-// scan before the next round).
-__global__ void k_mark_fresh(const uint32_t *list, const unsigned long long *n, uint8_t *fresh, int nbx, int nby) {
-    const i64 nb = (i64)*n;
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += (i64)gridDim.x * blockDim.x) {
-        const uint32_t e = list[i];
-        fresh[(e & 0x7FF) + (i64)nbx * (((e >> 11) & 0x7FF) + (i64)nby * (e >> 22))] = 1;
-    }
-}
-__global__ void k_list_keep(Grid g, Lists L, Lists T, const uint8_t *fresh, int sx, int sy, int sz, int nbx, int nby) {
-    const i64 n0 = min((i64)L.n[0], L.cap[0]), n1 = min((i64)L.n[1], L.cap[1]), n2 = min((i64)L.n[2], L.cap[2]),
-              n3 = min((i64)L.n[3], L.cap[3]);
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n0 + n1 + n2 + n3; i += (i64)gridDim.x * blockDim.x) {
-        int k;
-        i64 code;
-        if (i < n0) {
-            k = 0;
-            code = L.l[0][i];
-        } else if (i < n0 + n1) {
-            k = 1;
-            code = L.l[1][i - n0];
-        } else if (i < n0 + n1 + n2) {
-            k = 2;
-            code = L.l[2][i - n0 - n1];
-        } else {
-            k = 3;
-            code = L.l[3][i - n0 - n1 - n2];
-        }
-        int x, y, z;
-        decode_v(g, code >> 5, x, y, z);
-        if (fresh[x / sx + (i64)nbx * (y / sy + (i64)nby * (z / sz))]) continue;
-        push_list(T, k, code);
-    }
-}
-// the anchors of the fresh bricks (one block per listed brick step)
-__global__ void k_scan_fresh(Grid g, const uint32_t *crit_d, const uint32_t *crit_o, Lists T, const uint32_t *blist,
-                             const unsigned long long *bn, int sx, int sy, int sz, int want_saddles) {
-    const i64 nb = (i64)*bn;
-    const int per = sx * sy * sz;
-    for (i64 b = blockIdx.x; b < nb; b += gridDim.x) {
-        const uint32_t e = blist[b];
-        const int x0 = (e & 0x7FF) * sx, y0 = ((e >> 11) & 0x7FF) * sy, z0 = (e >> 22) * sz;
-        for (int t = threadIdx.x; t < per; t += blockDim.x) {
-            const int x = x0 + t % sx, y = y0 + (t / sx) % sy, z = z0 + t / (sx * sy);
-            if (x >= g.W || y >= g.H || z >= g.D) continue;
-            const i64 v = x + (i64)y * g.W + (i64)z * g.WH;
-            uint32_t d = crit_d[v] ^ crit_o[v];
-            if (!want_saddles) d &= 1u | (0x3Fu << 20);
-            push_cells(T, v, d);
-        }
-    }
-}
-// T back into L (counts included; entries past a list's capacity were not
-// stored, and the count shows the overflow)
-__global__ void k_list_back(Lists T, Lists L) {
-    const i64 n0 = min((i64)T.n[0], T.cap[0]), n1 = min((i64)T.n[1], T.cap[1]), n2 = min((i64)T.n[2], T.cap[2]),
-              n3 = min((i64)T.n[3], T.cap[3]);
-    const i64 tid = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    for (i64 i = tid; i < n0 + n1 + n2 + n3; i += (i64)gridDim.x * blockDim.x) {
-        if (i < n0) L.l[0][i] = T.l[0][i];
-        else if (i < n0 + n1) L.l[1][i - n0] = T.l[1][i - n0];
-        else if (i < n0 + n1 + n2) L.l[2][i - n0 - n1] = T.l[2][i - n0 - n1];
-        else L.l[3][i - n0 - n1 - n2] = T.l[3][i - n0 - n1 - n2];
-    }
-    if (tid < 4) L.n[tid] = T.n[tid];
 }
 
 // Dirty bricks.  A cell's pairing depends on the star of its highest vertex,
@@ -145,26 +56,33 @@ __global__ void k_list_back(Lists T, Lists L) {
 // or a neighbour of it: anchors 2 below to 1 above per axis.  Every brick with
 // such an anchor is marked (one byte per brick; writers all store 1).
 constexpr int kReachLow = 2, kReachHigh = 1;
-__global__ void k_mark_dirty(Grid g, int nbx, int nby, int sx, int sy, int sz, const i64 *verts,
-                             const unsigned long long *nverts, uint8_t *flags) {
-    const i64 n = (i64)*nverts;
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        int x, y, z;
-        decode_v(g, verts[i], x, y, z);
-        const int x0 = max(x - kReachLow, 0) / sx, x1 = min(x + kReachHigh, g.W - 1) / sx;
-        const int y0 = max(y - kReachLow, 0) / sy, y1 = min(y + kReachHigh, g.H - 1) / sy;
-        const int z0 = max(z - kReachLow, 0) / sz, z1 = min(z + kReachHigh, g.D - 1) / sz;
-        for (int bz = z0; bz <= z1; bz++)
-            for (int by = y0; by <= y1; by++)
-                for (int bx = x0; bx <= x1; bx++) flags[bx + (i64)nbx * (by + (i64)nby * bz)] = 1;
-    }
+struct BrickMarks {
+    uint8_t *flags;  // nullptr: not kept
+    int nbx, nby, shx, shy, shz;
+};
+__device__ __forceinline__ void mark_dirty(const Grid &g, const BrickMarks &B, i64 v) {
+    int x, y, z;
+    decode_v(g, v, x, y, z);
+    const int x0 = max(x - kReachLow, 0) >> B.shx, x1 = min(x + kReachHigh, g.W - 1) >> B.shx;
+    const int y0 = max(y - kReachLow, 0) >> B.shy, y1 = min(y + kReachHigh, g.H - 1) >> B.shy;
+    const int z0 = max(z - kReachLow, 0) >> B.shz, z1 = min(z + kReachHigh, g.D - 1) >> B.shz;
+    for (int bz = z0; bz <= z1; bz++)
+        for (int by = y0; by <= y1; by++)
+            for (int bx = x0; bx <= x1; bx++) B.flags[bx + (i64)B.nbx * (by + (i64)B.nby * bz)] = 1;
 }
-// the marked bricks as a list, and the marks cleared for the next round (four
-// marks to a word)
-__global__ void k_compact_bricks(int nbx, int nby, int nbz, uint32_t *flags, uint32_t *list, unsigned long long *n) {
+__global__ void k_mark_dirty(Grid g, BrickMarks B, const i64 *verts, const unsigned long long *nverts) {
+    const i64 n = (i64)*nverts;
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x)
+        mark_dirty(g, B, verts[i]);
+}
+// the marked bricks as a list and in `fresh`, and the marks cleared for the
+// next round (four marks to a word)
+__global__ void k_compact_bricks(int nbx, int nby, int nbz, uint32_t *flags, uint32_t *fresh, uint32_t *list,
+                                 unsigned long long *n) {
     const i64 nb = (i64)nbx * nby * nbz;
     for (i64 w = (i64)blockIdx.x * blockDim.x + threadIdx.x; w < (nb + 3) / 4; w += (i64)gridDim.x * blockDim.x) {
         const uint32_t word = flags[w];
+        fresh[w] = word;
         if (!word) continue;
         flags[w] = 0;
         for (int q = 0; q < 4; q++) {
@@ -681,8 +599,8 @@ static_assert(cxt::TOPO_FACE_NCOF[0] == 2 && cxt::TOPO_FACE_NCOF[5] == 2 && cxt:
 // bricks its paths visit.  A path is false only if a marked tetrahedron's
 // pairing differs.  Per brick, two flags say whether it holds such a
 // tetrahedron (as), or an original 1-saddle with a differing endpoint (ds);
-// k_path_flags sets them once and the gradient kernel refreshes them for the
-// bricks it re-pairs (a changed value reaches exactly their anchors).  A
+// the gradient kernels set them with the decompressed field's gradient (a
+// changed value reaches exactly the re-paired bricks' anchors).  A
 // detection then walks from the 2-saddles whose box holds a flagged brick and looks
 // at the 1-saddles of flagged bricks, and at nothing else.
 //
@@ -874,33 +792,13 @@ __device__ __forceinline__ i64 ds_differs(const Grid &g, const uint8_t *pvP, con
     if (pb != 15 && pb != pvQ[b]) return b;
     return -1;
 }
-// both flags of every brick (zero at launch)
-__global__ void k_path_flags(Grid g, PathFlags F, const uint32_t *tcQ, const uint8_t *pvQ, int nbx, int nby, int shx, int shy,
-                             int shz) {
-    for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += (i64)gridDim.x * blockDim.x) {
-        const uint32_t m = (F.critP[v] >> 1) & 0x7Fu;
-        bool ds = false;
-        if (m)
-            DMTZ_FOR(7, K, {
-                constexpr int k = decltype(K)::value;
-                if ((m >> k) & 1u) ds |= ds_differs<k>(g, F.pvP, pvQ, v) >= 0;
-            });
-        const bool as = tet_path_differs(F.tcP[v], tcQ[v]);
-        if (!as && !ds) continue;
-        int x, y, z;
-        decode_v(g, v, x, y, z);
-        const i64 b = (x >> shx) + (i64)nbx * ((y >> shy) + (i64)nby * (z >> shz));
-        if (as) F.as[b] = 1;
-        if (ds) F.ds[b] = 1;
-    }
-}
-
 // One detection: the first gridDim.x - ds_blocks blocks take the 2-saddles and
 // the segments of long paths, the others the bricks with a differing 1-saddle
 // endpoint (strict: none, k_ds_strict does those).
 constexpr int kQueue = 512;
 __global__ void __launch_bounds__(kBlock) k_path_detect(Grid g, PathFlags F, const i64 *sad2, const unsigned long long *nsad,
-                                                       const unsigned long long *box, const uint32_t *tcQ,
+                                                       const unsigned long long *box, const uint32_t *critP,
+                                                       const uint32_t *tcQ,
                                                        const uint8_t *pvQ, LongPaths L, PathRec R,
                                                        unsigned long long *ticket, int nbx, int nby, int nbz, int shape_x,
                                                        int shape_y, int shape_z, int ds_blocks) {
@@ -919,7 +817,7 @@ __global__ void __launch_bounds__(kBlock) k_path_detect(Grid g, PathFlags F, con
                     const int x = x0 + t % shape_x, y = y0 + (t / shape_x) % shape_y, z = z0 + t / (shape_x * shape_y);
                     if (x >= g.W || y >= g.H || z >= g.D) continue;
                     const i64 v = x + (i64)y * g.W + (i64)z * g.WH;
-                    const uint32_t c = (F.critP[v] >> 1) & 0x7Fu;
+                    const uint32_t c = (critP[v] >> 1) & 0x7Fu;
                     if (!c) continue;
                     DMTZ_FOR(7, K, {
                         constexpr int k = decltype(K)::value;
@@ -1169,7 +1067,8 @@ __global__ void __launch_bounds__(kBlock) k_fix_path(const __grid_constant__ Rul
 // The delta is what the reference's buffer holds: get_delta(v), with the
 // buffer's "no request" sentinel -2000*range (a request whose delta is not
 // above the sentinel leaves the buffer unchanged under edit_type 0).
-__global__ void k_apply(const __grid_constant__ RuleCtx c, double range, int preserve_type, int update, uint8_t *changed, double *delta_out) {
+__global__ void k_apply(const __grid_constant__ RuleCtx c, double range, int preserve_type, int update, uint8_t *changed, double *delta_out,
+                        BrickMarks B) {
     const i64 n = (i64)*c.reqn;
     const double sentinel = -2000.0 * range;
     const double tiny = 1e-15 * range;
@@ -1196,6 +1095,7 @@ __global__ void k_apply(const __grid_constant__ RuleCtx c, double range, int pre
             if (c.progress && (cv != 6 || gv != lowb)) *c.progress = 1ull;
         }
         if (changed) changed[v] = 1;
+        if (B.flags) mark_dirty(c.g, B, v);
     }
 }
 
@@ -1587,7 +1487,7 @@ struct dmtz_ctx {
     // separatrix checks (see k_path_detect): the box of bricks of each 2-saddle's
     // paths, and two flags per brick (path_keep: repairs refresh them)
     unsigned long long *path_box = nullptr;
-    uint8_t *path_as = nullptr, *path_ds = nullptr;
+    uint8_t *path_as = nullptr, *path_ds = nullptr;  // one allocation, capB each
     i64 capPB = 0;
     int path_keep = 0;
     Segment *seg = nullptr;  // segments of long paths, capSeg; per 2-saddle with one: capSlot
@@ -1606,7 +1506,8 @@ struct dmtz_ctx {
                                              // [20..23] rebuilt mismatch lists, [25,26]
                                              // path segments and their slots, [27] ticket of
                                              // the separatrix walks, [28] original 1-saddles, [29]
-                                             // ticket of the strict descending walks
+                                             // ticket of the strict descending walks, [30] blocks of
+                                             // k_round_end that are done
     int *errword = nullptr;
     uint8_t *changed = nullptr;
     int64_t launches = 0;  // kernels launched by the current call
@@ -1615,6 +1516,7 @@ struct dmtz_ctx {
     std::vector<dmtz_ctx *> pool;  // worker contexts of dmtz_correct_batch
     uint8_t *mm = nullptr;         // mismatch bytes of the learned proposal's features
     i64 capMM = 0;
+    unsigned long long *report = nullptr;  // pinned: counts of the last round (k_round_end), hc's layout
     int march_blocks = 0;          // blocks of k_grad_march the device holds at once (0: not asked yet)
     void *loopctl = nullptr;       // device copy of the graph loop's control block (kept: a
                                    // cudaFree per call would synchronise the whole device)
@@ -1653,7 +1555,7 @@ void free_all(dmtz_ctx *c) {
     cudaFree(c->as_tet); cudaFree(c->as_cur); cudaFree(c->ds_edge); cudaFree(c->ds_vert);
     cudaFree(c->counters); cudaFree(c->errword); cudaFree(c->changed);
     cudaFree(c->sad2); cudaFree(c->brick_flags); cudaFree(c->brick_list);
-    cudaFree(c->path_box); cudaFree(c->path_as); cudaFree(c->path_ds);
+    cudaFree(c->path_box); cudaFree(c->path_as);
     c->path_box = nullptr; c->path_as = c->path_ds = nullptr;
     cudaFree(c->seg); cudaFree(c->seg_sad); cudaFree(c->seg_res);
     c->seg = nullptr; c->seg_sad = nullptr; c->seg_res = nullptr;
@@ -1719,8 +1621,9 @@ dmtz_status ensure(dmtz_ctx *ctx, const Grid &g) {
     CK(cudaMemset(ctx->reqbits, 0, sizeof(uint32_t) * (size_t)((V + 31) / 32 + 1)));
     CK(dalloc(&ctx->reqlist, V));
     CK(dalloc(&ctx->brick_flags, (nbr + 3) / 4)); CK(dalloc(&ctx->brick_list, nbr));
-    CK(dalloc(&ctx->brick_fresh, nbr));
-    CK(dalloc(&ctx->path_as, nbr)); CK(dalloc(&ctx->path_ds, nbr));
+    CK(dalloc(&ctx->brick_fresh, (nbr + 3) / 4 * 4));
+    CK(dalloc(&ctx->path_as, 2 * nbr));
+    ctx->path_ds = ctx->path_as + nbr;
     CK(dalloc(&ctx->brick_n, 8));
     CK(cudaMemset(ctx->brick_flags, 0, sizeof(uint32_t) * (size_t)((nbr + 3) / 4)));
     ctx->capB = nbr;
@@ -1766,7 +1669,7 @@ bool shape_fits(const Grid &g, int shape) {
 }
 
 PathFlags path_flags(const dmtz_ctx *ctx) {
-    return PathFlags{ctx->path_as, ctx->path_ds, ctx->P.tcode, ctx->P.crit, ctx->P.pv};
+    return PathFlags{ctx->path_as, ctx->path_ds, ctx->P.tcode, ctx->P.pv};
 }
 LongPaths long_paths(const dmtz_ctx *ctx) {
     return LongPaths{ctx->seg, ctx->seg_sad, ctx->seg_res, ctx->counters + 25, ctx->capSeg, ctx->capSlot};
@@ -1786,13 +1689,14 @@ unsigned brick_grid(const dmtz_ctx *ctx, i64 nb) {
     return (unsigned)std::max<i64>(1, std::min<i64>(nb, cap));
 }
 
-// the gradient of a set of bricks
+// the gradient of a set of bricks (and the old mismatch lists' entries, see KeepOps)
 void grad_bricks(const Grid &g, const FieldState &s, const BrickList &bl, unsigned grid, cudaStream_t st,
-                 const PathFlags &F = PathFlags{}) {
+                 const GradOps &O = GradOps{}, const KeepOps &K = KeepOps{}) {
+    grid += K.blocks;
     switch (bl.shape) {
-    case 1: k_grad_bricks<16, 4, 2><<<grid, brick_threads<16, 4, 2>(), 0, st>>>(g, s, bl, F); break;
-    case 2: k_grad_bricks<32, 2, 2><<<grid, brick_threads<32, 2, 2>(), 0, st>>>(g, s, bl, F); break;
-    default: k_grad_bricks<8, 4, 4><<<grid, brick_threads<8, 4, 4>(), 0, st>>>(g, s, bl, F); break;
+    case 1: k_grad_bricks<16, 4, 2><<<grid, brick_threads<16, 4, 2>(), 0, st>>>(g, s, bl, O, K); break;
+    case 2: k_grad_bricks<32, 2, 2><<<grid, brick_threads<32, 2, 2>(), 0, st>>>(g, s, bl, O, K); break;
+    default: k_grad_bricks<8, 4, 4><<<grid, brick_threads<8, 4, 4>(), 0, st>>>(g, s, bl, O, K); break;
     }
 }
 
@@ -1815,22 +1719,27 @@ BrickList all_bricks(const Grid &g, int shape, i64 &nb) {
 // blocks and 48 registers 935 us at 256^3 and 51 us instead of 43 us at 97 x 61 x
 // 75; 32 x 8 with three blocks 874 and 51 us; 64 x 8 1035 and 58 us.
 constexpr int kMarchX = 32, kMarchY = 16, kMarchBlocks = 1;
-void grad_full(dmtz_ctx *ctx, const Grid &g, const FieldState &s) {
-    {
-        i64 nb;
-        const BrickList bl = all_bricks(g, ctx->tune_shape, nb);
-        if (nb <= (i64)(persistent_grid() / 8) * 3) {
-            grad_bricks(g, s, bl, (unsigned)nb, ctx->stream);
-            ctx->launches++;
-            return;
-        }
+bool grad_marches(const dmtz_ctx *ctx, const Grid &g) {
+    i64 nb;
+    all_bricks(g, ctx->tune_shape, nb);
+    return nb > (i64)(persistent_grid() / 8) * 3;
+}
+// Not counted in ctx->launches (also used while capturing the graph loop).
+void grad_full(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const GradOps &O = GradOps{}) {
+    i64 nb;
+    const BrickList bl = all_bricks(g, ctx->tune_shape, nb);
+    if (!grad_marches(ctx, g)) {
+        grad_bricks(g, s, bl, (unsigned)nb, ctx->stream, O);
+        return;
     }
     using M = March<kMarchX, kMarchY>;
-    auto kern = k_grad_march<kMarchX, kMarchY, kMarchBlocks>;
+    auto plain = k_grad_march<kMarchX, kMarchY, kMarchBlocks, false>;
+    auto track = k_grad_march<kMarchX, kMarchY, kMarchBlocks, true>;
     if (!ctx->march_blocks) {
         int per_sm = 0;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, M::NT, M::smem);
+        cudaFuncSetAttribute(plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::smem);
+        cudaFuncSetAttribute(track, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, plain, M::NT, M::smem);
         ctx->march_blocks = std::max(1, per_sm) * (int)(persistent_grid() / 8);
     }
     const int ntx = (g.W + kMarchX - 1) / kMarchX, nty = (g.H + kMarchY - 1) / kMarchY;
@@ -1847,71 +1756,117 @@ void grad_full(dmtz_ctx *ctx, const Grid &g, const FieldState &s) {
         }
     }
     const i64 blocks = tiles * ((g.D + chunk - 1) / chunk);
-    kern<<<(unsigned)blocks, M::NT, M::smem, ctx->stream>>>(g, s, ntx, nty, chunk);
-    ctx->launches++;
+    int sh[3];
+    shape_shifts(ctx->tune_shape, sh);
+    if (O.critP) {
+        if (O.F.as) cudaMemsetAsync(O.F.as, 0, 2 * (size_t)ctx->capB, ctx->stream);
+        track<<<(unsigned)blocks, M::NT, M::smem, ctx->stream>>>(g, s, ntx, nty, chunk, O, sh[0], sh[1], sh[2], bl.nbx, bl.nby);
+    } else {
+        plain<<<(unsigned)blocks, M::NT, M::smem, ctx->stream>>>(g, s, ntx, nty, chunk, O, sh[0], sh[1], sh[2], bl.nbx, bl.nby);
+    }
 }
 
-// mismatch lists of the decompressed gradient against crit_o
-void scan_mismatch(dmtz_ctx *ctx, const Grid &g, const uint32_t *crit_d, const uint32_t *crit_o, int want_saddles) {
+Lists mismatch_lists(const dmtz_ctx *ctx) {
     Lists L;
     for (int k = 0; k < 4; k++) {
         L.l[k] = ctx->lists[k];
         L.cap[k] = ctx->capL[k];
     }
     L.n = ctx->counters;
+    return L;
+}
+Lists rebuilt_lists(const dmtz_ctx *ctx) {
+    Lists T = mismatch_lists(ctx);
+    for (int k = 0; k < 4; k++) T.l[k] = ctx->list_tmp[k];
+    T.n = ctx->counters + 20;
+    return T;
+}
+// cells a mismatch list holds, as bits of FieldState::crit
+uint32_t want_bits(int want_saddles) { return want_saddles ? 0x3FFFFFFu : (1u | (0x3Fu << 20)); }
+
+// mismatch lists of the decompressed gradient against crit_o
+void scan_mismatch(dmtz_ctx *ctx, const Grid &g, const uint32_t *crit_d, const uint32_t *crit_o, int want_saddles) {
     cudaMemsetAsync(ctx->counters, 0, 4 * sizeof(unsigned long long), ctx->stream);
-    k_mismatch_scan<<<persistent_grid(), kBlock, 0, ctx->stream>>>(g, crit_d, crit_o, L, want_saddles);
+    k_mismatch_scan<<<persistent_grid(), kBlock, 0, ctx->stream>>>(g, crit_d, crit_o, mismatch_lists(ctx), want_saddles);
     ctx->launches++;
 }
 
-// full gradient of one field (and its mismatch lists when crit_o is given)
+// full gradient of one field (and its mismatch lists when crit_o is given, and
+// the bricks' path flags when they are kept)
 void run_pairing(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32_t *crit_o, int want_saddles) {
-    grad_full(ctx, g, s);
-    if (crit_o) scan_mismatch(ctx, g, s.crit, crit_o, want_saddles);
+    GradOps O{};
+    if (crit_o) {
+        cudaMemsetAsync(ctx->counters, 0, 4 * sizeof(unsigned long long), ctx->stream);
+        O.T = mismatch_lists(ctx);
+        O.critP = crit_o;
+        O.want = want_bits(want_saddles);
+        if (ctx->path_keep) O.F = path_flags(ctx);
+    }
+    grad_full(ctx, g, s, O);
+    ctx->launches++;
 }
 
-// re-pair only the bricks near the vertices the last update requested
-// (ctx->reqlist), then rebuild the mismatch lists
-void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32_t *crit_o, int want_saddles) {
-    int nbx, nby, nbz;
-    const int shape = ctx->tune_shape;
-    i64 nb = bricks_of(g, shape, nbx, nby, nbz);
+BrickMarks brick_marks(const dmtz_ctx *ctx, const Grid &g) {
+    BrickMarks B;
+    int nbz, sh[3];
+    B.flags = reinterpret_cast<uint8_t *>(ctx->brick_flags);
+    bricks_of(g, ctx->tune_shape, B.nbx, B.nby, nbz);
+    shape_shifts(ctx->tune_shape, sh);
+    B.shx = sh[0];
+    B.shy = sh[1];
+    B.shz = sh[2];
+    return B;
+}
+
+// Re-pair only the bricks near the vertices the last update requested (marked
+// already by k_apply, or else from ctx->reqlist); the mismatch lists are then rebuilt
+// into list_tmp (inc_scan; k_round_end takes them back) or scanned for.  The
+// brick count is zero at the start (k_round_end, or the caller).
+void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32_t *crit_o, int want_saddles, bool marked) {
+    const BrickMarks B = brick_marks(ctx, g);
     cudaStream_t st = ctx->stream;
-    cudaMemsetAsync(ctx->brick_n, 0, sizeof(unsigned long long), st);
-    k_mark_dirty<<<persistent_grid(), kBlock, 0, st>>>(g, nbx, nby, DMTZ_SHAPES[shape][0], DMTZ_SHAPES[shape][1],
-                                                        DMTZ_SHAPES[shape][2], ctx->reqlist, ctx->counters + 4,
-                                                        reinterpret_cast<uint8_t *>(ctx->brick_flags));
-    k_compact_bricks<<<persistent_grid(), kBlock, 0, st>>>(nbx, nby, nbz, ctx->brick_flags, ctx->brick_list, ctx->brick_n);
-    ctx->launches += 2;
-    if (ctx->inc_scan) {
-        cudaMemsetAsync(ctx->brick_fresh, 0, (size_t)nb, st);
-        k_mark_fresh<<<persistent_grid(), kBlock, 0, st>>>(ctx->brick_list, ctx->brick_n, ctx->brick_fresh, nbx, nby);
+    i64 nb;
+    BrickList bl = all_bricks(g, ctx->tune_shape, nb);
+    if (!marked) {
+        k_mark_dirty<<<persistent_grid(), kBlock, 0, st>>>(g, B, ctx->reqlist, ctx->counters + 4);
         ctx->launches++;
     }
-    BrickList bl = all_bricks(g, shape, nb);
+    k_compact_bricks<<<(unsigned)std::min<i64>(persistent_grid(), grid_for((nb + 3) / 4)), kBlock, 0, st>>>(
+        bl.nbx, bl.nby, bl.nbz, ctx->brick_flags, reinterpret_cast<uint32_t *>(ctx->brick_fresh), ctx->brick_list, ctx->brick_n);
     bl.list = ctx->brick_list;
     bl.n = ctx->brick_n;
-    grad_bricks(g, s, bl, brick_grid(ctx, nb), st, ctx->path_keep ? path_flags(ctx) : PathFlags{});
-    ctx->launches++;
-    if (!ctx->inc_scan) {
-        scan_mismatch(ctx, g, s.crit, crit_o, want_saddles);
-        return;
+    GradOps O{};
+    KeepOps K{};
+    if (ctx->path_keep || ctx->inc_scan) O.critP = crit_o;
+    if (ctx->path_keep) O.F = path_flags(ctx);
+    if (ctx->inc_scan) {
+        O.T = rebuilt_lists(ctx);
+        O.want = want_bits(want_saddles);
+        K.L = mismatch_lists(ctx);
+        K.fresh = ctx->brick_fresh;
+        K.shx = B.shx;
+        K.shy = B.shy;
+        K.shz = B.shz;
+        K.nbx = B.nbx;
+        K.nby = B.nby;
+        K.blocks = persistent_grid() / 8;
     }
-    Lists L, T;
-    for (int k = 0; k < 4; k++) {
-        L.l[k] = ctx->lists[k];
-        T.l[k] = ctx->list_tmp[k];
-        L.cap[k] = T.cap[k] = ctx->capL[k];
-    }
-    L.n = ctx->counters;
-    T.n = ctx->counters + 20;
-    const int sx = DMTZ_SHAPES[shape][0], sy = DMTZ_SHAPES[shape][1], sz = DMTZ_SHAPES[shape][2];
-    const unsigned pg = persistent_grid();
-    cudaMemsetAsync(ctx->counters + 20, 0, 4 * sizeof(unsigned long long), st);
-    k_list_keep<<<pg, kBlock, 0, st>>>(g, L, T, ctx->brick_fresh, sx, sy, sz, nbx, nby);
-    k_scan_fresh<<<pg, kBlock, 0, st>>>(g, s.crit, crit_o, T, ctx->brick_list, ctx->brick_n, sx, sy, sz, want_saddles);
-    k_list_back<<<pg, kBlock, 0, st>>>(T, L);
-    ctx->launches += 3;
+    grad_bricks(g, s, bl, brick_grid(ctx, nb), st, O, K);
+    ctx->launches += 2;
+    if (!ctx->inc_scan) scan_mismatch(ctx, g, s.crit, crit_o, want_saddles);
+}
+// a round's re-pairing when its lists are long (the whole grid, lists and flags in place)
+void repair_full(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32_t *crit_o, int want_saddles) {
+    run_pairing(ctx, g, s, crit_o, want_saddles);
+}
+// Lists with at least this many cells mean a repair of the whole grid: their
+// updates reach most bricks then, and the march's halo is smaller (256^3 with 189 k
+// listed cells and 131 k bricks: 96 % of the bricks, 1.81 ms by bricks, 0.9 ms
+// by the march, which is even at half of the bricks).
+i64 heavy_cells(const dmtz_ctx *ctx, const Grid &g) {
+    i64 nb;
+    all_bricks(g, ctx->tune_shape, nb);
+    return grad_marches(ctx, g) ? std::max<i64>(1, nb / 2) : INT64_MAX;
 }
 
 double key_to_double(unsigned long long k) {
@@ -2095,27 +2050,12 @@ dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g) {
     return trace_paths(ctx, g);
 }
 
-// the bricks' path flags, from both gradients; repairs keep them from here on
-dmtz_status init_path_flags(dmtz_ctx *ctx, const Grid &g) {
-    int nbx, nby, nbz, sh[3];
-    const i64 nb = bricks_of(g, ctx->tune_shape, nbx, nby, nbz);
-    shape_shifts(ctx->tune_shape, sh);
-    CK(cudaMemsetAsync(ctx->path_as, 0, (size_t)nb, ctx->stream));
-    CK(cudaMemsetAsync(ctx->path_ds, 0, (size_t)nb, ctx->stream));
-    k_path_flags<<<persistent_grid(), kBlock, 0, ctx->stream>>>(g, path_flags(ctx), ctx->Q.tcode, ctx->Q.pv, nbx, nby, sh[0],
-                                                                sh[1], sh[2]);
-    ctx->launches++;
-    ctx->path_keep = 1;
-    CK(cudaGetLastError());
-    return DMTZ_OK;
-}
-
 // separatrix detection (ascending and descending) into the path records
 // geometry mode (conn = 0) or connectivity mode (conn = 1); no launch counting
 // (also used while capturing the graph loop)
+// (counters 5, 6 and 27 are zero: the caller, or the round's end in the graph loop)
 void launch_detect(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const PathRec &R, unsigned grid, int conn) {
     cudaStream_t st = ctx->stream;
-    cudaMemsetAsync(ctx->counters + 5, 0, 2 * sizeof(unsigned long long), st);
     if (conn) {
         k_conn_as<<<grid, kBlock, 0, st>>>(g, ctx->P.crit, ctx->Q.crit, ctx->P.tcode, ctx->Q.tcode, R,
                                            g.T + 16, ctx->errword);
@@ -2125,9 +2065,8 @@ void launch_detect(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const PathRe
         const int shape = ctx->tune_shape, *sx = DMTZ_SHAPES[shape];
         const i64 nb = bricks_of(g, shape, nbx, nby, nbz);
         const int ds_blocks = ctx->strict_ds ? 0 : (int)std::min<i64>((nb + 255) / 256, grid / 8);
-        cudaMemsetAsync(ctx->counters + 27, 0, sizeof(unsigned long long), st);  // the walks' ticket
         k_path_detect<<<grid + (unsigned)ds_blocks, kBlock, 0, st>>>(g, path_flags(ctx), ctx->sad2, ctx->counters + 10,
-                                                                     ctx->path_box, ctx->Q.tcode, ctx->Q.pv, long_paths(ctx),
+                                                                     ctx->path_box, ctx->P.crit, ctx->Q.tcode, ctx->Q.pv, long_paths(ctx),
                                                                      R, ctx->counters + 27, nbx, nby, nbz, sx[0], sx[1],
                                                                      sx[2], ds_blocks);
         k_path_long<<<grid / 8, kBlock, 0, st>>>(g, long_paths(ctx), R);
@@ -2141,6 +2080,8 @@ void launch_detect(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const PathRe
 // kernels one detection launches
 int detect_kernels(const dmtz_ctx *ctx, int conn) { return conn ? 2 : (ctx->strict_ds ? 3 : 2); }
 void detect_paths(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const PathRec &R, unsigned grid, int conn = 0) {
+    cudaMemsetAsync(ctx->counters + 5, 0, 2 * sizeof(unsigned long long), ctx->stream);
+    cudaMemsetAsync(ctx->counters + 27, 0, sizeof(unsigned long long), ctx->stream);
     launch_detect(ctx, g, rc, R, grid, conn);
     ctx->launches += detect_kernels(ctx, conn);
 }
@@ -2444,6 +2385,7 @@ void dmtz_ctx_destroy(dmtz_ctx *ctx) {
     free_all(ctx);
     cudaFree(ctx->mm);
     cudaFree(ctx->loopctl);
+    cudaFreeHost(ctx->report);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->side) cudaStreamDestroy(ctx->side);
     if (ctx->side_done) cudaEventDestroy(ctx->side_done);
@@ -2484,13 +2426,21 @@ dmtz_status dmtz_extract(dmtz_ctx *ctx, int W, int H, int D, const double *data,
 }
 
 // shared set-up of the two complexes for the parity entry points
-static dmtz_status setup_pair(dmtz_ctx *ctx, const Grid &g, const double *orig, const double *decp) {
+// (paths: with the original paths and the bricks' path flags)
+static dmtz_status setup_pair(dmtz_ctx *ctx, const Grid &g, const double *orig, const double *decp, bool paths = false) {
     dmtz_status s;
+    ctx->path_keep = 0;
     if ((s = ensure(ctx, g)) != DMTZ_OK) return s;
     if ((s = upload(ctx, ctx->f, orig, g.V, 0)) != DMTZ_OK) return s;
     if ((s = upload(ctx, ctx->g, decp, g.V, 0)) != DMTZ_OK) return s;
     run_pairing(ctx, g, view(ctx->P, ctx->f), nullptr, 1);
+    if (paths) {
+        CK(cudaMemsetAsync(ctx->errword, 0, sizeof(int), ctx->stream));
+        if ((s = prep_paths(ctx, g)) != DMTZ_OK) return s;
+        ctx->path_keep = 1;
+    }
     run_pairing(ctx, g, view(ctx->Q, ctx->g), ctx->P.crit, 1);
+    ctx->path_keep = 0;
     CK(cudaGetLastError());
     unsigned long long hc[4];
     CK(cudaMemcpyAsync(hc, ctx->counters, sizeof(hc), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2551,7 +2501,7 @@ dmtz_status dmtz_fix_round(dmtz_ctx *ctx, int W, int H, int D, const double *ori
     std::vector<double> fill((size_t)g.V, sentinel);
     CK(cudaMemcpyAsync(dd, fill.data(), sizeof(double) * (size_t)g.V, cudaMemcpyHostToDevice, ctx->stream));
     // report the deltas the rules requested, without updating the field
-    k_apply<<<persistent_grid(), kBlock, 0, ctx->stream>>>(rc, range, 0, 0, nullptr, dd);
+    k_apply<<<persistent_grid(), kBlock, 0, ctx->stream>>>(rc, range, 0, 0, nullptr, dd, BrickMarks{});
     CK(cudaMemcpyAsync(delta_out, dd, sizeof(double) * (size_t)g.V, cudaMemcpyDeviceToHost, ctx->stream));
     int err = 0;
     CK(cudaMemcpyAsync(&err, ctx->errword, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2570,12 +2520,8 @@ static dmtz_status path_detect_impl(dmtz_ctx *ctx, int W, int H, int D, const do
     if (s != DMTZ_OK) return s;
     ctx->strict_ds = strict && !conn;
     CK(cudaSetDevice(ctx->device));
-    if ((s = setup_pair(ctx, g, orig, decp)) != DMTZ_OK) return s;
-    CK(cudaMemsetAsync(ctx->errword, 0, sizeof(int), ctx->stream));
+    if ((s = setup_pair(ctx, g, orig, decp, true)) != DMTZ_OK) return s;
     RuleCtx rc = rule_ctx(ctx, g, 0.0, 0);
-    if ((s = prep_paths(ctx, g)) != DMTZ_OK) return s;
-    if ((s = init_path_flags(ctx, g)) != DMTZ_OK) return s;
-    ctx->path_keep = 0;
     unsigned long long hc[2];
     int err = 0;
     for (int attempt = 0; attempt < 2; attempt++) {
@@ -2654,10 +2600,8 @@ dmtz_status dmtz_wall_detect(dmtz_ctx *ctx, int W, int H, int D, const double *o
     if (s != DMTZ_OK) return s;
     if (!count) return fail(ctx, DMTZ_ERR_ARG, "null count");
     CK(cudaSetDevice(ctx->device));
-    if ((s = setup_pair(ctx, g, orig, decp)) != DMTZ_OK) return s;
-    CK(cudaMemsetAsync(ctx->errword, 0, sizeof(int), ctx->stream));
+    if ((s = setup_pair(ctx, g, orig, decp, true)) != DMTZ_OK) return s;
     RuleCtx rc = rule_ctx(ctx, g, 0.0, 0);
-    if ((s = prep_paths(ctx, g)) != DMTZ_OK) return s;
     i64 n = 0;
     if ((s = detect_walls(ctx, g, rc, n)) != DMTZ_OK) return s;
     *count = (int64_t)n;
@@ -2690,15 +2634,17 @@ dmtz_status dmtz_wall_detect(dmtz_ctx *ctx, int W, int H, int D, const double *o
 //   PFIX   path phase on the records PCHECK just made (the reference detects
 //          them again at the start of its next outer iteration; same inputs,
 //          same records)
+//   CPF    a critical-point round with long lists: the whole grid is re-paired
 namespace {
-enum { LS_CP = 0, LS_PDF = 1, LS_PCHECK = 2, LS_PFIX = 3, LS_DONE = 4 };
+enum { LS_CP = 0, LS_PDF = 1, LS_PCHECK = 2, LS_PFIX = 3, LS_CPF = 4, LS_DONE = 5, LS_STATES = 5 };
 struct LoopCtl {
     int state, pvp, converged, pad;
     long long rounds, max_rounds, outer, cp_rounds, path_rounds;
     long long cc[4];
     long long n_as, n_ds;
-    long long runs[4];  // body executions per state
-    long long cap[4];   // mismatch list capacities
+    long long runs[LS_STATES];  // body executions per state
+    long long cap[4];           // mismatch list capacities
+    long long heavy;            // listed cells from which a round re-pairs the whole grid
     int overflow;       // a scan overflowed a list: stop, grow, scan again, resume at `state`
     int last;           // state of the last body run
     int break_stalls;   // stop when a round changed nothing (the host breaks the stall)
@@ -2710,25 +2656,27 @@ __global__ void k_set_switch(const LoopCtl *ctl, cudaGraphConditionalHandle h) {
     cudaGraphSetConditional(h, (unsigned)ctl->state);
 }
 
-__global__ void k_loop_ctl(LoopCtl *ctl, const unsigned long long *counters, cudaGraphConditionalHandle hwhile) {
-    LoopCtl c = *ctl;
+// the state after a body run, from the counters it left
+__device__ __forceinline__ LoopCtl loop_next(LoopCtl c, const unsigned long long *counters) {
     const int st = c.state;
     c.runs[st]++;
     if (st != LS_PCHECK)
         for (int k = 0; k < 4; k++) c.cc[k] = (long long)counters[k];
-    const bool cp_any = c.cc[0] > 0 || c.cc[1] > 0 || c.cc[2] > 0 || c.cc[3] > 0;
+    const long long cells = c.cc[0] + c.cc[1] + c.cc[2] + c.cc[3];
+    const bool cp_any = cells > 0;
+    const int cp = cells >= c.heavy ? LS_CPF : LS_CP;
     int next;
-    if (st == LS_CP) {
+    if (st == LS_CP || st == LS_CPF) {
         c.rounds++;
         c.cp_rounds++;
-        next = cp_any ? LS_CP : (c.pvp ? LS_PDF : LS_DONE);
+        next = cp_any ? cp : (c.pvp ? LS_PDF : LS_DONE);
     } else if (st == LS_PDF || st == LS_PFIX) {
         c.rounds++;
         c.path_rounds++;
         c.n_as = c.n_ds = 0;
         if (cp_any) {
             c.outer++;
-            next = LS_CP;
+            next = cp;
         } else {
             next = LS_PCHECK;
         }
@@ -2753,11 +2701,61 @@ __global__ void k_loop_ctl(LoopCtl *ctl, const unsigned long long *counters, cud
     // counters[7]: set by the update when it changed something; a path round
     // counts only if its detection had records (counters[5], [6])
     if (c.break_stalls && next != LS_DONE && counters[7] == 0 &&
-        (st == LS_CP || ((st == LS_PDF || st == LS_PFIX) && counters[5] + counters[6] > 0)))
+        (st == LS_CP || st == LS_CPF || ((st == LS_PDF || st == LS_PFIX) && counters[5] + counters[6] > 0)))
         c.stalled = 1;
     c.state = next;
-    *ctl = c;
-    cudaGraphSetConditional(hwhile, (next != LS_DONE && !c.overflow && !c.stalled) ? 1u : 0u);
+    return c;
+}
+
+// The end of a round: the rebuilt mismatch lists back into the lists (T.n ==
+// nullptr: none were rebuilt; entries past a list's capacity were not stored,
+// and the count shows the overflow), then the last block to finish clears the
+// round's counters and either decides the graph loop's next state (ctl) or
+// leaves the counts for the host (report, in pinned memory).
+__global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Lists T, const __grid_constant__ Lists L, unsigned long long *counters, unsigned long long *brick_n,
+                                                     LoopCtl *ctl, cudaGraphConditionalHandle hwhile,
+                                                     unsigned long long *report) {
+    __shared__ bool last;
+    const int st = ctl ? ctl->state : LS_CP;
+    const bool copy = T.n && st != LS_PCHECK && st != LS_CPF;
+    if (copy) {
+        const i64 n0 = min((i64)T.n[0], T.cap[0]), n1 = min((i64)T.n[1], T.cap[1]), n2 = min((i64)T.n[2], T.cap[2]),
+                  n3 = min((i64)T.n[3], T.cap[3]);
+        const i64 tid = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+        for (i64 i = tid; i < n0 + n1 + n2 + n3; i += (i64)gridDim.x * blockDim.x) {
+            if (i < n0) L.l[0][i] = T.l[0][i];
+            else if (i < n0 + n1) L.l[1][i - n0] = T.l[1][i - n0];
+            else if (i < n0 + n1 + n2) L.l[2][i - n0 - n1] = T.l[2][i - n0 - n1];
+            else L.l[3][i - n0 - n1 - n2] = T.l[3][i - n0 - n1 - n2];
+        }
+    }
+    __syncthreads();  // the block has read T.n and the state
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(&counters[30], 1ull) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last || threadIdx.x != 0) return;
+    __threadfence();
+    counters[30] = 0;
+    *brick_n = 0;
+    if (copy)
+        for (int k = 0; k < 4; k++) {
+            L.n[k] = T.n[k];
+            T.n[k] = 0;
+        }
+    bool stop = false;
+    if (ctl) {
+        const LoopCtl c = loop_next(*ctl, counters);
+        *ctl = c;
+        stop = c.state == LS_DONE || c.overflow || c.stalled;
+        cudaGraphSetConditional(hwhile, stop ? 0u : 1u);
+        if (!stop && (c.state == LS_PDF || c.state == LS_PCHECK)) counters[5] = counters[6] = counters[27] = 0;
+    } else {
+        for (int k = 0; k < 8; k++) report[k] = counters[k];
+        __threadfence_system();
+    }
+    if (!stop) counters[4] = counters[7] = 0;  // a stalled round's requests were applied: the host starts afresh
 }
 
 // ----------------------------------------------------------------------------- phase timers
@@ -2798,6 +2796,7 @@ struct PhaseTimer {
 }  // namespace
 
 // Build and run the graph-driven loop.  Returns the final LoopCtl in *out.
+// The states' counters (requests, progress, separatrix records) as its first state needs them.
 static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const CpLists &L,
                                   const PathRec &PR, const FieldState &Qs, double range, int ps, int pt, int conn,
                                   LoopCtl init, LoopCtl *out) {
@@ -2806,6 +2805,11 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
     if (!ctx->loopctl) CK(cudaMalloc(&ctx->loopctl, sizeof(LoopCtl)));
     LoopCtl *dctl = static_cast<LoopCtl *>(ctx->loopctl);
     CK(cudaMemcpyAsync(dctl, &init, sizeof(LoopCtl), cudaMemcpyHostToDevice, st));
+    CK(cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), st));
+    CK(cudaMemsetAsync(ctx->counters + 7, 0, sizeof(unsigned long long), st));
+    CK(cudaMemsetAsync(ctx->counters + 27, 0, sizeof(unsigned long long), st));
+    CK(cudaMemsetAsync(ctx->brick_n, 0, sizeof(unsigned long long), st));
+    if (init.state != LS_PFIX) CK(cudaMemsetAsync(ctx->counters + 5, 0, 2 * sizeof(unsigned long long), st));
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     dmtz_status res = DMTZ_OK;
@@ -2826,7 +2830,7 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
         cudaGraph_t body = wp.conditional.phGraph_out[0];
         cudaGraphConditionalHandle hsw;
         if (cudaGraphConditionalHandleCreate(&hsw, body, 0, 0) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
-        // body: set the switch from the state, switch over the four states, decide
+        // body: set the switch from the state, switch over the states, end the round
         cudaGraphNode_t n_set, n_sw, n_ctl;
         {
             if (cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
@@ -2843,9 +2847,9 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
         sp.type = cudaGraphNodeTypeConditional;
         sp.conditional.handle = hsw;
         sp.conditional.type = cudaGraphCondTypeSwitch;
-        sp.conditional.size = 4;
+        sp.conditional.size = LS_STATES;
         if (cudaGraphAddNode(&n_sw, body, &n_set, nullptr, 1, &sp) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
-        for (int state = 0; state < 4 && res == DMTZ_OK; state++) {
+        for (int state = 0; state < LS_STATES && res == DMTZ_OK; state++) {
             cudaGraph_t child = sp.conditional.phGraph_out[state];
             if (cudaStreamBeginCaptureToGraph(st, child, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
                 res = DMTZ_ERR_CUDA;
@@ -2853,12 +2857,14 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
             }
             if (state == LS_PDF || state == LS_PCHECK) launch_detect(ctx, g, rc, PR, pgrid, conn);
             if (state != LS_PCHECK) {
-                cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), st);
-                cudaMemsetAsync(ctx->counters + 7, 0, sizeof(unsigned long long), st);
-                if (state == LS_CP) k_fix_cp<<<pgrid, kBlock, 0, st>>>(rc, L, ps);
+                const bool cp = state == LS_CP || state == LS_CPF;
+                const int want = cp ? (ps == 1) : 1;
+                if (cp) k_fix_cp<<<pgrid, kBlock, 0, st>>>(rc, L, ps);
                 else k_fix_path<<<pgrid, kBlock, 0, st>>>(rc, PR);
-                k_apply<<<pgrid, kBlock, 0, st>>>(rc, range, pt, 1, ctx->changed, nullptr);
-                repair_dirty(ctx, g, Qs, ctx->P.crit, state == LS_CP ? (ps == 1) : 1);
+                k_apply<<<pgrid, kBlock, 0, st>>>(rc, range, pt, 1, ctx->changed, nullptr,
+                                                  state == LS_CPF ? BrickMarks{} : brick_marks(ctx, g));
+                if (state == LS_CPF) repair_full(ctx, g, Qs, ctx->P.crit, want);
+                else repair_dirty(ctx, g, Qs, ctx->P.crit, want, true);
             }
             cudaGraph_t tmp;
             if (cudaStreamEndCapture(st, &tmp) != cudaSuccess) res = DMTZ_ERR_CUDA;
@@ -2869,7 +2875,8 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
                 res = DMTZ_ERR_CUDA;
                 break;
             }
-            k_loop_ctl<<<1, 1, 0, st>>>(dctl, ctx->counters, hwhile);
+            k_round_end<<<pgrid / 8, kBlock, 0, st>>>(ctx->inc_scan ? rebuilt_lists(ctx) : Lists{}, mismatch_lists(ctx),
+                                                      ctx->counters, ctx->brick_n, dctl, hwhile, nullptr);
             cudaGraph_t tmp;
             if (cudaStreamEndCapture(st, &tmp) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
             (void)n_ctl;
@@ -2890,6 +2897,14 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
 }
 
 // ----------------------------------------------------------------------------- the correction loop
+// the round's end of the host-driven loop (its counts then stand in ctx->report once the stream is done)
+static void host_round_end(dmtz_ctx *ctx) {
+    k_round_end<<<persistent_grid() / 8, kBlock, 0, ctx->stream>>>(ctx->inc_scan ? rebuilt_lists(ctx) : Lists{},
+                                                                   mismatch_lists(ctx), ctx->counters, ctx->brick_n, nullptr,
+                                                                   cudaGraphConditionalHandle{}, ctx->report);
+    ctx->launches++;
+}
+
 // features of (ctx->f, ctx->g) from the current gradients ctx->P / ctx->Q
 static dmtz_status features_into(dmtz_ctx *ctx, const Grid &g, double bound, __nv_bfloat16 *feat, uint8_t *active) {
     if (g.V > ctx->capMM) {
@@ -2930,7 +2945,8 @@ static dmtz_status learned_start(dmtz_ctx *ctx, dmtz_cnn *net, const Grid &g, do
     ctx->launches += 5;
     // re-pair only the bricks within the passes' radii of the edited vertices
     // (the mismatch lists are rebuilt by a full scan: the loop has not started)
-    repair_dirty(ctx, g, view(ctx->Q, ctx->g), ctx->P.crit, 1);
+    CK(cudaMemsetAsync(ctx->brick_n, 0, sizeof(unsigned long long), ctx->stream));
+    repair_dirty(ctx, g, view(ctx->Q, ctx->g), ctx->P.crit, 1, false);
     CK(cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), ctx->stream));
     CK(cudaGetLastError());
     return DMTZ_OK;
@@ -2938,7 +2954,7 @@ static dmtz_status learned_start(dmtz_ctx *ctx, dmtz_cnn *net, const Grid &g, do
 
 // a round made no progress: reset the values around the remaining mismatched
 // cells (cp = 1) or separatrix records (cp = 0) to the original ones, re-pair
-// there, and clear the request bits (see k_snap_cells)
+// there, and clear the request bits (see k_snap_mask)
 static dmtz_status break_stall(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const PathRec &PR,
                                const FieldState &Qs, int cp, int want_saddles, int64_t nbreaks,
                                const WallRec *WR = nullptr) {
@@ -2959,8 +2975,10 @@ static dmtz_status break_stall(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, 
         k_dilate_axis<<<grid_for(g.V / n), kBlock, 0, st>>>(g, ctx->changed, axis, std::min(radius, n));
     }
     k_snap_mask<<<pgrid, kBlock, 0, st>>>(rc, ctx->changed);
-    repair_dirty(ctx, g, Qs, ctx->P.crit, want_saddles);
+    CK(cudaMemsetAsync(ctx->brick_n, 0, sizeof(unsigned long long), st));
+    repair_dirty(ctx, g, Qs, ctx->P.crit, want_saddles, false);
     k_clear_req<<<pgrid, kBlock, 0, st>>>(ctx->reqlist, ctx->counters + 4, g.V, ctx->reqbits);
+    host_round_end(ctx);
     ctx->launches += 6;
     CK(cudaGetLastError());
     return DMTZ_OK;
@@ -2989,6 +3007,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     CK(cudaSetDevice(ctx->device));
     if ((s = ensure(ctx, g)) != DMTZ_OK) return s;
     cudaStream_t st = ctx->stream;
+    if (!ctx->report) CK(cudaHostAlloc((void **)&ctx->report, 8 * sizeof(unsigned long long), cudaHostAllocDefault));
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
@@ -3014,6 +3033,8 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     CK(cudaMemsetAsync(ctx->errword, 0, sizeof(int), st));
     CK(cudaMemsetAsync(ctx->changed, 0, (size_t)g.V, st));
     CK(cudaMemsetAsync(ctx->counters, 0, 8 * sizeof(unsigned long long), st));
+    CK(cudaMemsetAsync(ctx->counters + 20, 0, 11 * sizeof(unsigned long long), st));
+    CK(cudaMemsetAsync(ctx->brick_n, 0, sizeof(unsigned long long), st));
     const FieldState Ps = view(ctx->P, ctx->f), Qs = view(ctx->Q, ctx->g);
     run_pairing(ctx, g, Ps, nullptr, 1);
     if (pvp == 1 && (s = prep_paths(ctx, g)) != DMTZ_OK) return s;
@@ -3024,10 +3045,10 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         k_filter<<<grid_for(g.V), kBlock, 0, st>>>(g, ctx->P.crit, ctx->f, ctx->g, bound);
         ctx->launches++;
     }
+    ctx->path_keep = pvp == 1 && !conn;
     run_pairing(ctx, g, Qs, ctx->P.crit, 1);
     k_fill_i32<<<grid_for(g.V), kBlock, 0, st>>>(ctx->cnt, 1, g.V);
     ctx->launches++;
-    if (pvp == 1 && !conn && (s = init_path_flags(ctx, g)) != DMTZ_OK) return s;
     pt_.end();
     unsigned long long hc[8];
     auto read_counts = [&]() -> dmtz_status {
@@ -3035,12 +3056,13 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         CK(cudaStreamSynchronize(st));
         return DMTZ_OK;
     };
-    // counts after a mismatch scan; lists that overflowed grow and are rebuilt
+    // counts after a round's end; lists that overflowed grow and are rebuilt
     auto read_fit = [&](int want_saddles) -> dmtz_status {
-        dmtz_status q = read_counts();
-        return q != DMTZ_OK ? q : fit_lists(ctx, g, want_saddles, hc);
+        CK(cudaStreamSynchronize(st));
+        for (int k = 0; k < 8; k++) hc[k] = ctx->report[k];
+        return fit_lists(ctx, g, want_saddles, hc);
     };
-    if ((s = read_fit(1)) != DMTZ_OK) return s;
+    if ((s = read_counts()) != DMTZ_OK || (s = fit_lists(ctx, g, 1, hc)) != DMTZ_OK) return s;
     dmtz_report R;
     memset(&R, 0, sizeof(R));
     for (int k = 0; k < 4; k++) R.initial_mismatch[k] = (int64_t)hc[k];
@@ -3048,13 +3070,15 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         pt_.begin(PH_SETUP);
         if ((s = learned_start(ctx, net, g, bound)) != DMTZ_OK) return s;
         pt_.end();
-        if ((s = read_fit(1)) != DMTZ_OK) return s;
+        if ((s = read_counts()) != DMTZ_OK || (s = fit_lists(ctx, g, 1, hc)) != DMTZ_OK) return s;
     }
     i64 cc[4] = {(i64)hc[0], (i64)hc[1], (i64)hc[2], (i64)hc[3]};
     i64 n_as = 1, n_ds = 1, n_wall = 1;
-    // every scan of the loop asks for saddles when preserve_saddles = 1: the
-    // repairs can then rebuild the lists from the re-paired bricks alone
-    ctx->inc_scan = ps == 1 ? 1 : 0;
+    // every scan of the loop asks for saddles when preserve_saddles = 1, and none
+    // does in runs without separatrix rounds otherwise: the repairs can then rebuild
+    // the lists from the re-paired bricks alone
+    ctx->inc_scan = ps == 1 || pvp == 0 ? 1 : 0;
+    const i64 heavy = heavy_cells(ctx, g);
     i64 rounds = 0;
     int converged = 1;
     const unsigned pgrid = persistent_grid();
@@ -3074,7 +3098,9 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         c.outer = 1;
         c.break_stalls = opts->break_stalls ? 1 : 0;
         for (int k = 0; k < 4; k++) c.cc[k] = cc[k];
-        c.state = cp_any() ? LS_CP : (pvp ? LS_PDF : LS_DONE);
+        c.heavy = heavy;
+        auto cp_state = [&](i64 cells) { return cells >= heavy ? LS_CPF : LS_CP; };
+        c.state = cp_any() ? cp_state(cc[0] + cc[1] + cc[2] + cc[3]) : (pvp ? LS_PDF : LS_DONE);
         LoopCtl fin = c;
         if (c.state != LS_DONE) {
             pt_.begin(PH_PAIR);
@@ -3087,11 +3113,11 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
                 // a scan outgrew a list: grow it, rebuild the lists and resume
                 unsigned long long h4[4];
                 for (int k = 0; k < 4; k++) h4[k] = (unsigned long long)fin.cc[k];
-                if ((s = fit_lists(ctx, g, fin.last == LS_CP ? (ps == 1) : 1, h4)) != DMTZ_OK) return s;
+                if ((s = fit_lists(ctx, g, fin.last == LS_CP || fin.last == LS_CPF ? (ps == 1) : 1, h4)) != DMTZ_OK) return s;
                 cur = fin;
                 cur.overflow = 0;
                 if (fin.stalled) {  // the round changed nothing: break the stall, then go on
-                    const int cpst = fin.last == LS_CP;
+                    const int cpst = fin.last == LS_CP || fin.last == LS_CPF;
                     if ((s = break_stall(ctx, g, rc, PR, Qs, cpst, cpst ? (ps == 1) : 1, R.stall_breaks)) != DMTZ_OK)
                         return s;
                     R.stall_breaks++;
@@ -3100,9 +3126,9 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
                     for (int k = 0; k < 4; k++) cur.cc[k] = (long long)hc[k];
                     const bool any = hc[0] || hc[1] || hc[2] || hc[3];
                     if (cpst) {  // on with the critical-point loop, or to a separatrix round
-                        cur.state = any ? LS_CP : (pvp ? LS_PDF : LS_DONE);
+                        cur.state = any ? cp_state(hc[0] + hc[1] + hc[2] + hc[3]) : (pvp ? LS_PDF : LS_DONE);
                     } else {  // a new outer iteration, or the separatrix re-check
-                        cur.state = any ? LS_CP : LS_PCHECK;
+                        cur.state = any ? cp_state(hc[0] + hc[1] + hc[2] + hc[3]) : LS_PCHECK;
                         if (any) cur.outer++;
                     }
                     if (cur.state == LS_DONE) {
@@ -3112,13 +3138,15 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
                 }
             }
             pt_.end();
-            // kernels per body run: switch + control, plus each state's own
+            // kernels per body run: switch + round's end, plus each state's own: a
+            // fix round is fix + update, then the repair (compaction, gradient, and
+            // the scan where the lists are not rebuilt), or the whole gradient
             const int64_t det = detect_kernels(ctx, conn);  // separatrix detection kernels
-            // a fix round: fix + update, then the repair (dirty marks, compaction,
-            // fresh marks, the gradient, the list rebuild)
-            const int64_t rnd = 2 + 2 + (ctx->inc_scan ? 1 : 0) + 1 + (ctx->inc_scan ? 3 : 1);
-            ctx->launches += 2 * (fin.runs[0] + fin.runs[1] + fin.runs[2] + fin.runs[3]) + rnd * fin.runs[LS_CP] +
-                             (rnd + det) * fin.runs[LS_PDF] + det * fin.runs[LS_PCHECK] + rnd * fin.runs[LS_PFIX];
+            const int64_t rnd = 2 + 2 + (ctx->inc_scan ? 0 : 1);
+            int64_t bodies = 0;
+            for (int k = 0; k < LS_STATES; k++) bodies += fin.runs[k];
+            ctx->launches += 2 * bodies + rnd * fin.runs[LS_CP] + (rnd + det) * fin.runs[LS_PDF] + det * fin.runs[LS_PCHECK] +
+                             rnd * fin.runs[LS_PFIX] + 3 * fin.runs[LS_CPF];
         }
         R.outer_iterations = fin.outer;
         R.cp_rounds = fin.cp_rounds;
@@ -3142,17 +3170,25 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             rounds++;
             R.cp_rounds++;
             paths_fresh = false;
-            CK(cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), st));
-            CK(cudaMemsetAsync(ctx->counters + 7, 0, sizeof(unsigned long long), st));
+            const bool full = cc[0] + cc[1] + cc[2] + cc[3] >= heavy;
             pt_.begin(PH_FIXCP);
             k_fix_cp<<<pgrid, kBlock, 0, st>>>(rc, cp_lists(ctx), ps);
             pt_.end();
             pt_.begin(PH_APPLY);
-            k_apply<<<pgrid, kBlock, 0, st>>>(rc, range, pt, 1, ctx->changed, nullptr);
+            k_apply<<<pgrid, kBlock, 0, st>>>(rc, range, pt, 1, ctx->changed, nullptr, full ? BrickMarks{} : brick_marks(ctx, g));
             pt_.end();
             ctx->launches += 2;
             pt_.begin(PH_PAIR);
-            repair_dirty(ctx, g, Qs, ctx->P.crit, ps == 1);
+            if (full) {  // lists in place: nothing to take back
+                repair_full(ctx, g, Qs, ctx->P.crit, ps == 1);
+                const int inc = ctx->inc_scan;
+                ctx->inc_scan = 0;
+                host_round_end(ctx);
+                ctx->inc_scan = inc;
+            } else {
+                repair_dirty(ctx, g, Qs, ctx->P.crit, ps == 1, true);
+                host_round_end(ctx);
+            }
             pt_.end();
             if ((s = read_fit(ps == 1)) != DMTZ_OK) return s;
             if (opts->break_stalls && hc[7] == 0 && rounds < max_rounds && (hc[0] || hc[1] || hc[2] || hc[3])) {
@@ -3178,8 +3214,6 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         }
         const i64 walls_fixed = walls ? n_wall : 0;
         paths_fresh = false;
-        CK(cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), st));
-        CK(cudaMemsetAsync(ctx->counters + 7, 0, sizeof(unsigned long long), st));
         pt_.begin(PH_FIXPATH);
         k_fix_path<<<pgrid, kBlock, 0, st>>>(rc, PR);
         if (walls_fixed > 0) {
@@ -3188,11 +3222,12 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         }
         pt_.end();
         pt_.begin(PH_APPLY);
-        k_apply<<<pgrid, kBlock, 0, st>>>(rc, range, pt, 1, ctx->changed, nullptr);
+        k_apply<<<pgrid, kBlock, 0, st>>>(rc, range, pt, 1, ctx->changed, nullptr, brick_marks(ctx, g));
         pt_.end();
         ctx->launches += 2;
         pt_.begin(PH_PAIR);
-        repair_dirty(ctx, g, Qs, ctx->P.crit, 1);
+        repair_dirty(ctx, g, Qs, ctx->P.crit, 1, true);
+        host_round_end(ctx);
         pt_.end();
         if ((s = read_fit(1)) != DMTZ_OK) return s;
         if (opts->break_stalls && hc[7] == 0 && rounds < max_rounds && hc[5] + hc[6] + walls_fixed > 0) {

@@ -270,7 +270,8 @@ __host__ __device__ __forceinline__ void take_lower(uint64_t &bk, uint32_t &sel,
 //        vertex's pair where the vertex is the edge's higher-id end
 //   w.y: pointing bits, B layout; bits 12..23: order bits, B layout; bits
 //        24..30: the family where the vertex is the lower-id end
-//   w.z: order bits of its edges, A layout
+//   w.z: order bits of its edges, A layout; bit 24: its steepest descent is not
+//        the original's (set by the kernels that keep PathFlags)
 //   w.w: pointing bits of its triangles; bits 24..29: tetrahedron order bits (2 3)
 //   w4:  tetrahedron order bits
 // km, k0, kp: the anchor's key in the planes z-1, z, z+1, rows ROW apart.
@@ -351,13 +352,14 @@ __host__ __device__ __forceinline__ StarWords grad_stage1(const uint64_t *km, co
 // The choice of the triangles and tetrahedra of one anchor:
 //   pa: the paired edge of each triangle, A layout; bits 24..30: edges (by
 //       family) paired with their vertex; bit 31: the vertex is critical
-//   pb: the same, B layout; bits 12..23: triangles paired with an edge
+//   pb: the same, B layout; bits 12..23: triangles paired with an edge; bits
+//       24..30 (TRACK): edges (by family) with an end whose descent differs
 //   r:  the paired facet of each tetrahedron
 // w: words of the plane z (w0) and z + 1 (w1) at the anchor, rows ROW apart.
 struct CellWords {
     uint32_t pa, pb, r;
 };
-template <int ROW>
+template <int ROW, bool TRACK = false>
 __host__ __device__ __forceinline__ CellWords grad_stage2(const uint4 *w0, const uint4 *w1, const uint32_t *f0,
                                                           const uint32_t *f1) {
     const uint4 a = w0[0], ax = w0[1], ay = w0[ROW], az = w1[0], ayz = w1[ROW];
@@ -406,6 +408,15 @@ __host__ __device__ __forceinline__ CellWords grad_stage2(const uint4 *w0, const
         const uint32_t vcrit = ((a.x | a.y) & 0x7F000000u) ? 0u : 0x80000000u;
         o.pa = p0 | (p1 << 12) | (vclaim << v) | vcrit;
         o.pb = p2 | ((p0 | p1 | p2) << 12);
+        if (TRACK) {
+            uint32_t d = 0;
+            if (a.z >> 24) d |= cxt::edges_at(0);
+            if (ax.z >> 24) d |= cxt::edges_at(1);
+            if (ay.z >> 24) d |= cxt::edges_at(2);
+            if (az.z >> 24) d |= cxt::edges_at(4);
+            if (ayz.z >> 24) d |= cxt::edges_at(6);
+            o.pb |= d << 24;
+        }
     }
     {   // tetrahedra, the same with four corners (labels = id order); garbage above
         // bit 5 of the shifted vectors is masked by s
@@ -532,16 +543,91 @@ __device__ __forceinline__ void brick_coords(const BrickList &bl, i64 b, int &bx
     }
 }
 
+// ---------------------------------------------------------------------------
+// Cell codes: anchor vertex * 32 + the cell's bit of FieldState::crit (0 the
+// vertex, 1..7 edges, 8..19 triangles, 20..25 tetrahedra).
+__host__ __device__ __forceinline__ i64 cell_code(i64 anchor, int bit) { return anchor * 32 + bit; }
+
+// The lists of mismatched cells (criticality differs between the two
+// gradients), by kind: min, 1-saddle, 2-saddle, max.
+struct Lists {
+    i64 *l[4];                  // cell codes
+    unsigned long long *n;      // 4 counters
+    i64 cap[4];                 // capacities; a counter above its capacity = overflow,
+                                // the host grows the list and scans again
+};
+// every lane of a warp appends the mismatched cells d (bits of
+// FieldState::crit) of its anchor v, with one atomic per kind and warp
+__device__ __forceinline__ void push_warp(const Lists &L, i64 v, uint32_t d) {
+    const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
+    if (!__any_sync(full, d != 0)) return;
+    const unsigned long long mine = (unsigned long long)(d & 1u) | ((unsigned long long)__popc(d & 0xFEu) << 16) |
+                                    ((unsigned long long)__popc(d & 0xFFF00u) << 32) |
+                                    ((unsigned long long)__popc(d & 0x3F00000u) << 48);
+    unsigned long long incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(full, incl, o);
+        if (lane >= (unsigned)o) incl += y;
+    }
+    const unsigned long long total = __shfl_sync(full, incl, 31);
+    const unsigned cnt = lane < 4 ? (unsigned)(total >> (16 * lane)) & 0xFFFFu : 0u;
+    unsigned long long base = 0;
+    if (cnt) base = atomicAdd(&L.n[lane], (unsigned long long)cnt);
+    const unsigned long long excl = incl - mine;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        unsigned long long at = __shfl_sync(full, base, k) + ((excl >> (16 * k)) & 0xFFFFull);
+        const uint32_t kind = k == 0 ? 1u : k == 1 ? 0xFEu : k == 2 ? 0xFFF00u : 0x3F00000u;
+        for (uint32_t m = d & kind; m; m &= m - 1, at++)
+            if ((i64)at < L.cap[k]) L.l[k][at] = cell_code(v, __ffs(m) - 1);
+    }
+}
+
 // Separatrix flags of the bricks (see k_path_detect), refreshed with a brick's gradient.
 struct PathFlags {
     uint8_t *as, *ds;            // per brick; nullptr: not kept
-    const uint32_t *tcP, *critP; // original tetrahedron codes with path bits (18 + slot), original criticality
+    const uint32_t *tcP;         // original tetrahedron codes with path bits (18 + slot)
     const uint8_t *pvP;          // original steepest descent
+};
+// What a gradient kernel does with its anchors besides storing their state
+struct GradOps {
+    PathFlags F;
+    Lists T;               // receives the anchors' mismatched cells
+    const uint32_t *critP; // original criticality; nullptr: no flags, no lists
+    uint32_t want;         // cell bits the lists take (0: no lists)
 };
 // does a tetrahedron on an original path pair differently?
 __host__ __device__ __forceinline__ bool tet_path_differs(uint32_t tcP, uint32_t tcQ) {
     const uint32_t x = tcP ^ tcQ, on = tcP >> 18;
     return on && ((x | (x >> 1) | (x >> 2)) & 0x9249u & spread3(on));
+}
+
+// Incremental mismatch lists.  A cell's mismatch status changes only where its
+// anchor's criticality is recomputed, i.e. in the repair's bricks (marked
+// fresh).  The new lists are the old entries outside fresh bricks, appended by
+// some extra blocks of the repair, plus what the repair itself finds.  Valid when every scan of
+// the run uses the same saddle flag and the old lists were complete (an
+// overflow is followed by a full scan before the next round).
+struct KeepOps {
+    Lists L;               // the old lists
+    const uint8_t *fresh;  // per brick
+    int shx, shy, shz, nbx, nby;
+    unsigned blocks;       // extra blocks; 0: nothing to carry over
+};
+__device__ __forceinline__ void keep_lists(const Grid &g, const GradOps &O, const KeepOps &K, unsigned block) {
+    const bool sad = (O.want & 0xFFFFEu) != 0;  // the run's lists hold saddles
+    const i64 n0 = min((i64)K.L.n[0], K.L.cap[0]), n1 = sad ? min((i64)K.L.n[1], K.L.cap[1]) : 0,
+              n2 = sad ? min((i64)K.L.n[2], K.L.cap[2]) : 0, n3 = min((i64)K.L.n[3], K.L.cap[3]);
+    for (i64 i = (i64)block * blockDim.x + threadIdx.x; i < n0 + n1 + n2 + n3; i += (i64)K.blocks * blockDim.x) {
+        const int k = i < n0 ? 0 : i < n0 + n1 ? 1 : i < n0 + n1 + n2 ? 2 : 3;
+        const i64 code = K.L.l[k][i - (k > 0 ? n0 : 0) - (k > 1 ? n1 : 0) - (k > 2 ? n2 : 0)];
+        int x, y, z;
+        decode_v(g, code >> 5, x, y, z);
+        if (K.fresh[(x >> K.shx) + (i64)K.nbx * ((y >> K.shy) + (i64)K.nby * (z >> K.shz))]) continue;
+        const unsigned long long at = agg_slot(&O.T.n[k]);
+        if ((i64)at < O.T.cap[k]) O.T.l[k][at] = code;
+    }
 }
 
 // The gradient of the listed bricks, one block per brick step.  One thread per
@@ -554,7 +640,8 @@ __host__ __device__ constexpr int brick_threads() {
 }
 template <int SX, int SY, int SZ>
 __global__ void __launch_bounds__((brick_threads<SX, SY, SZ>()), SX == 8 ? 3 : 2) k_grad_bricks(Grid g, FieldState s, BrickList bl,
-                                                                                        PathFlags F) {
+                                                                                        const __grid_constant__ GradOps O,
+                                                                                        const __grid_constant__ KeepOps K) {
     static_assert(SX * SY * SZ == DMTZ_BRICK, "a brick is 128 anchors");
     constexpr int NT = brick_threads<SX, SY, SZ>();
     constexpr int KX = SX + 4, KY = SY + 4, KZ = SZ + 4, NK = KX * KY * KZ;  // keys: two layers around
@@ -564,14 +651,17 @@ __global__ void __launch_bounds__((brick_threads<SX, SY, SZ>()), SX == 8 ? 3 : 2
     __shared__ uint4 sw[NW];
     __shared__ uint32_t sf[NW];
     __shared__ CellWords sc[NC];
-    __shared__ uint8_t sp[NW], sq[NW];  // steepest descent of this field and of the original one
     __shared__ uint32_t flag;  // bit 0: as, bit 1: ds
     const int t = threadIdx.x;
     const int wx = t % WX, wy = (t / WX) % WY, wz = t / (WX * WY);
     const int cx = t % CX, cy = (t / CX) % CY, cz = t / (CX * CY);
     const int ox = t % SX, oy = (t / SX) % SY, oz = t / (SX * SY);
+    if (blockIdx.x >= gridDim.x - K.blocks) {  // the blocks that carry the old lists over
+        keep_lists(g, O, K, blockIdx.x - (gridDim.x - K.blocks));
+        return;
+    }
     const i64 n = brick_count(bl);
-    for (i64 b = blockIdx.x; b < n; b += gridDim.x) {
+    for (i64 b = blockIdx.x; b < n; b += gridDim.x - K.blocks) {
         int bx, by, bz;
         brick_coords(bl, b, bx, by, bz);
         const int x0 = bx * SX, y0 = by * SY, z0 = bz * SZ;
@@ -580,27 +670,25 @@ __global__ void __launch_bounds__((brick_threads<SX, SY, SZ>()), SX == 8 ? 3 : 2
             const bool in = ux >= 0 && uy >= 0 && uz >= 0 && ux < g.W && uy < g.H && uz < g.D;
             sk[e] = in ? okey(s.val[ux + (i64)uy * g.W + (i64)uz * g.WH]) : kKeyAbsent;
         }
-        // what the path flags compare with, loaded with the keys
+        // what the flags and lists compare with, loaded with the keys
         uint32_t tcP = 0, critP = 0;
-        if (F.as) {
+        int pvP = 15;
+        if (O.critP) {
             const int x = x0 + wx - 1, y = y0 + wy - 1, z = z0 + wz - 1;
-            if (t < NW) {
-                const bool in = x >= 0 && y >= 0 && z >= 0 && x < g.W && y < g.H && z < g.D;
-                sq[t] = in ? F.pvP[x + (i64)y * g.W + (i64)z * g.WH] : (uint8_t)15;
-            }
+            if (O.F.as && t < NW && x >= 0 && y >= 0 && z >= 0 && x < g.W && y < g.H && z < g.D)
+                pvP = O.F.pvP[x + (i64)y * g.W + (i64)z * g.WH];
             if (t < DMTZ_BRICK && x0 + ox < g.W && y0 + oy < g.H && z0 + oz < g.D) {
                 const i64 v = (x0 + ox) + (i64)(y0 + oy) * g.W + (i64)(z0 + oz) * g.WH;
-                tcP = F.tcP[v];
-                critP = F.critP[v];
+                if (O.F.as) tcP = O.F.tcP[v];
+                critP = O.critP[v];
             }
         }
         __syncthreads();
         if (t < NW) {
             const uint64_t *k0 = sk + (wx + 1) + KX * ((wy + 1) + KY * (wz + 1));
             const StarWords w = grad_stage1<KX>(k0 - KX * KY, k0, k0 + KX * KY);
-            sw[t] = make_uint4(w.x, w.y, w.z, w.w);
+            sw[t] = make_uint4(w.x, w.y, w.z | (pvP != 15 && pvP != w.pv ? 1u << 24 : 0u), w.w);
             sf[t] = w.w4;
-            sp[t] = (uint8_t)w.pv;
             const int x = x0 + wx - 1, y = y0 + wy - 1, z = z0 + wz - 1;
             if (wx >= 1 && wy >= 1 && wz >= 1 && wx <= SX && wy <= SY && wz <= SZ && x < g.W && y < g.H && z < g.D)
                 s.pv[x + (i64)y * g.W + (i64)z * g.WH] = (uint8_t)w.pv;
@@ -609,41 +697,33 @@ __global__ void __launch_bounds__((brick_threads<SX, SY, SZ>()), SX == 8 ? 3 : 2
         if (t < NC) {
             if (t == 0) flag = 0;
             const int i = cx + WX * (cy + WY * cz);
-            sc[t] = grad_stage2<WX>(sw + i, sw + i + WX * WY, sf + i, sf + i + WX * WY);
+            sc[t] = grad_stage2<WX, true>(sw + i, sw + i + WX * WY, sf + i, sf + i + WX * WY);
         }
         __syncthreads();
         if (t < DMTZ_BRICK) {
             const int x = x0 + ox, y = y0 + oy, z = z0 + oz;
+            const i64 v = x + (i64)y * g.W + (i64)z * g.WH;
+            uint32_t differ = 0;
             if (x < g.W && y < g.H && z < g.D) {
                 const int i = (ox + 1) + CX * ((oy + 1) + CY * (oz + 1));
                 const uint32_t last = (x == g.W - 1 ? 1u : 0u) | (y == g.H - 1 ? 2u : 0u) | (z == g.D - 1 ? 4u : 0u);
                 const AnchorOut o = grad_stage3<CX>(sc + i - CX * CY, sc + i, last);
-                const i64 v = x + (i64)y * g.W + (i64)z * g.WH;
                 s.eup[v] = o.eup;
                 s.fup[v] = o.fup;
                 if (s.crit) s.crit[v] = o.crit;
                 if (s.tcode) s.tcode[v] = o.tcode;
-                if (F.as) {
-                    // an original 1-saddle with an endpoint whose descent differs: the
-                    // anchor and the corners its edges reach
-                    const uint32_t m = (critP >> 1) & 0x7Fu;
-                    uint32_t differ = 0;  // bit per corner
-                    DMTZ_FOR(5, C, {
-                        constexpr int c = decltype(C)::value == 3 ? 4 : decltype(C)::value == 4 ? 6 : decltype(C)::value;
-                        const int i = (ox + 1 + cxt::ccx(c)) + WX * ((oy + 1 + cxt::ccy(c)) + WY * (oz + 1 + cxt::ccz(c)));
-                        if (sq[i] != 15 && sq[i] != sp[i]) differ |= cxt::edges_at(c);
-                    });
-                    const uint32_t f = (tet_path_differs(tcP, o.tcode) ? 1u : 0u) | ((m & differ) ? 2u : 0u);
-                    if (f) atomicOr(&flag, f);
-                }
+                differ = (o.crit ^ critP) & O.want;
+                const uint32_t f = (tet_path_differs(tcP, o.tcode) ? 1u : 0u) | (((critP >> 1) & (sc[i].pb >> 24) & 0x7Fu) ? 2u : 0u);
+                if (f) atomicOr(&flag, f);
             }
+            if (O.want) push_warp(O.T, v, differ);
         }
-        if (F.as) {
+        if (O.F.as) {
             __syncthreads();
             if (t == 0) {
                 const i64 b = bx + (i64)bl.nbx * (by + (i64)bl.nby * bz);
-                F.as[b] = (uint8_t)(flag & 1u);
-                F.ds[b] = (uint8_t)(flag >> 1);
+                O.F.as[b] = (uint8_t)(flag & 1u);
+                O.F.ds[b] = (uint8_t)(flag >> 1);
             }
         }
         // the next brick's keys may land now: stage 1 of this one is behind two
@@ -667,8 +747,11 @@ struct March {
     static constexpr size_t smem = 4 * NK * sizeof(uint64_t) + 3 * NW * (sizeof(uint4) + sizeof(uint32_t)) +
                                    3 * NC * sizeof(CellWords);
 };
-template <int TX, int TY, int MINB>
-__global__ void __launch_bounds__((March<TX, TY>::NT), MINB) k_grad_march(Grid g, FieldState s, int ntx, int nty, int chunk) {
+// TRACK: flags and lists as GradOps says (brick flags zero at launch).
+template <int TX, int TY, int MINB, bool TRACK>
+__global__ void __launch_bounds__((March<TX, TY>::NT), MINB) k_grad_march(Grid g, FieldState s, int ntx, int nty, int chunk,
+                                                                          const __grid_constant__ GradOps O, int shx, int shy, int shz, int nbx,
+                                                                          int nby) {
     using M = March<TX, TY>;
     constexpr int KX = M::KX, NK = M::NK, WX = M::WX, NW = M::NW, CX = M::CX, NC = M::NC, NT = M::NT, NL = M::NL;
     extern __shared__ __align__(16) unsigned char march_smem[];
@@ -700,6 +783,7 @@ __global__ void __launch_bounds__((March<TX, TY>::NT), MINB) k_grad_march(Grid g
     const int wx = t % WX, wy = t / WX, ki = (wx + 1) + KX * (wy + 1);
     const bool pv_in = t < NW && wx >= 1 && wy >= 1 && wx <= TX && wy <= TY && x0 + wx - 1 < g.W && y0 + wy - 1 < g.H;
     const i64 pv_col = (x0 + wx - 1) + (i64)(y0 + wy - 1) * g.W;
+    const bool st1_in = t < NW && x0 + wx >= 1 && y0 + wy >= 1 && x0 + wx - 1 < g.W && y0 + wy - 1 < g.H;
     // stage 2 and stage 3 columns
     const int wi = t % CX + WX * (t / CX);
     const int ox = t % TX, oy = t / TX, x = x0 + ox, y = y0 + oy, ci = (ox + 1) + CX * (oy + 1);
@@ -712,24 +796,48 @@ __global__ void __launch_bounds__((March<TX, TY>::NT), MINB) k_grad_march(Grid g
         uint64_t nk[NL];
 #pragma unroll
         for (int l = 0; l < NL; l++) nk[l] = p < z1 ? load_key(l, p + 2) : kKeyAbsent;
+        // what the flags and lists compare with
+        const i64 v3 = out_col + (i64)(p - 3) * g.WH;
+        int pvP = 15;
+        uint32_t tcP = 0, critP = 0;
+        if (TRACK) {
+            if (O.F.as && st1_in && p >= 0 && p < g.D) pvP = O.F.pvP[pv_col + (i64)p * g.WH];
+            if (p - 3 >= z0 && out_in) {
+                if (O.F.as) tcP = O.F.tcP[v3];
+                critP = O.critP[v3];
+            }
+        }
         const int s3m1 = s3 == 0 ? 2 : s3 - 1, s3m2 = s3m1 == 0 ? 2 : s3m1 - 1;  // slots of planes p - 1, p - 2
         if (p <= z1 && t < NW) {
             const StarWords w = grad_stage1<KX>(sk + ((s4 + 2) & 3) * NK + ki, sk + ((s4 + 3) & 3) * NK + ki, sk + s4 * NK + ki);
-            sw[s3 * NW + t] = make_uint4(w.x, w.y, w.z, w.w);
+            sw[s3 * NW + t] = make_uint4(w.x, w.y, w.z | (TRACK && pvP != 15 && pvP != w.pv ? 1u << 24 : 0u), w.w);
             sf[s3 * NW + t] = w.w4;
             if (pv_in && p >= z0 && p < z1) s.pv[pv_col + (i64)p * g.WH] = (uint8_t)w.pv;
         }
         // cell words of plane q live in the slot star words of plane q had
         if (p - 2 >= z0 - 1 && p - 2 < z1 && t < NC)
-            sc[s3m2 * NC + t] = grad_stage2<WX>(sw + s3m2 * NW + wi, sw + s3m1 * NW + wi, sf + s3m2 * NW + wi, sf + s3m1 * NW + wi);
-        if (p - 3 >= z0 && out_in) {  // plane p - 3 in slot s3, plane p - 4 in slot s3m1
+            sc[s3m2 * NC + t] = grad_stage2<WX, TRACK>(sw + s3m2 * NW + wi, sw + s3m1 * NW + wi, sf + s3m2 * NW + wi, sf + s3m1 * NW + wi);
+        if (p - 3 >= z0 && t < TX * TY) {  // plane p - 3 in slot s3, plane p - 4 in slot s3m1
             const int z = p - 3;
-            const AnchorOut o = grad_stage3<CX>(sc + s3m1 * NC + ci, sc + s3 * NC + ci, last_xy | (z == g.D - 1 ? 4u : 0u));
-            const i64 v = out_col + (i64)z * g.WH;
-            s.eup[v] = o.eup;
-            s.fup[v] = o.fup;
-            if (s.crit) s.crit[v] = o.crit;
-            if (s.tcode) s.tcode[v] = o.tcode;
+            uint32_t differ = 0;
+            if (out_in) {
+                const CellWords *c0 = sc + s3 * NC + ci;
+                const AnchorOut o = grad_stage3<CX>(sc + s3m1 * NC + ci, c0, last_xy | (z == g.D - 1 ? 4u : 0u));
+                s.eup[v3] = o.eup;
+                s.fup[v3] = o.fup;
+                if (s.crit) s.crit[v3] = o.crit;
+                if (s.tcode) s.tcode[v3] = o.tcode;
+                if (TRACK) {
+                    differ = (o.crit ^ critP) & O.want;
+                    const bool as = tet_path_differs(tcP, o.tcode), ds = ((critP >> 1) & (c0->pb >> 24) & 0x7Fu) != 0;
+                    if (O.F.as && (as || ds)) {
+                        const i64 b = (x >> shx) + (i64)nbx * ((y >> shy) + (i64)nby * (z >> shz));
+                        if (as) O.F.as[b] = 1;
+                        if (ds) O.F.ds[b] = 1;
+                    }
+                }
+            }
+            if (TRACK && O.want) push_warp(O.T, v3, differ);
         }
         s4 = (s4 + 1) & 3;
 #pragma unroll

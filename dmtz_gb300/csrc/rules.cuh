@@ -395,7 +395,6 @@ __device__ __forceinline__ void load_rule_tab(RuleTab &t) {
 }
 
 enum { KIND_VERTEX = 0, KIND_EDGE, KIND_FACE, KIND_TET };
-__host__ __device__ __forceinline__ i64 cell_code(i64 anchor, int bit) { return anchor * 32 + bit; }
 __host__ __device__ __forceinline__ i64 edge_code(i64 anchor, int k) { return anchor * 32 + 1 + k; }
 __host__ __device__ __forceinline__ i64 face_code(i64 anchor, int s) { return anchor * 32 + 8 + s; }
 __host__ __device__ __forceinline__ i64 tet_code(i64 anchor, int t) { return anchor * 32 + 20 + t; }
