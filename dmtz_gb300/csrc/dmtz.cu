@@ -1239,68 +1239,83 @@ __global__ void k_filter(Grid g, const uint32_t *crit_o, const double *f, double
 // tetrahedron) its ascending path (is_false's walk, main_3d.cu:4437-4497)
 // reaches, or -1 when the path leaves through the boundary.  Both by pointer
 // jumping: lab <- lab[lab] until nothing changes.
-__global__ void k_desc_init(Grid g, const uint8_t *pv, i64 *lab) {
+//
+// I: int32 where every tetrahedron index fits (below 2^31 / 6 vertices), else int64.
+template <class I>
+__global__ void k_desc_init(Grid g, const uint8_t *pv, I *lab) {
     for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += (i64)gridDim.x * blockDim.x) {
         const int d = pv[v];
-        lab[v] = d == 15 ? v : v + g.doff[d];
+        lab[v] = (I)(d == 15 ? v : v + g.doff[d]);
     }
 }
-__global__ void k_asc_init(Grid g, const uint32_t *tcode, i64 *lab) {
+// one thread per anchor, its six tetrahedra
+template <class I>
+__global__ void __launch_bounds__(kBlock) k_asc_init(Grid g, const uint32_t *tcode, I *lab) {
     __shared__ AscTab tab;
     load_asc_tab(tab);
-    for (i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x; t < 6 * g.V; t += (i64)gridDim.x * blockDim.x) {
-        const i64 v = t / 6;
-        const int ts = (int)(t - 6 * v);
+    for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += (i64)gridDim.x * blockDim.x) {
         int x, y, z;
         decode_v(g, v, x, y, z);
-        if (!cell_ok(g, x, y, z, 1, 1, 1)) {
-            lab[t] = -2;  // no such tetrahedron
-            continue;
+        const bool cube = cell_ok(g, x, y, z, 1, 1, 1);
+        const uint32_t code = tcode[v];
+        I out[6];
+#pragma unroll
+        for (int ts = 0; ts < 6; ts++) {
+            const int j = (code >> (3 * ts)) & 7;
+            int nx = x, ny = y, nz = z, s = ts;
+            if (!cube) out[ts] = -2;                    // no such tetrahedron
+            else if (j == 7) out[ts] = (I)(6 * v + ts); // a maximum
+            else if (!asc_move(g, tab, nx, ny, nz, s, j)) out[ts] = -1;  // leaves through the boundary
+            else out[ts] = (I)((nx + (i64)ny * g.W + (i64)nz * g.WH) * 6 + s);
         }
-        const int j = (tcode[v] >> (3 * ts)) & 7;
-        if (j == 7) {
-            lab[t] = t;  // a maximum
-            continue;
-        }
-        int s = ts;
-        const bool in = asc_move(g, tab, x, y, z, s, j);
-        lab[t] = in ? (x + (i64)y * g.W + (i64)z * g.WH) * 6 + s : -1;  // -1: leaves through the boundary
+#pragma unroll
+        for (int ts = 0; ts < 6; ts++) lab[6 * v + ts] = out[ts];
     }
 }
-__global__ void k_jump(i64 *lab, i64 n, int *changed) {
-    int any = 0;
+// Every label to its root, following at most kHops links per element and
+// call; *unsettled is set when a root was not reached.  A link read while other threads
+// shorten theirs is an older or a newer one of the same path.  (One link per
+// call, and a look at the flag from the host after each: 8-10 calls per label
+// array.)
+constexpr int kHops = 64;
+template <class I>
+__global__ void __launch_bounds__(kBlock) k_jump(I *lab, i64 n, int *unsettled) {
+    int left = 0;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        const i64 l = lab[i];
+        const I l = lab[i];
         if (l < 0) continue;
-        const i64 ll = lab[l];
-        if (ll != l) {
-            lab[i] = ll;
-            any = 1;
+        I r = l;
+        int h = 0;
+        for (; h < kHops && r >= 0; h++) {
+            const I q = lab[r];
+            if (q == r) break;
+            r = q;
         }
+        if (r != l) lab[i] = r;
+        left |= h == kHops;
     }
-    if (__syncthreads_or(any) && threadIdx.x == 0) atomicOr(changed, 1);
+    if (__syncthreads_or(left) && threadIdx.x == 0) atomicOr(unsettled, 1);
 }
-// reference ids of the labels
-__global__ void k_desc_out(Grid g, const i64 *lab, int32_t *out) {
-    for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += (i64)gridDim.x * blockDim.x)
-        out[v] = (int32_t)lab[v];
-}
-__global__ void k_asc_out(Grid g, const i64 *lab, int32_t *out) {
-    for (i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x; t < 6 * g.V; t += (i64)gridDim.x * blockDim.x) {
-        const i64 v = t / 6;
-        const int ts = (int)(t - 6 * v);
+// reference ids of the tetrahedra's labels (a vertex's label is its id)
+template <class I>
+__global__ void k_asc_out(Grid g, const I *lab, int32_t *out) {
+    for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += (i64)gridDim.x * blockDim.x) {
         int x, y, z;
         decode_v(g, v, x, y, z);
         if (!cell_ok(g, x, y, z, 1, 1, 1)) continue;
-        const i64 l = lab[t];
-        int32_t r = -1;
-        if (l >= 0) {
-            const i64 lv = l / 6;
-            int lx, ly, lz;
-            decode_v(g, lv, lx, ly, lz);
-            r = (int32_t)tet_ref(g, lx, ly, lz, (int)(l - 6 * lv));
+        int32_t *o = out + tet_ref(g, x, y, z, 0);
+#pragma unroll
+        for (int ts = 0; ts < 6; ts++) {
+            const I l = lab[6 * v + ts];
+            int32_t r = -1;
+            if (l >= 0) {
+                const i64 lv = l / 6;
+                int lx, ly, lz;
+                decode_v(g, lv, lx, ly, lz);
+                r = (int32_t)tet_ref(g, lx, ly, lz, (int)(l - 6 * lv));
+            }
+            o[ts] = r;
         }
-        out[tet_ref(g, x, y, z, ts)] = r;
     }
 }
 
@@ -1516,6 +1531,10 @@ struct dmtz_ctx {
     std::vector<dmtz_ctx *> pool;  // worker contexts of dmtz_correct_batch
     uint8_t *mm = nullptr;         // mismatch bytes of the learned proposal's features
     i64 capMM = 0;
+    // results of the calls that hand arrays to the host (pairing arrays, labels):
+    // kept between calls up to kWorkKeep bytes, so that a call neither maps nor unmaps memory
+    unsigned char *work = nullptr;
+    size_t work_bytes = 0;
     unsigned long long *report = nullptr;  // pinned: counts of the last round (k_round_end), hc's layout
     int march_blocks = 0;          // blocks of k_grad_march the device holds at once (0: not asked yet)
     void *loopctl = nullptr;       // device copy of the graph loop's control block (kept: a
@@ -1538,6 +1557,29 @@ template <class T>
 cudaError_t dalloc(T **p, i64 n) {
     return cudaMalloc((void **)p, sizeof(T) * (size_t)std::max<i64>(n, 1));
 }
+
+// scratch of one call: take, then cut pieces off it; done gives a large one back
+constexpr size_t kWorkKeep = (size_t)1 << 30;
+cudaError_t work_take(dmtz_ctx *c, size_t bytes) {
+    if (bytes <= c->work_bytes) return cudaSuccess;
+    cudaFree(c->work);
+    c->work = nullptr;
+    c->work_bytes = 0;
+    const cudaError_t e = cudaMalloc((void **)&c->work, bytes);
+    if (e == cudaSuccess) c->work_bytes = bytes;
+    return e;
+}
+void work_done(dmtz_ctx *c) {
+    if (c->work_bytes <= kWorkKeep) return;
+    cudaFree(c->work);
+    c->work = nullptr;
+    c->work_bytes = 0;
+}
+struct WorkDone {  // gives a large scratch back on every way out
+    dmtz_ctx *c;
+    ~WorkDone() { work_done(c); }
+};
+size_t work_round(size_t b) { return (b + 255) / 256 * 256; }
 
 void free_field(DevField &d) {
     cudaFree(d.pv); cudaFree(d.eup); cudaFree(d.fup); cudaFree(d.crit); cudaFree(d.tcode);
@@ -1862,11 +1904,13 @@ void repair_full(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32
 // Lists with at least this many cells mean a repair of the whole grid: their
 // updates reach most bricks then, and the march's halo is smaller (256^3 with 189 k
 // listed cells and 131 k bricks: 96 % of the bricks, 1.81 ms by bricks, 0.9 ms
-// by the march, which is even at half of the bricks).
+// by the march, which is even at half of the bricks).  Below 8192 bricks the march's
+// pipeline costs what all bricks do (64^3, 2048 bricks: 29 us either way; 97 x 61
+// x 75, 3952 bricks: 56 and 53 us), so such grids are always repaired by bricks.
 i64 heavy_cells(const dmtz_ctx *ctx, const Grid &g) {
     i64 nb;
     all_bricks(g, ctx->tune_shape, nb);
-    return grad_marches(ctx, g) ? std::max<i64>(1, nb / 2) : INT64_MAX;
+    return nb >= 8192 ? nb / 2 : INT64_MAX;
 }
 
 double key_to_double(unsigned long long k) {
@@ -2316,8 +2360,9 @@ __global__ void k_link_classes(Grid g, const double *data, uint8_t *out, unsigne
 // ascending labels of its cofaces, in the original field (dP, aP) and in the
 // decompressed one (dQ, aQ).  out: [0] endpoints compared, [1] equal, [2]
 // cofaces compared, [3] equal, [4] anchor cells whose criticality differs.
-__global__ void k_sep_agree(Grid g, const uint32_t *critP, const uint32_t *critQ, const i64 *dP, const i64 *dQ,
-                            const i64 *aP, const i64 *aQ, unsigned long long *out) {
+template <class I>
+__global__ void k_sep_agree(Grid g, const uint32_t *critP, const uint32_t *critQ, const I *dP, const I *dQ,
+                            const I *aP, const I *aQ, unsigned long long *out) {
     unsigned long long c[5] = {0, 0, 0, 0, 0};
     for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < g.V; v += (i64)gridDim.x * blockDim.x) {
         const uint32_t cp = critP[v];
@@ -2385,6 +2430,7 @@ void dmtz_ctx_destroy(dmtz_ctx *ctx) {
     free_all(ctx);
     cudaFree(ctx->mm);
     cudaFree(ctx->loopctl);
+    cudaFree(ctx->work);
     cudaFreeHost(ctx->report);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->side) cudaStreamDestroy(ctx->side);
@@ -2414,13 +2460,16 @@ dmtz_status dmtz_extract(dmtz_ctx *ctx, int W, int H, int D, const double *data,
     run_pairing(ctx, g, fs, nullptr, 1);
     int32_t *d[4];
     const i64 n[4] = {g.V, g.E, g.F, g.T};
-    for (int k = 0; k < 4; k++) CK(dalloc(&d[k], n[k]));
+    size_t at[5] = {0, 0, 0, 0, 0};
+    for (int k = 0; k < 4; k++) at[k + 1] = at[k] + work_round(sizeof(int32_t) * (size_t)n[k]);
+    WorkDone done{ctx};
+    CK(work_take(ctx, at[4]));
+    for (int k = 0; k < 4; k++) d[k] = reinterpret_cast<int32_t *>(ctx->work + at[k]);
     k_export<<<grid_for(g.V), kBlock, 0, ctx->stream>>>(g, fs, d[0], d[1], d[2], d[3]);
     int32_t *h[4] = {PV, PE, PF, PT};
     for (int k = 0; k < 4; k++)
         CK(cudaMemcpyAsync(h[k], d[k], sizeof(int32_t) * (size_t)n[k], cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    for (int k = 0; k < 4; k++) cudaFree(d[k]);
     CK(cudaGetLastError());
     return DMTZ_OK;
 }
@@ -3362,18 +3411,22 @@ dmtz_status dmtz_features(dmtz_ctx *ctx, int W, int H, int D, const double *orig
     return DMTZ_OK;
 }
 
-// pointer jumping to a fixed point; false if it does not settle within the cap
-static dmtz_status jump_to_roots(dmtz_ctx *ctx, i64 *lab, i64 n) {
+}  // extern "C"
+// pointer jumping to a fixed point of several label arrays
+template <class I>
+static dmtz_status jump_to_roots(dmtz_ctx *ctx, I *const *lab, const i64 *n, int arrays) {
     for (int round = 0; round < 64; round++) {
         CK(cudaMemsetAsync(ctx->errword, 0, sizeof(int), ctx->stream));
-        k_jump<<<persistent_grid(), kBlock, 0, ctx->stream>>>(lab, n, ctx->errword);
-        int changed = 0;
-        CK(cudaMemcpyAsync(&changed, ctx->errword, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        for (int k = 0; k < arrays; k++)
+            k_jump<I><<<persistent_grid(), kBlock, 0, ctx->stream>>>(lab[k], n[k], ctx->errword);
+        int left = 0;
+        CK(cudaMemcpyAsync(&left, ctx->errword, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        if (!changed) return DMTZ_OK;
+        if (!left) return DMTZ_OK;
     }
     return fail(ctx, DMTZ_ERR_CYCLE, "manifold labels did not settle (cycle in the gradient paths)");
 }
+extern "C" {
 
 dmtz_status dmtz_labels(dmtz_ctx *ctx, int W, int H, int D, const double *data, int on_device, int32_t *desc,
                         int32_t *asc) {
@@ -3385,30 +3438,58 @@ dmtz_status dmtz_labels(dmtz_ctx *ctx, int W, int H, int D, const double *data, 
     if ((s = ensure(ctx, g)) != DMTZ_OK) return s;
     if ((s = upload(ctx, ctx->f, data, g.V, on_device)) != DMTZ_OK) return s;
     run_pairing(ctx, g, view(ctx->P, ctx->f), nullptr, 1);
-    i64 *dl = nullptr, *al = nullptr;
-    int32_t *dout = nullptr, *aout = nullptr;
-    CK(dalloc(&dl, g.V));
-    CK(dalloc(&al, 6 * g.V));
-    CK(dalloc(&dout, g.V));
-    CK(dalloc(&aout, g.T));
+    // int32 labels: 6 V is below F, and F below 2^31, but for columns of 2 x 2 vertices, which
+    // are short.  The vertices' labels are the result itself.
+    const size_t nd = work_round(sizeof(int32_t) * (size_t)g.V), na = work_round(sizeof(int32_t) * 6 * (size_t)g.V);
+    WorkDone done{ctx};
+    CK(work_take(ctx, nd + 2 * na));
+    int32_t *dl = reinterpret_cast<int32_t *>(ctx->work), *al = reinterpret_cast<int32_t *>(ctx->work + nd),
+            *aout = reinterpret_cast<int32_t *>(ctx->work + nd + na);
     const unsigned pg = persistent_grid();
-    k_desc_init<<<pg, kBlock, 0, ctx->stream>>>(g, ctx->P.pv, dl);
-    k_asc_init<<<pg, kBlock, 0, ctx->stream>>>(g, ctx->P.tcode, al);
-    if ((s = jump_to_roots(ctx, dl, g.V)) == DMTZ_OK) s = jump_to_roots(ctx, al, 6 * g.V);
-    if (s == DMTZ_OK) {
-        k_desc_out<<<pg, kBlock, 0, ctx->stream>>>(g, dl, dout);
-        k_asc_out<<<pg, kBlock, 0, ctx->stream>>>(g, al, aout);
-        CK(cudaMemcpyAsync(desc, dout, sizeof(int32_t) * (size_t)g.V, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaMemcpyAsync(asc, aout, sizeof(int32_t) * (size_t)g.T, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-    }
-    cudaFree(dl);
-    cudaFree(al);
-    cudaFree(dout);
-    cudaFree(aout);
+    k_desc_init<int32_t><<<pg, kBlock, 0, ctx->stream>>>(g, ctx->P.pv, dl);
+    k_asc_init<int32_t><<<pg, kBlock, 0, ctx->stream>>>(g, ctx->P.tcode, al);
+    int32_t *lab[2] = {dl, al};
+    const i64 n[2] = {g.V, 6 * g.V};
+    if ((s = jump_to_roots<int32_t>(ctx, lab, n, 2)) != DMTZ_OK) return s;
+    k_asc_out<int32_t><<<pg, kBlock, 0, ctx->stream>>>(g, al, aout);
+    CK(cudaMemcpyAsync(desc, dl, sizeof(int32_t) * (size_t)g.V, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(asc, aout, sizeof(int32_t) * (size_t)g.T, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaGetLastError());
-    return s;
+    return DMTZ_OK;
 }
+
+}  // extern "C"
+template <class I>
+static dmtz_status agreement(dmtz_ctx *ctx, const Grid &g, int64_t out[5]) {
+    cudaStream_t st = ctx->stream;
+    const size_t nd = work_round(sizeof(I) * (size_t)g.V), na = work_round(sizeof(I) * 6 * (size_t)g.V);
+    WorkDone done{ctx};
+    if (work_take(ctx, 2 * nd + 2 * na + 256) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(ctx, DMTZ_ERR_CUDA, "cannot allocate label buffers");
+    }
+    I *lab[4];
+    const i64 n[4] = {g.V, g.V, 6 * g.V, 6 * g.V};
+    for (int k = 0; k < 4; k++) lab[k] = reinterpret_cast<I *>(ctx->work + (k < 2 ? k * nd : 2 * nd + (k - 2) * na));
+    unsigned long long *cnt = reinterpret_cast<unsigned long long *>(ctx->work + 2 * nd + 2 * na);
+    const unsigned pg = persistent_grid();
+    k_desc_init<I><<<pg, kBlock, 0, st>>>(g, ctx->P.pv, lab[0]);
+    k_desc_init<I><<<pg, kBlock, 0, st>>>(g, ctx->Q.pv, lab[1]);
+    k_asc_init<I><<<pg, kBlock, 0, st>>>(g, ctx->P.tcode, lab[2]);
+    k_asc_init<I><<<pg, kBlock, 0, st>>>(g, ctx->Q.tcode, lab[3]);
+    const dmtz_status s = jump_to_roots<I>(ctx, lab, n, 4);
+    if (s != DMTZ_OK) return s;
+    unsigned long long h[5];
+    CK(cudaMemsetAsync(cnt, 0, sizeof(h), st));
+    k_sep_agree<I><<<pg, kBlock, 0, st>>>(g, ctx->P.crit, ctx->Q.crit, lab[0], lab[1], lab[2], lab[3], cnt);
+    CK(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    for (int k = 0; k < 5; k++) out[k] = (int64_t)h[k];
+    CK(cudaGetLastError());
+    return DMTZ_OK;
+}
+extern "C" {
 
 dmtz_status dmtz_separatrix_agreement(dmtz_ctx *ctx, int W, int H, int D, const double *orig, const double *decp,
                                       int on_device, int64_t out[5]) {
@@ -3420,41 +3501,9 @@ dmtz_status dmtz_separatrix_agreement(dmtz_ctx *ctx, int W, int H, int D, const 
     if ((s = ensure(ctx, g)) != DMTZ_OK) return s;
     if ((s = upload(ctx, ctx->f, orig, g.V, on_device)) != DMTZ_OK) return s;
     if ((s = upload(ctx, ctx->g, decp, g.V, on_device)) != DMTZ_OK) return s;
-    cudaStream_t st = ctx->stream;
     run_pairing(ctx, g, view(ctx->P, ctx->f), nullptr, 1);
     run_pairing(ctx, g, view(ctx->Q, ctx->g), nullptr, 1);
-    i64 *dP = nullptr, *dQ = nullptr, *aP = nullptr, *aQ = nullptr;
-    unsigned long long *cnt = nullptr;
-    auto release = [&]() {
-        cudaFree(dP); cudaFree(dQ); cudaFree(aP); cudaFree(aQ); cudaFree(cnt);
-    };
-    if (dalloc(&dP, g.V) != cudaSuccess || dalloc(&dQ, g.V) != cudaSuccess || dalloc(&aP, 6 * g.V) != cudaSuccess ||
-        dalloc(&aQ, 6 * g.V) != cudaSuccess || dalloc(&cnt, 5) != cudaSuccess) {
-        release();
-        return fail(ctx, DMTZ_ERR_CUDA, "cannot allocate label buffers");
-    }
-    const unsigned pg = persistent_grid();
-    k_desc_init<<<pg, kBlock, 0, st>>>(g, ctx->P.pv, dP);
-    k_desc_init<<<pg, kBlock, 0, st>>>(g, ctx->Q.pv, dQ);
-    k_asc_init<<<pg, kBlock, 0, st>>>(g, ctx->P.tcode, aP);
-    k_asc_init<<<pg, kBlock, 0, st>>>(g, ctx->Q.tcode, aQ);
-    s = jump_to_roots(ctx, dP, g.V);
-    if (s == DMTZ_OK) s = jump_to_roots(ctx, dQ, g.V);
-    if (s == DMTZ_OK) s = jump_to_roots(ctx, aP, 6 * g.V);
-    if (s == DMTZ_OK) s = jump_to_roots(ctx, aQ, 6 * g.V);
-    if (s == DMTZ_OK) {
-        unsigned long long h[5];
-        if (cudaMemsetAsync(cnt, 0, 5 * sizeof(unsigned long long), st) != cudaSuccess) s = DMTZ_ERR_CUDA;
-        k_sep_agree<<<pg, kBlock, 0, st>>>(g, ctx->P.crit, ctx->Q.crit, dP, dQ, aP, aQ, cnt);
-        if (s == DMTZ_OK && (cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                             cudaStreamSynchronize(st) != cudaSuccess))
-            s = fail(ctx, DMTZ_ERR_CUDA, "label comparison failed");
-        if (s == DMTZ_OK)
-            for (int k = 0; k < 5; k++) out[k] = (int64_t)h[k];
-    }
-    release();
-    CK(cudaGetLastError());
-    return s;
+    return 6 * g.V <= INT32_MAX ? agreement<int32_t>(ctx, g, out) : agreement<i64>(ctx, g, out);
 }
 
 dmtz_status dmtz_link_classes(dmtz_ctx *ctx, int W, int H, int D, const double *data, int on_device, uint8_t *out,
@@ -3467,20 +3516,19 @@ dmtz_status dmtz_link_classes(dmtz_ctx *ctx, int W, int H, int D, const double *
     if ((s = ensure(ctx, g)) != DMTZ_OK) return s;
     if ((s = upload(ctx, ctx->f, data, g.V, on_device)) != DMTZ_OK) return s;
     cudaStream_t st = ctx->stream;
-    uint8_t *dout = nullptr;
-    unsigned long long *cnt = nullptr;
-    if ((out && dalloc(&dout, g.V) != cudaSuccess) || dalloc(&cnt, 6) != cudaSuccess) {
-        cudaFree(dout);
+    WorkDone done{ctx};
+    if (work_take(ctx, 256 + (out ? (size_t)g.V : 0)) != cudaSuccess) {
+        cudaGetLastError();
         return fail(ctx, DMTZ_ERR_CUDA, "cannot allocate link buffers");
     }
+    unsigned long long *cnt = reinterpret_cast<unsigned long long *>(ctx->work);
+    uint8_t *dout = out ? ctx->work + 256 : nullptr;
     unsigned long long h[6];
     cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(h), st);
     k_link_classes<<<persistent_grid(), kBlock, 0, st>>>(g, ctx->f, dout, cnt);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess && out) e = cudaMemcpyAsync(out, dout, (size_t)g.V, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(dout);
-    cudaFree(cnt);
     if (e != cudaSuccess) return fail(ctx, DMTZ_ERR_CUDA, cudaGetErrorString(e));
     for (int k = 0; k < 6; k++) counts[k] = (int64_t)h[k];
     CK(cudaGetLastError());
