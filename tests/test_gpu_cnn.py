@@ -356,3 +356,27 @@ def test_mma_shape_ceiling(net):
     for bad in (40, 272):  # DmtzError: N is one of 32, 48, 64, 96, 128, 256
         with pytest.raises(RuntimeError):
             net.mma_ceiling(bad)
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2), (32, 8, 4), (33, 9, 5), (31, 7, 3), (65, 2, 9)])
+@pytest.mark.parametrize("scale", [1.0, 1e-306])
+def test_features_tile_edges(gpu_ctx, dims, scale):
+    """Grids at the edges of the feature kernel's 32 x 8 x 4 tiles; with values
+    whose bound has no normal reciprocal the quotients are divided out."""
+    r = np.random.default_rng(sum(dims))
+    V = dims[0] * dims[1] * dims[2]
+    f = r.standard_normal(V) * scale
+    rel = 1e-2 if scale == 1.0 else 1e-3
+    g = f + rel * (f.max() - f.min()) * r.uniform(-1, 1, V)
+    fd, gd = torch.from_numpy(f).cuda(), torch.from_numpy(g).cuda()
+    feat = torch.empty((V, 16), dtype=torch.bfloat16, device="cuda")
+    active = torch.empty(V, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    gpu_ctx.features(fd.data_ptr(), gd.data_ptr(), dims, rel, feat.data_ptr(), active.data_ptr())
+    got = R.from_bf16_bits(feat.view(torch.int16).cpu().numpy().view(np.uint16)).reshape(*dims[::-1], 16)
+    ref, ref_act = _features_ref(f, g, dims, rel)
+    assert np.array_equal(got[..., 1], ref[..., 1])
+    assert np.array_equal(active.cpu().numpy().reshape(*dims[::-1]).astype(bool), ref_act)
+    # one bf16 rounding step (2^-8 relative) around a float32 value, whose own error is far smaller
+    other = [0] + list(range(2, 16))
+    assert (np.abs(got - ref)[..., other] <= 2 ** -8 * np.abs(ref)[..., other] + 2 ** -126).all()
