@@ -20,7 +20,8 @@
 //            cp.async double buffer; operands reach registers by ldmatrix.
 //            The data gradient is the same kernel with transposed weights,
 //            mirrored taps and a ReLU-derivative epilogue.
-//   k_wgrad  weight + bias gradient: per tile, all 27 taps x out x in
+//   k_wgrad_tc  weight + bias gradient on tcgen05 (the default; see its comment).
+//   k_wgrad  the same on mma.sync: per tile, all 27 taps x out x in
 //            products reduced over the tile's 256 vertices on the same MMA
 //            (operands by ldmatrix.trans from the channels-last tiles);
 //            per-block partial sums, then a fixed-order reduction
@@ -941,13 +942,238 @@ __global__ void __launch_bounds__(512, 1) k_wgrad(Dims d, const bf16 *__restrict
     }
 }
 
-// grad[i] = scale * sum over blocks (in block order) of part[b][i]
-__global__ void k_reduce(const float *__restrict__ part, int nblk, i64 n, const float *__restrict__ scale,
-                         float *__restrict__ grad) {
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int b = 0; b < nblk; b++) s += part[(i64)b * n + i];
-        grad[i] = s * *scale;
+// --------------------------------------------- weight gradient on tcgen05
+// The same sums as matrix products with the vertices as K.  With u = v + (0, 0, dz):
+//   dW[dx, dy, dz][n][c] = sum_u dz[u - (0, 0, dz)][n] act[u + (dx, dy, 0)][c],
+// so one product of M = 3 COUT rows (z shift, n), N = 3 CIN columns (y shift, c)
+// and K = 16 vertices of an x-line serves nine taps, and the three x shifts have an
+// accumulator each: 27 taps in three products per line.  A tile is 16 x 8 x 2
+// vertices; its operands arrive by two TMA copies whose boxes put the lines
+// where the products want them:
+//   dz  as [y 8][z 4][channel group][x 16][8 channels], z from z0 - 1: the
+//       groups of three consecutive z lines are 256 bytes apart throughout (M)
+//   act as [z 2][y 10][channel group][x 18][8 channels], from x0 - 1, y0 - 1:
+//       the groups of three consecutive y lines are 288 bytes apart (N), an x
+//       shift is 16 bytes of the start address
+// Both operands are MN-major without swizzle: 8 vertices of one group are one
+// core matrix of 128 contiguous bytes, the next 8 vertices the next 128 bytes
+// (leading offset), the next group one stride offset on.  M is 128: the rows
+// past 3 COUT multiply whatever follows in shared memory and are not read.
+// Zeros outside the grid make every edge right.  The accumulators stay in
+// tensor memory over all tiles of a block and are written once, as this
+// block's partial sums.  Warps 2..5 sum the bias gradient from the same tiles.
+// Roles and bounded waits as in k_conv_tc, three stages; empty[s] takes the
+// MMAs' commit and one arrival per bias warp.
+//
+// Bound by the 16-byte rows of the copies (3488 per 32 -> 32 tile) and the
+// products' shared-memory reads (7 KB each, 48 per tile).  100 x 75 x 53: 35 us
+// for 32 -> 32, 30 us for 16 -> 32 and 32 -> 16 (mma.sync: 98, 68 and 60).
+constexpr int WG_X = 16, WG_Y = 8, WG_Z = 2, WG_ST = 3;
+template <int CIN, int COUT>
+struct WgradTc {
+    static constexpr uint32_t ALINE = (WG_Z + 2) * (COUT / 8) * WG_X * 16, ABYTES = WG_Y * ALINE;
+    static constexpr uint32_t BLINE = (CIN / 8) * (WG_X + 2) * 16, BPLANE = (WG_Y + 2) * BLINE, BBYTES = WG_Z * BPLANE;
+    static constexpr uint32_t STAGE = ABYTES + BBYTES;
+    static constexpr uint32_t N = 3 * CIN, COLS = N <= 64 ? 64 : 128, ALLOC = 3 * COLS <= 256 ? 256 : 512;
+    static constexpr size_t smem = 128 + (size_t)WG_ST * STAGE;
+    // the rows past 3 COUT of the last line stay inside the stage
+    static_assert((WG_Y - 1) * ALINE + (COUT / 8) * 256 + 16 * 256 <= STAGE, "operand reads stay inside the stage");
+    static_assert(ABYTES % 128 == 0 && STAGE % 128 == 0, "copies start on 128-byte boundaries");
+};
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kConvThreads, 1) k_wgrad_tc(const __grid_constant__ CUtensorMap tdz,
+                                                            const __grid_constant__ CUtensorMap tact, int ntx, int nty,
+                                                            i64 ntiles, float *__restrict__ part, int *err) {
+    using T = WgradTc<CIN, COUT>;
+    constexpr int CO8 = COUT / 8;
+    constexpr i64 NPAR = 27LL * COUT * CIN + COUT;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ uint32_t tmem_slot;
+    __shared__ __align__(8) uint64_t bar_full[WG_ST], bar_empty[WG_ST], bar_done;
+    __shared__ float red[4][COUT];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t base = smem_addr(smem_raw) + ((128 - (smem_addr(smem_raw) & 127)) & 127);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&tmem_slot)),
+                     "n"(T::ALLOC));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+    }
+    auto full = [&](int s) { return smem_addr(&bar_full[s]); };
+    auto empty = [&](int s) { return smem_addr(&bar_empty[s]); };
+    const uint32_t done = smem_addr(&bar_done);
+    if (tid == 0) {
+        for (int s = 0; s < WG_ST; s++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(full(s)));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 5;\n" ::"r"(empty(s)));
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(done));
+        asm volatile("fence.mbarrier_init.release.cluster;\n");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n");
+    const uint32_t tmem = tmem_slot;
+    const i64 first = blockIdx.x, stride = gridDim.x;
+    const int ntile = first < ntiles ? (int)((ntiles - 1 - first) / stride + 1) : 0;
+    bool failed = false;
+
+    if (warp == 0) {
+        if (lane == 0) {  // MMA issuer
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((T::N >> 3) << 17) |
+                                   ((uint32_t)(128 >> 4) << 24);
+            int s = 0;
+            uint32_t ph = 0;
+            for (int it = 0; it < ntile; it++) {
+                if (!mbar_wait(full(s), ph, kConvWaitPolls)) {
+                    failed = true;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;\n");
+                const uint32_t ab = base + (uint32_t)s * T::STAGE;
+                const uint64_t a0 = smem_desc(ab, 128, WG_X * 16), b0 = smem_desc(ab + T::ABYTES, 128, (WG_X + 2) * 16);
+#pragma unroll
+                for (int q = 0; q < WG_Z; q++)
+#pragma unroll
+                    for (int y = 0; y < WG_Y; y++)
+#pragma unroll
+                        for (int tx = 0; tx < 3; tx++)
+                            tc_mma(tmem + (uint32_t)tx * T::COLS, a0 + ((y * T::ALINE + q * CO8 * WG_X * 16) >> 4),
+                                   b0 + ((q * T::BPLANE + y * T::BLINE + tx * 16) >> 4), idesc, (it | q | y) != 0);
+                asm volatile(
+                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(empty(s)));
+                if (++s == WG_ST) {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(done));
+            if (!mbar_wait(done, 0u, kConvWaitPolls)) failed = true;  // every MMA issued is done
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {  // operand producer
+            int issued = 0, s = 0;
+            uint32_t ph = 0;
+            for (int it = 0; it < ntile; it++) {
+                if (it >= WG_ST && !mbar_wait(empty(s), ph ^ 1u, kConvWaitPolls)) {
+                    failed = true;
+                    break;
+                }
+                const i64 tile = first + it * stride;
+                const int x0 = (int)(tile % ntx) * WG_X, y0 = (int)((tile / ntx) % nty) * WG_Y,
+                          z0 = (int)(tile / ((i64)ntx * nty)) * WG_Z;
+                const uint32_t dst = base + (uint32_t)s * T::STAGE, bar = full(s);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(T::STAGE));
+                asm volatile(
+                    "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, "
+                    "{%2, %3, %4, %5, %6}], [%7];\n" ::"r"(dst),
+                    "l"(reinterpret_cast<uint64_t>(&tdz)), "r"(0), "r"(x0), "r"(0), "r"(z0 - 1), "r"(y0), "r"(bar)
+                    : "memory");
+                asm volatile(
+                    "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, "
+                    "{%2, %3, %4, %5, %6}], [%7];\n" ::"r"(dst + T::ABYTES),
+                    "l"(reinterpret_cast<uint64_t>(&tact)), "r"(0), "r"(x0 - 1), "r"(0), "r"(y0 - 1), "r"(z0), "r"(bar)
+                    : "memory");
+                issued = it + 1;
+                if (++s == WG_ST) {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+            // the copies still in flight land before the block leaves
+            for (int j = issued - WG_ST; j < issued; j++)
+                if (j >= 0) mbar_wait(full(j % WG_ST), (uint32_t)(j / WG_ST) & 1u, kConvWaitPolls);
+        }
+        __syncwarp();
+    } else {  // bias gradient, then the accumulators
+        const int w = warp - 2;
+        float b[COUT];
+#pragma unroll
+        for (int c = 0; c < COUT; c++) b[c] = 0.f;
+        int s = 0;
+        uint32_t ph = 0;
+        for (int it = 0; it < ntile; it++) {
+            if (!mbar_wait(full(s), ph, kConvWaitPolls)) {
+                failed = true;
+                break;
+            }
+            // lines 2 w and 2 w + 1 of both planes: lane = x + 16 * plane
+            const uint32_t ab = base + (uint32_t)s * T::STAGE + (uint32_t)((lane >> 4) + 1) * (CO8 * WG_X * 16) + (lane & 15) * 16;
+#pragma unroll
+            for (int y = 0; y < 2; y++)
+#pragma unroll
+                for (int gch = 0; gch < CO8; gch++) {
+                    uint32_t r[4];
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n"
+                                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                                 : "r"(ab + (uint32_t)(2 * w + y) * T::ALINE + gch * (WG_X * 16)));
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        b[gch * 8 + 2 * k] += __uint_as_float(r[k] << 16);
+                        b[gch * 8 + 2 * k + 1] += __uint_as_float(r[k] & 0xFFFF0000u);
+                    }
+                }
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(empty(s)) : "memory");
+            if (++s == WG_ST) {
+                s = 0;
+                ph ^= 1;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < COUT; c++) {
+            for (int o = 16; o > 0; o >>= 1) b[c] += __shfl_xor_sync(0xffffffffu, b[c], o);
+            if (lane == 0) red[w][c] = b[c];
+        }
+        if (!mbar_wait(done, 0u, kConvWaitPolls)) failed = true;
+        asm volatile("tcgen05.fence::after_thread_sync;\n");
+        const int quarter = warp & 3, row = quarter * 32 + lane, sh = row / COUT, n = row % COUT;
+        float *p = part + (i64)blockIdx.x * NPAR;
+        if (quarter * 32 < 3 * COUT) {  // whole warps: the loads are warp-wide
+#pragma unroll 1
+            for (int tx = 0; tx < 3; tx++)
+#pragma unroll 1
+                for (int ty = 0; ty < 3; ty++) {
+                    uint32_t r[CIN];
+                    tmem_ld<CIN>(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)tx * T::COLS + (uint32_t)ty * CIN, r);
+                    tmem_wait();
+                    if (sh < 3) {  // z shift sh holds dz = 1 - sh
+                        float4 *q = reinterpret_cast<float4 *>(p + ((i64)((2 - sh) * 9 + ty * 3 + tx) * COUT + n) * CIN);
+#pragma unroll
+                        for (int k = 0; k < CIN / 4; k++)
+                            q[k] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]),
+                                               __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
+                    }
+                }
+        }
+    }
+    if (failed) atomicOr(err, 1);
+    asm volatile("tcgen05.fence::before_thread_sync;\n");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n");
+    if (tid < COUT)
+        part[(i64)blockIdx.x * NPAR + 27LL * COUT * CIN + tid] = (red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]);
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(T::ALLOC));
+}
+
+// grad[i] = scale * sum over blocks of part[b][i], in a fixed order: eight
+// threads per parameter take every eighth block, then their sums are added
+// pairwise (one thread per parameter: 304 loads in turn, 19 us; so: 7)
+constexpr int kRedWays = 8;
+__global__ void __launch_bounds__(256) k_reduce(const float *__restrict__ part, int nblk, i64 n,
+                                                const float *__restrict__ scale, float *__restrict__ grad) {
+    __shared__ float sm[kRedWays][32];
+    const int col = threadIdx.x & 31, way = threadIdx.x >> 5;
+    const i64 i = (i64)blockIdx.x * 32 + col;
+    float s = 0.f;
+    if (i < n)
+        for (int b = way; b < nblk; b += kRedWays) s += part[(i64)b * n + i];
+    sm[way][col] = s;
+    __syncthreads();
+    if (way == 0 && i < n) {
+        const float a = (sm[0][col] + sm[1][col]) + (sm[2][col] + sm[3][col]);
+        const float b = (sm[4][col] + sm[5][col]) + (sm[6][col] + sm[7][col]);
+        grad[i] = (a + b) * *scale;
     }
 }
 
@@ -997,14 +1223,28 @@ __global__ void k_loss(i64 V, const float *__restrict__ o, const float *__restri
     }
 }
 // res[0] = mean loss, res[1] = sum of weights; scale = 1 / that (0 if none)
-__global__ void k_loss_final(const double *__restrict__ part, int nblk, double *__restrict__ res,
-                             float *__restrict__ scale) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// (one block of 256 threads; a fixed order.  By one thread 109 us, so 6)
+__global__ void __launch_bounds__(256) k_loss_final(const double *__restrict__ part, int nblk, double *__restrict__ res,
+                                                    float *__restrict__ scale) {
+    __shared__ double sa[256], sb[256];
     double a = 0.0, b = 0.0;
-    for (int i = 0; i < nblk; i++) {
+    for (int i = threadIdx.x; i < nblk; i += 256) {
         a += part[2 * i];
         b += part[2 * i + 1];
     }
+    sa[threadIdx.x] = a;
+    sb[threadIdx.x] = b;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if (threadIdx.x < o) {
+            sa[threadIdx.x] += sa[threadIdx.x + o];
+            sb[threadIdx.x] += sb[threadIdx.x + o];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x != 0) return;
+    a = sa[0];
+    b = sb[0];
     res[0] = b > 0 ? a / b : 0.0;
     res[1] = b;
     *scale = b > 0 ? (float)(1.0 / b) : 0.f;
@@ -1126,29 +1366,47 @@ dmtz_status launch_persistent(dmtz_cnn *net, K kernel, int threads, size_t smem,
     return DMTZ_OK;
 }
 
-// tensor map of a channels-last bf16 activation tensor for the TMA boxes of
-// k_conv_tc and k_conv_tcx (the CUDA driver's encoder, looked up once through
-// the runtime)
-dmtz_status box_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, int W, int H, int D, int bx = GX,
-                    int by = GY, int bz = GZ) {
-    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-    if (!encode) {
+// the CUDA driver's tensor-map encoder, looked up once through the runtime
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+    static const PFN_cuTensorMapEncodeTiled_v12000 encode = []() -> PFN_cuTensorMapEncodeTiled_v12000 {
         cudaDriverEntryPointQueryResult q;
         void *fn = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) !=
-                cudaSuccess ||
-            q != cudaDriverEntryPointSuccess || !fn)
-            return nfail(net, DMTZ_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-        encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-    }
-    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D};
-    const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)C * 2 * W, (cuuint64_t)C * 2 * W * H};
-    const cuuint32_t box[4] = {8, (cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz}, estr[4] = {1, 1, 1, 1};
-    const CUresult r = encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16 *>(act), dims, strides, box,
-                              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            return nullptr;
+        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    }();
+    return encode;
+}
+dmtz_status encode_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int rank, const cuuint64_t *dims,
+                       const cuuint64_t *strides, const cuuint32_t *box) {
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const auto encode = tensor_map_encoder();
+    if (!encode) return nfail(net, DMTZ_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+    const CUresult r = encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<bf16 *>(act), dims, strides,
+                              box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return nfail(net, DMTZ_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     return DMTZ_OK;
+}
+// tensor map of a channels-last bf16 activation tensor for the TMA boxes of
+// k_conv_tc and k_conv_tcx
+dmtz_status box_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, int W, int H, int D, int bx = GX,
+                    int by = GY, int bz = GZ) {
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D};
+    const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)C * 2 * W, (cuuint64_t)C * 2 * W * H};
+    const cuuint32_t box[4] = {8, (cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
+    return encode_map(net, tm, act, 4, dims, strides, box);
+}
+// tensor map of the same tensor as (8 channels, x, channel group, third, fourth)
+// for k_wgrad_tc's boxes; z_inner: third = z and fourth = y, else the other way round
+dmtz_status line_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, int W, int H, int D, bool z_inner, int bx,
+                     int b3, int b4) {
+    const cuuint64_t sx = (cuuint64_t)C * 2, sy = sx * W, sz = sy * H;
+    const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)C / 8, (cuuint64_t)(z_inner ? D : H), (cuuint64_t)(z_inner ? H : D)};
+    const cuuint64_t strides[4] = {sx, 16, z_inner ? sz : sy, z_inner ? sy : sz};
+    const cuuint32_t box[5] = {8, (cuuint32_t)bx, (cuuint32_t)C / 8, (cuuint32_t)b3, (cuuint32_t)b4};
+    return encode_map(net, tm, act, 5, dims, strides, box);
 }
 
 template <int CIN, int COUT, int MODE, bool FLIP>
@@ -1185,15 +1443,28 @@ dmtz_status conv(dmtz_cnn *net, const Dims &d, const bf16 *in, const bf16 *w, co
 
 template <int CIN, int COUT>
 dmtz_status wgrad(dmtz_cnn *net, const Dims &d, const bf16 *act, const bf16 *dz, float *grad_out, cudaStream_t st) {
-    Dims dd = d;
     float *part = net->part;
-    void *args[] = {&dd, &act, &dz, &part};
     int used = 0;
-    dmtz_status s = launch_persistent(net, k_wgrad<CIN, COUT>, 512, wgrad_smem<CIN, COUT>(), d.ntiles,
-                                      net->part_blocks, &used, st, args);
+    dmtz_status s;
+    if (net->tensor_path) {
+        CUtensorMap tdz, tact;
+        if ((s = line_map(net, &tdz, dz, COUT, d.W, d.H, d.D, true, WG_X, WG_Z + 2, WG_Y)) != DMTZ_OK ||
+            (s = line_map(net, &tact, act, CIN, d.W, d.H, d.D, false, WG_X + 2, WG_Y + 2, WG_Z)) != DMTZ_OK)
+            return s;
+        int ntx = (d.W + WG_X - 1) / WG_X, nty = (d.H + WG_Y - 1) / WG_Y, *err = net->tc_err;
+        i64 ntiles = (i64)ntx * nty * ((d.D + WG_Z - 1) / WG_Z);
+        void *args[] = {&tdz, &tact, &ntx, &nty, &ntiles, &part, &err};
+        s = launch_persistent(net, k_wgrad_tc<CIN, COUT>, kConvThreads, WgradTc<CIN, COUT>::smem, ntiles, net->nsm, &used, st,
+                              args);
+    } else {
+        Dims dd = d;
+        void *args[] = {&dd, &act, &dz, &part};
+        s = launch_persistent(net, k_wgrad<CIN, COUT>, 512, wgrad_smem<CIN, COUT>(), d.ntiles, net->part_blocks, &used, st,
+                              args);
+    }
     if (s != DMTZ_OK) return s;
     const i64 n = 27LL * COUT * CIN + COUT;
-    k_reduce<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(net->part, used, n, net->scale, grad_out);
+    k_reduce<<<(unsigned)((n + 31) / 32), 256, 0, st>>>(net->part, used, n, net->scale, grad_out);
     NCK(cudaGetLastError());
     return DMTZ_OK;
 }
@@ -1474,7 +1745,7 @@ dmtz_status dmtz_cnn_backward(dmtz_cnn *net, int W, int H, int D, const float *t
     const Dims d = make_dims(W, H, D);
     const i64 V = (i64)W * H * D;
     k_loss<<<kLossBlocks, 256, 0, st>>>(V, net->last_out, target, active, net->dz4, net->lpart);
-    k_loss_final<<<1, 32, 0, st>>>(net->lpart, kLossBlocks, net->lres, net->scale);
+    k_loss_final<<<1, 256, 0, st>>>(net->lpart, kLossBlocks, net->lres, net->scale);
     NCK(cudaGetLastError());
     bf16 *a1 = net->a[0], *a2 = net->a[1], *a3 = net->a[2];
     float *gr = net->grad;

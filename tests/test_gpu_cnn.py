@@ -380,3 +380,28 @@ def test_features_tile_edges(gpu_ctx, dims, scale):
     # one bf16 rounding step (2^-8 relative) around a float32 value, whose own error is far smaller
     other = [0] + list(range(2, 16))
     assert (np.abs(got - ref)[..., other] <= 2 ** -8 * np.abs(ref)[..., other] + 2 ** -126).all()
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2), (14, 8, 2), (16, 8, 2), (17, 9, 3), (31, 7, 5), (2, 17, 12)])
+def test_gradient_tile_edges(net, dims):
+    """Grids at the edges of the convolutions' 14 x 8 x 2 and the weight
+    gradient's 16 x 8 x 2 tiles (tolerances as in the backward test)."""
+    W, H, D = dims
+    p = _params(11)
+    net.set_params(p)
+    feat_h, feat_d = _feat(12, dims)
+    target = np.random.default_rng(13).uniform(-0.9, 0.9, (D, H, W))
+    out = torch.empty(W * H * D, dtype=torch.float32, device="cuda")
+    tgt = torch.from_numpy(target.reshape(-1).astype(np.float32)).cuda()
+    act = torch.ones(W * H * D, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    net.forward(feat_d.data_ptr(), out.data_ptr(), dims, train=True)
+    loss = net.backward(tgt.data_ptr(), act.data_ptr(), dims)
+    grads = net.get_grads().astype(np.float64)
+    ref_loss, ref_g = R.loss_and_grad(feat_h, p.astype(np.float64), target, np.ones((D, H, W), bool))
+    assert abs(loss - ref_loss) < 2e-3 * ref_loss
+    o = 0
+    for l, (ci, co) in enumerate(R.LAYERS):
+        n = 27 * ci * co + co
+        assert _rel(grads[o:o + n], ref_g[o:o + n]) < 2e-2, l
+        o += n
