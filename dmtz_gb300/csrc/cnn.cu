@@ -11,9 +11,10 @@
 // tap = (dz+1)*9 + (dy+1)*3 + (dx+1).
 //
 // Kernels (all persistent: one or two blocks per SM loop over tiles):
-//   k_conv_tc  the convolutions (forward and data gradient) on tcgen05: a
-//            tile of 128 vertices per MMA chain, accumulator in tensor
-//            memory (the default path; see its comment).
+//   k_conv_tcx  the convolutions (forward and data gradient) on tcgen05: the
+//            128 rows of a product are a plane across x, which marches (the
+//            default path; see its comment).
+//   k_conv_tc  the same with a box of vertices per MMA chain.
 //   k_conv   the same convolution on mma.sync.m16n8k16 (bf16 in, f32
 //            accumulate).  A block keeps all 27 x out x in weights in shared
 //            memory and streams 8x8x4-vertex tiles (+1 halo) through a
@@ -299,11 +300,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int lim
             : "r"(bar), "r"(parity));
     return done != 0;
 }
-// this warp's 32 accumulator rows, columns 0..N-1 (N = 16 or 32), into r;
+// this warp's 32 accumulator rows, columns 0..N-1 (N = 1, 16 or 32), into r;
 // the registers are valid after tmem_wait()
 template <int N>
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[N]) {
-    if constexpr (N == 32) {
+    if constexpr (N == 1) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n" : "=r"(r[0]) : "r"(taddr));
+    } else if constexpr (N == 32) {
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
             "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
@@ -552,229 +555,335 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv_tc(const __grid_consta
 }
 
 // ---------------------------------------- convolution on tcgen05, x-taps folded
-// The same convolution with wider products.  For each (dy, dz) offset one
-// MMA multiplies the rows shifted by (-1, dy, dz) with the three x-taps'
-// weight blocks side by side (N = 3 COUT): columns [t COUT, (t+1) COUT) of
-// row r hold the contribution of x-tap t (dx = t - 1) to the output t
-// vertices before row r's along x, so
-//   out[r] = D[r][0, COUT) + D[r+1][COUT, 2 COUT) + D[r+2][2 COUT, 3 COUT),
-// summed in the epilogue with two warp shuffles per channel.  A tile's 128
-// rows are 8 lines of 16 x-neighbours (two core matrices per line, so the
-// 8-row groups are 128 bytes apart throughout), of which the first 14 are
-// outputs; tiles step 14 along x and overlap by two rows.  The box needs no
-// halo along +x (16 x 10 x (QZ2 + 2) vertices).  9 x CIN/16 x QZ2 MMAs per
-// tile of 14 x 8 x QZ2 outputs.  Roles, barriers and bounded waits as in
-// k_conv_tc; FLIP mirrors the taps through the weight layout.
-constexpr int XF_TX = 14, XF_GX = 16, XF_TY = 8, XF_GY = XF_TY + 2, XF_QZ = 2, XF_GZ = XF_QZ + 2;
-constexpr int XF_GVOX = XF_GX * XF_GY * XF_GZ;
-constexpr uint32_t XF_PLANE = XF_GVOX * 16;  // a multiple of 128
-inline Dims make_xf_dims(int W, int H, int D) {
-    Dims d{W, H, D, (W + XF_TX - 1) / XF_TX, (H + XF_TY - 1) / XF_TY, (D + XF_QZ - 1) / XF_QZ, 0};
-    d.ntiles = (i64)d.ntx * d.nty * d.ntz;
-    return d;
+// The same convolution with wider products, marching along x.  A tile is a
+// column: 8 x 16 vertices of the plane across x (axes a and b: y and z, or z
+// and y when that pads fewer rows) are the 128 rows of every product.  The
+// input arrives as slices of constant x (10 x 18 vertices with the halo), each
+// once.  Slice x contributes to the outputs x + 1, x and x - 1 through the
+// taps dx = -1, 0, 1; their weight blocks side by side make one MMA of N =
+// 3 COUT per (dy, dz) offset: 9 x CIN/16 MMAs per slice.  The three
+// contributions to an output lie in the same lanes of three successive
+// slices' accumulators, so the epilogue adds them in registers as it goes.
+//
+// Blocks take equal contiguous runs of outputs, column after column; a run
+// that starts or ends inside a column reads one more slice there.  A vertex is
+// one row of CIN channels in shared memory, swizzled over its own width (64 or
+// 32 bytes); the swizzle goes by address bits, so an operand may start at any
+// row, and a slice is a TMA box whose rows are whole vertices.
+//
+// Roles: warps 0 and 1 issue the MMAs of every other copy (two slices): the
+// tensor pipe takes a product only when one before it is done, so the 400
+// cycles that a warp spends on waits and commits would be idle, were there no
+// other.  The whole warp walks and one elected lane issues: inside a branch on
+// the lane, the descriptors would be moved to uniform registers one by one,
+// which took longer than the products.  Warp 2 brings the copies (full / empty
+// barriers), warps 3..10 the weights, and then they run the epilogue, half of
+// the channels of a lane quarter each, from four accumulators in turn.  Waits
+// are bounded as in k_conv_tc.
+//
+// Bound by the products: 59 cycles for N = 96, the rate of back-to-back MMAs of
+// that shape, and 47 for N = 48 (and for anything narrower).  161 x 127 x 110,
+// against 14 x 8 x 2 tiles with halo boxes, where one lane issued and the shifts
+// were warp shuffles: 32 -> 32 76 us (148), 16 -> 32 50 (101), 32 -> 16 59 (128);
+// at 100 x 75 x 53 24 (40), 19 (30), 20 (35), data gradients 29 (47) and 23 (45).
+constexpr int CX_A = 8, CX_B = 16, CX_GA = CX_A + 2, CX_GB = CX_B + 2, CX_NX = 2, CX_ACC = 4, CX_ST = 6;
+constexpr int CX_EPI = 8, CX_THREADS = 96 + 32 * CX_EPI;
+struct March {
+    int W, na, nb;  // extents along x, a, b
+    i64 sa, sb;     // vertex strides of a and b
+    int swapped;    // a = z and b = y
+    int nta;        // columns along a
+    i64 outputs;    // of all columns
+};
+inline March make_march(int W, int H, int D) {
+    auto up = [](i64 n, i64 m) { return (n + m - 1) / m * m; };
+    const bool swap = up(D, CX_A) * up(H, CX_B) < up(H, CX_A) * up(D, CX_B);
+    March m{};
+    m.W = W;
+    m.na = swap ? D : H;
+    m.nb = swap ? H : D;
+    m.sa = swap ? (i64)W * H : W;
+    m.sb = swap ? W : (i64)W * H;
+    m.swapped = swap;
+    m.nta = (m.na + CX_A - 1) / CX_A;
+    m.outputs = (i64)m.nta * ((m.nb + CX_B - 1) / CX_B) * W;
+    return m;
 }
-// accumulator columns of one slice: 3 COUT rounded up to a power of two
-template <int COUT>
-__host__ __device__ constexpr uint32_t xf_cols() {
-    return COUT == 32 ? 128u : 64u;
+// the part of a run that lies in one column: outputs [o0, o1) from slices j0..j1
+struct Stretch {
+    int a0, b0, o0, o1, j0, j1;
+    __device__ __forceinline__ Stretch(const March &m, i64 g, i64 end) {
+        const i64 col = g / m.W;
+        a0 = (int)(col % m.nta) * CX_A;
+        b0 = (int)(col / m.nta) * CX_B;
+        o0 = (int)(g - col * m.W);
+        o1 = (int)min((i64)m.W, o0 + (end - g));
+        j0 = max(o0 - 1, 0);
+        j1 = min(o1, m.W - 1);
+    }
+};
+template <int CIN>
+__host__ __device__ constexpr uint32_t cx_stage() {  // bytes of a copy's slices, to the next 1024
+    return (CX_NX * CX_GB * CX_GA * CIN * 2 + 1023) / 1024 * 1024;
 }
 template <int CIN, int COUT>
-constexpr size_t xf_smem() {
-    return 128 + (size_t)9 * (CIN / 8) * (3 * COUT) * 16 + 2 * (size_t)(CIN / 8) * XF_PLANE;
+constexpr size_t cx_smem() {
+    return 1024 + (size_t)CX_ST * cx_stage<CIN>() + (size_t)9 * (CIN / 8) * (3 * COUT) * 16;
+}
+// descriptor of a K-major operand whose rows are as wide as their swizzle (64
+// or 32 bytes), groups of eight rows `group` bytes apart
+template <int ROW>
+__device__ __forceinline__ uint64_t swizzled_desc(uint32_t addr, uint32_t group) {
+    static_assert(ROW == 64 || ROW == 32, "row widths");
+    return smem_desc(addr, 16, group) | ((uint64_t)(ROW == 64 ? 4 : 6) << 61);
+}
+// one lane of a converged warp (elect.sync: always the same one)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar));
+}
+struct alignas(32) Vec8 {
+    uint32_t v[8];
+};
+__device__ __forceinline__ Vec8 ld32(const void *p) {  // 32 bytes, issued where it stands
+    Vec8 r;
+    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]),
+                   "=r"(r.v[7])
+                 : "l"(p));
+    return r;
+}
+__device__ __forceinline__ void st32(void *p, const Vec8 &r) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p), "r"(r.v[0]), "r"(r.v[1]), "r"(r.v[2]),
+                 "r"(r.v[3]), "r"(r.v[4]), "r"(r.v[5]), "r"(r.v[6]), "r"(r.v[7])
+                 : "memory");
 }
 template <int CIN, int COUT, int MODE, bool FLIP>
-__global__ void __launch_bounds__(kConvThreads, 1) k_conv_tcx(const __grid_constant__ CUtensorMap tmap, Dims d,
-                                                            const bf16 *__restrict__ wt,
-                                                            const float *__restrict__ bias, void *out,
-                                                            const bf16 *__restrict__ aux, int *err) {
-    constexpr int KCH = CIN / 8, N = 3 * COUT;
-    constexpr uint32_t WGRP = N * 16, WBYTES = 9 * KCH * WGRP, XBYTES = KCH * XF_PLANE;
-    constexpr uint32_t SCOLS = xf_cols<COUT>(), ACC_COLS = XF_QZ * SCOLS, ALLOC = 2 * ACC_COLS;
+__global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constant__ CUtensorMap tmap, const March m,
+                                                          const bf16 *__restrict__ wt, const float *__restrict__ bias,
+                                                          void *out, const bf16 *__restrict__ aux, int *err) {
+    constexpr int KCH = CIN / 8, N = 3 * COUT, ROW = CIN * 2;
+    constexpr uint32_t WGRP = N * 16, LINE = CX_GA * ROW, SLICE = CX_GB * LINE, STAGE = cx_stage<CIN>();
+    constexpr uint32_t COLS = COUT == 32 ? 128 : 64, ALLOC = CX_ACC * COLS;
+    constexpr int EPI = MODE == 1 ? 4 : CX_EPI;  // warps of the epilogue: one channel needs no second half
     static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "tile shapes");
-    static_assert(WGRP % 128 == 0 && XF_PLANE % 128 == 0, "operand blocks stay 128-byte aligned");
     static_assert(ALLOC == 256 || ALLOC == 512, "tensor-memory allocation is a power of two");
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint32_t tmem_slot;
-    __shared__ __align__(8) uint64_t bar_full[2], bar_mma[2], bar_free[2];
-    unsigned char *ws = smem_raw + ((128 - (smem_addr(smem_raw) & 127)) & 127);
+    __shared__ __align__(8) uint64_t bar_full[CX_ST], bar_empty[CX_ST], bar_mma[CX_ACC], bar_free[CX_ACC], bar_w, bar_done;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // weights: per (dy, dz) offset u and channel group kc, rows n = t COUT + c
-    // hold tap (t - 1, dy, dz) of output channel c (mirrored under FLIP)
-    for (int i = tid; i < 9 * KCH * N; i += blockDim.x) {
-        const int u = i / (KCH * N), rem = i - u * (KCH * N), kc = rem / N, n = rem - kc * N;
-        const int t = n / COUT, c = n - t * COUT;
-        const int tap = FLIP ? 26 - (t + 3 * u) : t + 3 * u;
-        cp16(ws + (u * KCH + kc) * WGRP + n * 16, wt + ((i64)tap * COUT + c) * CIN + kc * 8, 16);
-    }
-    cp_commit();
+    const uint32_t ring = (smem_addr(smem_raw) + 1023) & ~1023u, wbase = ring + CX_ST * STAGE;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                          smem_addr(&tmem_slot)),
                      "n"(ALLOC));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
-    const uint32_t full0 = smem_addr(&bar_full[0]), full1 = smem_addr(&bar_full[1]);
-    const uint32_t mma0 = smem_addr(&bar_mma[0]), mma1 = smem_addr(&bar_mma[1]);
-    const uint32_t fre0 = smem_addr(&bar_free[0]), fre1 = smem_addr(&bar_free[1]);
-    auto full = [&](int b) { return b ? full1 : full0; };
-    auto mma = [&](int b) { return b ? mma1 : mma0; };
-    auto fre = [&](int b) { return b ? fre1 : fre0; };
-    const uint32_t wbase = smem_addr(ws), xbase0 = wbase + WBYTES;
+    auto full = [&](int s) { return smem_addr(&bar_full[s]); };
+    auto empty = [&](int s) { return smem_addr(&bar_empty[s]); };
+    auto mma = [&](int q) { return smem_addr(&bar_mma[q % CX_ACC]); };
+    auto fre = [&](int q) { return smem_addr(&bar_free[q % CX_ACC]); };
+    const uint32_t wbar = smem_addr(&bar_w), done = smem_addr(&bar_done);
     if (tid == 0) {
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(full(b)));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mma(b)));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;\n" ::"r"(fre(b)));
+        auto init = [](uint32_t bar, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(n)); };
+        for (int s = 0; s < CX_ST; s++) {
+            init(full(s), 1);
+            init(empty(s), 1);
         }
+        for (int q = 0; q < CX_ACC; q++) {
+            init(mma(q), 1);
+            init(fre(q), EPI);
+        }
+        init(wbar, 32 * CX_EPI);
+        init(done, 2);
         asm volatile("fence.mbarrier_init.release.cluster;\n");
     }
-    cp_wait<0>();
-    asm volatile("fence.proxy.async.shared::cta;\n");
     asm volatile("tcgen05.fence::before_thread_sync;\n");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n");
     const uint32_t tmem = tmem_slot;
-    const i64 first = blockIdx.x, stride = gridDim.x;
-    const int ntile = first < d.ntiles ? (int)((d.ntiles - 1 - first) / stride + 1) : 0;
-    auto origin = [&](i64 tile, int &x0, int &y0, int &z0) {
-        x0 = (int)(tile % d.ntx) * XF_TX;
-        y0 = (int)((tile / d.ntx) % d.nty) * XF_TY;
-        z0 = (int)(tile / ((i64)d.ntx * d.nty)) * XF_QZ;
-    };
+    // this block's run of outputs
+    const i64 per = m.outputs / gridDim.x, rest = m.outputs - per * gridDim.x;
+    const i64 first = blockIdx.x * per + min((i64)blockIdx.x, rest), end = first + per + (blockIdx.x < rest);
     bool failed = false;
 
-    if (warp == 0) {
-        if (lane == 0) {  // MMA issuer
-            const uint32_t idesc =
-                (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-            const uint64_t b0 = smem_desc(wbase, WGRP, 128);
-            int committed = 0;
-            for (int it = 0; it < ntile; it++) {
-                const int b = it & 1;
-                if (!mbar_wait(full(b), (uint32_t)(it >> 1) & 1u, kConvWaitPolls) ||
-                    (it >= 2 && !mbar_wait(fre(b), (uint32_t)((it >> 1) - 1) & 1u, kConvWaitPolls))) {
-                    failed = true;
-                    break;
+    if (warp < 2) {  // MMA issuers
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint64_t b0 = smem_desc(wbase, WGRP, 128);
+        const uint32_t dy = (m.swapped ? LINE : ROW) >> 4, dz = (m.swapped ? ROW : LINE) >> 4;
+        if (!mbar_wait(wbar, 0u, kConvWaitPolls)) failed = true;
+        int c = 0, q = 0;  // copies and slices so far
+        for (i64 g = first; g < end && !failed;) {
+            const Stretch t(m, g, end);
+            for (int j = t.j0; j <= t.j1 && !failed; j += CX_NX, c++) {
+                const int n = min(CX_NX, t.j1 - j + 1), s = c % CX_ST;
+                if ((c & 1) == warp) {
+                    // the copy, and the accumulators' last readers: a barrier per lane
+                    const int mine = lane == 2 && n == 2 ? q + 1 : q;
+                    const bool copy = lane == 0 || mine < CX_ACC;
+                    if (!__all_sync(0xffffffffu, mbar_wait(copy ? full(s) : fre(mine),
+                                                           (uint32_t)(copy ? c / CX_ST : mine / CX_ACC - 1) & 1u,
+                                                           kConvWaitPolls))) {
+                        failed = true;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;\n");
+                    if (elect_one()) {
+                        for (int e = 0; e < n; e++) {
+                            const uint64_t a0 = swizzled_desc<ROW>(ring + s * STAGE + e * SLICE, LINE);
+                            const uint32_t acc = tmem + (uint32_t)((q + e) % CX_ACC) * COLS;
+#pragma unroll
+                            for (int u = 0; u < 9; u++)
+#pragma unroll
+                                for (int kk = 0; kk < KCH / 2; kk++)
+                                    tc_mma(acc, a0 + (u % 3 * dy + u / 3 * dz + kk * 2),
+                                           b0 + (((u * KCH + kk * 2) * WGRP) >> 4), idesc, (u | kk) != 0);
+                            tc_commit(mma(q + e));
+                        }
+                        tc_commit(empty(s));
+                    }
+                    __syncwarp();
                 }
-                asm volatile("tcgen05.fence::after_thread_sync;\n");
-                const uint64_t a0 = smem_desc(xbase0 + b * XBYTES, XF_PLANE, 128);
-                const uint32_t acc = tmem + (uint32_t)b * ACC_COLS;
-#pragma unroll
-                for (int u = 0; u < 9; u++) {
-                    const int sy = u % 3, sz = u / 3;  // dy + 1, dz + 1
-#pragma unroll
-                    for (int kk = 0; kk < KCH / 2; kk++)
-#pragma unroll
-                        for (int q = 0; q < XF_QZ; q++)
-                            tc_mma(acc + (uint32_t)q * SCOLS,
-                                   a0 + ((((q + sz) * XF_GY + sy) * XF_GX * 16 + kk * 2 * XF_PLANE) >> 4),
-                                   b0 + (((u * KCH + kk * 2) * WGRP) >> 4), idesc, (u | kk) != 0);
-                }
-                asm volatile(
-                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mma(b)));
-                committed = it + 1;
+                q += n;
             }
-            if (committed > 0)
-                mbar_wait(mma((committed - 1) & 1), (uint32_t)((committed - 1) >> 1) & 1u, kConvWaitPolls);
+            g += t.o1 - t.o0;
         }
+        if (elect_one()) tc_commit(done);
         __syncwarp();
-    } else if (warp == 1) {
-        if (lane == 0) {  // box producer
+        if (!mbar_wait(done, 0u, kConvWaitPolls)) failed = true;  // every MMA issued is done
+    } else if (warp == 2) {
+        if (lane == 0) {  // copies
             int issued = 0;
-            for (int it = 0; it < ntile; it++) {
-                const int b = it & 1;
-                if (it >= 2 && !mbar_wait(mma(b), (uint32_t)((it >> 1) - 1) & 1u, kConvWaitPolls)) {
-                    failed = true;
-                    break;
-                }
-                int x0, y0, z0;
-                origin(first + it * stride, x0, y0, z0);
-                const uint32_t dst = xbase0 + b * XBYTES, bar = full(b);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar),
-                             "r"((uint32_t)(KCH * XF_GVOX * 16)));
-#pragma unroll
-                for (int c = 0; c < KCH; c++)
+            for (i64 g = first; g < end && !failed;) {
+                const Stretch t(m, g, end);
+                for (int j = t.j0; j <= t.j1; j += CX_NX) {
+                    const int s = issued % CX_ST;
+                    if (issued >= CX_ST && !mbar_wait(empty(s), (uint32_t)(issued / CX_ST - 1) & 1u, kConvWaitPolls)) {
+                        failed = true;
+                        break;
+                    }
+                    const uint32_t bar = full(s);
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(CX_NX * SLICE));
                     asm volatile(
                         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, "
-                        "{%2, %3, %4, %5}], [%6];\n" ::"r"(dst + c * XF_PLANE),
-                        "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(c * 8), "r"(x0 - 1), "r"(y0 - 1), "r"(z0 - 1),
-                        "r"(bar)
+                        "{%2, %3, %4, %5}], [%6];\n" ::"r"(ring + s * STAGE),
+                        "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(0), "r"(t.a0 - 1), "r"(t.b0 - 1), "r"(j), "r"(bar)
                         : "memory");
-                issued = it + 1;
+                    issued++;
+                }
+                g += t.o1 - t.o0;
             }
-            for (int j = issued - 2; j < issued; j++)
-                if (j >= 0) mbar_wait(full(j & 1), (uint32_t)(j >> 1) & 1u, kConvWaitPolls);
+            // the copies still in flight land before the block leaves
+            for (int j = issued - CX_ST; j < issued; j++)
+                if (j >= 0) mbar_wait(full(j % CX_ST), (uint32_t)(j / CX_ST) & 1u, kConvWaitPolls);
         }
         __syncwarp();
-    } else {  // epilogue: warps 2..5
-        const int quarter = warp & 3;
-        const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16);
-        float bsh[COUT];
+    } else {
+        // weights: per offset u = (dy + 1) + 3 (dz + 1) and channel group kc, rows
+        // n = t COUT + c hold tap dx = t - 1 of output channel c (mirrored under FLIP)
+        unsigned char *ws = smem_raw + (wbase - smem_addr(smem_raw));
+        for (int i = tid - 96; i < 9 * KCH * N; i += 32 * CX_EPI) {
+            const int u = i / (KCH * N), rem = i - u * (KCH * N), kc = rem / N, n = rem - kc * N;
+            const int t = n / COUT, c = n - t * COUT;
+            const int tap = FLIP ? 26 - (t + 3 * u) : t + 3 * u;
+            cp16(ws + (u * KCH + kc) * WGRP + n * 16, wt + ((i64)tap * COUT + c) * CIN + kc * 8, 16);
+        }
+        cp_commit();
+        cp_wait<0>();
+        asm volatile("fence.proxy.async.shared::cta;\n");
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(wbar) : "memory");
+
+        // the epilogue: channels [c0, c0 + NC) of lane quarter `quarter`
+        constexpr int NC = MODE == 1 ? 1 : COUT * 4 / CX_EPI;
+        static_assert(MODE == 1 || NC == 16, "a thread stores 32 bytes");
+        const int quarter = warp & 3, half = (warp - 3) >> 2, c0 = half * NC;
+        const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
+        float bsh[MODE == 2 ? 1 : NC];
+        if constexpr (MODE != 2) {
 #pragma unroll
-        for (int c = 0; c < COUT; c++) bsh[c] = MODE == 2 ? 0.f : (MODE == 1 && c > 0 ? 0.f : bias[c]);
-        const int r = quarter * 32 + lane, rx = r & 15, ry = r >> 4;
-        for (int it = 0; it < ntile; it++) {
-            const int b = it & 1;
-            if (!mbar_wait(mma(b), (uint32_t)(it >> 1) & 1u, kConvWaitPolls)) {
-                failed = true;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;\n");
-            int x0, y0, z0;
-            origin(first + it * stride, x0, y0, z0);
-            const int gx = x0 + rx, gy = y0 + ry;
-#pragma unroll 1
-            for (int zq = 0; zq < XF_QZ; zq++) {
-                uint32_t p0[COUT], p1[COUT], p2[COUT];
-                const uint32_t col = taddr + (uint32_t)b * ACC_COLS + (uint32_t)zq * SCOLS;
-                tmem_ld<COUT>(col, p0);
-                tmem_ld<COUT>(col + COUT, p1);
-                tmem_ld<COUT>(col + 2 * COUT, p2);
-                tmem_wait();
-                if (zq == XF_QZ - 1) {  // the accumulator set is read: hand it back
-                    asm volatile("tcgen05.fence::before_thread_sync;\n");
-                    __syncwarp();
-                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(fre(b)) : "memory");
-                }
-                float acc[COUT];
+            for (int c = 0; c < NC; c++) bsh[c] = bias[c0 + c];
+        }
+        const int r = quarter * 32 + lane;
+        int q = 0;
+        for (i64 g = half < EPI / 4 ? first : end; g < end && !failed;) {
+            const Stretch t(m, g, end);
+            const int a = t.a0 + (r & 7), b = t.b0 + (r >> 3);
+            const bool row = a < m.na && b < m.nb;
+            const i64 v0 = a * m.sa + b * m.sb;
+            // contributions of the slices before j: to output j, and to output j - 1
+            float next[NC], cur[NC];
 #pragma unroll
-                for (int c = 0; c < COUT; c++)  // rows r+1 and r+2 are lanes lane+1, lane+2 (same x-line)
-                    acc[c] = __uint_as_float(p0[c]) + __shfl_down_sync(0xffffffffu, __uint_as_float(p1[c]), 1) +
-                             __shfl_down_sync(0xffffffffu, __uint_as_float(p2[c]), 2);
-                const int gz = z0 + zq;
-                if (rx < XF_TX && gx < d.W && gy < d.H && gz < d.D) {
-                    const i64 v = gx + (i64)gy * d.W + (i64)gz * d.W * d.H;
-                    if constexpr (MODE == 1) {
-                        reinterpret_cast<float *>(out)[v] = acc[0] + bsh[0];
-                    } else {
-                        uint4 *o = reinterpret_cast<uint4 *>(reinterpret_cast<bf16 *>(out) + v * COUT);
-                        const uint4 *ax = MODE == 2 ? reinterpret_cast<const uint4 *>(aux + v * COUT) : nullptr;
+            for (int c = 0; c < NC; c++) next[c] = cur[c] = 0.f;
+            auto store = [&](int o, const Vec8 &mk) {  // cur is complete: output o
+                if (!row) return;
+                const i64 v = v0 + o;
+                if constexpr (MODE == 1) {
+                    reinterpret_cast<float *>(out)[v] = cur[0] + bsh[0];
+                } else {
+                    Vec8 pk;
 #pragma unroll
-                        for (int q = 0; q < COUT / 8; q++) {
-                            uint4 mk = make_uint4(0, 0, 0, 0);
-                            if constexpr (MODE == 2) mk = ax[q];
-                            const bf16 *mb = reinterpret_cast<const bf16 *>(&mk);
-                            uint4 pk;
-                            __nv_bfloat162 *p2h = reinterpret_cast<__nv_bfloat162 *>(&pk);
-#pragma unroll
-                            for (int h = 0; h < 4; h++) {
-                                const int ch = q * 8 + 2 * h;
-                                float v0 = acc[ch], v1 = acc[ch + 1];
-                                if constexpr (MODE == 0) {
-                                    v0 = fmaxf(v0 + bsh[ch], 0.f);
-                                    v1 = fmaxf(v1 + bsh[ch + 1], 0.f);
-                                } else {
-                                    if (!(__bfloat162float(mb[2 * h]) > 0.f)) v0 = 0.f;
-                                    if (!(__bfloat162float(mb[2 * h + 1]) > 0.f)) v1 = 0.f;
-                                }
-                                p2h[h] = __floats2bfloat162_rn(v0, v1);
-                            }
-                            o[q] = pk;
+                    for (int i = 0; i < 8; i++) {
+                        float x0 = cur[2 * i], x1 = cur[2 * i + 1];
+                        if constexpr (MODE == 0) {
+                            x0 = fmaxf(x0 + bsh[2 * i], 0.f);
+                            x1 = fmaxf(x1 + bsh[2 * i + 1], 0.f);
+                        } else {
+                            if (!(__uint_as_float(mk.v[i] << 16) > 0.f)) x0 = 0.f;
+                            if (!(__uint_as_float(mk.v[i] & 0xFFFF0000u) > 0.f)) x1 = 0.f;
                         }
+                        const __nv_bfloat162 two = __floats2bfloat162_rn(x0, x1);
+                        pk.v[i] = *reinterpret_cast<const uint32_t *>(&two);
                     }
+                    st32(reinterpret_cast<bf16 *>(out) + v * COUT + c0, pk);
+                }
+            };
+            auto mask = [&](int o) {
+                Vec8 mk{};
+                if (MODE == 2 && row && o >= t.o0 && o < t.o1) mk = ld32(aux + (v0 + o) * COUT + c0);
+                return mk;
+            };
+            auto slice = [&](int j, const Vec8 &mk) {
+                if (!mbar_wait(mma(q), (uint32_t)(q / CX_ACC) & 1u, kConvWaitPolls)) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;\n");
+                const uint32_t at = lanes + (uint32_t)(q % CX_ACC) * COLS;
+                uint32_t p0[NC], p1[NC], p2[NC];
+                tmem_ld<NC>(at, p0);
+                tmem_ld<NC>(at + COUT, p1);
+                tmem_ld<NC>(at + 2 * COUT, p2);
+                tmem_wait();
+                asm volatile("tcgen05.fence::before_thread_sync;\n");
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(fre(q)) : "memory");
+#pragma unroll
+                for (int c = 0; c < NC; c++) cur[c] += __uint_as_float(p2[c]);
+                if (j > t.o0) store(j - 1, mk);
+#pragma unroll
+                for (int c = 0; c < NC; c++) {
+                    cur[c] = next[c] + __uint_as_float(p1[c]);
+                    next[c] = __uint_as_float(p0[c]);
+                }
+                q++;
+                return true;
+            };
+            // mk[i] is the mask of output j0 - 1 + i mod 4, loaded three slices before its use
+            constexpr int AHEAD = MODE == 2 ? 4 : 1;
+            Vec8 mk[AHEAD];
+#pragma unroll
+            for (int e = 0; e < AHEAD - 1; e++) mk[e] = mask(t.j0 - 1 + e);
+            for (int j = t.j0; j <= t.j1 && !failed; j += AHEAD) {
+#pragma unroll
+                for (int e = 0; e < AHEAD; e++) {
+                    if (j + e > t.j1 || failed) break;
+                    mk[(e + AHEAD - 1) % AHEAD] = mask(j + e + AHEAD - 2);
+                    if (!slice(j + e, mk[e])) failed = true;
                 }
             }
+            if (t.j1 < t.o1 && !failed) store(t.o1 - 1, mask(t.o1 - 1));  // the column's last output: nothing follows it
+            g += t.o1 - t.o0;
         }
     }
     if (failed) atomicOr(err, 1);
@@ -1379,24 +1488,30 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return encode;
 }
 dmtz_status encode_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int rank, const cuuint64_t *dims,
-                       const cuuint64_t *strides, const cuuint32_t *box) {
+                       const cuuint64_t *strides, const cuuint32_t *box,
+                       CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE) {
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     const auto encode = tensor_map_encoder();
     if (!encode) return nfail(net, DMTZ_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
     const CUresult r = encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<bf16 *>(act), dims, strides,
-                              box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return nfail(net, DMTZ_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     return DMTZ_OK;
 }
-// tensor map of a channels-last bf16 activation tensor for the TMA boxes of
-// k_conv_tc and k_conv_tcx
-dmtz_status box_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, int W, int H, int D, int bx = GX,
-                    int by = GY, int bz = GZ) {
+// tensor map of a channels-last bf16 activation tensor for k_conv_tc's boxes
+dmtz_status box_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, int W, int H, int D) {
     const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D};
     const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)C * 2 * W, (cuuint64_t)C * 2 * W * H};
-    const cuuint32_t box[4] = {8, (cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
+    const cuuint32_t box[4] = {8, GX, GY, GZ};
     return encode_map(net, tm, act, 4, dims, strides, box);
+}
+// and for k_conv_tcx's slices: whole vertices, axes (channel, a, b, x)
+dmtz_status slice_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, const March &m) {
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)m.na, (cuuint64_t)m.nb, (cuuint64_t)m.W}, row = (cuuint64_t)C * 2;
+    const cuuint64_t strides[3] = {row * m.sa, row * m.sb, row};
+    const cuuint32_t box[4] = {(cuuint32_t)C, CX_GA, CX_GB, CX_NX};
+    return encode_map(net, tm, act, 4, dims, strides, box, C == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 // tensor map of the same tensor as (8 channels, x, channel group, third, fourth)
 // for k_wgrad_tc's boxes; z_inner: third = z and fourth = y, else the other way round
@@ -1413,17 +1528,14 @@ template <int CIN, int COUT, int MODE, bool FLIP>
 dmtz_status conv(dmtz_cnn *net, const Dims &d, const bf16 *in, const bf16 *w, const float *bias, void *out,
                  const bf16 *aux, cudaStream_t st) {
     if (net->tensor_path == 2) {
-        Dims dt = make_xf_dims(d.W, d.H, d.D);
+        March m = make_march(d.W, d.H, d.D);
         CUtensorMap tm;
-        dmtz_status s = box_map(net, &tm, in, CIN, d.W, d.H, d.D, XF_GX, XF_GY, XF_GZ);
+        dmtz_status s = slice_map(net, &tm, in, CIN, m);
         if (s != DMTZ_OK) return s;
         int *err = net->tc_err;
-        void *args[] = {&tm, &dt, &w, &bias, &out, &aux, &err};
-        // each block holds 2 x 2 x 64 or 2 x 2 x 128 tensor-memory columns; no more blocks per SM
-        // than the 512 columns hold (a second block's allocation would wait for the first to exit)
-        const int cap = net->nsm * (int)(512 / (4 * xf_cols<COUT>()));
-        return launch_persistent(net, k_conv_tcx<CIN, COUT, MODE, FLIP>, kConvThreads, xf_smem<CIN, COUT>(),
-                                 dt.ntiles, cap, nullptr, st, args);
+        void *args[] = {&tm, &m, &w, &bias, &out, &aux, &err};
+        return launch_persistent(net, k_conv_tcx<CIN, COUT, MODE, FLIP>, CX_THREADS, cx_smem<CIN, COUT>(), m.outputs, net->nsm,
+                                 nullptr, st, args);
     }
     if (net->tensor_path) {
         Dims dt = make_tc_dims(d.W, d.H, d.D);

@@ -405,3 +405,21 @@ def test_gradient_tile_edges(net, dims):
         n = 27 * ci * co + co
         assert _rel(grads[o:o + n], ref_g[o:o + n]) < 2e-2, l
         o += n
+
+
+@pytest.mark.parametrize("dims", [(2, 8, 16), (3, 17, 9), (3, 9, 17), (1, 40, 33), (160, 2, 3), (37, 16, 8)])
+def test_forward_column_edges(net, dims):
+    """Grids at the edges of the default convolution's 8 x 16 columns, in both
+    orientations, with columns shorter and longer than a block's run
+    (tolerances as in the forward test)."""
+    W, H, D = dims
+    p = _params(14)
+    net.set_params(p)
+    feat_h, feat_d = _feat(15, dims)
+    out = torch.empty(W * H * D, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    net.forward(feat_d.data_ptr(), out.data_ptr(), dims)
+    got = out.cpu().numpy().reshape(D, H, W).astype(np.float64)
+    ref, _ = R.forward(feat_h, p.astype(np.float64))
+    assert _rel(got, ref) < 3e-3
+    assert np.abs(got - ref).max() < 2e-2 * np.abs(ref).max()
