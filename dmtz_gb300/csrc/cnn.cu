@@ -27,7 +27,7 @@
 //            (operands by ldmatrix.trans from the channels-last tiles);
 //            per-block partial sums, then a fixed-order reduction
 //            (deterministic).
-//   k_loss, k_loss_final, k_reduce, k_adam, k_pack: loss, gradient scaling,
+//   k_loss, k_reduce, k_adam, k_pack: loss, gradient scaling,
 //            Adam, bf16 weight refresh.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -1058,50 +1058,58 @@ __global__ void __launch_bounds__(512, 1) k_wgrad(Dims d, const bf16 *__restrict
 // and K = 16 vertices of an x-line serves nine taps, and the three x shifts have an
 // accumulator each: 27 taps in three products per line.  A tile is 16 x 8 x 2
 // vertices; its operands arrive by two TMA copies whose boxes put the lines
-// where the products want them:
-//   dz  as [y 8][z 4][channel group][x 16][8 channels], z from z0 - 1: the
-//       groups of three consecutive z lines are 256 bytes apart throughout (M)
-//   act as [z 2][y 10][channel group][x 18][8 channels], from x0 - 1, y0 - 1:
-//       the groups of three consecutive y lines are 288 bytes apart (N), an x
-//       shift is 16 bytes of the start address
-// Both operands are MN-major without swizzle: 8 vertices of one group are one
-// core matrix of 128 contiguous bytes, the next 8 vertices the next 128 bytes
-// (leading offset), the next group one stride offset on.  M is 128: the rows
-// past 3 COUT multiply whatever follows in shared memory and are not read.
-// Zeros outside the grid make every edge right.  The accumulators stay in
-// tensor memory over all tiles of a block and are written once, as this
-// block's partial sums.  Warps 2..5 sum the bias gradient from the same tiles.
-// Roles and bounded waits as in k_conv_tc, three stages; empty[s] takes the
-// MMAs' commit and one arrival per bias warp.
+// where the products want them, a vertex as one row of its channels, swizzled
+// over its own width (64 or 32 bytes):
+//   dz  as [y 8][z 4][x 16], z from z0 - 1: three consecutive z lines are M
+//   act as [z 2][y 10][x 18], from x0 - 1, y0 - 1: three consecutive y lines
+//       are N, an x shift is a row of the start address (the swizzle goes by
+//       address bits, so an operand may start at any row)
+// Both operands are MN-major: the channels of 8 vertices are one swizzle atom,
+// the next 8 vertices the next (stride offset), the next line of the operand
+// one leading offset on.  M is 128: the rows past 3 COUT multiply whatever
+// follows in the stage and are not read.  Zeros outside the grid make every
+// edge right.  The accumulators stay in tensor memory over all tiles of a block
+// and are written once, as this block's partial sums.
 //
-// Bound by the 16-byte rows of the copies (3488 per 32 -> 32 tile) and the
-// products' shared-memory reads (7 KB each, 48 per tile).  100 x 75 x 53: 35 us
-// for 32 -> 32, 30 us for 16 -> 32 and 32 -> 16 (mma.sync: 98, 68 and 60).
-constexpr int WG_X = 16, WG_Y = 8, WG_Z = 2, WG_ST = 3;
+// Roles: warps 0..2 issue one x shift each, so that one's waits are hidden
+// behind the others' products and every accumulator has its order; warp 3 brings
+// the tiles; warps 4..7 sum the bias gradient from the same tiles and write the
+// accumulators at the end.  empty[s] takes the commits of the three issuers and
+// one arrival per bias warp.  Waits are bounded as in k_conv_tc.
+//
+// Bound by the products: 48 per tile at 59 cycles (N = 96), a quarter of their
+// rows unused.  100 x 75 x 53: 29 us for 32 -> 32, 23 for 16 -> 32, 27 for 32 ->
+// 16 (mma.sync: 98, 68 and 60; 16-byte copy rows and one issuing lane: 35, 30, 30).
+constexpr int WG_X = 16, WG_Y = 8, WG_Z = 2, WG_ST = 4, WG_THREADS = 256;
 template <int CIN, int COUT>
 struct WgradTc {
-    static constexpr uint32_t ALINE = (WG_Z + 2) * (COUT / 8) * WG_X * 16, ABYTES = WG_Y * ALINE;
-    static constexpr uint32_t BLINE = (CIN / 8) * (WG_X + 2) * 16, BPLANE = (WG_Y + 2) * BLINE, BBYTES = WG_Z * BPLANE;
-    static constexpr uint32_t STAGE = ABYTES + BBYTES;
+    static constexpr uint32_t AROW = COUT * 2, ALINE = WG_X * AROW, ABYTES = WG_Y * (WG_Z + 2) * ALINE;
+    static constexpr uint32_t BROW = CIN * 2, BLINE = (WG_X + 2) * BROW, BPLANE = (WG_Y + 2) * BLINE, BBYTES = WG_Z * BPLANE;
+    static constexpr uint32_t STAGE = (ABYTES + BBYTES + 1023) / 1024 * 1024;
     static constexpr uint32_t N = 3 * CIN, COLS = N <= 64 ? 64 : 128, ALLOC = 3 * COLS <= 256 ? 256 : 512;
-    static constexpr size_t smem = 128 + (size_t)WG_ST * STAGE;
+    static constexpr size_t smem = 1024 + (size_t)WG_ST * STAGE;
     // the rows past 3 COUT of the last line stay inside the stage
-    static_assert((WG_Y - 1) * ALINE + (COUT / 8) * 256 + 16 * 256 <= STAGE, "operand reads stay inside the stage");
-    static_assert(ABYTES % 128 == 0 && STAGE % 128 == 0, "copies start on 128-byte boundaries");
+    static_assert(ABYTES - 3 * ALINE + (128 / COUT) * ALINE <= STAGE, "operand reads stay inside the stage");
+    static_assert(ABYTES % 1024 == 0, "both boxes start on a swizzle pattern");
 };
+// descriptor of an MN-major operand of such rows, `line` bytes from one line to the next
+template <int ROW>
+__device__ __forceinline__ uint64_t lines_desc(uint32_t addr, uint32_t line) {
+    static_assert(ROW == 64 || ROW == 32, "row widths");
+    return smem_desc(addr, line, 8 * ROW) | ((uint64_t)(ROW == 64 ? 4 : 6) << 61);
+}
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kConvThreads, 1) k_wgrad_tc(const __grid_constant__ CUtensorMap tdz,
+__global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_tc(const __grid_constant__ CUtensorMap tdz,
                                                             const __grid_constant__ CUtensorMap tact, int ntx, int nty,
                                                             i64 ntiles, float *__restrict__ part, int *err) {
     using T = WgradTc<CIN, COUT>;
-    constexpr int CO8 = COUT / 8;
     constexpr i64 NPAR = 27LL * COUT * CIN + COUT;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(8) uint64_t bar_full[WG_ST], bar_empty[WG_ST], bar_done;
     __shared__ float red[4][COUT];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t base = smem_addr(smem_raw) + ((128 - (smem_addr(smem_raw) & 127)) & 127);
+    const uint32_t base = (smem_addr(smem_raw) + 1023) & ~1023u;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&tmem_slot)),
                      "n"(T::ALLOC));
@@ -1113,80 +1121,86 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_wgrad_tc(const __grid_const
     if (tid == 0) {
         for (int s = 0; s < WG_ST; s++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(full(s)));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 5;\n" ::"r"(empty(s)));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 7;\n" ::"r"(empty(s)));
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(done));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 3;\n" ::"r"(done));
         asm volatile("fence.mbarrier_init.release.cluster;\n");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n");
     const uint32_t tmem = tmem_slot;
-    const i64 first = blockIdx.x, stride = gridDim.x;
-    const int ntile = first < ntiles ? (int)((ntiles - 1 - first) / stride + 1) : 0;
+    // this block's run of tiles, x fastest
+    const i64 per = ntiles / gridDim.x, rest = ntiles - per * gridDim.x;
+    const i64 first = blockIdx.x * per + min((i64)blockIdx.x, rest);
+    const int ntile = (int)per + (blockIdx.x < rest);
     bool failed = false;
 
-    if (warp == 0) {
-        if (lane == 0) {  // MMA issuer
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((T::N >> 3) << 17) |
-                                   ((uint32_t)(128 >> 4) << 24);
-            int s = 0;
-            uint32_t ph = 0;
-            for (int it = 0; it < ntile; it++) {
-                if (!mbar_wait(full(s), ph, kConvWaitPolls)) {
-                    failed = true;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;\n");
+    if (warp < 3) {  // MMA issuers, one x shift each
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((T::N >> 3) << 17) |
+                               ((uint32_t)(128 >> 4) << 24);
+        int s = 0;
+        uint32_t ph = 0;
+        for (int it = 0; it < ntile; it++) {
+            if (!__all_sync(0xffffffffu, mbar_wait(full(s), ph, kConvWaitPolls))) {
+                failed = true;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n");
+            if (elect_one()) {
                 const uint32_t ab = base + (uint32_t)s * T::STAGE;
-                const uint64_t a0 = smem_desc(ab, 128, WG_X * 16), b0 = smem_desc(ab + T::ABYTES, 128, (WG_X + 2) * 16);
+                const uint64_t a0 = lines_desc<T::AROW>(ab, T::ALINE),
+                               b0 = lines_desc<T::BROW>(ab + T::ABYTES + warp * T::BROW, T::BLINE);
 #pragma unroll
                 for (int q = 0; q < WG_Z; q++)
 #pragma unroll
                     for (int y = 0; y < WG_Y; y++)
-#pragma unroll
-                        for (int tx = 0; tx < 3; tx++)
-                            tc_mma(tmem + (uint32_t)tx * T::COLS, a0 + ((y * T::ALINE + q * CO8 * WG_X * 16) >> 4),
-                                   b0 + ((q * T::BPLANE + y * T::BLINE + tx * 16) >> 4), idesc, (it | q | y) != 0);
-                asm volatile(
-                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(empty(s)));
-                if (++s == WG_ST) {
-                    s = 0;
-                    ph ^= 1;
-                }
+                        tc_mma(tmem + (uint32_t)warp * T::COLS, a0 + (((y * (WG_Z + 2) + q) * T::ALINE) >> 4),
+                               b0 + ((q * T::BPLANE + y * T::BLINE) >> 4), idesc, (it | q | y) != 0);
+                tc_commit(empty(s));
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(done));
-            if (!mbar_wait(done, 0u, kConvWaitPolls)) failed = true;  // every MMA issued is done
+            __syncwarp();
+            if (++s == WG_ST) {
+                s = 0;
+                ph ^= 1;
+            }
         }
+        if (elect_one()) tc_commit(done);
         __syncwarp();
-    } else if (warp == 1) {
+        if (!mbar_wait(done, 0u, kConvWaitPolls)) failed = true;  // every MMA issued is done
+    } else if (warp == 3) {
         if (lane == 0) {  // operand producer
             int issued = 0, s = 0;
             uint32_t ph = 0;
+            int x = (int)(first % ntx), y = (int)((first / ntx) % nty), z = (int)(first / ((i64)ntx * nty));
             for (int it = 0; it < ntile; it++) {
                 if (it >= WG_ST && !mbar_wait(empty(s), ph ^ 1u, kConvWaitPolls)) {
                     failed = true;
                     break;
                 }
-                const i64 tile = first + it * stride;
-                const int x0 = (int)(tile % ntx) * WG_X, y0 = (int)((tile / ntx) % nty) * WG_Y,
-                          z0 = (int)(tile / ((i64)ntx * nty)) * WG_Z;
                 const uint32_t dst = base + (uint32_t)s * T::STAGE, bar = full(s);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(T::STAGE));
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(T::ABYTES + T::BBYTES));
                 asm volatile(
-                    "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, "
-                    "{%2, %3, %4, %5, %6}], [%7];\n" ::"r"(dst),
-                    "l"(reinterpret_cast<uint64_t>(&tdz)), "r"(0), "r"(x0), "r"(0), "r"(z0 - 1), "r"(y0), "r"(bar)
+                    "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, "
+                    "{%2, %3, %4, %5}], [%6];\n" ::"r"(dst),
+                    "l"(reinterpret_cast<uint64_t>(&tdz)), "r"(0), "r"(x * WG_X), "r"(z * WG_Z - 1), "r"(y * WG_Y), "r"(bar)
                     : "memory");
                 asm volatile(
-                    "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, "
-                    "{%2, %3, %4, %5, %6}], [%7];\n" ::"r"(dst + T::ABYTES),
-                    "l"(reinterpret_cast<uint64_t>(&tact)), "r"(0), "r"(x0 - 1), "r"(0), "r"(y0 - 1), "r"(z0), "r"(bar)
+                    "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, "
+                    "{%2, %3, %4, %5}], [%6];\n" ::"r"(dst + T::ABYTES),
+                    "l"(reinterpret_cast<uint64_t>(&tact)), "r"(0), "r"(x * WG_X - 1), "r"(y * WG_Y - 1), "r"(z * WG_Z), "r"(bar)
                     : "memory");
                 issued = it + 1;
                 if (++s == WG_ST) {
                     s = 0;
                     ph ^= 1;
+                }
+                if (++x == ntx) {
+                    x = 0;
+                    if (++y == nty) {
+                        y = 0;
+                        z++;
+                    }
                 }
             }
             // the copies still in flight land before the block leaves
@@ -1195,7 +1209,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_wgrad_tc(const __grid_const
         }
         __syncwarp();
     } else {  // bias gradient, then the accumulators
-        const int w = warp - 2;
+        const int w = warp - 4;
         float b[COUT];
 #pragma unroll
         for (int c = 0; c < COUT; c++) b[c] = 0.f;
@@ -1206,16 +1220,18 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_wgrad_tc(const __grid_const
                 failed = true;
                 break;
             }
-            // lines 2 w and 2 w + 1 of both planes: lane = x + 16 * plane
-            const uint32_t ab = base + (uint32_t)s * T::STAGE + (uint32_t)((lane >> 4) + 1) * (CO8 * WG_X * 16) + (lane & 15) * 16;
+            // lines 2 w and 2 w + 1 of both planes: lane = x + 16 * plane; the row's
+            // 16-byte chunks are permuted by the address bits above a pair of rows
+            const uint32_t row = (uint32_t)((lane >> 4) + 1) * T::ALINE + (lane & 15) * T::AROW;
+            const uint32_t ab = base + (uint32_t)s * T::STAGE + row, turn = (row >> 7) & (COUT / 8 - 1);
 #pragma unroll
             for (int y = 0; y < 2; y++)
 #pragma unroll
-                for (int gch = 0; gch < CO8; gch++) {
+                for (int gch = 0; gch < COUT / 8; gch++) {
                     uint32_t r[4];
                     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n"
                                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                                 : "r"(ab + (uint32_t)(2 * w + y) * T::ALINE + gch * (WG_X * 16)));
+                                 : "r"(ab + (uint32_t)(2 * w + y) * ((WG_Z + 2) * T::ALINE) + ((gch ^ turn) << 4)));
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
                         b[gch * 8 + 2 * k] += __uint_as_float(r[k] << 16);
@@ -1267,22 +1283,33 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_wgrad_tc(const __grid_const
 
 // grad[i] = scale * sum over blocks of part[b][i], in a fixed order: eight
 // threads per parameter take every eighth block, then their sums are added
-// pairwise (one thread per parameter: 304 loads in turn, 19 us; so: 7)
+// pairwise.  One launch for all layers, whose sums lie one after the other (one
+// thread per parameter and a launch per layer: 304 loads in turn, 4 x 19 us; so:
+// 15 us)
 constexpr int kRedWays = 8;
-__global__ void __launch_bounds__(256) k_reduce(const float *__restrict__ part, int nblk, i64 n,
-                                                const float *__restrict__ scale, float *__restrict__ grad) {
+struct Partials {
+    const float *part[NLAYER];
+    int nblk[NLAYER], first[NLAYER + 1];  // blocks that wrote; first block here
+    i64 n[NLAYER], grad[NLAYER];
+};
+__global__ void __launch_bounds__(256) k_reduce(const Partials p, const float *__restrict__ scale, float *__restrict__ grad) {
     __shared__ float sm[kRedWays][32];
-    const int col = threadIdx.x & 31, way = threadIdx.x >> 5;
-    const i64 i = (i64)blockIdx.x * 32 + col;
+    int l = 0;
+    while ((int)blockIdx.x >= p.first[l + 1]) l++;
+    const float *part = p.part[l];
+    const int nblk = p.nblk[l], col = threadIdx.x & 31, way = threadIdx.x >> 5;
+    const i64 n = p.n[l], i = (i64)((int)blockIdx.x - p.first[l]) * 32 + col;
     float s = 0.f;
-    if (i < n)
+    if (i < n) {
+#pragma unroll 8
         for (int b = way; b < nblk; b += kRedWays) s += part[(i64)b * n + i];
+    }
     sm[way][col] = s;
     __syncthreads();
     if (way == 0 && i < n) {
         const float a = (sm[0][col] + sm[1][col]) + (sm[2][col] + sm[3][col]);
         const float b = (sm[4][col] + sm[5][col]) + (sm[6][col] + sm[7][col]);
-        grad[i] = (a + b) * *scale;
+        grad[p.grad[l] + i] = (a + b) * *scale;
     }
 }
 
@@ -1290,11 +1317,17 @@ __global__ void __launch_bounds__(256) k_reduce(const float *__restrict__ part, 
 // Weighted over vertices (weight = the byte active[v], 0 = ignored):
 // L = sum w (tanh(o) - target)^2 / sum w.  Writes dL/do without the 1/sum w
 // factor (applied by k_reduce) into channel 0 of dz (16 channels, the others
-// 0), and per-block (weighted sum, sum of weights) partials.
-constexpr int kLossBlocks = 1024;
-__global__ void k_loss(i64 V, const float *__restrict__ o, const float *__restrict__ target,
-                       const uint8_t *__restrict__ active, bf16 *__restrict__ dz, double *__restrict__ part) {
-    double ls = 0.0, cnt = 0.0;
+// 0), and per-block (weighted sum, sum of weights) partials; the block that
+// finishes last adds those in a fixed order: res[0] = mean loss, res[1] = sum of
+// weights, scale = 1 / that (0 if none).  (Added by one thread of a kernel of
+// its own: 14 + 109 us at 100 x 75 x 53; so: 13)
+constexpr int kLossBlocks = 608;  // few: the blocks' sums are in double precision, which is slow here
+__global__ void __launch_bounds__(256) k_loss(i64 V, const float *__restrict__ o, const float *__restrict__ target,
+                                              const uint8_t *__restrict__ active, bf16 *__restrict__ dz,
+                                              double *__restrict__ part, unsigned *__restrict__ ticket,
+                                              double *__restrict__ res, float *__restrict__ scale) {
+    double ls = 0.0;
+    i64 cnt = 0;  // whole weights
     for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (i64)gridDim.x * blockDim.x) {
         float gval = 0.f;
         const float w = (float)active[v];
@@ -1302,15 +1335,15 @@ __global__ void k_loss(i64 V, const float *__restrict__ o, const float *__restri
             const float y = tanhf(o[v]);
             const float e = y - target[v];
             ls += (double)w * e * e;
-            cnt += w;
+            cnt += active[v];
             gval = 2.f * w * e * (1.f - y * y);
         }
         const __nv_bfloat162 lo = __floats2bfloat162_rn(gval, 0.f);
-        uint4 first = make_uint4(*reinterpret_cast<const uint32_t *>(&lo), 0u, 0u, 0u);
-        reinterpret_cast<uint4 *>(dz + v * 16)[0] = first;
-        reinterpret_cast<uint4 *>(dz + v * 16)[1] = make_uint4(0u, 0u, 0u, 0u);
+        st32(dz + v * 16, Vec8{{*reinterpret_cast<const uint32_t *>(&lo), 0u, 0u, 0u, 0u, 0u, 0u, 0u}});
     }
-    __shared__ double sl[32], sc[32];
+    __shared__ double sl[256];
+    __shared__ i64 sc[256];
+    __shared__ unsigned turn;
     for (int off = 16; off > 0; off >>= 1) {
         ls += __shfl_down_sync(0xffffffffu, ls, off);
         cnt += __shfl_down_sync(0xffffffffu, cnt, off);
@@ -1322,41 +1355,43 @@ __global__ void k_loss(i64 V, const float *__restrict__ o, const float *__restri
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double a = 0.0, b = 0.0;
+        double a = 0.0;
+        i64 b = 0;
         for (int i = 0; i < (int)(blockDim.x >> 5); i++) {
             a += sl[i];
             b += sc[i];
         }
         part[2 * blockIdx.x] = a;
-        part[2 * blockIdx.x + 1] = b;
+        part[2 * blockIdx.x + 1] = (double)b;
+        __threadfence();
+        turn = atomicAdd(ticket, 1u);
     }
-}
-// res[0] = mean loss, res[1] = sum of weights; scale = 1 / that (0 if none)
-// (one block of 256 threads; a fixed order.  By one thread 109 us, so 6)
-__global__ void __launch_bounds__(256) k_loss_final(const double *__restrict__ part, int nblk, double *__restrict__ res,
-                                                    float *__restrict__ scale) {
-    __shared__ double sa[256], sb[256];
-    double a = 0.0, b = 0.0;
-    for (int i = threadIdx.x; i < nblk; i += 256) {
-        a += part[2 * i];
-        b += part[2 * i + 1];
-    }
-    sa[threadIdx.x] = a;
-    sb[threadIdx.x] = b;
     __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) {
-            sa[threadIdx.x] += sa[threadIdx.x + o];
-            sb[threadIdx.x] += sb[threadIdx.x + o];
+    if (turn != gridDim.x - 1) return;
+    __threadfence();
+    double a = 0.0;
+    i64 n = 0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += 256) {
+        a += __ldcg(part + 2 * i);
+        n += (i64)__ldcg(part + 2 * i + 1);
+    }
+    sl[threadIdx.x] = a;
+    sc[threadIdx.x] = n;
+    __syncthreads();
+    for (int k = 128; k > 0; k >>= 1) {
+        if (threadIdx.x < k) {
+            sl[threadIdx.x] += sl[threadIdx.x + k];
+            sc[threadIdx.x] += sc[threadIdx.x + k];
         }
         __syncthreads();
     }
     if (threadIdx.x != 0) return;
-    a = sa[0];
-    b = sb[0];
+    a = sl[0];
+    const double b = (double)sc[0];
     res[0] = b > 0 ? a / b : 0.0;
     res[1] = b;
     *scale = b > 0 ? (float)(1.0 / b) : 0.f;
+    *ticket = 0u;
 }
 
 // ------------------------------------------------------------ Adam + weights
@@ -1394,8 +1429,7 @@ struct dmtz_cnn {
     std::string err;
     float *w = nullptr, *grad = nullptr, *m1 = nullptr, *m2 = nullptr;  // kParams each
     bf16 *wf = nullptr, *wt = nullptr;  // bf16 weights, forward and transposed, per layer at woff[l]
-    float *part = nullptr;              // weight-gradient partials, part_blocks x (largest layer)
-    int part_blocks = 0;
+    float *part = nullptr;              // weight-gradient partials: nsm x all layers, or 2 nsm x one layer (mma.sync)
     double *lpart = nullptr, *lres = nullptr;
     float *scale = nullptr;
     i64 step = 0;
@@ -1409,6 +1443,7 @@ struct dmtz_cnn {
     const float *last_out = nullptr;
     // convolutions on tcgen05 (1, the default) or on mma.sync (0)
     int tensor_path = 2;
+    unsigned *lticket = nullptr;
     int *tc_err = nullptr;  // set by a tcgen05 convolution whose wait timed out
     // warm-start scratch
     i64 capS = 0;
@@ -1513,15 +1548,15 @@ dmtz_status slice_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, co
     const cuuint32_t box[4] = {(cuuint32_t)C, CX_GA, CX_GB, CX_NX};
     return encode_map(net, tm, act, 4, dims, strides, box, C == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
-// tensor map of the same tensor as (8 channels, x, channel group, third, fourth)
-// for k_wgrad_tc's boxes; z_inner: third = z and fourth = y, else the other way round
-dmtz_status line_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, int W, int H, int D, bool z_inner, int bx,
-                     int b3, int b4) {
-    const cuuint64_t sx = (cuuint64_t)C * 2, sy = sx * W, sz = sy * H;
-    const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)C / 8, (cuuint64_t)(z_inner ? D : H), (cuuint64_t)(z_inner ? H : D)};
-    const cuuint64_t strides[4] = {sx, 16, z_inner ? sz : sy, z_inner ? sy : sz};
-    const cuuint32_t box[5] = {8, (cuuint32_t)bx, (cuuint32_t)C / 8, (cuuint32_t)b3, (cuuint32_t)b4};
-    return encode_map(net, tm, act, 5, dims, strides, box);
+// and for k_wgrad_tc's lines: whole vertices, axes (channel, x, third, fourth);
+// z_inner: third = z and fourth = y, else the other way round
+dmtz_status line_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, const Dims &d, bool z_inner, int bx, int b3,
+                     int b4) {
+    const cuuint64_t sx = (cuuint64_t)C * 2, sy = sx * d.W, sz = sy * d.H;
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)d.W, (cuuint64_t)(z_inner ? d.D : d.H), (cuuint64_t)(z_inner ? d.H : d.D)};
+    const cuuint64_t strides[3] = {sx, z_inner ? sz : sy, z_inner ? sy : sz};
+    const cuuint32_t box[4] = {(cuuint32_t)C, (cuuint32_t)bx, (cuuint32_t)b3, (cuuint32_t)b4};
+    return encode_map(net, tm, act, 4, dims, strides, box, C == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
 template <int CIN, int COUT, int MODE, bool FLIP>
@@ -1553,32 +1588,48 @@ dmtz_status conv(dmtz_cnn *net, const Dims &d, const bf16 *in, const bf16 *w, co
                              nullptr, st, args);
 }
 
+// gradients of layers [from, to) from their blocks' partial sums
+dmtz_status reduce(dmtz_cnn *net, Partials &p, int from, int to, cudaStream_t st) {
+    int blocks = 0;
+    for (int l = 0; l < NLAYER; l++) {
+        p.first[l] = blocks;
+        p.grad[l] = layer_offset(l);
+        p.n[l] = layer_params(l);
+        if (l >= from && l < to) blocks += (int)((p.n[l] + 31) / 32);
+    }
+    p.first[NLAYER] = blocks;
+    k_reduce<<<blocks, 256, 0, st>>>(p, net->scale, net->grad);
+    NCK(cudaGetLastError());
+    return DMTZ_OK;
+}
+// the blocks' partial sums of a layer; on the tcgen05 paths the caller reduces
+// all layers at once
 template <int CIN, int COUT>
-dmtz_status wgrad(dmtz_cnn *net, const Dims &d, const bf16 *act, const bf16 *dz, float *grad_out, cudaStream_t st) {
+dmtz_status wgrad(dmtz_cnn *net, const Dims &d, const bf16 *act, const bf16 *dz, int layer, Partials &p, cudaStream_t st) {
     float *part = net->part;
     int used = 0;
     dmtz_status s;
     if (net->tensor_path) {
+        part += net->nsm * layer_offset(layer);
         CUtensorMap tdz, tact;
-        if ((s = line_map(net, &tdz, dz, COUT, d.W, d.H, d.D, true, WG_X, WG_Z + 2, WG_Y)) != DMTZ_OK ||
-            (s = line_map(net, &tact, act, CIN, d.W, d.H, d.D, false, WG_X + 2, WG_Y + 2, WG_Z)) != DMTZ_OK)
+        if ((s = line_map(net, &tdz, dz, COUT, d, true, WG_X, WG_Z + 2, WG_Y)) != DMTZ_OK ||
+            (s = line_map(net, &tact, act, CIN, d, false, WG_X + 2, WG_Y + 2, WG_Z)) != DMTZ_OK)
             return s;
         int ntx = (d.W + WG_X - 1) / WG_X, nty = (d.H + WG_Y - 1) / WG_Y, *err = net->tc_err;
         i64 ntiles = (i64)ntx * nty * ((d.D + WG_Z - 1) / WG_Z);
         void *args[] = {&tdz, &tact, &ntx, &nty, &ntiles, &part, &err};
-        s = launch_persistent(net, k_wgrad_tc<CIN, COUT>, kConvThreads, WgradTc<CIN, COUT>::smem, ntiles, net->nsm, &used, st,
-                              args);
+        s = launch_persistent(net, k_wgrad_tc<CIN, COUT>, WG_THREADS, WgradTc<CIN, COUT>::smem, ntiles, net->nsm, &used,
+                              st, args);
     } else {
         Dims dd = d;
         void *args[] = {&dd, &act, &dz, &part};
-        s = launch_persistent(net, k_wgrad<CIN, COUT>, 512, wgrad_smem<CIN, COUT>(), d.ntiles, net->part_blocks, &used, st,
+        s = launch_persistent(net, k_wgrad<CIN, COUT>, 512, wgrad_smem<CIN, COUT>(), d.ntiles, 2 * net->nsm, &used, st,
                               args);
     }
     if (s != DMTZ_OK) return s;
-    const i64 n = 27LL * COUT * CIN + COUT;
-    k_reduce<<<(unsigned)((n + 31) / 32), 256, 0, st>>>(net->part, used, n, net->scale, grad_out);
-    NCK(cudaGetLastError());
-    return DMTZ_OK;
+    p.part[layer] = part;
+    p.nblk[layer] = used;
+    return net->tensor_path ? DMTZ_OK : reduce(net, p, layer, layer + 1, st);
 }
 
 dmtz_status pack(dmtz_cnn *net, cudaStream_t st) {
@@ -1704,15 +1755,13 @@ dmtz_status dmtz_cnn_create(dmtz_cnn **out, int device, uint64_t seed) {
     if (cudaDeviceGetAttribute(&net->nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
         return bail(DMTZ_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(DMTZ_ERR_CUDA);
-    net->part_blocks = 2 * net->nsm;
-    i64 largest = 0;
-    for (int l = 0; l < NLAYER; l++) largest = std::max(largest, layer_params(l));
     if (nalloc(&net->w, kParams) || nalloc(&net->grad, kParams) || nalloc(&net->m1, kParams) ||
         nalloc(&net->m2, kParams) || nalloc(&net->wf, kWeights) || nalloc(&net->wt, kWeights) ||
-        nalloc(&net->part, (i64)net->part_blocks * largest) || nalloc(&net->lpart, 2 * kLossBlocks) ||
-        nalloc(&net->lres, 2) || nalloc(&net->scale, 1) || nalloc(&net->tc_err, 1))
+        nalloc(&net->part, net->nsm * kParams) || nalloc(&net->lpart, 2 * kLossBlocks) ||
+        nalloc(&net->lres, 2) || nalloc(&net->lticket, 1) || nalloc(&net->scale, 1) || nalloc(&net->tc_err, 1))
         return bail(DMTZ_ERR_CUDA);
-    if (cudaMemset(net->tc_err, 0, sizeof(int)) != cudaSuccess) return bail(DMTZ_ERR_CUDA);
+    if (cudaMemset(net->tc_err, 0, sizeof(int)) != cudaSuccess || cudaMemset(net->lticket, 0, sizeof(unsigned)) != cudaSuccess)
+        return bail(DMTZ_ERR_CUDA);
     // He-uniform weights (bound sqrt(6 / fan_in)); the output layer 0.1x and
     // only its channel 0 nonzero; zero biases
     std::vector<float> h((size_t)kParams, 0.f);
@@ -1738,7 +1787,7 @@ void dmtz_cnn_destroy(dmtz_cnn *net) {
     cudaSetDevice(net->device);
     if (net->stream) cudaStreamSynchronize(net->stream);
     for (void *p : {(void *)net->w, (void *)net->grad, (void *)net->m1, (void *)net->m2, (void *)net->wf,
-                    (void *)net->wt, (void *)net->part, (void *)net->lpart, (void *)net->lres, (void *)net->scale,
+                    (void *)net->wt, (void *)net->part, (void *)net->lpart, (void *)net->lres, (void *)net->lticket, (void *)net->scale,
                     (void *)net->a[0], (void *)net->a[1], (void *)net->dz4, (void *)net->gA, (void *)net->gB,
                     (void *)net->feat, (void *)net->active, (void *)net->out, (void *)net->tc_err})
         cudaFree(p);
@@ -1856,22 +1905,23 @@ dmtz_status dmtz_cnn_backward(dmtz_cnn *net, int W, int H, int D, const float *t
     cudaStream_t st = net->stream;
     const Dims d = make_dims(W, H, D);
     const i64 V = (i64)W * H * D;
-    k_loss<<<kLossBlocks, 256, 0, st>>>(V, net->last_out, target, active, net->dz4, net->lpart);
-    k_loss_final<<<1, 256, 0, st>>>(net->lpart, kLossBlocks, net->lres, net->scale);
+    k_loss<<<kLossBlocks, 256, 0, st>>>(V, net->last_out, target, active, net->dz4, net->lpart, net->lticket, net->lres,
+                                         net->scale);
     NCK(cudaGetLastError());
     bf16 *a1 = net->a[0], *a2 = net->a[1], *a3 = net->a[2];
-    float *gr = net->grad;
+    Partials p{};
     // layer 4: data gradient into a3's space (ReLU mask of a3), weight gradient
     if ((s = conv<16, 32, 2, true>(net, d, net->dz4, net->wt + woff(3), nullptr, net->gA, a3, st)) != DMTZ_OK) return s;
-    if ((s = wgrad<32, 16>(net, d, a3, net->dz4, gr + layer_offset(3), st)) != DMTZ_OK) return s;
+    if ((s = wgrad<32, 16>(net, d, a3, net->dz4, 3, p, st)) != DMTZ_OK) return s;
     // layer 3
     if ((s = conv<32, 32, 2, true>(net, d, net->gA, net->wt + woff(2), nullptr, net->gB, a2, st)) != DMTZ_OK) return s;
-    if ((s = wgrad<32, 32>(net, d, a2, net->gA, gr + layer_offset(2), st)) != DMTZ_OK) return s;
+    if ((s = wgrad<32, 32>(net, d, a2, net->gA, 2, p, st)) != DMTZ_OK) return s;
     // layer 2
     if ((s = conv<32, 32, 2, true>(net, d, net->gB, net->wt + woff(1), nullptr, net->gA, a1, st)) != DMTZ_OK) return s;
-    if ((s = wgrad<32, 32>(net, d, a1, net->gB, gr + layer_offset(1), st)) != DMTZ_OK) return s;
+    if ((s = wgrad<32, 32>(net, d, a1, net->gB, 1, p, st)) != DMTZ_OK) return s;
     // layer 1 (no data gradient of the features)
-    if ((s = wgrad<16, 32>(net, d, net->last_feat, net->gA, gr + layer_offset(0), st)) != DMTZ_OK) return s;
+    if ((s = wgrad<16, 32>(net, d, net->last_feat, net->gA, 0, p, st)) != DMTZ_OK) return s;
+    if (net->tensor_path && (s = reduce(net, p, 0, NLAYER, st)) != DMTZ_OK) return s;
     double res[2] = {0, 0};
     NCK(cudaMemcpyAsync(res, net->lres, sizeof(res), cudaMemcpyDeviceToHost, st));
     NCK(cudaStreamSynchronize(st));
@@ -1950,8 +2000,13 @@ extern "C" dmtz_status dmtz_cnn_profile(dmtz_cnn *net, int W, int H, int D, cons
             },
             ms[2]);
     if (s == DMTZ_OK)
-        s = timed([&]() { return wgrad<32, 32>(net, d, net->a[1], net->gB, net->grad + layer_offset(2), st); },
-                  ms[3]);
+        s = timed(
+            [&]() {
+                Partials p{};
+                const dmtz_status r = wgrad<32, 32>(net, d, net->a[1], net->gB, 2, p, st);
+                return r == DMTZ_OK && net->tensor_path ? reduce(net, p, 2, 3, st) : r;
+            },
+            ms[3]);
     cudaEventDestroy(e[0]);
     cudaEventDestroy(e[1]);
     cudaMemcpyAsync(net->w, keep, sizeof(float) * kParams, cudaMemcpyDeviceToDevice, st);
