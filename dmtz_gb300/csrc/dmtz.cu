@@ -159,6 +159,17 @@ struct CpLists {
     i64 cap[4];
 };
 
+// Cells per warp for n cells (a power of two).  The cells of a warp take different
+// branches of a rule, each a chain of loads, one after the other, so as long as
+// there are warps to spare a warp takes few cells: 256-thread blocks of the rules
+// run three to an SM, and the grid is eight blocks per SM.
+__device__ __forceinline__ int cells_per_warp(i64 n) {
+    const i64 warps = (i64)gridDim.x * 3;
+    int c = 1;
+    while (c < 32 && n > c * warps) c *= 2;
+    return c;
+}
+
 // fix_minimum, [fix_saddle, fix_2saddle], fix_maximum over the current lists
 // (the host never runs this on an overflowed list; the clamp only keeps
 // every read inside the allocation).  The four lists are taken one behind the
@@ -167,25 +178,31 @@ struct CpLists {
 // rounds of noisy fields: millions of cells) all warps of the GPU are in the
 // same rule's code.  The rules only set request bits, so the order does not
 // matter.
-__global__ void __launch_bounds__(kBlock) k_fix_cp(const __grid_constant__ RuleCtx c, CpLists L, int preserve_saddles) {
+__global__ void __launch_bounds__(kBlock) k_fix_cp(const __grid_constant__ RuleCtx c, const __grid_constant__ CpLists L, int preserve_saddles) {
     __shared__ RuleTab tab;
     const i64 n0 = min((i64)L.n[0], L.cap[0]), n1 = preserve_saddles ? min((i64)L.n[1], L.cap[1]) : 0,
               n2 = preserve_saddles ? min((i64)L.n[2], L.cap[2]) : 0, n3 = min((i64)L.n[3], L.cap[3]);
-    const i64 e0 = (n0 + 31) & ~31ll, e1 = e0 + ((n1 + 31) & ~31ll), e2 = e1 + ((n2 + 31) & ~31ll), e3 = e2 + n3;
-    i64 i = (i64)blockIdx.x * blockDim.x;
-    if (i >= e3) return;
+    const int per = cells_per_warp(n0 + n1 + n2 + n3), lane = threadIdx.x & 31;
+    auto warps = [&](i64 n) { return (n + per - 1) / per; };
+    const i64 w0 = warps(n0), w1 = w0 + warps(n1), w2 = w1 + warps(n2), w3 = w2 + warps(n3);
+    constexpr int NW = kBlock / 32;
+    if ((i64)blockIdx.x * NW >= w3) return;
     load_rule_tab(tab);
     const Rules R{c, tab};
-    for (i += threadIdx.x; i < e3; i += (i64)gridDim.x * blockDim.x) {
-        if (i < e0) {
-            if (i < n0) rule_min(R, L.l[0][i]);
-        } else if (i < e1) {
-            if (i - e0 < n1) rule_saddle(R, L.l[1][i - e0]);
-        } else if (i < e2) {
-            if (i - e1 < n2) rule_2saddle(R, L.l[2][i - e1]);
-        } else {
-            rule_max(R, L.l[3][i - e2]);
+    for (i64 w = (i64)blockIdx.x * NW + (threadIdx.x >> 5); w < w3; w += (i64)gridDim.x * NW) {
+        Lowered o;
+        const int k = w < w0 ? 0 : w < w1 ? 1 : w < w2 ? 2 : 3;
+        const i64 i = (w - (k == 0 ? 0 : k == 1 ? w0 : k == 2 ? w1 : w2)) * per + lane;
+        if (lane < per && i < (k == 0 ? n0 : k == 1 ? n1 : k == 2 ? n2 : n3)) {
+            const i64 code = L.l[k][i];
+            if (k == 0) rule_min(R, code, o);
+            else if (k == 1) rule_saddle(R, code, o);
+            else if (k == 2) rule_2saddle(R, code, o);
+            else rule_max(R, code, o);
         }
+        __syncwarp();
+        rescan_warp(c, o);
+        request_warp(c, o);
     }
 }
 
@@ -1049,16 +1066,27 @@ __global__ void k_ds_strict(const __grid_constant__ RuleCtx c, PathRec R, const 
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_fix_path(const __grid_constant__ RuleCtx c, PathRec P) {
+__global__ void __launch_bounds__(kBlock) k_fix_path(const __grid_constant__ RuleCtx c, const __grid_constant__ PathRec P) {
     __shared__ RuleTab tab;
-    const i64 na = min((i64)P.n[0], P.cap_as), nd = min((i64)P.n[1], P.cap_ds), ea = (na + 31) & ~31ll;
-    i64 i = (i64)blockIdx.x * blockDim.x;
-    if (i >= ea + nd) return;
+    const i64 na = min((i64)P.n[0], P.cap_as), nd = min((i64)P.n[1], P.cap_ds);
+    const int per = cells_per_warp(na + nd), lane = threadIdx.x & 31;
+    const i64 wa = (na + per - 1) / per, wd = wa + (nd + per - 1) / per;
+    constexpr int NW = kBlock / 32;
+    if ((i64)blockIdx.x * NW >= wd) return;
     load_rule_tab(tab);
     const Rules R{c, tab};
-    for (i += threadIdx.x; i < ea + nd; i += (i64)gridDim.x * blockDim.x) {
-        if (i < na) rule_as_path(R, P.as_cur[i]);
-        else if (i >= ea) rule_ds_path(R, P.ds_vert[i - ea]);
+    for (i64 w = (i64)blockIdx.x * NW + (threadIdx.x >> 5); w < wd; w += (i64)gridDim.x * NW) {
+        Lowered o;
+        const i64 i = (w < wa ? w : w - wa) * per + lane;
+        if (lane < per) {
+            if (w < wa) {
+                if (i < na) rule_as_path(R, P.as_cur[i], o);
+            } else if (i < nd) {
+                rule_ds_path(R, P.ds_vert[i], o);
+            }
+        }
+        __syncwarp();
+        request_warp(c, o);
     }
 }
 

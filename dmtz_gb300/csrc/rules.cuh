@@ -21,7 +21,10 @@
 // hundred instructions each, fetched cold in every launch) and the rule context was copied
 // to each thread's stack for the accessors that were called: a critical-point
 // round took 82 us on average on a noisy 97 x 61 x 75 field and 78 us at 16^3,
-// now 20 and 22 us (cold caches); 134 -> 54 us at 256^3.
+// then 20 and 22 us (cold caches); 134 -> 54 us at 256^3.  What was left were the
+// branches of a warp's cells one after the other and rescans by one thread: with a
+// cell per warp as long as there are warps, and the rescans by the warp, a cell
+// takes 4 to 6 k cycles of loads and at most 11 k (36 k before).
 //
 // A rule "lowers" a vertex: it asks for d_deltaBuffer[v] = get_delta(v).
 // get_delta depends only on v's own value and counter, which no rule
@@ -263,6 +266,131 @@ __device__ __forceinline__ double get_delta(const RuleCtx &c, i64 v) {
     if (c.edit_type == 1) return -ldexp(1.0, -c.cnt[v]) * c.bound;
     return __dmul_rn(__dsub_rn(__dsub_rn(c.f[v], c.bound), c.gv[v]), 0.5);  // x / 2, rounded the same
 }
+// The vertices that a rule lowers, at most four.  They are requested once the warp
+// is back together: a rule's branches hold no atomics, and the atomics of several
+// vertices do not wait for one another.  `rescan`: the two (edge) or three
+// (triangle) vertices are lowered only if rescan_warp finds no neighbour to lower
+// in their place.
+struct Lowered {
+    static constexpr i64 NONE = LLONG_MIN;
+    i64 v[4] = {NONE, NONE, NONE, NONE};
+    int rescan = 0;
+    __device__ __forceinline__ void add(i64 w) {
+        v[3] = v[2];
+        v[2] = v[1];
+        v[1] = v[0];
+        v[0] = w;
+    }
+};
+// components of the 14 neighbour directions, plus one, two bits each
+__host__ __device__ constexpr uint32_t pack_dirs(int axis) {
+    uint32_t w = 0;
+    for (int i = 0; i < 14; i++) w |= (uint32_t)(cxt::TOPO_DIRS[i][axis] + 1) << (2 * i);
+    return w;
+}
+// the directions as a set of (dx + 1) + 3 (dy + 1) + 9 (dz + 1)
+__host__ __device__ constexpr uint32_t mask_dirs() {
+    uint32_t m = 0;
+    for (int i = 0; i < 14; i++)
+        m |= 1u << ((cxt::TOPO_DIRS[i][0] + 1) + 3 * (cxt::TOPO_DIRS[i][1] + 1) + 9 * (cxt::TOPO_DIRS[i][2] + 1));
+    return m;
+}
+__device__ __forceinline__ bool is_neighbour(int dx, int dy, int dz) {
+    constexpr uint32_t M = mask_dirs();
+    return (unsigned)(dx + 1) < 3u && (unsigned)(dy + 1) < 3u && (unsigned)(dz + 1) < 3u &&
+           (M >> ((dx + 1) + 3 * (dy + 1) + 9 * (dz + 1)) & 1u);
+}
+// The rescans of a warp's rules.  Edge (v1, v2): argmin over the common neighbours n
+// with exactly one of v1, v2 above n in the ORIGINAL field (the rescan of
+// fix_saddle, main_3d.cu:2942-3015); triangle: argmin over those below exactly
+// two of its vertices (get_smallest_vertex, main_3d.cu:2115-2194).  A neighbour per lane,
+// two cells at a time: by one thread, a rescan took 10 k (edge) or 15 k cycles,
+// where the rest of a rule takes 4 to 6 k.
+__device__ __forceinline__ void rescan_warp(const RuleCtx &c, Lowered &o) {
+    const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
+    constexpr uint32_t X = pack_dirs(0), Y = pack_dirs(1), Z = pack_dirs(2);
+    unsigned pending = __ballot_sync(full, o.rescan != 0);
+    while (pending) {
+        const int a = __ffs(pending) - 1;
+        pending &= pending - 1;
+        const int b = pending ? __ffs(pending) - 1 : a;
+        pending &= pending - 1;  // 0 stays 0
+        const int src = lane < 16 ? a : b, i = lane & 15;
+        const int nv = __shfl_sync(full, o.rescan, src);
+        const i64 v1 = __shfl_sync(full, o.v[0], src), v2 = __shfl_sync(full, o.v[1], src), v3 = __shfl_sync(full, o.v[2], src);
+        uint64_t bk = ~0ull;
+        i64 bid = LLONG_MAX;
+        if (i < 14) {
+            const int dx = (int)(X >> (2 * i) & 3u) - 1, dy = (int)(Y >> (2 * i) & 3u) - 1, dz = (int)(Z >> (2 * i) & 3u) - 1;
+            int x, y, z, x2, y2, z2, x3 = 0, y3 = 0, z3 = 0;
+            decode_v(c.g, v1, x, y, z);
+            decode_v(c.g, v2, x2, y2, z2);
+            if (nv == 3) decode_v(c.g, v3, x3, y3, z3);
+            x += dx;
+            y += dy;
+            z += dz;
+            if (inb(c.g, x, y, z) && is_neighbour(x - x2, y - y2, z - z2) &&
+                (nv == 2 || is_neighbour(x - x3, y - y3, z - z3))) {
+                const i64 n = x + (i64)y * c.g.W + (i64)z * c.g.WH;
+                const uint64_t kn = okey(c.f[n]), k1 = okey(c.f[v1]), k2 = okey(c.f[v2]), k3 = nv == 3 ? okey(c.f[v3]) : 0;
+                const int above = (k1 > kn || (k1 == kn && v1 > n)) + (k2 > kn || (k2 == kn && v2 > n)) +
+                                  (nv == 3 && (k3 > kn || (k3 == kn && v3 > n)));
+                // (the reference starts from DBL_MAX and INT_MAX)
+                if (above == nv - 1 && (kn < DMTZ_KEY_DBL_MAX || (kn == DMTZ_KEY_DBL_MAX && n < INT_MAX))) {
+                    bk = kn;
+                    bid = n;
+                }
+            }
+        }
+#pragma unroll
+        for (int s = 8; s > 0; s >>= 1) {
+            const uint64_t ok = __shfl_xor_sync(full, bk, s);
+            const i64 oid = __shfl_xor_sync(full, bid, s);
+            if (ok < bk || (ok == bk && oid < bid)) {
+                bk = ok;
+                bid = oid;
+            }
+        }
+        const i64 ma = __shfl_sync(full, bid, 0), mb = __shfl_sync(full, bid, 16);
+        const i64 m = (int)lane == a ? ma : mb;
+        if (((int)lane == a || (int)lane == b) && m != LLONG_MAX) {
+            o.v[0] = m;
+            o.v[1] = o.v[2] = Lowered::NONE;
+        }
+    }
+}
+// every lane of a warp requests its vertices: one atomic per vertex, one per warp
+__device__ __forceinline__ void request_warp(const RuleCtx &c, const Lowered &o) {
+    const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
+    bool fresh[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        fresh[k] = false;
+        if (o.v[k] == Lowered::NONE) continue;
+        if (o.v[k] < 0 || o.v[k] >= c.g.V) {
+            atomicOr(c.err, ERR_OOB);
+            continue;
+        }
+        const uint32_t bit = 1u << (o.v[k] & 31);
+        fresh[k] = !(atomicOr(&c.reqbits[o.v[k] >> 5], bit) & bit);
+    }
+    unsigned m[4], total = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        m[k] = __ballot_sync(full, fresh[k]);
+        total += __popc(m[k]);
+    }
+    if (!total) return;
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(c.reqn, (unsigned long long)total);
+    at = __shfl_sync(full, at, 0);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const unsigned long long mine = at + __popc(m[k] & ((1u << lane) - 1u));
+        if (fresh[k] && (i64)mine < c.reqcap) c.reqlist[mine] = o.v[k];
+        at += __popc(m[k]);
+    }
+}
 // "lower v": the reference's swap(v, get_delta(v))
 __device__ __forceinline__ void lower(const RuleCtx &c, i64 v) {
     if (v < 0 || v >= c.g.V) {
@@ -289,61 +417,6 @@ __device__ __forceinline__ i64 fourth_of(i64 a, i64 b, i64 cc, i64 d, i64 v1, i6
     else if (cc != v1 && cc != v2 && cc != v3) v4 = cc;
     return v4;
 }
-// argmin over the common neighbours n of (v1, v2) with exactly one of v1, v2
-// above n in the ORIGINAL field (the rescan of fix_saddle, main_3d.cu:2942-3015)
-__device__ DMTZ_SHARED_CODE i64 rescan_edge(const RuleCtx &c, i64 v1, i64 v2) {
-    int x1, y1, z1, x2, y2, z2;
-    decode_v(c.g, v1, x1, y1, z1);
-    decode_v(c.g, v2, x2, y2, z2);
-    uint64_t bk = DMTZ_KEY_DBL_MAX;
-    i64 bid = INT_MAX;
-    bool found = false;
-    for (int i = 0; i < 14; i++) {
-        const int nx = x1 + TOPO_DIRS[i][0], ny = y1 + TOPO_DIRS[i][1], nz = z1 + TOPO_DIRS[i][2];
-        if (!inb(c.g, nx, ny, nz)) continue;
-        if (dir_of(nx - x2, ny - y2, nz - z2) < 0) continue;
-        const i64 n = nx + (i64)ny * c.g.W + (i64)nz * c.g.WH;
-        if (above_f(c, v1, n) != above_f(c, v2, n)) {
-            const uint64_t kn = okey(c.f[n]);
-            if (kn < bk || (kn == bk && n < bid)) {
-                bk = kn;
-                bid = n;
-                found = true;
-            }
-        }
-    }
-    return found ? bid : -1;
-}
-
-// get_smallest_vertex (main_3d.cu:2115-2194): common neighbours of a triangle
-// below exactly two of its vertices in the ORIGINAL field, argmin
-__device__ DMTZ_SHARED_CODE i64 smallest_vertex(const RuleCtx &c, i64 v1, i64 v2, i64 v3) {
-    int x1, y1, z1, x2, y2, z2, x3, y3, z3;
-    decode_v(c.g, v1, x1, y1, z1);
-    decode_v(c.g, v2, x2, y2, z2);
-    decode_v(c.g, v3, x3, y3, z3);
-    uint64_t bk = DMTZ_KEY_DBL_MAX;
-    i64 bid = INT_MAX;
-    bool found = false;
-    for (int i = 0; i < 14; i++) {
-        const int nx = x1 + TOPO_DIRS[i][0], ny = y1 + TOPO_DIRS[i][1], nz = z1 + TOPO_DIRS[i][2];
-        if (!inb(c.g, nx, ny, nz)) continue;
-        if (dir_of(nx - x2, ny - y2, nz - z2) < 0 || dir_of(nx - x3, ny - y3, nz - z3) < 0) continue;
-        const i64 n = nx + (i64)ny * c.g.W + (i64)nz * c.g.WH;
-        if (n == v1 || n == v2 || n == v3) continue;
-        const bool c1 = above_f(c, v1, n), c2 = above_f(c, v2, n), c3 = above_f(c, v3, n);
-        if ((c1 && c2 && !c3) || (c1 && !c2 && c3) || (!c1 && c2 && c3)) {
-            const uint64_t kn = okey(c.f[n]);
-            if (kn < bk || (kn == bk && n < bid)) {
-                bk = kn;
-                bid = n;
-                found = true;
-            }
-        }
-    }
-    return found ? bid : -1;
-}
-
 // --------------------------------------------------------------- cells as codes
 // Tables of the code arithmetic.  Offsets are (dx+1) | (dy+1) << 2 | (dz+1) <<
 // 4 (six bits), corners dx + 2 dy + 4 dz (three bits).
@@ -500,13 +573,13 @@ struct Rules {
 };
 
 // --------------------------------------------------------------- A8 fix_minimum
-__device__ __forceinline__ void rule_min(const Rules &R, i64 v) {
+__device__ __forceinline__ void rule_min(const Rules &R, i64 v, Lowered &o) {
     const i64 w = R.below(R.c.P, v >> 5);
-    lower(R.c, w >= 0 ? w : v >> 5);
+    o.add(w >= 0 ? w : v >> 5);
 }
 
 // --------------------------------------------------------------- A9 fix_saddle
-__device__ __forceinline__ void rule_saddle(const Rules &R, i64 id) {
+__device__ __forceinline__ void rule_saddle(const Rules &R, i64 id, Lowered &o) {
     const RuleCtx &c = R.c;
     i64 v1, v2;
     R.verts(id, v1, v2);
@@ -517,12 +590,12 @@ __device__ __forceinline__ void rule_saddle(const Rules &R, i64 id) {
         const i64 false_v2 = R.below(c.Q, v1);
         if (false_v2 < 0) return;
         const double a = gval(c, v2), b = gval(c, false_v2);
-        if (a > b || (a == b && v2 > false_v2)) lower(c, v2);
+        if (a > b || (a == b && v2 > false_v2)) o.add(v2);
         return;
     }
     const i64 qe = pe == -1 ? R.edge_partner(c.Q, id) : -1;
     if (pe == -1 && (qe == -1 || cell_kind(qe) == KIND_VERTEX)) {
-        if (qe != -1) lower(c, qe >> 5);
+        if (qe != -1) o.add(qe >> 5);
         return;
     }
     const i64 face = pe != -1 ? pe : qe;
@@ -530,7 +603,7 @@ __device__ __forceinline__ void rule_saddle(const Rules &R, i64 id) {
     const bool g1 = above_g(c, v1, v3), g2 = above_g(c, v2, v3), f1 = above_f(c, v1, v3), f2 = above_f(c, v2, v3);
     if (pe != -1) {  // originally paired with this face
         if ((g1 && g2) || (f1 && f2)) {
-            lower(c, v3);
+            o.add(v3);
             return;
         }
         const i64 qf = R.face_partner(c.Q, face);
@@ -542,35 +615,31 @@ __device__ __forceinline__ void rule_saddle(const Rules &R, i64 id) {
             if (above_f(c, w2, w3) && above_f(c, w1, w3)) {
                 const i64 pfe = R.edge_partner(c.P, qf);
                 if (pfe != -1 && cell_kind(pfe) == KIND_FACE) {
-                    lower(c, R.third(pfe, w1, w2));
+                    o.add(R.third(pfe, w1, w2));
                     return;
                 }
             }
-            if (fabs(get_delta(c, false_v)) > 0) lower(c, false_v);
+            if (fabs(get_delta(c, false_v)) > 0) o.add(false_v);
         } else if (f1 && !g1) {
-            lower(c, g1 ? v1 : v3);
+            o.add(g1 ? v1 : v3);
         } else {
-            lower(c, g2 ? v2 : v3);
+            o.add(g2 ? v2 : v3);
         }
         return;
     }
     // originally critical, now paired with this face
     if (g1 == g2) {
-        if (g2 != f2) lower(c, v2);
-        if (g1 != f1) lower(c, v1);
+        if (g2 != f2) o.add(v2);
+        if (g1 != f1) o.add(v1);
     } else {
-        const i64 m = rescan_edge(c, v1, v2);
-        if (m != -1) {
-            lower(c, m);
-        } else {
-            lower(c, v1);
-            lower(c, v2);
-        }
+        o.add(v2);
+        o.add(v1);
+        o.rescan = 2;
     }
 }
 
 // --------------------------------------------------------------- A10 fix_2saddle
-__device__ __forceinline__ void rule_2saddle(const Rules &R, i64 id) {
+__device__ __forceinline__ void rule_2saddle(const Rules &R, i64 id, Lowered &o) {
     const RuleCtx &c = R.c;
     const Grid &G = c.g;
     const i64 pf = R.face_partner(c.P, id);
@@ -580,7 +649,7 @@ __device__ __forceinline__ void rule_2saddle(const Rules &R, i64 id) {
         const i64 v3 = R.third(id, v1, v2);
         const bool g1 = above_g(c, v2, v3), g2 = above_g(c, v1, v3), f1 = above_f(c, v2, v3), f2 = above_f(c, v1, v3);
         if (g1 && g2) {  // the edge's original face is this one
-            lower(c, v3);
+            o.add(v3);
         } else if (f1 != f2 && g1 != g2) {
             const i64 ff = R.edge_partner(c.Q, pf);
             i64 w = v3;
@@ -589,9 +658,9 @@ __device__ __forceinline__ void rule_2saddle(const Rules &R, i64 id) {
                 const bool h1 = above_f(c, v2, u), h2 = above_f(c, v1, u);
                 if (above_g(c, v2, u) && above_g(c, v1, u) && h1 != h2) w = !h1 ? v2 : v1;
             }
-            lower(c, w);
+            o.add(w);
         } else if (!g1 || !g2) {
-            lower(c, v3);
+            o.add(v3);
         }
         return;
     }
@@ -600,12 +669,12 @@ __device__ __forceinline__ void rule_2saddle(const Rules &R, i64 id) {
         R.verts(id, v1, v2, v3);
         const i64 v4 = R.fourth(pf, v1, v2, v3);
         if (above_f(c, v3, v4) && above_f(c, v2, v4) && above_f(c, v1, v4)) {
-            lower(c, v4);
+            o.add(v4);
             return;
         }
         const i64 pff = R.tet_partner(c.Q, pf);
         if (pff == -1) {
-            lower(c, v4);
+            o.add(v4);
             return;
         }
         i64 u1, u2, u3;
@@ -613,9 +682,9 @@ __device__ __forceinline__ void rule_2saddle(const Rules &R, i64 id) {
         const bool ga = above_g(c, u3, v4) && above_g(c, u2, v4) && above_g(c, u1, v4);
         const bool fa = above_f(c, u3, v4) && above_f(c, u2, v4) && above_f(c, u1, v4);
         if (ga || fa) {
-            lower(c, u1);
-            lower(c, u2);
-            lower(c, u3);
+            o.add(u1);
+            o.add(u2);
+            o.add(u3);
             return;
         }
         const i64 id2 = R.face_partner(c.P, pff);
@@ -623,7 +692,7 @@ __device__ __forceinline__ void rule_2saddle(const Rules &R, i64 id) {
         if (cell_kind(id2) == KIND_EDGE) {
             i64 w1, w2;
             R.verts(id2, w1, w2);
-            lower(c, third_of(u1, u2, u3, w1, w2));
+            o.add(third_of(u1, u2, u3, w1, w2));
         } else {
             // as the reference has it: the fourth vertex is replaced by one of the
             // face's when an earlier one is not on the face
@@ -632,10 +701,10 @@ __device__ __forceinline__ void rule_2saddle(const Rules &R, i64 id) {
             if (t1 != u1 && t1 != u2 && t1 != u3) t4 = u1;
             else if (t2 != u1 && t2 != u2 && t2 != u3) t4 = u2;
             else if (t3 != u1 && t3 != u2 && t3 != u3) t4 = u3;
-            lower(c, t1);
-            lower(c, t2);
-            lower(c, t3);
-            lower(c, t4);
+            o.add(t1);
+            o.add(t2);
+            o.add(t3);
+            o.add(t4);
         }
         return;
     }
@@ -647,10 +716,10 @@ __device__ __forceinline__ void rule_2saddle(const Rules &R, i64 id) {
         const i64 tf = R.edge_partner(c.P, qf);
         if (tf == -1) return;
         if (cell_kind(tf) == KIND_FACE) {
-            lower(c, R.third(tf, v1, v2));
+            o.add(R.third(tf, v1, v2));
         } else {
-            lower(c, v1);
-            lower(c, v2);
+            o.add(v1);
+            o.add(v2);
         }
         return;
     }
@@ -660,22 +729,17 @@ __device__ __forceinline__ void rule_2saddle(const Rules &R, i64 id) {
     const bool g1 = above_g(c, v3, v4), g2 = above_g(c, v2, v4), g3 = above_g(c, v1, v4);
     const bool f1 = above_f(c, v3, v4), f2 = above_f(c, v2, v4), f3 = above_f(c, v1, v4);
     if (g1 && g2 && g3) {
-        if (!f1) lower(c, v3);
-        else if (!f2) lower(c, v2);
-        else if (!f3) lower(c, v1);
+        if (!f1) o.add(v3);
+        else if (!f2) o.add(v2);
+        else if (!f3) o.add(v1);
         return;
     }
     // the reference compares this face id with the number of tetrahedra
     const i64 true_cell = R.tet_partner(c.P, qf);
-    i64 m = -1;
-    if (!(true_cell != -1 && code_ref(G, true_cell) < G.T)) m = smallest_vertex(c, v1, v2, v3);
-    if (m != -1) {
-        lower(c, m);
-    } else {
-        lower(c, v1);
-        lower(c, v2);
-        lower(c, v3);
-    }
+    o.add(v3);
+    o.add(v2);
+    o.add(v1);
+    if (!(true_cell != -1 && code_ref(G, true_cell) < G.T)) o.rescan = 3;
 }
 
 // --------------------------------------------------------------- A11 fix_maximum
@@ -686,7 +750,7 @@ __device__ DMTZ_SHARED_CODE i64 literal_fourth(const Grid &G, i64 id, i64 v1, i6
     tet_verts(G, id, p, q, r, w);
     return fourth_of(p, q, r, w, v1, v2, v3);
 }
-__device__ __forceinline__ void rule_max(const Rules &R, i64 id) {
+__device__ __forceinline__ void rule_max(const Rules &R, i64 id, Lowered &o) {
     const RuleCtx &c = R.c;
     const i64 pt = R.tet_partner(c.P, id);
     const i64 face = pt != -1 ? pt : R.tet_partner(c.Q, id);
@@ -697,7 +761,7 @@ __device__ __forceinline__ void rule_max(const Rules &R, i64 id) {
     const bool f1 = above_f(c, v1, v4), f2 = above_f(c, v2, v4), f3 = above_f(c, v3, v4);
     if (pt != -1) {
         if (f1 && f2 && f3) {
-            lower(c, v4);
+            o.add(v4);
             return;
         }
         const i64 fc = R.face_partner(c.Q, face);
@@ -708,44 +772,44 @@ __device__ __forceinline__ void rule_max(const Rules &R, i64 id) {
             R.verts(fc, e1, e2);
             w = above_g(c, e1, e2) ? e1 : e2;
         }
-        lower(c, w);
+        o.add(w);
         return;
     }
     const bool g1 = above_g(c, v1, v4), g2 = above_g(c, v2, v4), g3 = above_g(c, v3, v4);
     if (g1 && g2 && g3) {
-        if (!f1) lower(c, v1);
-        if (!f2) lower(c, v2);
-        if (!f3) lower(c, v3);
+        if (!f1) o.add(v1);
+        if (!f2) o.add(v2);
+        if (!f3) o.add(v3);
         if (f1 && f2 && f3) {
             const i64 it = R.face_partner(c.P, face);
             if (it != -1)
-                lower(c, cell_kind(it) == KIND_TET ? R.fourth(it, v1, v2, v3)
+                o.add(cell_kind(it) == KIND_TET ? R.fourth(it, v1, v2, v3)
                                                    : literal_fourth(c.g, code_ref(c.g, it), v1, v2, v3, c.err));
         }
         return;
     }
     const i64 pid = R.face_partner(c.P, face);
     if (pid == -1) {
-        if (!f1) lower(c, v1);
-        if (!f2) lower(c, v2);
-        if (!f3) lower(c, v3);
+        if (!f1) o.add(v1);
+        if (!f2) o.add(v2);
+        if (!f3) o.add(v3);
     } else if (cell_kind(pid) == KIND_EDGE) {
         i64 e1, e2;
         R.verts(pid, e1, e2);
-        lower(c, e1);
-        lower(c, e2);
+        o.add(e1);
+        o.add(e2);
     } else {
         i64 p, q, r, w;
         R.verts(pid, p, q, r, w);
-        lower(c, p);
-        lower(c, q);
-        lower(c, r);
-        lower(c, w);
+        o.add(p);
+        o.add(q);
+        o.add(r);
+        o.add(w);
     }
 }
 
 // --------------------------------------------------------------- A15 fix_as_vpath (type 2)
-__device__ __forceinline__ void rule_as_path(const Rules &R, i64 tet) {
+__device__ __forceinline__ void rule_as_path(const Rules &R, i64 tet, Lowered &o) {
     const RuleCtx &c = R.c;
     const i64 tf = R.tet_partner(c.P, tet), ff = R.tet_partner(c.Q, tet);
     i64 v1, v2, v3, a = -1, b = -1, tv3 = -1;
@@ -756,25 +820,24 @@ __device__ __forceinline__ void rule_as_path(const Rules &R, i64 tet) {
         R.verts(ff, a, b, tv3);
         const i64 pfe = R.face_partner(c.P, ff);
         if (pfe != -1 && cell_kind(pfe) == KIND_TET) {
-            lower(c, R.fourth(pfe, a, b, tv3));
+            o.add(R.fourth(pfe, a, b, tv3));
             return;
         }
     }
     if (tf == -1) tri_verts(c.g, -1, v1, v2, v3);
     else R.verts(tf, v1, v2, v3);
-    lower(c, fourth_of(a, b, tv3, tv3, v1, v2, v3));
+    o.add(fourth_of(a, b, tv3, tv3, v1, v2, v3));
 }
 // A14 fix_ds_vpath (type 0)
-__device__ DMTZ_SHARED_CODE void literal_ds_path(const RuleCtx &c, i64 v) {
+__device__ DMTZ_SHARED_CODE i64 literal_ds_path(const RuleCtx &c, i64 v) {
     const i64 tpe = pv_ref(c, c.P, v);
     i64 v1, v2;
     edge_verts(c.g, tpe, v1, v2);
-    lower(c, v == v1 ? v2 : v1);
+    return v == v1 ? v2 : v1;
 }
-__device__ __forceinline__ void rule_ds_path(const Rules &R, i64 v) {
+__device__ __forceinline__ void rule_ds_path(const Rules &R, i64 v, Lowered &o) {
     const i64 w = v >= 0 && v < R.c.g.V ? R.below(R.c.P, v) : -1;
-    if (w >= 0) lower(R.c, w);
-    else literal_ds_path(R.c, v);  // no vertex (-1), or a critical one
+    o.add(w >= 0 ? w : literal_ds_path(R.c, v));  // literal: no vertex (-1), or a critical one
 }
 
 // fix_ds_wall (main_3d.cu:5297-5413) for the wall record edge e: the edge's
