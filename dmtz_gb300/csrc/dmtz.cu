@@ -54,43 +54,51 @@ __global__ void __launch_bounds__(kBlock) k_mismatch_scan(Grid g, const uint32_t
 // Dirty bricks.  A cell's pairing depends on the star of its highest vertex,
 // so a changed value reaches the cells whose highest vertex is the changed one
 // or a neighbour of it: anchors 2 below to 1 above per axis.  Every brick with
-// such an anchor is marked (one byte per brick; writers all store 1).
+// such an anchor is marked (one byte per brick, four to a word) and listed by
+// whoever marks it first; the marks stay until the round's end, where the list
+// says which ones to clear.  (A kernel that made the list from the marks took 5 of
+// a short round's 45 us.)
 constexpr int kReachLow = 2, kReachHigh = 1;
 struct BrickMarks {
-    uint8_t *flags;  // nullptr: not kept
+    uint32_t *flags;  // nullptr: not kept
+    uint32_t *list;   // packed brick coordinates
+    unsigned long long *n;
     int nbx, nby, shx, shy, shz;
+    int lanes;  // per vertex: 8 where the reach spans at most two bricks per axis, else 32 (three)
 };
-__device__ __forceinline__ void mark_dirty(const Grid &g, const BrickMarks &B, i64 v) {
-    int x, y, z;
-    decode_v(g, v, x, y, z);
-    const int x0 = max(x - kReachLow, 0) >> B.shx, x1 = min(x + kReachHigh, g.W - 1) >> B.shx;
-    const int y0 = max(y - kReachLow, 0) >> B.shy, y1 = min(y + kReachHigh, g.H - 1) >> B.shy;
-    const int z0 = max(z - kReachLow, 0) >> B.shz, z1 = min(z + kReachHigh, g.D - 1) >> B.shz;
-    for (int bz = z0; bz <= z1; bz++)
-        for (int by = y0; by <= y1; by++)
-            for (int bx = x0; bx <= x1; bx++) B.flags[bx + (i64)B.nbx * (by + (i64)B.nby * bz)] = 1;
-}
-__global__ void k_mark_dirty(Grid g, BrickMarks B, const i64 *verts, const unsigned long long *nverts) {
-    const i64 n = (i64)*nverts;
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x)
-        mark_dirty(g, B, verts[i]);
-}
-// the marked bricks as a list and in `fresh`, and the marks cleared for the
-// next round (four marks to a word)
-__global__ void k_compact_bricks(int nbx, int nby, int nbz, uint32_t *flags, uint32_t *fresh, uint32_t *list,
-                                 unsigned long long *n) {
-    const i64 nb = (i64)nbx * nby * nbz;
-    for (i64 w = (i64)blockIdx.x * blockDim.x + threadIdx.x; w < (nb + 3) / 4; w += (i64)gridDim.x * blockDim.x) {
-        const uint32_t word = flags[w];
-        fresh[w] = word;
-        if (!word) continue;
-        flags[w] = 0;
-        for (int q = 0; q < 4; q++) {
-            if (!((word >> (8 * q)) & 0xFFu)) continue;
-            const i64 b = 4 * w + q;
-            const int bx = (int)(b % nbx), by = (int)((b / nbx) % nby), bz = (int)(b / ((i64)nbx * nby));
-            list[agg_slot(n)] = (uint32_t)bx | ((uint32_t)by << 11) | ((uint32_t)bz << 22);
+// Every lane of a warp takes part: lane j of a vertex's lanes has the j-th brick of
+// its reach, so that the marks, and then the list's slots, wait for memory once.
+__device__ __forceinline__ void mark_dirty(const Grid &g, const BrickMarks &B, bool on, i64 v, int j) {
+    uint32_t entry = 0;
+    bool first = false;
+    if (on) {
+        int x, y, z;
+        decode_v(g, v, x, y, z);
+        const int span = B.lanes == 8 ? 2 : 3;
+        const int bx = (max(x - kReachLow, 0) >> B.shx) + j % span, by = (max(y - kReachLow, 0) >> B.shy) + (j / span) % span,
+                  bz = (max(z - kReachLow, 0) >> B.shz) + j / (span * span);
+        if (bx <= min(x + kReachHigh, g.W - 1) >> B.shx && by <= min(y + kReachHigh, g.H - 1) >> B.shy &&
+            bz <= min(z + kReachHigh, g.D - 1) >> B.shz) {
+            const i64 b = bx + (i64)B.nbx * (by + (i64)B.nby * bz);
+            const uint32_t bit = 1u << (8 * (int)(b & 3));
+            if (!(__ldcg(B.flags + (b >> 2)) & bit)) first = !(atomicOr(B.flags + (b >> 2), bit) & bit);
+            entry = (uint32_t)bx | ((uint32_t)by << 11) | ((uint32_t)bz << 22);
         }
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, first), lane = threadIdx.x & 31u;
+    if (!m) return;
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(B.n, (unsigned long long)__popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (first) B.list[at + __popc(m & ((1u << lane) - 1u))] = entry;
+}
+__global__ void __launch_bounds__(kBlock) k_mark_dirty(Grid g, BrickMarks B, const i64 *verts, const unsigned long long *nverts) {
+    const i64 n = (i64)*nverts;
+    const int lane = threadIdx.x & 31, per = 32 / B.lanes, j = lane % B.lanes;
+    const i64 step = (i64)gridDim.x * (kBlock / 32) * per;
+    for (i64 b = ((i64)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)) * per; b < n; b += step) {
+        const i64 i = b + lane / B.lanes;
+        mark_dirty(g, B, i < n, i < n ? verts[i] : 0, j);
     }
 }
 
@@ -1095,35 +1103,48 @@ __global__ void __launch_bounds__(kBlock) k_fix_path(const __grid_constant__ Rul
 // The delta is what the reference's buffer holds: get_delta(v), with the
 // buffer's "no request" sentinel -2000*range (a request whose delta is not
 // above the sentinel leaves the buffer unchanged under edit_type 0).
-__global__ void k_apply(const __grid_constant__ RuleCtx c, double range, int preserve_type, int update, uint8_t *changed, double *delta_out,
-                        BrickMarks B) {
-    const i64 n = (i64)*c.reqn;
+// Where bricks are marked, a vertex has as many lanes as its reach has bricks
+// (see mark_dirty) and the first of them updates it.
+__global__ void __launch_bounds__(kBlock) k_apply(const __grid_constant__ RuleCtx c, double range, int preserve_type, int update,
+                                                 uint8_t *changed, double *delta_out, const __grid_constant__ BrickMarks B) {
+    const i64 n = min((i64)*c.reqn, c.reqcap);
     const double sentinel = -2000.0 * range;
     const double tiny = 1e-15 * range;
     double *g = const_cast<double *>(c.gv);
     int *cnt = const_cast<int *>(c.cnt);
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n && i < c.reqcap; i += (i64)gridDim.x * blockDim.x) {
-        const i64 v = c.reqlist[i];
-        c.reqbits[v >> 5] = 0;  // every bit of this word belongs to listed vertices
-        const double d = get_delta(c, v);
-        const bool req = c.edit_type == 0 ? (d > sentinel) : (d != sentinel);
-        if (delta_out) delta_out[v] = req ? d : sentinel;
-        if (!req || !update) continue;
-        const double f = c.f[v];
-        const double gv = g[v];
-        const int cv = cnt[v];
-        const double lowb = __dsub_rn(f, c.bound);
-        if (preserve_type == 0 && fabs(d) > tiny && cv < 5 && fabs(__dsub_rn(f, __dadd_rn(gv, d))) <= c.bound) {
-            g[v] = __dadd_rn(gv, d);
-            cnt[v] = cv + 1;
-            if (c.progress) *c.progress = 1ull;
-        } else {
-            cnt[v] = 6;
-            g[v] = lowb;
-            if (c.progress && (cv != 6 || gv != lowb)) *c.progress = 1ull;
+    const int lane = threadIdx.x & 31, lanes = B.flags ? B.lanes : 1, per = 32 / lanes, j = lane % lanes;
+    const i64 step = (i64)gridDim.x * (kBlock / 32) * per;
+    for (i64 base = ((i64)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)) * per; base < n; base += step) {
+        const i64 i = base + lane / lanes;
+        const i64 v = i < n ? c.reqlist[i] : 0;
+        double d = 0, f = 0, gv = 0;
+        int cv = 0;
+        if (i < n) {
+            d = get_delta(c, v);
+            f = c.f[v];
+            gv = g[v];
+            cv = cnt[v];
         }
-        if (changed) changed[v] = 1;
-        if (B.flags) mark_dirty(c.g, B, v);
+        const bool req = i < n && (c.edit_type == 0 ? (d > sentinel) : (d != sentinel));
+        __syncwarp();  // every lane has read what the first one changes
+        if (i < n && j == 0) {
+            c.reqbits[v >> 5] = 0;  // every bit of this word belongs to listed vertices
+            if (delta_out) delta_out[v] = req ? d : sentinel;
+            if (req && update) {
+                const double lowb = __dsub_rn(f, c.bound);
+                if (preserve_type == 0 && fabs(d) > tiny && cv < 5 && fabs(__dsub_rn(f, __dadd_rn(gv, d))) <= c.bound) {
+                    g[v] = __dadd_rn(gv, d);
+                    cnt[v] = cv + 1;
+                    if (c.progress) *c.progress = 1ull;
+                } else {
+                    cnt[v] = 6;
+                    g[v] = lowb;
+                    if (c.progress && (cv != 6 || gv != lowb)) *c.progress = 1ull;
+                }
+                if (changed) changed[v] = 1;
+            }
+        }
+        if (B.flags) mark_dirty(c.g, B, req && update, v, j);
     }
 }
 
@@ -1555,8 +1576,7 @@ struct dmtz_ctx {
     i64 list_min = 1 << 20;
     i64 *as_tet = nullptr, *as_cur = nullptr, *ds_edge = nullptr, *ds_vert = nullptr;
     i64 capAS = 0, capDS = 0, capSad2 = 0;
-    uint32_t *brick_flags = nullptr;  // per brick (a byte each, four to a word): in the next repair
-    uint8_t *brick_fresh = nullptr;   // per brick: re-paired by the current round's criticality pass
+    uint32_t *brick_flags = nullptr;  // per brick (a byte each, four to a word): in this round's repair
     int inc_scan = 0;                 // repairs rebuild the mismatch lists incrementally (see k_list_keep)
     int strict_ds = 0;                // descending separatrix checks walk whole paths (k_ds_strict)
     i64 *list_tmp[4] = {nullptr, nullptr, nullptr, nullptr};  // rebuilt mismatch lists, capL entries each
@@ -1656,8 +1676,6 @@ void free_all(dmtz_ctx *c) {
     cudaFree(c->cnt); cudaFree(c->reqbits); cudaFree(c->reqlist);
     for (auto &l : c->lists) { cudaFree(l); l = nullptr; }
     for (auto &l : c->list_tmp) { cudaFree(l); l = nullptr; }
-    cudaFree(c->brick_fresh);
-    c->brick_fresh = nullptr;
     for (auto &k : c->capL) k = 0;
     c->capAS = c->capDS = c->capSad2 = 0;
     cudaFree(c->as_tet); cudaFree(c->as_cur); cudaFree(c->ds_edge); cudaFree(c->ds_vert);
@@ -1729,7 +1747,6 @@ dmtz_status ensure(dmtz_ctx *ctx, const Grid &g) {
     CK(cudaMemset(ctx->reqbits, 0, sizeof(uint32_t) * (size_t)((V + 31) / 32 + 1)));
     CK(dalloc(&ctx->reqlist, V));
     CK(dalloc(&ctx->brick_flags, (nbr + 3) / 4)); CK(dalloc(&ctx->brick_list, nbr));
-    CK(dalloc(&ctx->brick_fresh, (nbr + 3) / 4 * 4));
     CK(dalloc(&ctx->path_as, 2 * nbr));
     ctx->path_ds = ctx->path_as + nbr;
     CK(dalloc(&ctx->brick_n, 8));
@@ -1917,19 +1934,27 @@ void run_pairing(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32
 BrickMarks brick_marks(const dmtz_ctx *ctx, const Grid &g) {
     BrickMarks B;
     int nbz, sh[3];
-    B.flags = reinterpret_cast<uint8_t *>(ctx->brick_flags);
+    B.flags = ctx->brick_flags;
+    B.list = ctx->brick_list;
+    B.n = ctx->brick_n;
     bricks_of(g, ctx->tune_shape, B.nbx, B.nby, nbz);
     shape_shifts(ctx->tune_shape, sh);
     B.shx = sh[0];
     B.shy = sh[1];
     B.shz = sh[2];
+    B.lanes = std::min(sh[0], std::min(sh[1], sh[2])) >= 2 ? 8 : 32;
     return B;
 }
 
+// no brick marked and none listed
+void clear_marks(dmtz_ctx *ctx) {
+    cudaMemsetAsync(ctx->brick_n, 0, sizeof(unsigned long long), ctx->stream);
+    cudaMemsetAsync(ctx->brick_flags, 0, (size_t)(ctx->capB + 3) / 4 * sizeof(uint32_t), ctx->stream);
+}
 // Re-pair only the bricks near the vertices the last update requested (marked
 // already by k_apply, or else from ctx->reqlist); the mismatch lists are then rebuilt
 // into list_tmp (inc_scan; k_round_end takes them back) or scanned for.  The
-// brick count is zero at the start (k_round_end, or the caller).
+// marks are clear at the start (k_round_end, or the caller).
 void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32_t *crit_o, int want_saddles, bool marked) {
     const BrickMarks B = brick_marks(ctx, g);
     cudaStream_t st = ctx->stream;
@@ -1939,8 +1964,6 @@ void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint3
         k_mark_dirty<<<persistent_grid(), kBlock, 0, st>>>(g, B, ctx->reqlist, ctx->counters + 4);
         ctx->launches++;
     }
-    k_compact_bricks<<<(unsigned)std::min<i64>(persistent_grid(), grid_for((nb + 3) / 4)), kBlock, 0, st>>>(
-        bl.nbx, bl.nby, bl.nbz, ctx->brick_flags, reinterpret_cast<uint32_t *>(ctx->brick_fresh), ctx->brick_list, ctx->brick_n);
     bl.list = ctx->brick_list;
     bl.n = ctx->brick_n;
     GradOps O{};
@@ -1951,7 +1974,7 @@ void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint3
         O.T = rebuilt_lists(ctx);
         O.want = want_bits(want_saddles);
         K.L = mismatch_lists(ctx);
-        K.fresh = ctx->brick_fresh;
+        K.fresh = reinterpret_cast<const uint8_t *>(ctx->brick_flags);
         K.shx = B.shx;
         K.shy = B.shy;
         K.shz = B.shz;
@@ -1960,7 +1983,7 @@ void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint3
         K.blocks = persistent_grid() / 8;
     }
     grad_bricks(g, s, bl, brick_grid(ctx, nb), st, O, K);
-    ctx->launches += 2;
+    ctx->launches++;
     if (!ctx->inc_scan) scan_mismatch(ctx, g, s.crit, crit_o, want_saddles);
 }
 // a round's re-pairing when its lists are long (the whole grid, lists and flags in place)
@@ -2764,12 +2787,9 @@ struct LoopCtl {
     int last;           // state of the last body run
     int break_stalls;   // stop when a round changed nothing (the host breaks the stall)
     int stalled;
+    int begun;          // a body has run: a round's end has something to end
 };
 }  // namespace
-
-__global__ void k_set_switch(const LoopCtl *ctl, cudaGraphConditionalHandle h) {
-    cudaGraphSetConditional(h, (unsigned)ctl->state);
-}
 
 // the state after a body run, from the counters it left
 __device__ __forceinline__ LoopCtl loop_next(LoopCtl c, const unsigned long long *counters) {
@@ -2824,15 +2844,24 @@ __device__ __forceinline__ LoopCtl loop_next(LoopCtl c, const unsigned long long
 
 // The end of a round: the rebuilt mismatch lists back into the lists (T.n ==
 // nullptr: none were rebuilt; entries past a list's capacity were not stored,
-// and the count shows the overflow), then the last block to finish clears the
-// round's counters and either decides the graph loop's next state (ctl) or
-// leaves the counts for the host (report, in pinned memory).
-__global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Lists T, const __grid_constant__ Lists L, unsigned long long *counters, unsigned long long *brick_n,
-                                                     LoopCtl *ctl, cudaGraphConditionalHandle hwhile,
+// and the count shows the overflow) and the bricks' marks cleared, then the last
+// block to finish clears the round's counters and either decides the graph loop's
+// next state (ctl) or leaves the counts for the host (report, in pinned memory).
+// In the graph it stands before the switch that it sets, so the first one has no
+// round to end, and after the last one no state runs.
+__global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Lists T, const __grid_constant__ Lists L, unsigned long long *counters,
+                                                     const __grid_constant__ BrickMarks B, LoopCtl *ctl,
+                                                     cudaGraphConditionalHandle hwhile, cudaGraphConditionalHandle hswitch,
                                                      unsigned long long *report) {
     __shared__ bool last;
     const int st = ctl ? ctl->state : LS_CP;
-    const bool copy = T.n && st != LS_PCHECK && st != LS_CPF;
+    const bool begun = !ctl || ctl->begun;
+    const bool copy = begun && T.n && st != LS_PCHECK && st != LS_CPF;
+    const i64 nbrick = (i64)*B.n;
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < nbrick; i += (i64)gridDim.x * blockDim.x) {
+        const uint32_t e = B.list[i];
+        reinterpret_cast<uint8_t *>(B.flags)[(e & 0x7FF) + (i64)B.nbx * (((e >> 11) & 0x7FF) + (i64)B.nby * (e >> 22))] = 0;
+    }
     if (copy) {
         const i64 n0 = min((i64)T.n[0], T.cap[0]), n1 = min((i64)T.n[1], T.cap[1]), n2 = min((i64)T.n[2], T.cap[2]),
                   n3 = min((i64)T.n[3], T.cap[3]);
@@ -2853,7 +2882,7 @@ __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Li
     if (!last || threadIdx.x != 0) return;
     __threadfence();
     counters[30] = 0;
-    *brick_n = 0;
+    *B.n = 0;
     if (copy)
         for (int k = 0; k < 4; k++) {
             L.n[k] = T.n[k];
@@ -2861,9 +2890,12 @@ __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Li
         }
     bool stop = false;
     if (ctl) {
-        const LoopCtl c = loop_next(*ctl, counters);
+        LoopCtl c = *ctl;
+        if (begun) c = loop_next(c, counters);
+        c.begun = 1;
         *ctl = c;
         stop = c.state == LS_DONE || c.overflow || c.stalled;
+        cudaGraphSetConditional(hswitch, stop ? (unsigned)LS_STATES : (unsigned)c.state);
         cudaGraphSetConditional(hwhile, stop ? 0u : 1u);
         if (!stop && (c.state == LS_PDF || c.state == LS_PCHECK)) counters[5] = counters[6] = counters[27] = 0;
     } else {
@@ -2919,11 +2951,11 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
     const unsigned pgrid = persistent_grid();
     if (!ctx->loopctl) CK(cudaMalloc(&ctx->loopctl, sizeof(LoopCtl)));
     LoopCtl *dctl = static_cast<LoopCtl *>(ctx->loopctl);
+    init.begun = 0;
     CK(cudaMemcpyAsync(dctl, &init, sizeof(LoopCtl), cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), st));
     CK(cudaMemsetAsync(ctx->counters + 7, 0, sizeof(unsigned long long), st));
     CK(cudaMemsetAsync(ctx->counters + 27, 0, sizeof(unsigned long long), st));
-    CK(cudaMemsetAsync(ctx->brick_n, 0, sizeof(unsigned long long), st));
     if (init.state != LS_PFIX) CK(cudaMemsetAsync(ctx->counters + 5, 0, 2 * sizeof(unsigned long long), st));
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -2945,14 +2977,15 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
         cudaGraph_t body = wp.conditional.phGraph_out[0];
         cudaGraphConditionalHandle hsw;
         if (cudaGraphConditionalHandleCreate(&hsw, body, 0, 0) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
-        // body: set the switch from the state, switch over the states, end the round
-        cudaGraphNode_t n_set, n_sw, n_ctl;
+        // body: end the round before and set the switch, then switch over the states
+        cudaGraphNode_t n_set, n_sw;
         {
             if (cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
                 res = DMTZ_ERR_CUDA;
                 break;
             }
-            k_set_switch<<<1, 1, 0, st>>>(dctl, hsw);
+            k_round_end<<<pgrid / 8, kBlock, 0, st>>>(ctx->inc_scan ? rebuilt_lists(ctx) : Lists{}, mismatch_lists(ctx),
+                                                      ctx->counters, brick_marks(ctx, g), dctl, hwhile, hsw, nullptr);
             cudaGraph_t tmp;
             if (cudaStreamEndCapture(st, &tmp) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
             size_t nn = 1;
@@ -2985,17 +3018,6 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
             if (cudaStreamEndCapture(st, &tmp) != cudaSuccess) res = DMTZ_ERR_CUDA;
         }
         if (res != DMTZ_OK) break;
-        {
-            if (cudaStreamBeginCaptureToGraph(st, body, &n_sw, nullptr, 1, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
-                res = DMTZ_ERR_CUDA;
-                break;
-            }
-            k_round_end<<<pgrid / 8, kBlock, 0, st>>>(ctx->inc_scan ? rebuilt_lists(ctx) : Lists{}, mismatch_lists(ctx),
-                                                      ctx->counters, ctx->brick_n, dctl, hwhile, nullptr);
-            cudaGraph_t tmp;
-            if (cudaStreamEndCapture(st, &tmp) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
-            (void)n_ctl;
-        }
         if (cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
         if (cudaGraphLaunch(exec, st) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
         if (cudaMemcpyAsync(out, dctl, sizeof(LoopCtl), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -3013,10 +3035,11 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
 
 // ----------------------------------------------------------------------------- the correction loop
 // the round's end of the host-driven loop (its counts then stand in ctx->report once the stream is done)
-static void host_round_end(dmtz_ctx *ctx) {
+static void host_round_end(dmtz_ctx *ctx, const Grid &g) {
     k_round_end<<<persistent_grid() / 8, kBlock, 0, ctx->stream>>>(ctx->inc_scan ? rebuilt_lists(ctx) : Lists{},
-                                                                   mismatch_lists(ctx), ctx->counters, ctx->brick_n, nullptr,
-                                                                   cudaGraphConditionalHandle{}, ctx->report);
+                                                                   mismatch_lists(ctx), ctx->counters, brick_marks(ctx, g), nullptr,
+                                                                   cudaGraphConditionalHandle{}, cudaGraphConditionalHandle{},
+                                                                   ctx->report);
     ctx->launches++;
 }
 
@@ -3064,8 +3087,8 @@ static dmtz_status learned_start(dmtz_ctx *ctx, dmtz_cnn *net, const Grid &g, do
     ctx->launches += 5;
     // re-pair only the bricks within the passes' radii of the edited vertices
     // (the mismatch lists are rebuilt by a full scan: the loop has not started)
-    CK(cudaMemsetAsync(ctx->brick_n, 0, sizeof(unsigned long long), ctx->stream));
     repair_dirty(ctx, g, view(ctx->Q, ctx->g), ctx->P.crit, 1, false);
+    clear_marks(ctx);
     CK(cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), ctx->stream));
     CK(cudaGetLastError());
     return DMTZ_OK;
@@ -3094,10 +3117,9 @@ static dmtz_status break_stall(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, 
         k_dilate_axis<<<grid_for(g.V / n), kBlock, 0, st>>>(g, ctx->changed, axis, std::min(radius, n));
     }
     k_snap_mask<<<pgrid, kBlock, 0, st>>>(rc, ctx->changed);
-    CK(cudaMemsetAsync(ctx->brick_n, 0, sizeof(unsigned long long), st));
     repair_dirty(ctx, g, Qs, ctx->P.crit, want_saddles, false);
     k_clear_req<<<pgrid, kBlock, 0, st>>>(ctx->reqlist, ctx->counters + 4, g.V, ctx->reqbits);
-    host_round_end(ctx);
+    host_round_end(ctx, g);
     ctx->launches += 6;
     CK(cudaGetLastError());
     return DMTZ_OK;
@@ -3153,7 +3175,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     CK(cudaMemsetAsync(ctx->changed, 0, (size_t)g.V, st));
     CK(cudaMemsetAsync(ctx->counters, 0, 8 * sizeof(unsigned long long), st));
     CK(cudaMemsetAsync(ctx->counters + 20, 0, 11 * sizeof(unsigned long long), st));
-    CK(cudaMemsetAsync(ctx->brick_n, 0, sizeof(unsigned long long), st));
+    clear_marks(ctx);
     const FieldState Ps = view(ctx->P, ctx->f), Qs = view(ctx->Q, ctx->g);
     run_pairing(ctx, g, Ps, nullptr, 1);
     if (pvp == 1 && (s = prep_paths(ctx, g)) != DMTZ_OK) return s;
@@ -3257,14 +3279,14 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
                 }
             }
             pt_.end();
-            // kernels per body run: switch + round's end, plus each state's own: a
-            // fix round is fix + update, then the repair (compaction, gradient, and
-            // the scan where the lists are not rebuilt), or the whole gradient
+            // kernels per body run: the round's end, plus each state's own: a fix
+            // round is fix + update, then the repair (gradient, and the scan where
+            // the lists are not rebuilt), or the whole gradient; one end more
             const int64_t det = detect_kernels(ctx, conn);  // separatrix detection kernels
-            const int64_t rnd = 2 + 2 + (ctx->inc_scan ? 0 : 1);
+            const int64_t rnd = 2 + 1 + (ctx->inc_scan ? 0 : 1);
             int64_t bodies = 0;
             for (int k = 0; k < LS_STATES; k++) bodies += fin.runs[k];
-            ctx->launches += 2 * bodies + rnd * fin.runs[LS_CP] + (rnd + det) * fin.runs[LS_PDF] + det * fin.runs[LS_PCHECK] +
+            ctx->launches += 1 + bodies + rnd * fin.runs[LS_CP] + (rnd + det) * fin.runs[LS_PDF] + det * fin.runs[LS_PCHECK] +
                              rnd * fin.runs[LS_PFIX] + 3 * fin.runs[LS_CPF];
         }
         R.outer_iterations = fin.outer;
@@ -3302,11 +3324,11 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
                 repair_full(ctx, g, Qs, ctx->P.crit, ps == 1);
                 const int inc = ctx->inc_scan;
                 ctx->inc_scan = 0;
-                host_round_end(ctx);
+                host_round_end(ctx, g);
                 ctx->inc_scan = inc;
             } else {
                 repair_dirty(ctx, g, Qs, ctx->P.crit, ps == 1, true);
-                host_round_end(ctx);
+                host_round_end(ctx, g);
             }
             pt_.end();
             if ((s = read_fit(ps == 1)) != DMTZ_OK) return s;
@@ -3346,7 +3368,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         ctx->launches += 2;
         pt_.begin(PH_PAIR);
         repair_dirty(ctx, g, Qs, ctx->P.crit, 1, true);
-        host_round_end(ctx);
+        host_round_end(ctx, g);
         pt_.end();
         if ((s = read_fit(1)) != DMTZ_OK) return s;
         if (opts->break_stalls && hc[7] == 0 && rounds < max_rounds && hc[5] + hc[6] + walls_fixed > 0) {
