@@ -38,6 +38,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -1444,6 +1445,7 @@ struct dmtz_cnn {
     // convolutions on tcgen05 (1, the default) or on mma.sync (0)
     int tensor_path = 2;
     unsigned *lticket = nullptr;
+    std::map<const void *, int> per_sm;  // blocks of a kernel that an SM holds
     int *tc_err = nullptr;  // set by a tcgen05 convolution whose wait timed out
     // warm-start scratch
     i64 capS = 0;
@@ -1498,10 +1500,12 @@ constexpr size_t wgrad_smem() {
 template <class K>
 dmtz_status launch_persistent(dmtz_cnn *net, K kernel, int threads, size_t smem, i64 ntiles, int cap_blocks,
                               int *used_blocks, cudaStream_t st, void **args) {
-    NCK(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    NCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-    if (per_sm < 1) return nfail(net, DMTZ_ERR_CUDA, "convolution kernel does not fit on an SM");
+    int &per_sm = net->per_sm[(const void *)kernel];  // asked for once: the shared memory depends on the kernel alone
+    if (per_sm < 1) {
+        NCK(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        NCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+        if (per_sm < 1) return nfail(net, DMTZ_ERR_CUDA, "convolution kernel does not fit on an SM");
+    }
     i64 blocks = std::min<i64>(ntiles, (i64)per_sm * net->nsm);
     if (cap_blocks > 0) blocks = std::min<i64>(blocks, cap_blocks);
     blocks = std::max<i64>(blocks, 1);
@@ -1758,10 +1762,11 @@ dmtz_status dmtz_cnn_create(dmtz_cnn **out, int device, uint64_t seed) {
     if (nalloc(&net->w, kParams) || nalloc(&net->grad, kParams) || nalloc(&net->m1, kParams) ||
         nalloc(&net->m2, kParams) || nalloc(&net->wf, kWeights) || nalloc(&net->wt, kWeights) ||
         nalloc(&net->part, net->nsm * kParams) || nalloc(&net->lpart, 2 * kLossBlocks) ||
-        nalloc(&net->lres, 2) || nalloc(&net->lticket, 1) || nalloc(&net->scale, 1) || nalloc(&net->tc_err, 1))
+        nalloc(&net->lres, 3) || nalloc(&net->scale, 1))
         return bail(DMTZ_ERR_CUDA);
-    if (cudaMemset(net->tc_err, 0, sizeof(int)) != cudaSuccess || cudaMemset(net->lticket, 0, sizeof(unsigned)) != cudaSuccess)
-        return bail(DMTZ_ERR_CUDA);
+    net->tc_err = reinterpret_cast<int *>(net->lres + 2);  // behind the loss, so that one copy brings both
+    net->lticket = reinterpret_cast<unsigned *>(net->lres + 2) + 1;
+    if (cudaMemset(net->tc_err, 0, sizeof(double)) != cudaSuccess) return bail(DMTZ_ERR_CUDA);
     // He-uniform weights (bound sqrt(6 / fan_in)); the output layer 0.1x and
     // only its channel 0 nonzero; zero biases
     std::vector<float> h((size_t)kParams, 0.f);
@@ -1787,9 +1792,9 @@ void dmtz_cnn_destroy(dmtz_cnn *net) {
     cudaSetDevice(net->device);
     if (net->stream) cudaStreamSynchronize(net->stream);
     for (void *p : {(void *)net->w, (void *)net->grad, (void *)net->m1, (void *)net->m2, (void *)net->wf,
-                    (void *)net->wt, (void *)net->part, (void *)net->lpart, (void *)net->lres, (void *)net->lticket, (void *)net->scale,
+                    (void *)net->wt, (void *)net->part, (void *)net->lpart, (void *)net->lres, (void *)net->scale,
                     (void *)net->a[0], (void *)net->a[1], (void *)net->dz4, (void *)net->gA, (void *)net->gB,
-                    (void *)net->feat, (void *)net->active, (void *)net->out, (void *)net->tc_err})
+                    (void *)net->feat, (void *)net->active, (void *)net->out})
         cudaFree(p);
     if (net->cap_train) cudaFree(net->a[2]);
     if (net->stream) cudaStreamDestroy(net->stream);
@@ -1837,13 +1842,18 @@ dmtz_status dmtz_cnn_get_grads(dmtz_cnn *net, float *host) {
 
 // a tcgen05 convolution whose completion wait timed out leaves a flag (the
 // kernel itself returns); the synchronous calls report it
-static dmtz_status check_tc(dmtz_cnn *net) {
-    int e = 0;
-    NCK(cudaMemcpy(&e, net->tc_err, sizeof(int), cudaMemcpyDeviceToHost));
+// (res: the loss and its weight as well; waits for the network's stream)
+static dmtz_status check_tc(dmtz_cnn *net, double *res = nullptr) {
+    double h[3];
+    NCK(cudaMemcpyAsync(h, net->lres, sizeof(h), cudaMemcpyDeviceToHost, net->stream));
+    NCK(cudaStreamSynchronize(net->stream));
+    int e;
+    memcpy(&e, h + 2, sizeof(e));
     if (e) {
         NCK(cudaMemset(net->tc_err, 0, sizeof(int)));
         return nfail(net, DMTZ_ERR_CUDA, "a tensor-core convolution timed out waiting for its MMAs");
     }
+    if (res) *res = h[0];
     return DMTZ_OK;
 }
 
@@ -1890,7 +1900,6 @@ dmtz_status dmtz_cnn_forward(dmtz_cnn *net, int W, int H, int D, const void *fea
     if (!net) return DMTZ_ERR_ARG;
     dmtz_status s = forward_on(net, W, H, D, static_cast<const bf16 *>(feat), out, train, net->stream);
     if (s != DMTZ_OK) return s;
-    NCK(cudaStreamSynchronize(net->stream));
     return check_tc(net);
 }
 
@@ -1922,11 +1931,7 @@ dmtz_status dmtz_cnn_backward(dmtz_cnn *net, int W, int H, int D, const float *t
     // layer 1 (no data gradient of the features)
     if ((s = wgrad<16, 32>(net, d, net->last_feat, net->gA, 0, p, st)) != DMTZ_OK) return s;
     if (net->tensor_path && (s = reduce(net, p, 0, NLAYER, st)) != DMTZ_OK) return s;
-    double res[2] = {0, 0};
-    NCK(cudaMemcpyAsync(res, net->lres, sizeof(res), cudaMemcpyDeviceToHost, st));
-    NCK(cudaStreamSynchronize(st));
-    if (loss) *loss = res[0];
-    return check_tc(net);
+    return check_tc(net, loss);
 }
 
 dmtz_status dmtz_cnn_step(dmtz_cnn *net, float lr) {

@@ -1622,6 +1622,9 @@ struct dmtz_ctx {
     unsigned char *work = nullptr;
     size_t work_bytes = 0;
     unsigned long long *report = nullptr;  // pinned: counts of the last round (k_round_end), hc's layout
+    unsigned long long report_seq = 0;       // the last round's end; report[8] once it is done
+    std::vector<cudaEvent_t> events;         // of the phase timer
+    cudaEvent_t span[2] = {nullptr, nullptr};  // a correction's begin and end
     int march_blocks = 0;          // blocks of k_grad_march the device holds at once (0: not asked yet)
     void *loopctl = nullptr;       // device copy of the graph loop's control block (kept: a
                                    // cudaFree per call would synchronise the whole device)
@@ -2521,6 +2524,9 @@ void dmtz_ctx_destroy(dmtz_ctx *ctx) {
     cudaFree(ctx->loopctl);
     cudaFree(ctx->work);
     cudaFreeHost(ctx->report);
+    for (cudaEvent_t e : ctx->events) cudaEventDestroy(e);
+    for (cudaEvent_t e : ctx->span)
+        if (e) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->side) cudaStreamDestroy(ctx->side);
     if (ctx->side_done) cudaEventDestroy(ctx->side_done);
@@ -2852,7 +2858,7 @@ __device__ __forceinline__ LoopCtl loop_next(LoopCtl c, const unsigned long long
 __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Lists T, const __grid_constant__ Lists L, unsigned long long *counters,
                                                      const __grid_constant__ BrickMarks B, LoopCtl *ctl,
                                                      cudaGraphConditionalHandle hwhile, cudaGraphConditionalHandle hswitch,
-                                                     unsigned long long *report) {
+                                                     unsigned long long *report, unsigned long long seq) {
     __shared__ bool last;
     const int st = ctl ? ctl->state : LS_CP;
     const bool begun = !ctl || ctl->begun;
@@ -2901,6 +2907,7 @@ __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Li
     } else {
         for (int k = 0; k < 8; k++) report[k] = counters[k];
         __threadfence_system();
+        *reinterpret_cast<volatile unsigned long long *>(report + 8) = seq;
     }
     if (!stop) counters[4] = counters[7] = 0;  // a stalled round's requests were applied: the host starts afresh
 }
@@ -2908,36 +2915,41 @@ __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Li
 // ----------------------------------------------------------------------------- phase timers
 namespace {
 enum { PH_PAIR = 0, PH_FIXCP, PH_PATH, PH_FIXPATH, PH_APPLY, PH_SETUP, PH_N };
-// event pairs recorded on the context's stream around each phase; summed once
-// the stream has finished
+// Phase times from events on the context's stream: one at each boundary (a phase
+// ends where the next begins), from a pool that the context keeps.  reuse() adds up
+// what is complete and takes its events back, so a long host-driven loop needs
+// about 64 of them (two per phase, created and destroyed in every call: 1 ms of a
+// 16^3 field's 48 rounds).
 struct PhaseTimer {
     cudaStream_t st;
-    std::vector<cudaEvent_t> pool;
-    std::vector<std::pair<int, size_t>> marks;  // phase, index of its first event
+    std::vector<cudaEvent_t> &pool;
+    std::vector<std::pair<int, size_t>> marks;  // phase that begins (PH_N: none), its event
     size_t used = 0;
-    cudaEvent_t next() {
+    double total[PH_N] = {0, 0, 0, 0, 0, 0};
+    void mark(int ph) {
+        if (used >= 64 && marks.back().first == PH_N) {
+            cudaEventSynchronize(pool[used - 1]);
+            reuse();
+        }
         if (used == pool.size()) {
             cudaEvent_t e;
             cudaEventCreate(&e);
             pool.push_back(e);
         }
-        return pool[used++];
+        cudaEventRecord(pool[used], st);
+        marks.push_back({ph, used++});
     }
-    void begin(int ph) {
-        marks.push_back({ph, used});
-        cudaEventRecord(next(), st);
-    }
-    void end() { cudaEventRecord(next(), st); }
-    void sum(double out[PH_N]) {
-        for (int k = 0; k < PH_N; k++) out[k] = 0;
-        for (auto &m : marks) {
+    void stop() { mark(PH_N); }
+    // the events recorded so far are complete, and no phase is open
+    void reuse() {
+        for (size_t k = 0; k + 1 < marks.size(); k++) {
+            if (marks[k].first == PH_N) continue;
             float t = 0;
-            cudaEventElapsedTime(&t, pool[m.second], pool[m.second + 1]);
-            out[m.first] += t;
+            cudaEventElapsedTime(&t, pool[marks[k].second], pool[marks[k + 1].second]);
+            total[marks[k].first] += t;
         }
-    }
-    ~PhaseTimer() {
-        for (auto e : pool) cudaEventDestroy(e);
+        marks.clear();
+        used = 0;
     }
 };
 }  // namespace
@@ -2985,7 +2997,7 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
                 break;
             }
             k_round_end<<<pgrid / 8, kBlock, 0, st>>>(ctx->inc_scan ? rebuilt_lists(ctx) : Lists{}, mismatch_lists(ctx),
-                                                      ctx->counters, brick_marks(ctx, g), dctl, hwhile, hsw, nullptr);
+                                                      ctx->counters, brick_marks(ctx, g), dctl, hwhile, hsw, nullptr, 0);
             cudaGraph_t tmp;
             if (cudaStreamEndCapture(st, &tmp) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
             size_t nn = 1;
@@ -3039,7 +3051,7 @@ static void host_round_end(dmtz_ctx *ctx, const Grid &g) {
     k_round_end<<<persistent_grid() / 8, kBlock, 0, ctx->stream>>>(ctx->inc_scan ? rebuilt_lists(ctx) : Lists{},
                                                                    mismatch_lists(ctx), ctx->counters, brick_marks(ctx, g), nullptr,
                                                                    cudaGraphConditionalHandle{}, cudaGraphConditionalHandle{},
-                                                                   ctx->report);
+                                                                   ctx->report, ++ctx->report_seq);
     ctx->launches++;
 }
 
@@ -3148,10 +3160,15 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     CK(cudaSetDevice(ctx->device));
     if ((s = ensure(ctx, g)) != DMTZ_OK) return s;
     cudaStream_t st = ctx->stream;
-    if (!ctx->report) CK(cudaHostAlloc((void **)&ctx->report, 8 * sizeof(unsigned long long), cudaHostAllocDefault));
-    cudaEvent_t e0, e1;
-    CK(cudaEventCreate(&e0));
-    CK(cudaEventCreate(&e1));
+    if (!ctx->report) {
+        CK(cudaHostAlloc((void **)&ctx->report, 16 * sizeof(unsigned long long), cudaHostAllocDefault));
+        memset(ctx->report, 0, 16 * sizeof(unsigned long long));
+    }
+    if (!ctx->span[0]) {
+        CK(cudaEventCreate(&ctx->span[0]));
+        CK(cudaEventCreate(&ctx->span[1]));
+    }
+    const cudaEvent_t e0 = ctx->span[0], e1 = ctx->span[1];
     if ((s = upload(ctx, ctx->f, orig, g.V, on_device)) != DMTZ_OK) return s;
     // the decompressed field travels on a second stream while the original
     // field's gradient is computed; the work that reads it waits for it
@@ -3165,9 +3182,9 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     // range and bound exactly as the reference computes them (main_3d.cu:6303-6323)
     double mn, mx;
     ctx->launches = 0;
-    PhaseTimer pt_{st};
+    PhaseTimer pt_{st, ctx->events};
     CK(cudaEventRecord(e0, st));
-    pt_.begin(PH_SETUP);
+    pt_.mark(PH_SETUP);
     if ((s = device_minmax(ctx, ctx->f, g.V, mn, mx)) != DMTZ_OK) return s;
     const double bound = (mx - mn) * rel_eps;
     const double range = mx - mn;
@@ -3190,7 +3207,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     run_pairing(ctx, g, Qs, ctx->P.crit, 1);
     k_fill_i32<<<grid_for(g.V), kBlock, 0, st>>>(ctx->cnt, 1, g.V);
     ctx->launches++;
-    pt_.end();
+    pt_.stop();
     unsigned long long hc[8];
     auto read_counts = [&]() -> dmtz_status {
         CK(cudaMemcpyAsync(hc, ctx->counters, sizeof(hc), cudaMemcpyDeviceToHost, st));
@@ -3198,9 +3215,18 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         return DMTZ_OK;
     };
     // counts after a round's end; lists that overflowed grow and are rebuilt
+    // (the counts stand in pinned memory as soon as the round's end wrote them, some
+    // microseconds before a wait for the stream would return)
     auto read_fit = [&](int want_saddles) -> dmtz_status {
-        CK(cudaStreamSynchronize(st));
-        for (int k = 0; k < 8; k++) hc[k] = ctx->report[k];
+        volatile unsigned long long *report = ctx->report;
+        for (unsigned spin = 1; report[8] != ctx->report_seq; spin++) {
+            if (spin % 4096) continue;
+            const cudaError_t q = cudaStreamQuery(st);
+            if (q == cudaSuccess) break;
+            if (q != cudaErrorNotReady) CK(q);
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);
+        for (int k = 0; k < 8; k++) hc[k] = report[k];
         return fit_lists(ctx, g, want_saddles, hc);
     };
     if ((s = read_counts()) != DMTZ_OK || (s = fit_lists(ctx, g, 1, hc)) != DMTZ_OK) return s;
@@ -3208,9 +3234,9 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     memset(&R, 0, sizeof(R));
     for (int k = 0; k < 4; k++) R.initial_mismatch[k] = (int64_t)hc[k];
     if (net) {
-        pt_.begin(PH_SETUP);
+        pt_.mark(PH_SETUP);
         if ((s = learned_start(ctx, net, g, bound)) != DMTZ_OK) return s;
-        pt_.end();
+        pt_.stop();
         if ((s = read_counts()) != DMTZ_OK || (s = fit_lists(ctx, g, 1, hc)) != DMTZ_OK) return s;
     }
     i64 cc[4] = {(i64)hc[0], (i64)hc[1], (i64)hc[2], (i64)hc[3]};
@@ -3244,7 +3270,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         c.state = cp_any() ? cp_state(cc[0] + cc[1] + cc[2] + cc[3]) : (pvp ? LS_PDF : LS_DONE);
         LoopCtl fin = c;
         if (c.state != LS_DONE) {
-            pt_.begin(PH_PAIR);
+            pt_.mark(PH_PAIR);
             LoopCtl cur = c;
             while (true) {
                 for (int k = 0; k < 4; k++) cur.cap[k] = ctx->capL[k];
@@ -3278,7 +3304,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
                     }
                 }
             }
-            pt_.end();
+            pt_.stop();
             // kernels per body run: the round's end, plus each state's own: a fix
             // round is fix + update, then the repair (gradient, and the scan where
             // the lists are not rebuilt), or the whole gradient; one end more
@@ -3312,14 +3338,12 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             R.cp_rounds++;
             paths_fresh = false;
             const bool full = cc[0] + cc[1] + cc[2] + cc[3] >= heavy;
-            pt_.begin(PH_FIXCP);
+            pt_.mark(PH_FIXCP);
             k_fix_cp<<<pgrid, kBlock, 0, st>>>(rc, cp_lists(ctx), ps);
-            pt_.end();
-            pt_.begin(PH_APPLY);
+            pt_.mark(PH_APPLY);
             k_apply<<<pgrid, kBlock, 0, st>>>(rc, range, pt, 1, ctx->changed, nullptr, full ? BrickMarks{} : brick_marks(ctx, g));
-            pt_.end();
             ctx->launches += 2;
-            pt_.begin(PH_PAIR);
+            pt_.mark(PH_PAIR);
             if (full) {  // lists in place: nothing to take back
                 repair_full(ctx, g, Qs, ctx->P.crit, ps == 1);
                 const int inc = ctx->inc_scan;
@@ -3330,7 +3354,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
                 repair_dirty(ctx, g, Qs, ctx->P.crit, ps == 1, true);
                 host_round_end(ctx, g);
             }
-            pt_.end();
+            pt_.stop();
             if ((s = read_fit(ps == 1)) != DMTZ_OK) return s;
             if (opts->break_stalls && hc[7] == 0 && rounds < max_rounds && (hc[0] || hc[1] || hc[2] || hc[3])) {
                 if ((s = break_stall(ctx, g, rc, PR, Qs, 1, ps == 1, R.stall_breaks)) != DMTZ_OK) return s;
@@ -3348,28 +3372,26 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         rounds++;
         R.path_rounds++;
         if (!paths_fresh) {  // else the last re-check ran on this same state
-            pt_.begin(PH_PATH);
+            pt_.mark(PH_PATH);
             detect_paths(ctx, g, rc, PR, pgrid, conn);
             if (walls && (s = detect_walls(ctx, g, rc, n_wall)) != DMTZ_OK) return s;
-            pt_.end();
+            pt_.stop();
         }
         const i64 walls_fixed = walls ? n_wall : 0;
         paths_fresh = false;
-        pt_.begin(PH_FIXPATH);
+        pt_.mark(PH_FIXPATH);
         k_fix_path<<<pgrid, kBlock, 0, st>>>(rc, PR);
         if (walls_fixed > 0) {
             k_fix_wall<<<pgrid, kBlock, 0, st>>>(rc, WR);
             ctx->launches++;
         }
-        pt_.end();
-        pt_.begin(PH_APPLY);
+        pt_.mark(PH_APPLY);
         k_apply<<<pgrid, kBlock, 0, st>>>(rc, range, pt, 1, ctx->changed, nullptr, brick_marks(ctx, g));
-        pt_.end();
         ctx->launches += 2;
-        pt_.begin(PH_PAIR);
+        pt_.mark(PH_PAIR);
         repair_dirty(ctx, g, Qs, ctx->P.crit, 1, true);
         host_round_end(ctx, g);
-        pt_.end();
+        pt_.stop();
         if ((s = read_fit(1)) != DMTZ_OK) return s;
         if (opts->break_stalls && hc[7] == 0 && rounds < max_rounds && hc[5] + hc[6] + walls_fixed > 0) {
             if ((s = break_stall(ctx, g, rc, PR, Qs, 0, 1, R.stall_breaks, walls_fixed > 0 ? &WR : nullptr)) !=
@@ -3381,9 +3403,9 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         for (int k = 0; k < 4; k++) cc[k] = (i64)hc[k];
         n_as = n_ds = n_wall = 0;
         if (!cp_any()) {
-            pt_.begin(PH_PATH);
+            pt_.mark(PH_PATH);
             detect_paths(ctx, g, rc, PR, pgrid, conn);
-            pt_.end();
+            pt_.stop();
             if ((s = read_counts()) != DMTZ_OK) return s;
             n_as = (i64)hc[5];
             n_ds = (i64)hc[6];
@@ -3406,8 +3428,6 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     CK(cudaStreamSynchronize(st));
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     CK(cudaGetLastError());
     for (int k = 0; k < 4; k++) R.final_mismatch[k] = cc[k];
     R.final_paths[0] = n_as;
@@ -3418,7 +3438,8 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     R.error_flags = err;
     R.seconds = ms * 1e-3;
     R.kernel_launches = ctx->launches;
-    pt_.sum(R.phase_ms);
+    pt_.reuse();
+    for (int k = 0; k < PH_N; k++) R.phase_ms[k] = pt_.total[k];
     if (rep) *rep = R;
     if (err & ERR_OOB) return fail(ctx, DMTZ_ERR_OOB, "a fix rule indexed out of range");
     if (err & ERR_WALK) return fail(ctx, DMTZ_ERR_CYCLE, "ascending path walk exceeded its step cap");
