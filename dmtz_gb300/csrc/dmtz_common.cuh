@@ -220,6 +220,10 @@ __device__ __forceinline__ void tet_unref(const Grid &g, i64 t, int &x, int &y, 
 }
 
 // packed field accessors
+// The kernel launched behind this one (launch_next) may start; and, there: wait
+// until the kernel before is done and its memory visible.  No effect otherwise.
+__device__ __forceinline__ void let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A slot in a list whose length is *n: the converged lanes appending to the
 // same counter take one atomic between them (the leader's), so that a list
 // filled from every warp does not serialise on one address.

@@ -656,6 +656,8 @@ __global__ void __launch_bounds__((brick_threads<SX, SY, SZ>()), SX == 8 ? 3 : 2
     const int wx = t % WX, wy = (t / WX) % WY, wz = t / (WX * WY);
     const int cx = t % CX, cy = (t / CX) % CY, cz = t / (CX * CY);
     const int ox = t % SX, oy = (t / SX) % SY, oz = t / (SX * SY);
+    let_next();
+    after_previous();
     if (blockIdx.x >= gridDim.x - K.blocks) {  // the blocks that carry the old lists over
         keep_lists(g, O, K, blockIdx.x - (gridDim.x - K.blocks));
         return;
