@@ -14,7 +14,8 @@
 //   k_conv_tcx  the convolutions (forward and data gradient) on tcgen05: the
 //            128 rows of a product are a plane across x, which marches (the
 //            default path; see its comment).
-//   k_conv_tc  the same with a box of vertices per MMA chain.
+//   k_conv_out  the last layer, of which one channel is needed.
+//   k_conv_tc  all layers with a box of vertices per MMA chain.
 //   k_conv   the same convolution on mma.sync.m16n8k16 (bf16 in, f32
 //            accumulate).  A block keeps all 27 x out x in weights in shared
 //            memory and streams 8x8x4-vertex tiles (+1 halo) through a
@@ -587,18 +588,20 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv_tc(const __grid_consta
 // against 14 x 8 x 2 tiles with halo boxes, where one lane issued and the shifts
 // were warp shuffles: 32 -> 32 76 us (148), 16 -> 32 50 (101), 32 -> 16 59 (128);
 // at 100 x 75 x 53 24 (40), 19 (30), 20 (35), data gradients 29 (47) and 23 (45).
+// (The output layer, 32 -> 16, has its own kernel since: k_conv_out.)
 constexpr int CX_A = 8, CX_B = 16, CX_GA = CX_A + 2, CX_GB = CX_B + 2, CX_NX = 2, CX_ACC = 4, CX_ST = 6;
 constexpr int CX_EPI = 8, CX_THREADS = 96 + 32 * CX_EPI;
 struct March {
     int W, na, nb;  // extents along x, a, b
     i64 sa, sb;     // vertex strides of a and b
     int swapped;    // a = z and b = y
+    int ta, tb;     // a column's outputs along a and b
     int nta;        // columns along a
     i64 outputs;    // of all columns
 };
-inline March make_march(int W, int H, int D) {
+inline March make_march(int W, int H, int D, int ta = CX_A, int tb = CX_B) {
     auto up = [](i64 n, i64 m) { return (n + m - 1) / m * m; };
-    const bool swap = up(D, CX_A) * up(H, CX_B) < up(H, CX_A) * up(D, CX_B);
+    const bool swap = up(D, ta) * up(H, tb) < up(H, ta) * up(D, tb);
     March m{};
     m.W = W;
     m.na = swap ? D : H;
@@ -606,8 +609,10 @@ inline March make_march(int W, int H, int D) {
     m.sa = swap ? (i64)W * H : W;
     m.sb = swap ? W : (i64)W * H;
     m.swapped = swap;
-    m.nta = (m.na + CX_A - 1) / CX_A;
-    m.outputs = (i64)m.nta * ((m.nb + CX_B - 1) / CX_B) * W;
+    m.ta = ta;
+    m.tb = tb;
+    m.nta = (m.na + ta - 1) / ta;
+    m.outputs = (i64)m.nta * ((m.nb + tb - 1) / tb) * W;
     return m;
 }
 // the part of a run that lies in one column: outputs [o0, o1) from slices j0..j1
@@ -615,8 +620,8 @@ struct Stretch {
     int a0, b0, o0, o1, j0, j1;
     __device__ __forceinline__ Stretch(const March &m, i64 g, i64 end) {
         const i64 col = g / m.W;
-        a0 = (int)(col % m.nta) * CX_A;
-        b0 = (int)(col / m.nta) * CX_B;
+        a0 = (int)(col % m.nta) * m.ta;
+        b0 = (int)(col / m.nta) * m.tb;
         o0 = (int)(g - col * m.W);
         o1 = (int)min((i64)m.W, o0 + (end - g));
         j0 = max(o0 - 1, 0);
@@ -666,13 +671,12 @@ __device__ __forceinline__ void st32(void *p, const Vec8 &r) {
 template <int CIN, int COUT, int MODE, bool FLIP>
 __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constant__ CUtensorMap tmap, const March m,
                                                           const bf16 *__restrict__ wt, const float *__restrict__ bias,
-                                                          void *out, const bf16 *__restrict__ aux, int *err) {
+                                                          bf16 *out, const bf16 *__restrict__ aux, int *err) {
     constexpr int KCH = CIN / 8, N = 3 * COUT, ROW = CIN * 2;
     constexpr uint32_t WGRP = N * 16, LINE = CX_GA * ROW, SLICE = CX_GB * LINE, STAGE = cx_stage<CIN>();
-    constexpr uint32_t COLS = COUT == 32 ? 128 : 64, ALLOC = CX_ACC * COLS;
-    constexpr int EPI = MODE == 1 ? 4 : CX_EPI;  // warps of the epilogue: one channel needs no second half
-    static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "tile shapes");
-    static_assert(ALLOC == 256 || ALLOC == 512, "tensor-memory allocation is a power of two");
+    constexpr uint32_t COLS = 128, ALLOC = CX_ACC * COLS;
+    static_assert((CIN == 16 || CIN == 32) && COUT == 32 && MODE != 1, "tile shapes");
+    static_assert(ALLOC == 512, "all of the tensor memory");
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(8) uint64_t bar_full[CX_ST], bar_empty[CX_ST], bar_mma[CX_ACC], bar_free[CX_ACC], bar_w, bar_done;
@@ -697,7 +701,7 @@ __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constan
         }
         for (int q = 0; q < CX_ACC; q++) {
             init(mma(q), 1);
-            init(fre(q), EPI);
+            init(fre(q), CX_EPI);
         }
         init(wbar, 32 * CX_EPI);
         init(done, 2);
@@ -799,8 +803,8 @@ __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constan
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(wbar) : "memory");
 
         // the epilogue: channels [c0, c0 + NC) of lane quarter `quarter`
-        constexpr int NC = MODE == 1 ? 1 : COUT * 4 / CX_EPI;
-        static_assert(MODE == 1 || NC == 16, "a thread stores 32 bytes");
+        constexpr int NC = COUT * 4 / CX_EPI;
+        static_assert(NC == 16, "a thread stores 32 bytes");
         const int quarter = warp & 3, half = (warp - 3) >> 2, c0 = half * NC;
         const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
         float bsh[MODE == 2 ? 1 : NC];
@@ -810,7 +814,7 @@ __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constan
         }
         const int r = quarter * 32 + lane;
         int q = 0;
-        for (i64 g = half < EPI / 4 ? first : end; g < end && !failed;) {
+        for (i64 g = first; g < end && !failed;) {
             const Stretch t(m, g, end);
             const int a = t.a0 + (r & 7), b = t.b0 + (r >> 3);
             const bool row = a < m.na && b < m.nb;
@@ -822,25 +826,21 @@ __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constan
             auto store = [&](int o, const Vec8 &mk) {  // cur is complete: output o
                 if (!row) return;
                 const i64 v = v0 + o;
-                if constexpr (MODE == 1) {
-                    reinterpret_cast<float *>(out)[v] = cur[0] + bsh[0];
-                } else {
-                    Vec8 pk;
+                Vec8 pk;
 #pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        float x0 = cur[2 * i], x1 = cur[2 * i + 1];
-                        if constexpr (MODE == 0) {
-                            x0 = fmaxf(x0 + bsh[2 * i], 0.f);
-                            x1 = fmaxf(x1 + bsh[2 * i + 1], 0.f);
-                        } else {
-                            if (!(__uint_as_float(mk.v[i] << 16) > 0.f)) x0 = 0.f;
-                            if (!(__uint_as_float(mk.v[i] & 0xFFFF0000u) > 0.f)) x1 = 0.f;
-                        }
-                        const __nv_bfloat162 two = __floats2bfloat162_rn(x0, x1);
-                        pk.v[i] = *reinterpret_cast<const uint32_t *>(&two);
+                for (int i = 0; i < 8; i++) {
+                    float x0 = cur[2 * i], x1 = cur[2 * i + 1];
+                    if constexpr (MODE == 0) {
+                        x0 = fmaxf(x0 + bsh[2 * i], 0.f);
+                        x1 = fmaxf(x1 + bsh[2 * i + 1], 0.f);
+                    } else {
+                        if (!(__uint_as_float(mk.v[i] << 16) > 0.f)) x0 = 0.f;
+                        if (!(__uint_as_float(mk.v[i] & 0xFFFF0000u) > 0.f)) x1 = 0.f;
                     }
-                    st32(reinterpret_cast<bf16 *>(out) + v * COUT + c0, pk);
+                    const __nv_bfloat162 two = __floats2bfloat162_rn(x0, x1);
+                    pk.v[i] = *reinterpret_cast<const uint32_t *>(&two);
                 }
+                st32(out + v * COUT + c0, pk);
             };
             auto mask = [&](int o) {
                 Vec8 mk{};
@@ -884,6 +884,204 @@ __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constan
                 }
             }
             if (t.j1 < t.o1 && !failed) store(t.o1 - 1, mask(t.o1 - 1));  // the column's last output: nothing follows it
+            g += t.o1 - t.o0;
+        }
+    }
+    if (failed) atomicOr(err, 1);
+    asm volatile("tcgen05.fence::before_thread_sync;\n");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(ALLOC));
+}
+
+// ------------------------------------------------- the output layer on tcgen05
+// The last convolution needs one output channel, and a product of fewer than 48
+// columns takes as long as one of 48.  So the other direction is folded too: the
+// columns are the 27 taps (of channel 0; 5 more are zero), and one product per 16
+// channels gives what every vertex of a slice adds to its 27 neighbours: 2 MMAs
+// per slice instead of 18.  The rows are the slice's 8 x 16 vertices with the
+// halo, of which 6 x 14 are outputs; the x contributions are added in registers
+// from slice to slice, the nine of the plane through shared memory.
+//
+// Runs, copies (four slices each, three stages) and waits as in k_conv_tcx; two
+// blocks per SM.  Warp 0 issues, warp 1 copies, warps 2..5 are the epilogue; a
+// warp whose wait gave up goes on without waiting, so that the others find it at
+// their barrier.
+//
+// Bound by memory: 1.5 times the input through the caches.  161 x 127 x 110: 47 us
+// (59 as 18 products of 48 columns); 100 x 75 x 53: 15 (20).  Exchanging four outputs
+// at a time changed neither.
+constexpr int OL_A = 6, OL_B = 14, OL_ROWS = 128, OL_NX = 4, OL_ST = 3, OL_ACC = 8, OL_COLS = 32, OL_THREADS = 192;
+template <int CIN>
+struct OutLayer {
+    static constexpr uint32_t ROW = CIN * 2, SLICE = OL_ROWS * ROW, STAGE = OL_NX * SLICE, WBYTES = (CIN / 8) * 32 * 16;
+    static constexpr size_t smem = 1024 + (size_t)OL_ST * STAGE + WBYTES + 2 * 9 * OL_ROWS * sizeof(float);
+};
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(OL_THREADS, 2) k_conv_out(const __grid_constant__ CUtensorMap tmap, const March m,
+                                                          const bf16 *__restrict__ wt, const float *__restrict__ bias,
+                                                          float *__restrict__ out, int *err) {
+    using T = OutLayer<CIN>;
+    constexpr uint32_t ALLOC = OL_ACC * OL_COLS;
+    static_assert(ALLOC == 256 && OL_ACC == 2 * OL_NX, "two copies' accumulators");
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ uint32_t tmem_slot;
+    __shared__ __align__(8) uint64_t bar_full[OL_ST], bar_empty[OL_ST], bar_mma[2], bar_free[2], bar_done;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t ring = (smem_addr(smem_raw) + 1023) & ~1023u, wbase = ring + OL_ST * T::STAGE;
+    unsigned char *ws = smem_raw + (wbase - smem_addr(smem_raw));
+    float(*sum)[9][OL_ROWS] = reinterpret_cast<float(*)[9][OL_ROWS]>(ws + T::WBYTES);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
+                         smem_addr(&tmem_slot)),
+                     "n"(ALLOC));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+    }
+    auto full = [&](int s) { return smem_addr(&bar_full[s]); };
+    auto empty = [&](int s) { return smem_addr(&bar_empty[s]); };
+    auto mma = [&](int c) { return smem_addr(&bar_mma[c & 1]); };
+    auto fre = [&](int c) { return smem_addr(&bar_free[c & 1]); };
+    const uint32_t done = smem_addr(&bar_done);
+    if (tid == 0) {
+        auto init = [](uint32_t bar, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(n)); };
+        for (int s = 0; s < OL_ST; s++) {
+            init(full(s), 1);
+            init(empty(s), 1);
+        }
+        for (int c = 0; c < 2; c++) {
+            init(mma(c), 1);
+            init(fre(c), 4);
+        }
+        init(done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n");
+    }
+    // weights: per channel group, row n = 9 (dx + 1) + 3 (db + 1) + (da + 1) is that tap of output channel 0
+    for (int i = tid; i < (CIN / 8) * 32; i += OL_THREADS) {
+        const int kc = i / 32, n = i % 32, dx = n / 9, a = n % 3, b = n / 3 % 3;
+        const int tap = dx + (m.swapped ? 9 * a + 3 * b : 3 * a + 9 * b);
+        const uint4 v = n < 27 ? *reinterpret_cast<const uint4 *>(wt + (i64)tap * COUT * CIN + kc * 8) : make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4 *>(ws + i * 16) = v;
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n");
+    asm volatile("tcgen05.fence::before_thread_sync;\n");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n");
+    const uint32_t tmem = tmem_slot;
+    const i64 per = m.outputs / gridDim.x, rest = m.outputs - per * gridDim.x;
+    const i64 first = blockIdx.x * per + min((i64)blockIdx.x, rest), end = first + per + (blockIdx.x < rest);
+    bool failed = false;
+
+    if (warp == 0) {  // MMA issuer; c: copies so far
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((32u >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint64_t b0 = smem_desc(wbase, 32 * 16, 128);
+        int c = 0;
+        for (i64 g = first; g < end && !failed;) {
+            const Stretch t(m, g, end);
+            for (int j = t.j0; j <= t.j1; j += OL_NX, c++) {
+                const int n = min(OL_NX, t.j1 - j + 1), s = c % OL_ST;
+                const bool copy = lane == 0 || c < 2;  // the copy, and the accumulators' last readers: a barrier per lane
+                if (!__all_sync(0xffffffffu, mbar_wait(copy ? full(s) : fre(c), (uint32_t)(copy ? c / OL_ST : c / 2 - 1) & 1u,
+                                                       kConvWaitPolls))) {
+                    failed = true;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;\n");
+                if (elect_one()) {
+                    for (int e = 0; e < n; e++) {
+                        const uint64_t a0 = swizzled_desc<T::ROW>(ring + s * T::STAGE + e * T::SLICE, 8 * T::ROW);
+#pragma unroll
+                        for (int kk = 0; kk < CIN / 16; kk++)
+                            tc_mma(tmem + (uint32_t)((c & 1) * OL_NX + e) * OL_COLS, a0 + kk * 2,
+                                   b0 + ((kk * 2 * 32 * 16) >> 4), idesc, kk != 0);
+                    }
+                    tc_commit(mma(c));
+                    tc_commit(empty(s));
+                }
+                __syncwarp();
+            }
+            g += t.o1 - t.o0;
+        }
+        if (elect_one()) tc_commit(done);
+        __syncwarp();
+        if (!mbar_wait(done, 0u, kConvWaitPolls)) failed = true;  // every MMA issued is done
+    } else if (warp == 1) {
+        if (lane == 0) {  // copies
+            int issued = 0;
+            for (i64 g = first; g < end && !failed;) {
+                const Stretch t(m, g, end);
+                for (int j = t.j0; j <= t.j1; j += OL_NX) {
+                    const int s = issued % OL_ST;
+                    if (issued >= OL_ST && !mbar_wait(empty(s), (uint32_t)(issued / OL_ST - 1) & 1u, kConvWaitPolls)) {
+                        failed = true;
+                        break;
+                    }
+                    const uint32_t bar = full(s);
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(T::STAGE));
+                    asm volatile(
+                        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, "
+                        "{%2, %3, %4, %5}], [%6];\n" ::"r"(ring + s * T::STAGE),
+                        "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(0), "r"(t.a0 - 1), "r"(t.b0 - 1), "r"(j), "r"(bar)
+                        : "memory");
+                    issued++;
+                }
+                g += t.o1 - t.o0;
+            }
+            // the copies still in flight land before the block leaves
+            for (int j = issued - OL_ST; j < issued; j++)
+                if (j >= 0) mbar_wait(full(j % OL_ST), (uint32_t)(j / OL_ST) & 1u, kConvWaitPolls);
+        }
+        __syncwarp();
+    } else {
+        const int quarter = warp & 3, r = quarter * 32 + lane, ra = r & 7, rb = r >> 3;
+        const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
+        const bool inner = ra >= 1 && ra <= OL_A && rb >= 1 && rb <= OL_B;
+        const float b0 = bias[0];
+        int c = 0, buf = 0;
+        for (i64 g = first; g < end;) {
+            const Stretch t(m, g, end);
+            const int a = t.a0 + ra - 1, b = t.b0 + rb - 1;
+            const bool row = inner && a < m.na && b < m.nb;
+            const i64 v0 = a * m.sa + b * m.sb;
+            // what this row adds to its nine neighbours' outputs at j (next) and j - 1 (cur), from the slices before j
+            float next[9], cur[9];
+#pragma unroll
+            for (int u = 0; u < 9; u++) next[u] = cur[u] = 0.f;
+            auto store = [&](int o) {  // cur is complete: output o
+#pragma unroll
+                for (int u = 0; u < 9; u++) sum[buf][u][r] = cur[u];
+                asm volatile("bar.sync 1, 128;\n" ::: "memory");
+                if (row) {
+                    float x = 0.f;
+#pragma unroll
+                    for (int u = 0; u < 9; u++) x += sum[buf][u][r + (u % 3 - 1) + 8 * (u / 3 - 1)];
+                    out[v0 + o] = x + b0;
+                }
+                buf ^= 1;
+            };
+            for (int j = t.j0; j <= t.j1; j += OL_NX, c++) {
+                const int n = min(OL_NX, t.j1 - j + 1);
+                if (!failed && !mbar_wait(mma(c), (uint32_t)(c / 2) & 1u, kConvWaitPolls)) failed = true;
+                asm volatile("tcgen05.fence::after_thread_sync;\n");
+                for (int e = 0; e < n; e++) {
+                    uint32_t p[OL_COLS];
+                    tmem_ld<OL_COLS>(lanes + (uint32_t)((c & 1) * OL_NX + e) * OL_COLS, p);
+                    tmem_wait();
+                    if (e == n - 1) {
+                        asm volatile("tcgen05.fence::before_thread_sync;\n");
+                        __syncwarp();
+                        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(fre(c)) : "memory");
+                    }
+#pragma unroll
+                    for (int u = 0; u < 9; u++) cur[u] += __uint_as_float(p[18 + u]);
+                    if (j + e > t.o0) store(j + e - 1);
+#pragma unroll
+                    for (int u = 0; u < 9; u++) {
+                        cur[u] = next[u] + __uint_as_float(p[9 + u]);
+                        next[u] = __uint_as_float(p[u]);
+                    }
+                }
+            }
+            if (t.j1 < t.o1) store(t.o1 - 1);  // the column's last output: nothing follows it
             g += t.o1 - t.o0;
         }
     }
@@ -1545,11 +1743,11 @@ dmtz_status box_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, int 
     const cuuint32_t box[4] = {8, GX, GY, GZ};
     return encode_map(net, tm, act, 4, dims, strides, box);
 }
-// and for k_conv_tcx's slices: whole vertices, axes (channel, a, b, x)
-dmtz_status slice_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, const March &m) {
+// and for k_conv_tcx's and k_conv_out's slices with their halo: whole vertices, axes (channel, a, b, x)
+dmtz_status slice_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, const March &m, int nx) {
     const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)m.na, (cuuint64_t)m.nb, (cuuint64_t)m.W}, row = (cuuint64_t)C * 2;
     const cuuint64_t strides[3] = {row * m.sa, row * m.sb, row};
-    const cuuint32_t box[4] = {(cuuint32_t)C, CX_GA, CX_GB, CX_NX};
+    const cuuint32_t box[4] = {(cuuint32_t)C, (cuuint32_t)m.ta + 2, (cuuint32_t)m.tb + 2, (cuuint32_t)nx};
     return encode_map(net, tm, act, 4, dims, strides, box, C == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 // and for k_wgrad_tc's lines: whole vertices, axes (channel, x, third, fourth);
@@ -1567,14 +1765,22 @@ template <int CIN, int COUT, int MODE, bool FLIP>
 dmtz_status conv(dmtz_cnn *net, const Dims &d, const bf16 *in, const bf16 *w, const float *bias, void *out,
                  const bf16 *aux, cudaStream_t st) {
     if (net->tensor_path == 2) {
-        March m = make_march(d.W, d.H, d.D);
         CUtensorMap tm;
-        dmtz_status s = slice_map(net, &tm, in, CIN, m);
-        if (s != DMTZ_OK) return s;
+        dmtz_status s;
         int *err = net->tc_err;
-        void *args[] = {&tm, &m, &w, &bias, &out, &aux, &err};
-        return launch_persistent(net, k_conv_tcx<CIN, COUT, MODE, FLIP>, CX_THREADS, cx_smem<CIN, COUT>(), m.outputs, net->nsm,
-                                 nullptr, st, args);
+        if constexpr (MODE == 1) {
+            March m = make_march(d.W, d.H, d.D, OL_A, OL_B);
+            if ((s = slice_map(net, &tm, in, CIN, m, OL_NX)) != DMTZ_OK) return s;
+            void *args[] = {&tm, &m, &w, &bias, &out, &err};
+            return launch_persistent(net, k_conv_out<CIN, COUT>, OL_THREADS, OutLayer<CIN>::smem, m.outputs, 2 * net->nsm, nullptr,
+                                     st, args);
+        } else {
+            March m = make_march(d.W, d.H, d.D);
+            if ((s = slice_map(net, &tm, in, CIN, m, CX_NX)) != DMTZ_OK) return s;
+            void *args[] = {&tm, &m, &w, &bias, &out, &aux, &err};
+            return launch_persistent(net, k_conv_tcx<CIN, COUT, MODE, FLIP>, CX_THREADS, cx_smem<CIN, COUT>(), m.outputs,
+                                     net->nsm, nullptr, st, args);
+        }
     }
     if (net->tensor_path) {
         Dims dt = make_tc_dims(d.W, d.H, d.D);

@@ -423,3 +423,21 @@ def test_forward_column_edges(net, dims):
     ref, _ = R.forward(feat_h, p.astype(np.float64))
     assert _rel(got, ref) < 3e-3
     assert np.abs(got - ref).max() < 2e-2 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("dims", [(5, 6, 14), (4, 7, 15), (4, 15, 7), (1, 31, 13), (90, 3, 2), (23, 14, 6)])
+def test_output_layer_column_edges(net, dims):
+    """Grids at the edges of the output layer's 6 x 14 columns, in both
+    orientations, with stretches of every length modulo its four slices
+    (tolerances as in the forward test)."""
+    W, H, D = dims
+    p = _params(16)
+    net.set_params(p)
+    feat_h, feat_d = _feat(17, dims)
+    out = torch.empty(W * H * D, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    net.forward(feat_d.data_ptr(), out.data_ptr(), dims)
+    got = out.cpu().numpy().reshape(D, H, W).astype(np.float64)
+    ref, _ = R.forward(feat_h, p.astype(np.float64))
+    assert _rel(got, ref) < 3e-3
+    assert np.abs(got - ref).max() < 2e-2 * np.abs(ref).max()
