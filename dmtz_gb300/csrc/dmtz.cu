@@ -2981,23 +2981,39 @@ struct PhaseTimer {
 };
 }  // namespace
 
-// Build and run the graph-driven loop.  Returns the final LoopCtl in *out.
-// The states' counters (requests, progress, separatrix records) as its first state needs them.
-static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const CpLists &L,
-                                  const PathRec &PR, const FieldState &Qs, double range, int ps, int pt, int conn,
-                                  LoopCtl init, LoopCtl *out) {
-    cudaStream_t st = ctx->stream;
-    const unsigned pgrid = persistent_grid();
-    if (!ctx->loopctl) CK(cudaMalloc(&ctx->loopctl, sizeof(LoopCtl)));
-    LoopCtl *dctl = static_cast<LoopCtl *>(ctx->loopctl);
-    init.begun = 0;
-    CK(cudaMemcpyAsync(dctl, &init, sizeof(LoopCtl), cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), st));
-    CK(cudaMemsetAsync(ctx->counters + 7, 0, sizeof(unsigned long long), st));
-    CK(cudaMemsetAsync(ctx->counters + 27, 0, sizeof(unsigned long long), st));
-    if (init.state != LS_PFIX) CK(cudaMemsetAsync(ctx->counters + 5, 0, 2 * sizeof(unsigned long long), st));
+// The loop as an executable graph, with the lists' capacities that it was built for.
+// Building and instantiating takes 110 us of host time and destroying 60 to 100, so
+// the first is done while the set-up's kernels run and the last while the results travel.
+struct LoopGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    i64 cap[4] = {0, 0, 0, 0};
+    bool fits(const dmtz_ctx *ctx) const {
+        for (int k = 0; k < 4; k++)
+            if (cap[k] != ctx->capL[k]) return false;
+        return exec != nullptr;
+    }
+    void clear() {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
+        exec = nullptr;
+        graph = nullptr;
+    }
+    ~LoopGraph() { clear(); }
+};
+// (a capture: work already on the stream goes on)
+static dmtz_status build_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const PathRec &PR, const FieldState &Qs,
+                                    double range, int ps, int pt, int conn, LoopGraph &lg) {
+    cudaStream_t st = ctx->stream;
+    const unsigned pgrid = persistent_grid();
+    const CpLists L = cp_lists(ctx);
+    if (!ctx->loopctl) CK(cudaMalloc(&ctx->loopctl, sizeof(LoopCtl)));
+    LoopCtl *dctl = static_cast<LoopCtl *>(ctx->loopctl);
+    lg.clear();
+    for (int k = 0; k < 4; k++) lg.cap[k] = ctx->capL[k];
+    cudaGraph_t &graph = lg.graph;
+    cudaGraphExec_t &exec = lg.exec;
+    const auto launches = ctx->launches;  // of a capture: none
     dmtz_status res = DMTZ_OK;
     do {
         if (cudaGraphCreate(&graph, 0) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
@@ -3058,16 +3074,30 @@ static dmtz_status run_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx &r
         }
         if (res != DMTZ_OK) break;
         if (cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
-        if (cudaGraphLaunch(exec, st) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
-        if (cudaMemcpyAsync(out, dctl, sizeof(LoopCtl), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess)
-            res = DMTZ_ERR_CUDA;
     } while (0);
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
+    ctx->launches = launches;
     if (res != DMTZ_OK) {
+        lg.clear();
         cudaGetLastError();
-        return fail(ctx, res, "building or running the loop graph failed");
+        return fail(ctx, res, "building the loop graph failed");
+    }
+    return DMTZ_OK;
+}
+// Run it.  Returns the final LoopCtl in *out.  The states' counters (requests,
+// progress, separatrix records) are as the first state needs them.
+static dmtz_status run_graph_loop(dmtz_ctx *ctx, const LoopGraph &lg, LoopCtl init, LoopCtl *out) {
+    cudaStream_t st = ctx->stream;
+    init.begun = 0;
+    CK(cudaMemcpyAsync(ctx->loopctl, &init, sizeof(LoopCtl), cudaMemcpyHostToDevice, st));
+    CK(cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), st));
+    CK(cudaMemsetAsync(ctx->counters + 7, 0, sizeof(unsigned long long), st));
+    CK(cudaMemsetAsync(ctx->counters + 27, 0, sizeof(unsigned long long), st));
+    if (init.state != LS_PFIX) CK(cudaMemsetAsync(ctx->counters + 5, 0, 2 * sizeof(unsigned long long), st));
+    if (cudaGraphLaunch(lg.exec, st) != cudaSuccess ||
+        cudaMemcpyAsync(out, ctx->loopctl, sizeof(LoopCtl), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(ctx, DMTZ_ERR_CUDA, "running the loop graph failed");
     }
     return DMTZ_OK;
 }
@@ -3234,6 +3264,24 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     k_fill_i32<<<grid_for(g.V), kBlock, 0, st>>>(ctx->cnt, 1, g.V);
     ctx->launches++;
     pt_.stop();
+    const unsigned pgrid = persistent_grid();
+    RuleCtx rc = rule_ctx(ctx, g, bound, et);
+    rc.range = range;
+    const PathRec PR = path_rec(ctx);
+    // every scan of the loop asks for saddles when preserve_saddles = 1, and none
+    // does in runs without separatrix rounds otherwise: the repairs can then rebuild
+    // the lists from the re-paired bricks alone
+    const int inc = ps == 1 || pvp == 0 ? 1 : 0;
+    LoopGraph lg;
+    auto fit_graph = [&]() -> dmtz_status {  // (built for lists that the loop itself uses)
+        if (lg.fits(ctx)) return DMTZ_OK;
+        const int keep = ctx->inc_scan;
+        ctx->inc_scan = inc;
+        const dmtz_status r = build_graph_loop(ctx, g, rc, PR, Qs, range, ps, pt, conn, lg);
+        ctx->inc_scan = keep;
+        return r;
+    };
+    if (use_graph && pvp && (s = fit_graph()) != DMTZ_OK) return s;  // (without separatrix rounds it may not be needed)
     unsigned long long hc[8];
     auto read_counts = [&]() -> dmtz_status {
         CK(cudaMemcpyAsync(hc, ctx->counters, sizeof(hc), cudaMemcpyDeviceToHost, st));
@@ -3267,17 +3315,10 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     }
     i64 cc[4] = {(i64)hc[0], (i64)hc[1], (i64)hc[2], (i64)hc[3]};
     i64 n_as = 1, n_ds = 1, n_wall = 1;
-    // every scan of the loop asks for saddles when preserve_saddles = 1, and none
-    // does in runs without separatrix rounds otherwise: the repairs can then rebuild
-    // the lists from the re-paired bricks alone
-    ctx->inc_scan = ps == 1 || pvp == 0 ? 1 : 0;
+    ctx->inc_scan = inc;
     const i64 heavy = heavy_cells(ctx, g);
     i64 rounds = 0;
     int converged = 1;
-    const unsigned pgrid = persistent_grid();
-    RuleCtx rc = rule_ctx(ctx, g, bound, et);
-    rc.range = range;
-    const PathRec PR = path_rec(ctx);
     if (walls && (s = ensure_walls(ctx)) != DMTZ_OK) return s;
     const WallRec WR = wall_rec(ctx);
     auto cp_any = [&]() { return cc[0] > 0 || cc[1] > 0 || cc[2] > 0 || cc[3] > 0; };
@@ -3300,8 +3341,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             LoopCtl cur = c;
             while (true) {
                 for (int k = 0; k < 4; k++) cur.cap[k] = ctx->capL[k];
-                if ((s = run_graph_loop(ctx, g, rc, cp_lists(ctx), PR, Qs, range, ps, pt, conn, cur, &fin)) != DMTZ_OK)
-                    return s;
+                if ((s = fit_graph()) != DMTZ_OK || (s = run_graph_loop(ctx, lg, cur, &fin)) != DMTZ_OK) return s;
                 if (!fin.overflow && !fin.stalled) break;
                 // a scan outgrew a list: grow it, rebuild the lists and resume
                 unsigned long long h4[4];
@@ -3443,10 +3483,11 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     CK(cudaEventRecord(e1, st));
     CK(cudaMemsetAsync(ctx->counters + 12, 0, sizeof(unsigned long long), st));
     k_count_u8<<<persistent_grid(), kBlock, 0, st>>>(ctx->changed, g.V, ctx->counters + 12);
+    if (on_device) CK(cudaMemcpyAsync(decp, ctx->g, sizeof(double) * (size_t)g.V, cudaMemcpyDeviceToDevice, st));
+    lg.clear();
     unsigned long long n_edited = 0;
     CK(cudaMemcpyAsync(&n_edited, ctx->counters + 12, sizeof(n_edited), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(decp, ctx->g, sizeof(double) * (size_t)g.V,
-                       on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
+    if (!on_device) CK(cudaMemcpyAsync(decp, ctx->g, sizeof(double) * (size_t)g.V, cudaMemcpyDeviceToHost, st));
     if (edit_counter_out)
         CK(cudaMemcpyAsync(edit_counter_out, ctx->cnt, sizeof(int) * (size_t)g.V, cudaMemcpyDeviceToHost, st));
     int err = 0;
