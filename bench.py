@@ -539,8 +539,9 @@ def run_cnn(args):
     # the tensor pipe's own rate for the instruction shape the convolutions
     # use (128 x 32 x 16) and for wider ones, measured here
     ceil = {n: net.mma_ceiling(n) for n in (32, 64, 96, 128, 256)}
-    # path 2's MMAs are 128 x 96 x 16, of whose 128 rows (16 per x-line) 14 are outputs
-    shape_n, row_eff = (96, 14 / 16) if args.tensor_path == 2 else (32, 1.0)
+    # path 2's MMAs are 128 x 96 x 16; their rows are 8 x 16 vertices of the plane across x
+    pad = -(-size // 8) * 8 * (-(-size // 16) * 16)
+    shape_n, row_eff = (96, size * size / pad) if args.tensor_path == 2 else (32, 1.0)
     line = {"metric": "learned-proposal network, forward TFLOP/s (bf16 tensor cores)",
             "value": CNN_FLOP_PER_VOX * V / (ms[0] * 1e-3) / 1e12, "unit": "TFLOP/s", "n_gpus": 1,
             "steps": args.steps, "warmup": 1, "ms_per_step": ms[0], "higher_is_better": True, "dtype": "bf16",

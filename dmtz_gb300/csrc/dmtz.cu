@@ -1603,7 +1603,7 @@ struct dmtz_ctx {
     i64 *as_tet = nullptr, *as_cur = nullptr, *ds_edge = nullptr, *ds_vert = nullptr;
     i64 capAS = 0, capDS = 0, capSad2 = 0;
     uint32_t *brick_flags = nullptr;  // per brick (a byte each, four to a word): in this round's repair
-    int inc_scan = 0;                 // repairs rebuild the mismatch lists incrementally (see k_list_keep)
+    int inc_scan = 0;                 // repairs rebuild the mismatch lists incrementally (see KeepOps)
     int strict_ds = 0;                // descending separatrix checks walk whole paths (k_ds_strict)
     i64 *list_tmp[4] = {nullptr, nullptr, nullptr, nullptr};  // rebuilt mismatch lists, capL entries each
     uint32_t *brick_list = nullptr;   // the repair's bricks, capB entries
@@ -2803,9 +2803,10 @@ dmtz_status dmtz_wall_detect(dmtz_ctx *ctx, int W, int H, int D, const double *o
 
 // ----------------------------------------------------------------------------- graph-driven loop
 // The host loop of main_3d.cu:6784-7149 as a state machine that runs on the
-// device: a CUDA graph holds a WHILE node whose body switches on the state,
-// runs that state's kernels, then lets one thread decide the next state and
-// the loop condition from the device-side counters.  States:
+// device: a CUDA graph holds a WHILE node whose body lets one thread decide the
+// state and the loop condition from the device-side counters that the round
+// before left (k_round_end), then switches on the state and runs its kernels.
+// A pass takes 10 us besides the kernels (6 the loop, 4 the switch).  States:
 //   CP     one critical-point round (fix rules, update, re-pair, mismatch)
 //   PDF    path phase: detect separatrix records, fix, update, re-pair, mismatch
 //   PCHECK detect separatrix records only (the reference's end-of-round check)
