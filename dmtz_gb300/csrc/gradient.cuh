@@ -639,95 +639,107 @@ __host__ __device__ constexpr int brick_threads() {
     return ((SX + 2) * (SY + 2) * (SZ + 2) + 31) / 32 * 32;
 }
 template <int SX, int SY, int SZ>
-__global__ void __launch_bounds__((brick_threads<SX, SY, SZ>()), SX == 8 ? 3 : 2) k_grad_bricks(Grid g, FieldState s, BrickList bl,
-                                                                                        const __grid_constant__ GradOps O,
-                                                                                        const __grid_constant__ KeepOps K) {
+struct BrickMem {
+    static constexpr int KX = SX + 4, KY = SY + 4, KZ = SZ + 4, NK = KX * KY * KZ;  // keys: two layers around
+    static constexpr int WX = SX + 2, WY = SY + 2, WZ = SZ + 2, NW = WX * WY * WZ;  // star words: one layer around
+    static constexpr int CX = SX + 1, CY = SY + 1, CZ = SZ + 1, NC = CX * CY * CZ;  // cell words: one layer below
+    uint64_t sk[NK];
+    uint4 sw[NW];
+    uint32_t sf[NW];
+    CellWords sc[NC];
+    uint32_t flag;  // bit 0: as, bit 1: ds
+};
+// one brick, by a block of brick_threads
+template <int SX, int SY, int SZ>
+__device__ __forceinline__ void grad_brick(const Grid &g, const FieldState &s, const BrickList &bl, const GradOps &O, i64 b,
+                                           BrickMem<SX, SY, SZ> &M) {
     static_assert(SX * SY * SZ == DMTZ_BRICK, "a brick is 128 anchors");
+    using B = BrickMem<SX, SY, SZ>;
     constexpr int NT = brick_threads<SX, SY, SZ>();
-    constexpr int KX = SX + 4, KY = SY + 4, KZ = SZ + 4, NK = KX * KY * KZ;  // keys: two layers around
-    constexpr int WX = SX + 2, WY = SY + 2, WZ = SZ + 2, NW = WX * WY * WZ;  // star words: one layer around
-    constexpr int CX = SX + 1, CY = SY + 1, CZ = SZ + 1, NC = CX * CY * CZ;  // cell words: one layer below
-    __shared__ uint64_t sk[NK];
-    __shared__ uint4 sw[NW];
-    __shared__ uint32_t sf[NW];
-    __shared__ CellWords sc[NC];
-    __shared__ uint32_t flag;  // bit 0: as, bit 1: ds
+    constexpr int KX = B::KX, KY = B::KY, NK = B::NK, WX = B::WX, WY = B::WY, NW = B::NW, CX = B::CX, CY = B::CY, NC = B::NC;
     const int t = threadIdx.x;
     const int wx = t % WX, wy = (t / WX) % WY, wz = t / (WX * WY);
     const int cx = t % CX, cy = (t / CX) % CY, cz = t / (CX * CY);
     const int ox = t % SX, oy = (t / SX) % SY, oz = t / (SX * SY);
+    int bx, by, bz;
+    brick_coords(bl, b, bx, by, bz);
+    const int x0 = bx * SX, y0 = by * SY, z0 = bz * SZ;
+    for (int e = t; e < NK; e += NT) {
+        const int ux = x0 - 2 + e % KX, uy = y0 - 2 + (e / KX) % KY, uz = z0 - 2 + e / (KX * KY);
+        const bool in = ux >= 0 && uy >= 0 && uz >= 0 && ux < g.W && uy < g.H && uz < g.D;
+        M.sk[e] = in ? okey(s.val[ux + (i64)uy * g.W + (i64)uz * g.WH]) : kKeyAbsent;
+    }
+    // what the flags and lists compare with, loaded with the keys
+    uint32_t tcP = 0, critP = 0;
+    int pvP = 15;
+    if (O.critP) {
+        const int x = x0 + wx - 1, y = y0 + wy - 1, z = z0 + wz - 1;
+        if (O.F.as && t < NW && x >= 0 && y >= 0 && z >= 0 && x < g.W && y < g.H && z < g.D)
+            pvP = O.F.pvP[x + (i64)y * g.W + (i64)z * g.WH];
+        if (t < DMTZ_BRICK && x0 + ox < g.W && y0 + oy < g.H && z0 + oz < g.D) {
+            const i64 v = (x0 + ox) + (i64)(y0 + oy) * g.W + (i64)(z0 + oz) * g.WH;
+            if (O.F.as) tcP = O.F.tcP[v];
+            critP = O.critP[v];
+        }
+    }
+    __syncthreads();
+    if (t < NW) {
+        const uint64_t *k0 = M.sk + (wx + 1) + KX * ((wy + 1) + KY * (wz + 1));
+        const StarWords w = grad_stage1<KX>(k0 - KX * KY, k0, k0 + KX * KY);
+        M.sw[t] = make_uint4(w.x, w.y, w.z | (pvP != 15 && pvP != w.pv ? 1u << 24 : 0u), w.w);
+        M.sf[t] = w.w4;
+        const int x = x0 + wx - 1, y = y0 + wy - 1, z = z0 + wz - 1;
+        if (wx >= 1 && wy >= 1 && wz >= 1 && wx <= SX && wy <= SY && wz <= SZ && x < g.W && y < g.H && z < g.D)
+            s.pv[x + (i64)y * g.W + (i64)z * g.WH] = (uint8_t)w.pv;
+    }
+    __syncthreads();
+    if (t < NC) {
+        if (t == 0) M.flag = 0;
+        const int i = cx + WX * (cy + WY * cz);
+        M.sc[t] = grad_stage2<WX, true>(M.sw + i, M.sw + i + WX * WY, M.sf + i, M.sf + i + WX * WY);
+    }
+    __syncthreads();
+    if (t < DMTZ_BRICK) {
+        const int x = x0 + ox, y = y0 + oy, z = z0 + oz;
+        const i64 v = x + (i64)y * g.W + (i64)z * g.WH;
+        uint32_t differ = 0;
+        if (x < g.W && y < g.H && z < g.D) {
+            const int i = (ox + 1) + CX * ((oy + 1) + CY * (oz + 1));
+            const uint32_t last = (x == g.W - 1 ? 1u : 0u) | (y == g.H - 1 ? 2u : 0u) | (z == g.D - 1 ? 4u : 0u);
+            const AnchorOut o = grad_stage3<CX>(M.sc + i - CX * CY, M.sc + i, last);
+            s.eup[v] = o.eup;
+            s.fup[v] = o.fup;
+            if (s.crit) s.crit[v] = o.crit;
+            if (s.tcode) s.tcode[v] = o.tcode;
+            differ = (o.crit ^ critP) & O.want;
+            const uint32_t f = (tet_path_differs(tcP, o.tcode) ? 1u : 0u) | (((critP >> 1) & (M.sc[i].pb >> 24) & 0x7Fu) ? 2u : 0u);
+            if (f) atomicOr(&M.flag, f);
+        }
+        if (O.want) push_warp(O.T, v, differ);
+    }
+    if (O.F.as) {
+        __syncthreads();
+        if (t == 0) {
+            const i64 b = bx + (i64)bl.nbx * (by + (i64)bl.nby * bz);
+            O.F.as[b] = (uint8_t)(M.flag & 1u);
+            O.F.ds[b] = (uint8_t)(M.flag >> 1);
+        }
+    }
+}
+template <int SX, int SY, int SZ>
+__global__ void __launch_bounds__((brick_threads<SX, SY, SZ>()), SX == 8 ? 3 : 2) k_grad_bricks(Grid g, FieldState s, BrickList bl,
+                                                                                        const __grid_constant__ GradOps O,
+                                                                                        const __grid_constant__ KeepOps K) {
+    __shared__ BrickMem<SX, SY, SZ> M;
     let_next();
     after_previous();
     if (blockIdx.x >= gridDim.x - K.blocks) {  // the blocks that carry the old lists over
         keep_lists(g, O, K, blockIdx.x - (gridDim.x - K.blocks));
         return;
     }
-    const i64 n = brick_count(bl);
-    for (i64 b = blockIdx.x; b < n; b += gridDim.x - K.blocks) {
-        int bx, by, bz;
-        brick_coords(bl, b, bx, by, bz);
-        const int x0 = bx * SX, y0 = by * SY, z0 = bz * SZ;
-        for (int e = t; e < NK; e += NT) {
-            const int ux = x0 - 2 + e % KX, uy = y0 - 2 + (e / KX) % KY, uz = z0 - 2 + e / (KX * KY);
-            const bool in = ux >= 0 && uy >= 0 && uz >= 0 && ux < g.W && uy < g.H && uz < g.D;
-            sk[e] = in ? okey(s.val[ux + (i64)uy * g.W + (i64)uz * g.WH]) : kKeyAbsent;
-        }
-        // what the flags and lists compare with, loaded with the keys
-        uint32_t tcP = 0, critP = 0;
-        int pvP = 15;
-        if (O.critP) {
-            const int x = x0 + wx - 1, y = y0 + wy - 1, z = z0 + wz - 1;
-            if (O.F.as && t < NW && x >= 0 && y >= 0 && z >= 0 && x < g.W && y < g.H && z < g.D)
-                pvP = O.F.pvP[x + (i64)y * g.W + (i64)z * g.WH];
-            if (t < DMTZ_BRICK && x0 + ox < g.W && y0 + oy < g.H && z0 + oz < g.D) {
-                const i64 v = (x0 + ox) + (i64)(y0 + oy) * g.W + (i64)(z0 + oz) * g.WH;
-                if (O.F.as) tcP = O.F.tcP[v];
-                critP = O.critP[v];
-            }
-        }
-        __syncthreads();
-        if (t < NW) {
-            const uint64_t *k0 = sk + (wx + 1) + KX * ((wy + 1) + KY * (wz + 1));
-            const StarWords w = grad_stage1<KX>(k0 - KX * KY, k0, k0 + KX * KY);
-            sw[t] = make_uint4(w.x, w.y, w.z | (pvP != 15 && pvP != w.pv ? 1u << 24 : 0u), w.w);
-            sf[t] = w.w4;
-            const int x = x0 + wx - 1, y = y0 + wy - 1, z = z0 + wz - 1;
-            if (wx >= 1 && wy >= 1 && wz >= 1 && wx <= SX && wy <= SY && wz <= SZ && x < g.W && y < g.H && z < g.D)
-                s.pv[x + (i64)y * g.W + (i64)z * g.WH] = (uint8_t)w.pv;
-        }
-        __syncthreads();
-        if (t < NC) {
-            if (t == 0) flag = 0;
-            const int i = cx + WX * (cy + WY * cz);
-            sc[t] = grad_stage2<WX, true>(sw + i, sw + i + WX * WY, sf + i, sf + i + WX * WY);
-        }
-        __syncthreads();
-        if (t < DMTZ_BRICK) {
-            const int x = x0 + ox, y = y0 + oy, z = z0 + oz;
-            const i64 v = x + (i64)y * g.W + (i64)z * g.WH;
-            uint32_t differ = 0;
-            if (x < g.W && y < g.H && z < g.D) {
-                const int i = (ox + 1) + CX * ((oy + 1) + CY * (oz + 1));
-                const uint32_t last = (x == g.W - 1 ? 1u : 0u) | (y == g.H - 1 ? 2u : 0u) | (z == g.D - 1 ? 4u : 0u);
-                const AnchorOut o = grad_stage3<CX>(sc + i - CX * CY, sc + i, last);
-                s.eup[v] = o.eup;
-                s.fup[v] = o.fup;
-                if (s.crit) s.crit[v] = o.crit;
-                if (s.tcode) s.tcode[v] = o.tcode;
-                differ = (o.crit ^ critP) & O.want;
-                const uint32_t f = (tet_path_differs(tcP, o.tcode) ? 1u : 0u) | (((critP >> 1) & (sc[i].pb >> 24) & 0x7Fu) ? 2u : 0u);
-                if (f) atomicOr(&flag, f);
-            }
-            if (O.want) push_warp(O.T, v, differ);
-        }
-        if (O.F.as) {
-            __syncthreads();
-            if (t == 0) {
-                const i64 b = bx + (i64)bl.nbx * (by + (i64)bl.nby * bz);
-                O.F.as[b] = (uint8_t)(flag & 1u);
-                O.F.ds[b] = (uint8_t)(flag >> 1);
-            }
-        }
+    const unsigned n = (unsigned)brick_count(bl);  // (their coordinates fill 32 bits)
+    for (unsigned b = blockIdx.x; b < n; b += gridDim.x - K.blocks) {
+        grad_brick<SX, SY, SZ>(g, s, bl, O, b, M);
         // the next brick's keys may land now: stage 1 of this one is behind two
         // barriers, and the words stage 3 reads are not written before the next one
     }
