@@ -1855,12 +1855,12 @@ unsigned brick_grid(const dmtz_ctx *ctx, i64 nb) {
 
 // the gradient of a set of bricks (and the old mismatch lists' entries, see KeepOps)
 void grad_bricks(const Grid &g, const FieldState &s, const BrickList &bl, unsigned grid, cudaStream_t st,
-                 const GradOps &O = GradOps{}, const KeepOps &K = KeepOps{}) {
+                 const GradOps &O = GradOps{}, const KeepOps &K = KeepOps{}, const int *wanted = nullptr) {
     grid += K.blocks;
     switch (bl.shape) {
-    case 1: launch_next(k_grad_bricks<16, 4, 2>, grid, brick_threads<16, 4, 2>(), st, g, s, bl, O, K); break;
-    case 2: launch_next(k_grad_bricks<32, 2, 2>, grid, brick_threads<32, 2, 2>(), st, g, s, bl, O, K); break;
-    default: launch_next(k_grad_bricks<8, 4, 4>, grid, brick_threads<8, 4, 4>(), st, g, s, bl, O, K); break;
+    case 1: launch_next(k_grad_bricks<16, 4, 2>, grid, brick_threads<16, 4, 2>(), st, g, s, bl, O, K, wanted); break;
+    case 2: launch_next(k_grad_bricks<32, 2, 2>, grid, brick_threads<32, 2, 2>(), st, g, s, bl, O, K, wanted); break;
+    default: launch_next(k_grad_bricks<8, 4, 4>, grid, brick_threads<8, 4, 4>(), st, g, s, bl, O, K, wanted); break;
     }
 }
 
@@ -2011,7 +2011,8 @@ void repair_ops(const dmtz_ctx *ctx, const BrickMarks &B, const uint32_t *crit_o
 // already by k_apply, or else from ctx->reqlist); the mismatch lists are then rebuilt
 // into list_tmp (inc_scan; k_round_end takes them back) or scanned for.  The
 // marks are clear at the start (k_round_end, or the caller).
-void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32_t *crit_o, int want_saddles, bool marked) {
+void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32_t *crit_o, int want_saddles, bool marked,
+                  const int *wanted = nullptr) {
     const BrickMarks B = brick_marks(ctx, g);
     cudaStream_t st = ctx->stream;
     i64 nb;
@@ -2025,7 +2026,7 @@ void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint3
     GradOps O{};
     KeepOps K{};
     repair_ops(ctx, B, crit_o, want_saddles, O, K);
-    grad_bricks(g, s, bl, brick_grid(ctx, nb), st, O, K);
+    grad_bricks(g, s, bl, brick_grid(ctx, nb), st, O, K, wanted);
     ctx->launches++;
     if (!ctx->inc_scan) scan_mismatch(ctx, g, s.crit, crit_o, want_saddles);
 }
@@ -2828,8 +2829,14 @@ dmtz_status dmtz_wall_detect(dmtz_ctx *ctx, int W, int H, int D, const double *o
 //          them again at the start of its next outer iteration; same inputs,
 //          same records)
 //   CPF    a critical-point round with long lists: the whole grid is re-paired
+//   CPS    critical-point rounds with short lists, one after the other (k_short_rounds)
 namespace {
-enum { LS_CP = 0, LS_PDF = 1, LS_PCHECK = 2, LS_PFIX = 3, LS_CPF = 4, LS_DONE = 5, LS_STATES = 5 };
+enum { LS_CP = 0, LS_PDF = 1, LS_PCHECK = 2, LS_PFIX = 3, LS_CPF = 4, LS_CPS = 5, LS_DONE = 6, LS_STATES = 6 };
+// bodies of the loop graph's switch: the last one is CPF's or CPS's (a body more costs 50 us to
+// instantiate and destroy, 3 % of a 120 x 89 x 101 field's correction; grids that are ever
+// repaired whole have few rounds, the others many short ones)
+constexpr int LS_BODIES = 5;
+__host__ __device__ inline bool is_cp(int state) { return state == LS_CP || state == LS_CPF || state == LS_CPS; }
 struct LoopCtl {
     int state, pvp, converged, pad;
     long long rounds, max_rounds, outer, cp_rounds, path_rounds;
@@ -2843,6 +2850,9 @@ struct LoopCtl {
     int break_stalls;   // stop when a round changed nothing (the host breaks the stall)
     int stalled;
     int begun;          // a body has run: a round's end has something to end
+    int ended;          // and k_short_rounds has ended it
+    int pending;        // it left a round's repair to k_grad_bricks
+    long long few;      // listed cells up to which rounds are short
 };
 }  // namespace
 
@@ -2854,9 +2864,9 @@ __device__ __forceinline__ LoopCtl loop_next(LoopCtl c, const unsigned long long
         for (int k = 0; k < 4; k++) c.cc[k] = (long long)counters[k];
     const long long cells = c.cc[0] + c.cc[1] + c.cc[2] + c.cc[3];
     const bool cp_any = cells > 0;
-    const int cp = cells >= c.heavy ? LS_CPF : LS_CP;
+    const int cp = cells >= c.heavy ? LS_CPF : cells <= c.few ? LS_CPS : LS_CP;
     int next;
-    if (st == LS_CP || st == LS_CPF) {
+    if (is_cp(st)) {
         c.rounds++;
         c.cp_rounds++;
         next = cp_any ? cp : (c.pvp ? LS_PDF : LS_DONE);
@@ -2891,7 +2901,7 @@ __device__ __forceinline__ LoopCtl loop_next(LoopCtl c, const unsigned long long
     // counters[7]: set by the update when it changed something; a path round
     // counts only if its detection had records (counters[5], [6])
     if (c.break_stalls && next != LS_DONE && counters[7] == 0 &&
-        (st == LS_CP || st == LS_CPF || ((st == LS_PDF || st == LS_PFIX) && counters[5] + counters[6] > 0)))
+        (is_cp(st) || ((st == LS_PDF || st == LS_PFIX) && counters[5] + counters[6] > 0)))
         c.stalled = 1;
     c.state = next;
     return c;
@@ -2911,8 +2921,8 @@ __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Li
     __shared__ bool last;
     after_previous();
     const int st = ctl ? ctl->state : LS_CP;
-    const bool begun = !ctl || ctl->begun;
-    const bool copy = begun && T.n && st != LS_PCHECK && st != LS_CPF;
+    const bool ends = !ctl || (ctl->begun && !ctl->ended);
+    const bool copy = ends && T.n && st != LS_PCHECK && st != LS_CPF;
     const i64 nbrick = (i64)*B.n;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < nbrick; i += (i64)gridDim.x * blockDim.x) {
         const uint32_t e = B.list[i];
@@ -2947,11 +2957,12 @@ __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Li
     bool stop = false;
     if (ctl) {
         LoopCtl c = *ctl;
-        if (begun) c = loop_next(c, counters);
+        if (ends) c = loop_next(c, counters);
         c.begun = 1;
+        c.ended = c.pending = 0;
         *ctl = c;
         stop = c.state == LS_DONE || c.overflow || c.stalled;
-        cudaGraphSetConditional(hswitch, stop ? (unsigned)LS_STATES : (unsigned)c.state);
+        cudaGraphSetConditional(hswitch, stop ? (unsigned)LS_BODIES : (unsigned)min(c.state, LS_BODIES - 1));
         cudaGraphSetConditional(hwhile, stop ? 0u : 1u);
         if (!stop && (c.state == LS_PDF || c.state == LS_PCHECK)) counters[5] = counters[6] = counters[27] = 0;
     } else {
@@ -2970,10 +2981,12 @@ __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Li
 // loop ends when the lists are empty or hold more than kShortCells (then the whole
 // GPU does a round sooner), when a list overflowed, a round changed nothing (stop_stalled), or max_rounds
 // have run; with more than kShortBricks bricks marked it leaves the round to the
-// kernels that it stands for, after its update (report[10]).  report: [0..7] the
+// kernels that it stands for, after its update (report[10]).  In the loop graph
+// (ctl) it is the state CPS and goes on from round to round as k_round_end would.  report: [0..7] the
 // counters as after any round, [9] rounds, [11..13] nanoseconds of fix, update and
 // the rest.  Host-driven loops, 16^3: 2.81 -> 2.47 ms, 64^3 extrema: 10.3 -> 9.7; with 384
-// cells and 64 bricks 2.42 and 9.7, but a batch of eight got 3 % slower.
+// cells and 64 bricks 2.42 and 9.7, but a batch of eight got 3 % slower.  Graph loop, noisy
+// 97 x 61 x 75 field: 17.3 -> 16.5.
 constexpr unsigned kShortBlocks = 16;
 constexpr i64 kShortCells = 64, kShortBricks = 160, kShortRounds = 256;  // at most that many per launch
 __device__ __forceinline__ void cluster_barrier() {
@@ -2990,7 +3003,7 @@ __global__ void __launch_bounds__((brick_threads<8, 4, 4>()), 2)
                    const __grid_constant__ Lists T, int preserve_saddles, double range, int preserve_type, uint8_t *changed,
                    const __grid_constant__ BrickMarks B, const __grid_constant__ FieldState s, const __grid_constant__ BrickList bl,
                    const __grid_constant__ GradOps O, const __grid_constant__ KeepOps K, unsigned long long *counters,
-                   i64 max_rounds, int stop_stalled, unsigned long long *report, unsigned long long seq) {
+                   i64 max_rounds, int stop_stalled, LoopCtl *ctl, unsigned long long *report, unsigned long long seq) {
     __shared__ RuleTab tab;
     __shared__ BrickMem<8, 4, 4> M;
     const Grid &g = c.g;
@@ -2998,6 +3011,10 @@ __global__ void __launch_bounds__((brick_threads<8, 4, 4>()), 2)
     const bool first = block == 0 && threadIdx.x == 0;
     const i64 tid = (i64)block * blockDim.x + threadIdx.x, nt = (i64)blocks * blockDim.x;
     load_rule_tab(tab);
+    if (ctl) {
+        max_rounds = min((i64)(ctl->max_rounds - ctl->rounds), kShortRounds);
+        stop_stalled = ctl->break_stalls;
+    }
     i64 rounds = 0;
     bool left = false;
     unsigned long long ns[3] = {0, 0, 0}, t0 = nanoseconds(), t1;
@@ -3045,15 +3062,19 @@ __global__ void __launch_bounds__((brick_threads<8, 4, 4>()), 2)
                 T.n[k] = 0;
             }
             *B.n = 0;
-            if (stop)
-                for (int k = 0; k < 8; k++) report[k] = k == 7 ? moved : counters[k];
+            if (ctl) *ctl = loop_next(*ctl, counters);
+            else if (stop)
+                for (int k = 0; k < 8; k++) report[k] = counters[k];
             counters[4] = counters[7] = 0;
         }
         cluster_barrier();
         lap(2);
         if (stop) break;
     }
-    if (first) {
+    if (first && ctl) {
+        ctl->ended = !left;
+        ctl->pending = left;
+    } else if (first) {
         report[9] = (unsigned long long)rounds;
         report[10] = left;
         for (int k = 0; k < 3; k++) report[11 + k] = ns[k];
@@ -3103,6 +3124,60 @@ struct PhaseTimer {
     }
 };
 }  // namespace
+
+// Can this run's short rounds go to k_short_rounds?  (Lists rebuilt by the repairs,
+// the default brick shape, and a device that holds the cluster.)
+static bool short_rounds_fit(dmtz_ctx *ctx) {
+    if (!ctx->inc_scan || ctx->tune_shape != 0) return false;
+    if (!ctx->short_clusters) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kShortBlocks);
+        cfg.blockDim = dim3(brick_threads<8, 4, 4>());
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = kShortBlocks;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute((const void *)k_short_rounds, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, k_short_rounds, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        ctx->short_clusters = n > 0 ? n : -1;
+    }
+    return ctx->short_clusters > 0;
+}
+// in the loop graph: on grids that are never repaired whole
+static bool graph_short_rounds(dmtz_ctx *ctx, const Grid &g) { return heavy_cells(ctx, g) == INT64_MAX && short_rounds_fit(ctx); }
+static cudaError_t launch_short_rounds(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const FieldState &Qs, double range, int ps,
+                                       int pt, i64 max_rounds, int stop_stalled, LoopCtl *ctl = nullptr) {
+    const BrickMarks B = brick_marks(ctx, g);
+    i64 nb;
+    BrickList bl = all_bricks(g, ctx->tune_shape, nb);
+    bl.list = ctx->brick_list;
+    bl.n = ctx->brick_n;
+    GradOps O{};
+    KeepOps K{};
+    repair_ops(ctx, B, ctx->P.crit, ps == 1, O, K);
+    K.blocks = kShortBlocks;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kShortBlocks);
+    cfg.blockDim = dim3(brick_threads<8, 4, 4>());
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kShortBlocks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (!ctl) ctx->report_seq++;
+    ctx->launches++;
+    return cudaLaunchKernelEx(&cfg, k_short_rounds, rc, cp_lists(ctx), mismatch_lists(ctx), rebuilt_lists(ctx), ps, range, pt,
+                              ctx->changed, B, Qs, bl, O, K, ctx->counters, max_rounds, stop_stalled, ctl, ctx->report,
+                              ctx->report_seq);
+}
 
 // The loop as an executable graph, with the lists' capacities that it was built for.
 // Building and instantiating takes 110 us of host time and destroying 60 to 100, so
@@ -3173,17 +3248,22 @@ static dmtz_status build_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx 
         sp.type = cudaGraphNodeTypeConditional;
         sp.conditional.handle = hsw;
         sp.conditional.type = cudaGraphCondTypeSwitch;
-        sp.conditional.size = LS_STATES;
+        sp.conditional.size = LS_BODIES;
         if (cudaGraphAddNode(&n_sw, body, &n_set, nullptr, 1, &sp) != cudaSuccess) { res = DMTZ_ERR_CUDA; break; }
-        for (int state = 0; state < LS_STATES && res == DMTZ_OK; state++) {
-            cudaGraph_t child = sp.conditional.phGraph_out[state];
+        const bool short_rounds = graph_short_rounds(ctx, g);
+        for (int body = 0; body < LS_BODIES && res == DMTZ_OK; body++) {
+            cudaGraph_t child = sp.conditional.phGraph_out[body];
+            const int state = body == LS_CPF && short_rounds ? LS_CPS : body;
             if (cudaStreamBeginCaptureToGraph(st, child, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
                 res = DMTZ_ERR_CUDA;
                 break;
             }
             if (state == LS_PDF || state == LS_PCHECK) launch_detect(ctx, g, rc, PR, pgrid, conn);
-            if (state != LS_PCHECK) {
-                const bool cp = state == LS_CP || state == LS_CPF;
+            if (state == LS_CPS) {
+                if (launch_short_rounds(ctx, g, rc, Qs, range, ps, pt, 0, 0, dctl) != cudaSuccess) res = DMTZ_ERR_CUDA;
+                repair_dirty(ctx, g, Qs, ctx->P.crit, ps == 1, true, &dctl->pending);
+            } else if (state != LS_PCHECK) {
+                const bool cp = is_cp(state);
                 const int want = cp ? (ps == 1) : 1;
                 if (cp) k_fix_cp<<<pgrid, kBlock, 0, st>>>(rc, L, ps);
                 else k_fix_path<<<pgrid, kBlock, 0, st>>>(rc, PR);
@@ -3210,7 +3290,7 @@ static dmtz_status build_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx 
 // progress, separatrix records) are as the first state needs them.
 static dmtz_status run_graph_loop(dmtz_ctx *ctx, const LoopGraph &lg, LoopCtl init, LoopCtl *out) {
     cudaStream_t st = ctx->stream;
-    init.begun = 0;
+    init.begun = init.ended = init.pending = 0;
     CK(cudaMemcpyAsync(ctx->loopctl, &init, sizeof(LoopCtl), cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(ctx->counters + 4, 0, sizeof(unsigned long long), st));
     CK(cudaMemsetAsync(ctx->counters + 7, 0, sizeof(unsigned long long), st));
@@ -3313,57 +3393,6 @@ static dmtz_status break_stall(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, 
     host_round_end(ctx, g);
     ctx->launches += 6;
     CK(cudaGetLastError());
-    return DMTZ_OK;
-}
-
-// Can this run's short rounds go to k_short_rounds?  (Lists rebuilt by the repairs,
-// the default brick shape, and a device that holds the cluster.)
-static bool short_rounds_fit(dmtz_ctx *ctx) {
-    if (!ctx->inc_scan || ctx->tune_shape != 0) return false;
-    if (!ctx->short_clusters) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(kShortBlocks);
-        cfg.blockDim = dim3(brick_threads<8, 4, 4>());
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = kShortBlocks;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaFuncSetAttribute((const void *)k_short_rounds, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, k_short_rounds, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            n = 0;
-        }
-        ctx->short_clusters = n > 0 ? n : -1;
-    }
-    return ctx->short_clusters > 0;
-}
-static dmtz_status launch_short_rounds(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const FieldState &Qs, double range, int ps,
-                                       int pt, i64 max_rounds, int stop_stalled) {
-    const BrickMarks B = brick_marks(ctx, g);
-    i64 nb;
-    BrickList bl = all_bricks(g, ctx->tune_shape, nb);
-    bl.list = ctx->brick_list;
-    bl.n = ctx->brick_n;
-    GradOps O{};
-    KeepOps K{};
-    repair_ops(ctx, B, ctx->P.crit, ps == 1, O, K);
-    K.blocks = kShortBlocks;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(kShortBlocks);
-    cfg.blockDim = dim3(brick_threads<8, 4, 4>());
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = kShortBlocks;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    CK(cudaLaunchKernelEx(&cfg, k_short_rounds, rc, cp_lists(ctx), mismatch_lists(ctx), rebuilt_lists(ctx), ps, range, pt, ctx->changed,
-                          B, Qs, bl, O, K, ctx->counters, max_rounds, stop_stalled, ctx->report, ++ctx->report_seq));
-    ctx->launches++;
     return DMTZ_OK;
 }
 
@@ -3507,7 +3536,8 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         c.break_stalls = opts->break_stalls ? 1 : 0;
         for (int k = 0; k < 4; k++) c.cc[k] = cc[k];
         c.heavy = heavy;
-        auto cp_state = [&](i64 cells) { return cells >= heavy ? LS_CPF : LS_CP; };
+        c.few = graph_short_rounds(ctx, g) ? kShortCells : 0;
+        auto cp_state = [&](i64 cells) { return cells >= heavy ? LS_CPF : cells <= c.few ? LS_CPS : LS_CP; };
         c.state = cp_any() ? cp_state(cc[0] + cc[1] + cc[2] + cc[3]) : (pvp ? LS_PDF : LS_DONE);
         LoopCtl fin = c;
         if (c.state != LS_DONE) {
@@ -3520,11 +3550,11 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
                 // a scan outgrew a list: grow it, rebuild the lists and resume
                 unsigned long long h4[4];
                 for (int k = 0; k < 4; k++) h4[k] = (unsigned long long)fin.cc[k];
-                if ((s = fit_lists(ctx, g, fin.last == LS_CP || fin.last == LS_CPF ? (ps == 1) : 1, h4)) != DMTZ_OK) return s;
+                if ((s = fit_lists(ctx, g, is_cp(fin.last) ? (ps == 1) : 1, h4)) != DMTZ_OK) return s;
                 cur = fin;
                 cur.overflow = 0;
                 if (fin.stalled) {  // the round changed nothing: break the stall, then go on
-                    const int cpst = fin.last == LS_CP || fin.last == LS_CPF;
+                    const int cpst = is_cp(fin.last);
                     if ((s = break_stall(ctx, g, rc, PR, Qs, cpst, cpst ? (ps == 1) : 1, R.stall_breaks)) != DMTZ_OK)
                         return s;
                     R.stall_breaks++;
@@ -3551,7 +3581,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             const int64_t det = detect_kernels(ctx, conn);  // separatrix detection kernels
             const int64_t rnd = 2 + 1 + (ctx->inc_scan ? 0 : 1);
             int64_t bodies = 0;
-            for (int k = 0; k < LS_STATES; k++) bodies += fin.runs[k];
+            for (int k = 0; k < LS_STATES; k++) bodies += k == LS_CPS ? 0 : fin.runs[k];
             ctx->launches += 1 + bodies + rnd * fin.runs[LS_CP] + (rnd + det) * fin.runs[LS_PDF] + det * fin.runs[LS_PCHECK] +
                              rnd * fin.runs[LS_PFIX] + 3 * fin.runs[LS_CPF];
         }
@@ -3584,9 +3614,8 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             if (rounds >= max_rounds) break;
             paths_fresh = false;
             if (cc[0] + cc[1] + cc[2] + cc[3] <= kShortCells && short_rounds_fit(ctx)) {
-                if ((s = launch_short_rounds(ctx, g, rc, Qs, range, ps, pt, std::min(max_rounds - rounds, kShortRounds), opts->break_stalls)) != DMTZ_OK ||
-                    (s = read_fit(ps == 1)) != DMTZ_OK)
-                    return s;
+                CK(launch_short_rounds(ctx, g, rc, Qs, range, ps, pt, std::min(max_rounds - rounds, kShortRounds), opts->break_stalls));
+                if ((s = read_fit(ps == 1)) != DMTZ_OK) return s;
                 const unsigned long long *r = ctx->report;
                 rounds += (i64)r[9];
                 R.cp_rounds += (i64)r[9];

@@ -729,10 +729,12 @@ __device__ __forceinline__ void grad_brick(const Grid &g, const FieldState &s, c
 template <int SX, int SY, int SZ>
 __global__ void __launch_bounds__((brick_threads<SX, SY, SZ>()), SX == 8 ? 3 : 2) k_grad_bricks(Grid g, FieldState s, BrickList bl,
                                                                                         const __grid_constant__ GradOps O,
-                                                                                        const __grid_constant__ KeepOps K) {
+                                                                                        const __grid_constant__ KeepOps K,
+                                                                                        const int *wanted) {
     __shared__ BrickMem<SX, SY, SZ> M;
     let_next();
     after_previous();
+    if (wanted && !*wanted) return;
     if (blockIdx.x >= gridDim.x - K.blocks) {  // the blocks that carry the old lists over
         keep_lists(g, O, K, blockIdx.x - (gridDim.x - K.blocks));
         return;
