@@ -734,12 +734,12 @@ struct LongPaths {
 };
 // One lane per 2-saddle, both cofaces one after the other; a lane that is done
 // takes the chunk's next 2-saddle.
-__global__ void __launch_bounds__(kBlock) k_path_trace(Grid g, const i64 *sad2, const unsigned long long *nsad, uint32_t *tcP,
+__global__ void __launch_bounds__(kBlock) k_path_trace(Grid g, const i64 *sad2, const unsigned long long *nsad, i64 capsad, uint32_t *tcP,
                                                       unsigned long long *box, LongPaths L, int shx, int shy, int shz,
                                                       i64 cap, int *err, unsigned long long *ticket) {
     __shared__ AscTab tab;
     load_asc_tab(tab);
-    const i64 n = (i64)*nsad, chunk = chunk_size(n, 256);
+    const i64 n = min((i64)*nsad, capsad), chunk = chunk_size(n, 256);
     const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
     constexpr unsigned long long kEmpty = 1ull;  // x0 = 1 > x1 = 0
     bool first = true;
@@ -849,7 +849,7 @@ __device__ __forceinline__ i64 ds_differs(const Grid &g, const uint8_t *pvP, con
 // the segments of long paths, the others the bricks with a differing 1-saddle
 // endpoint (strict: none, k_ds_strict does those).
 constexpr int kQueue = 512;
-__global__ void __launch_bounds__(kBlock) k_path_detect(Grid g, PathFlags F, const i64 *sad2, const unsigned long long *nsad,
+__global__ void __launch_bounds__(kBlock) k_path_detect(Grid g, PathFlags F, const i64 *sad2, const unsigned long long *nsad, i64 capsad,
                                                        const unsigned long long *box, const uint32_t *critP,
                                                        const uint32_t *tcQ,
                                                        const uint8_t *pvQ, LongPaths L, PathRec R,
@@ -893,7 +893,7 @@ __global__ void __launch_bounds__(kBlock) k_path_detect(Grid g, PathFlags F, con
     __shared__ uint16_t queue[kBlock / 32][kQueue];  // per warp: the chunk's items to walk
     __shared__ AscTab tab;
     load_asc_tab(tab);
-    const i64 n2 = (i64)*nsad, n = n2 + min((i64)L.n[0], L.cap_seg);  // 2-saddles, then segments
+    const i64 n2 = min((i64)*nsad, capsad), n = n2 + min((i64)L.n[0], L.cap_seg);  // 2-saddles, then segments
     const i64 warps = (i64)as_blocks * (blockDim.x / 32);
     i64 chunk = (n / (warps * 8) + 31) / 32 * 32;
     chunk = chunk < 32 ? 32 : (chunk > kQueue ? kQueue : chunk);
@@ -2147,9 +2147,9 @@ dmtz_status trace_paths(dmtz_ctx *ctx, const Grid &g) {
             ctx->capSlot = need_slot;
         }
         CK(cudaMemsetAsync(ctx->counters + 25, 0, 3 * sizeof(unsigned long long), st));  // segments, slots, ticket
-        k_path_trace<<<persistent_grid(), kBlock, 0, st>>>(g, ctx->sad2, ctx->counters + 10, ctx->P.tcode, ctx->path_box,
-                                                           long_paths(ctx), sh[0], sh[1], sh[2], g.T + 16, ctx->errword,
-                                                           ctx->counters + 27);
+        k_path_trace<<<persistent_grid(), kBlock, 0, st>>>(g, ctx->sad2, ctx->counters + 10, ctx->capSad2, ctx->P.tcode,
+                                                           ctx->path_box, long_paths(ctx), sh[0], sh[1], sh[2], g.T + 16,
+                                                           ctx->errword, ctx->counters + 27);
         ctx->launches++;
         unsigned long long n[2] = {0, 0};
         CK(cudaMemcpyAsync(n, ctx->counters + 25, sizeof(n), cudaMemcpyDeviceToHost, st));
@@ -2180,13 +2180,19 @@ dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g) {
     if ((i64)n[1] > ctx->capAS) {
         cudaFree(ctx->as_tet);
         cudaFree(ctx->as_cur);
-        cudaFree(ctx->sad2);
-        ctx->as_tet = ctx->as_cur = ctx->sad2 = nullptr;
-        ctx->capAS = ctx->capSad2 = 0;
+        ctx->as_tet = ctx->as_cur = nullptr;
+        ctx->capAS = 0;
         CK(dalloc(&ctx->as_tet, (i64)n[1]));
         CK(dalloc(&ctx->as_cur, (i64)n[1]));
+        ctx->capAS = (i64)n[1];
+    }
+    // (of its own: a connectivity check grows the records alone)
+    if ((i64)n[1] > ctx->capSad2) {
+        cudaFree(ctx->sad2);
+        ctx->sad2 = nullptr;
+        ctx->capSad2 = 0;
         CK(dalloc(&ctx->sad2, (i64)n[1]));
-        ctx->capAS = ctx->capSad2 = (i64)n[1];
+        ctx->capSad2 = (i64)n[1];
     }
     // buffers exist even when a count is 0 (kernels take their addresses)
     if (!ctx->ds_edge) {
@@ -2196,8 +2202,8 @@ dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g) {
     if (!ctx->as_tet) {
         CK(dalloc(&ctx->as_tet, 1));
         CK(dalloc(&ctx->as_cur, 1));
-        CK(dalloc(&ctx->sad2, 1));
     }
+    if (!ctx->sad2) CK(dalloc(&ctx->sad2, 1));
     const i64 nbox = std::max<i64>((i64)n[1], 1);
     if (nbox > ctx->capPB) {
         cudaFree(ctx->path_box);
@@ -2243,9 +2249,9 @@ void launch_detect(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, const PathRe
         const i64 nb = bricks_of(g, shape, nbx, nby, nbz);
         const int ds_blocks = ctx->strict_ds ? 0 : (int)std::min<i64>((nb + 255) / 256, grid / 8);
         k_path_detect<<<grid + (unsigned)ds_blocks, kBlock, 0, st>>>(g, path_flags(ctx), ctx->sad2, ctx->counters + 10,
-                                                                     ctx->path_box, ctx->P.crit, ctx->Q.tcode, ctx->Q.pv, long_paths(ctx),
-                                                                     R, ctx->counters + 27, nbx, nby, nbz, sx[0], sx[1],
-                                                                     sx[2], ds_blocks);
+                                                                     ctx->capSad2, ctx->path_box, ctx->P.crit, ctx->Q.tcode,
+                                                                     ctx->Q.pv, long_paths(ctx), R, ctx->counters + 27, nbx,
+                                                                     nby, nbz, sx[0], sx[1], sx[2], ds_blocks);
         k_path_long<<<grid / 8, kBlock, 0, st>>>(g, long_paths(ctx), R);
         if (ctx->strict_ds) {  // whole-path descending checks of every 1-saddle, into the records
             cudaMemsetAsync(ctx->counters + 29, 0, sizeof(unsigned long long), st);  // the walks' ticket
