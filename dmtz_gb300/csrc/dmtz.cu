@@ -27,6 +27,7 @@
 #include "cnn.cuh"
 #include "dmtz_common.cuh"
 #include "gradient.cuh"
+#include "report_wait.cuh"
 #include "rules.cuh"
 
 using namespace dmtz;
@@ -3081,6 +3082,8 @@ __global__ void __launch_bounds__((brick_threads<8, 4, 4>()), 2)
         ctl->ended = !left;
         ctl->pending = left;
     } else if (first) {
+        if (left)
+            for (int k = 0; k < 8; k++) report[k] = counters[k];
         report[9] = (unsigned long long)rounds;
         report[10] = left;
         for (int k = 0; k < 3; k++) report[11 + k] = ns[k];
@@ -3499,16 +3502,13 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     };
     // counts after a round's end; lists that overflowed grow and are rebuilt
     // (the counts stand in pinned memory as soon as the round's end wrote them, some
-    // microseconds before a wait for the stream would return)
+    // microseconds before a wait for the stream would return; a launch of the round
+    // that failed shows here)
     auto read_fit = [&](int want_saddles) -> dmtz_status {
-        volatile unsigned long long *report = ctx->report;
-        for (unsigned spin = 1; report[8] != ctx->report_seq; spin++) {
-            if (spin % 4096) continue;
-            const cudaError_t q = cudaStreamQuery(st);
-            if (q == cudaSuccess) break;
-            if (q != cudaErrorNotReady) CK(q);
-        }
-        std::atomic_thread_fence(std::memory_order_acquire);
+        const cudaError_t waited = wait_report(ctx->report + 8, ctx->report_seq, [&]() { return cudaStreamQuery(st); });
+        CK(cudaGetLastError());
+        CK(waited);
+        const volatile unsigned long long *report = ctx->report;
         for (int k = 0; k < 8; k++) hc[k] = report[k];
         return fit_lists(ctx, g, want_saddles, hc);
     };
