@@ -45,3 +45,40 @@ def test_two_saddle_list_grows_after_a_connectivity_check(use_graph, strict):
         assert np.array_equal(out, field) and np.array_equal(gcnt, cnt)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("call", ["connectivity", "walls", "correct"])
+def test_no_paths_traced_where_none_are_read(call):
+    """Connectivity mode and the walls read no traced path: their calls leave no
+    room for segments (24 bytes per 16 vertices, 16 per 64) behind."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import dmtz_gb300 as dm
+
+    dims = (176, 176, 176)
+    n = dims[0] ** 3
+    z, y, x = np.meshgrid(*[np.arange(k, dtype=float) for k in dims[::-1]], indexing="ij")
+    f = (x + 0.37 * y + 0.11 * z).reshape(-1)  # few saddles: records and lists are small
+    g = f.copy()
+    g[n // 2] -= 3e-3 * (f.max() - f.min())
+    held = []
+    for paths in (False, True):
+        ctx = dm.Context(0)
+        ctx.mismatch(f, g, dims)
+        before = torch.cuda.mem_get_info()[0]
+        if not paths and call == "connectivity":
+            ctx.path_detect(f, g, dims, connectivity=True)
+        elif not paths and call == "walls":
+            ctx.wall_detect(f, g, dims)
+        elif not paths:
+            ctx.correct(f, g, 1e-2, (1, 1, 0, 0, 0, 0, 0), dims=dims)
+        elif call == "correct":
+            ctx.correct(f, g, 1e-2, (1, 1, 1, 0, 0, 0, 0), dims=dims)
+        else:
+            ctx.path_detect(f, g, dims)
+        held.append(before - torch.cuda.mem_get_info()[0])
+        ctx.close()
+    room = n // 16 * 24 + n // 64 * 16
+    assert held[1] >= room, held
+    assert held[0] < room // 2, held
