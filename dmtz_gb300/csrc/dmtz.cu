@@ -2853,7 +2853,8 @@ struct LoopCtl {
     long long rounds, max_rounds, outer, cp_rounds, path_rounds;
     long long cc[4];
     long long n_as, n_ds;
-    long long runs[LS_STATES];  // body executions per state
+    long long runs[LS_STATES];  // body executions per state (CPS: rounds)
+    long long shorts;           // body executions of CPS
     long long cap[4];           // mismatch list capacities
     long long heavy;            // listed cells from which a round re-pairs the whole grid
     int overflow;       // a scan overflowed a list: stop, grow, scan again, resume at `state`
@@ -3085,6 +3086,7 @@ __global__ void __launch_bounds__((brick_threads<8, 4, 4>()), 2)
     if (first && ctl) {
         ctl->ended = !left;
         ctl->pending = left;
+        ctl->shorts++;
     } else if (first) {
         if (left)
             for (int k = 0; k < 8; k++) report[k] = counters[k];
@@ -3553,7 +3555,9 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         if (c.state != LS_DONE) {
             pt_.mark(PH_PAIR);
             LoopCtl cur = c;
+            int64_t graphs = 0;
             while (true) {
+                graphs++;
                 for (int k = 0; k < 4; k++) cur.cap[k] = ctx->capL[k];
                 if ((s = fit_graph()) != DMTZ_OK || (s = run_graph_loop(ctx, lg, cur, &fin)) != DMTZ_OK) return s;
                 if (!fin.overflow && !fin.stalled) break;
@@ -3587,13 +3591,14 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             pt_.stop();
             // kernels per body run: the round's end, plus each state's own: a fix
             // round is fix + update, then the repair (gradient, and the scan where
-            // the lists are not rebuilt), or the whole gradient; one end more
+            // the lists are not rebuilt), or the whole gradient; short rounds are
+            // one kernel and the repair behind it; one end more per graph
             const int64_t det = detect_kernels(ctx, conn);  // separatrix detection kernels
             const int64_t rnd = 2 + 1 + (ctx->inc_scan ? 0 : 1);
             int64_t bodies = 0;
             for (int k = 0; k < LS_STATES; k++) bodies += k == LS_CPS ? 0 : fin.runs[k];
-            ctx->launches += 1 + bodies + rnd * fin.runs[LS_CP] + (rnd + det) * fin.runs[LS_PDF] + det * fin.runs[LS_PCHECK] +
-                             rnd * fin.runs[LS_PFIX] + 3 * fin.runs[LS_CPF];
+            ctx->launches += graphs + bodies + 3 * fin.shorts + rnd * fin.runs[LS_CP] + (rnd + det) * fin.runs[LS_PDF] +
+                             det * fin.runs[LS_PCHECK] + rnd * fin.runs[LS_PFIX] + 3 * fin.runs[LS_CPF];
         }
         R.outer_iterations = fin.outer;
         R.cp_rounds = fin.cp_rounds;
