@@ -346,8 +346,9 @@ class Context:
         return a.value, b.value
 
     def autotune(self, f, g, dims=None):
-        """Time the brick gradient kernel for every brick shape / blocks-per-SM choice on
-        (f, g); keep the fastest in this context.  Returns (shape, blocks_per_sm, ms)."""
+        """Time the first rounds of a correction of g for every brick shape / blocks-per-SM
+        choice; keep the fastest in this context.  Returns (shape, blocks_per_sm, ms of
+        the gradient kernel over every brick)."""
         dims = _dims_of(np.asarray(f), dims)
         ff, gg = _flat(f), _flat(g)
         best = (_int * 2)()

@@ -1,10 +1,10 @@
 """Autotuner front end: a JSON cache of sweep configurations.
 
 The library measures (`Context.autotune`): for each brick shape (8x4x4,
-16x4x2, 32x2x2 anchors) and 8/16/32/64 blocks per SM it times a full gradient
-sweep and keeps the fastest.  This module remembers the answer per
-(GPU name, grid size class, dtype) in a JSON file, so later runs on the same
-kind of input skip the measurement:
+16x4x2, 32x2x2 anchors) and 8/16/32/64 blocks per SM it times the first rounds
+of a correction and keeps the fastest.  This module remembers the answer per
+(GPU name, grid size class, dtype, what was timed) in a JSON file, so later runs
+on the same kind of input skip the measurement:
 
     from dmtz_gb300 import autotune
     autotune.tune(ctx, f, g)          # measures once, then reads the cache
@@ -45,8 +45,12 @@ def _store(path, data):
     os.replace(tmp, path)
 
 
+# what the library times; entries of files that timed something else are left alone
+MEASURED = "rounds"
+
+
 def key(ctx, dims, dtype) -> str:
-    return f"{ctx.device_name()}|{size_class(dims)}|{np.dtype(dtype).name}"
+    return f"{ctx.device_name()}|{size_class(dims)}|{np.dtype(dtype).name}|{MEASURED}"
 
 
 def tune(ctx, f, g, dims=None, dtype=np.float64, path=None, force=False):

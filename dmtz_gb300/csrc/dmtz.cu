@@ -1423,6 +1423,15 @@ __global__ void k_minmax(const double *a, i64 n, unsigned long long *kmin, unsig
     }
 }
 
+// largest |a - b| as an order key
+__global__ void k_max_gap(const double *a, const double *b, i64 n, unsigned long long *kmax) {
+    double gap = 0;
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) gap = fmax(gap, fabs(a[i] - b[i]));
+    unsigned long long k = okey(gap);
+    for (int o = 16; o > 0; o >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(kmax, k);
+}
+
 __global__ void k_count_u8(const uint8_t *a, i64 n, unsigned long long *out) {
     unsigned long long c = 0;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) c += a[i] != 0;
@@ -3993,6 +4002,15 @@ dmtz_status dmtz_get_tuning(const dmtz_ctx *ctx, int *shape, int *blocks_per_sm)
     return DMTZ_OK;
 }
 
+// What a choice is worth to corrections: the brick kernel over all bricks is not it, because
+// repairs take short lists of bricks, large grids march, and the other shapes lack short
+// rounds (64^3 Gaussian mixture, 108 rounds: 5.6 ms with 8 x 4 x 4, 6.7 with 16 x 4 x 2, 7.1
+// with 32 x 2 x 2).  So every choice corrects decp for kTuneRounds rounds, with the error
+// that decp has as its bound, and another choice than 8 x 4 x 4 and 32 has to be faster by
+// kTuneGain.
+static constexpr int kTuneRounds = 32;
+static constexpr double kTuneGain = 0.02;
+
 dmtz_status dmtz_autotune(dmtz_ctx *ctx, int W, int H, int D, const double *orig, const double *decp, int on_device,
                           int best[2], double *best_ms) {
     Grid g;
@@ -4009,8 +4027,7 @@ dmtz_status dmtz_autotune(dmtz_ctx *ctx, int W, int H, int D, const double *orig
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     static const int bps_opts[4] = {8, 16, 32, 64};
-    double best_t = 1e30;
-    int bs = 0, bb = 32;
+    float sweep[DMTZ_NSHAPES][4];  // ms of the brick kernel over all bricks
     for (int sh = 0; sh < DMTZ_NSHAPES; sh++) {
         if (!shape_fits(g, sh)) continue;
         for (int bi = 0; bi < 4; bi++) {
@@ -4030,22 +4047,75 @@ dmtz_status dmtz_autotune(dmtz_ctx *ctx, int W, int H, int D, const double *orig
                 cudaEventElapsedTime(&t, e0, e1);
                 t_min = std::min(t_min, t);
             }
-            if (t_min < best_t) {
-                best_t = t_min;
-                bs = sh;
-                bb = bps_opts[bi];
-            }
+            sweep[sh][bi] = t_min;
         }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    double mn, mx;
+    unsigned long long gap = 0;
+    if ((s = device_minmax(ctx, ctx->f, g.V, mn, mx)) != DMTZ_OK) return s;
+    CK(cudaMemsetAsync(ctx->counters + 9, 0, sizeof(gap), st));
+    k_max_gap<<<persistent_grid(), kBlock, 0, st>>>(ctx->f, ctx->g, g.V, ctx->counters + 9);
+    CK(cudaMemcpyAsync(&gap, ctx->counters + 9, sizeof(gap), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    const double rel = key_to_double(gap) / (mx - mn);
+    int bs = 0, bb = 2;
+    double *copy = nullptr;  // original, decompressed, corrected
+    bool can = std::isfinite(rel) && rel > 0;
+    if (can && dalloc(&copy, 3 * g.V) != cudaSuccess) {  // no room for them: the default shape
+        cudaGetLastError();
+        can = false;
+    }
+    if (can) {
+        const size_t bytes = sizeof(double) * (size_t)g.V;
+        cudaMemcpyAsync(copy, ctx->f, bytes, cudaMemcpyDeviceToDevice, st);
+        cudaMemcpyAsync(copy + g.V, ctx->g, bytes, cudaMemcpyDeviceToDevice, st);
+        const std::string err = ctx->err;
+        double best_t = 1e30;
+        auto rounds = [&](int sh, int bi) {  // seconds; a first run that takes long is not repeated
+            double t = 1e30;
+            ctx->tune_shape = sh;
+            ctx->tune_bps = bps_opts[bi];
+            for (int r = 0; r < 3; r++) {
+                dmtz_opts o{};
+                dmtz_report rep{};
+                o.preserve_saddles = o.preserve_vpath = o.preserve_geometry = o.break_stalls = 1;
+                o.max_rounds = kTuneRounds;
+                cudaMemcpyAsync(copy + 2 * g.V, copy + g.V, bytes, cudaMemcpyDeviceToDevice, st);
+                const dmtz_status q = dmtz_correct(ctx, W, H, D, copy, copy + 2 * g.V, 1, rel, &o, &rep, nullptr);
+                if (q != DMTZ_OK && q != DMTZ_ERR_NONCONVERGED) return 1e30;
+                t = std::min(t, rep.seconds);
+                if (t > 0.05) break;
+            }
+            return t;
+        };
+        best_t = rounds(bs, bb);
+        for (int sh = 0; sh < DMTZ_NSHAPES; sh++) {
+            if (!shape_fits(g, sh)) continue;
+            for (int bi = 0; bi < 4; bi++) {
+                if (sh == 0 && bi == 2) continue;
+                const double t = rounds(sh, bi);
+                if (t < (1 - kTuneGain) * best_t) {
+                    best_t = t;
+                    bs = sh;
+                    bb = bi;
+                }
+            }
+        }
+        cudaFree(copy);
+        ctx->err = err;
+    } else {
+        for (int bi = 0; bi < 4; bi++)
+            if (sweep[0][bi] < sweep[0][bb]) bb = bi;
+    }
     ctx->tune_shape = bs;
-    ctx->tune_bps = bb;
+    ctx->tune_bps = bps_opts[bb];
     if (best) {
         best[0] = bs;
-        best[1] = bb;
+        best[1] = bps_opts[bb];
     }
-    if (best_ms) *best_ms = best_t;
+    if (best_ms) *best_ms = sweep[bs][bb];
     CK(cudaGetLastError());
     return DMTZ_OK;
 }

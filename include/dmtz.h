@@ -262,10 +262,14 @@ dmtz_status dmtz_correct_batch(dmtz_ctx *ctx, int n, const dmtz_instance *inst, 
 
 /* Brick shape (0: 8x4x4, 1: 16x4x2, 2: 32x2x2 anchors) and blocks per SM
  * (counted for blocks of 128 threads) of the gradient kernel that re-pairs
- * bricks after an update.  Results do not depend on them, only speed.
- * dmtz_autotune times that kernel over every brick of `decp` for every shape
- * and 8, 16, 32, 64 blocks per SM, keeps the fastest in the context and returns
- * it in best[2]. */
+ * bricks after an update.  Results do not depend on them, only speed.  Runs of
+ * short rounds go to a kernel of their own with shape 0 alone.
+ * dmtz_autotune corrects copies of `decp` for up to 32 rounds with every shape
+ * and 8, 16, 32, 64 blocks per SM, keeps the fastest in the context (0 and 32
+ * unless another is faster by 2 %) and returns it in best[2]; best_ms is the
+ * time of the gradient kernel over every brick with that choice.  It needs 24
+ * bytes of device memory per vertex for the copies; without them, or where
+ * `decp` equals `orig`, it keeps shape 0 and chooses the blocks by that kernel. */
 dmtz_status dmtz_set_tuning(dmtz_ctx *ctx, int shape, int blocks_per_sm);
 /* Memory of the mismatch lists (critical cells that differ between the two
  * gradients).  Each of the four lists starts with room for `fraction` of the
