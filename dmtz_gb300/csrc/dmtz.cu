@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "../../include/dmtz.h"
+#include "alloc_retry.cuh"
 #include "cnn.cuh"
 #include "dmtz_common.cuh"
 #include "gradient.cuh"
@@ -1688,27 +1689,35 @@ dmtz_status fail(dmtz_ctx *c, dmtz_status s, const std::string &m) {
         if (e_ != cudaSuccess) return fail(ctx, DMTZ_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-template <class T>
-cudaError_t dalloc(T **p, i64 n) {
-    return cudaMalloc((void **)p, sizeof(T) * (size_t)std::max<i64>(n, 1));
-}
-
-// scratch of one call: take, then cut pieces off it; done gives a large one back
+// Scratch of one call: take, then cut pieces off it; done gives a large one back.  What is
+// kept goes when the context's buffers grow, and when an allocation would fail
+// otherwise (dalloc; no call allocates while it uses the scratch).
 constexpr size_t kWorkKeep = (size_t)1 << 30;
-cudaError_t work_take(dmtz_ctx *c, size_t bytes) {
-    if (bytes <= c->work_bytes) return cudaSuccess;
+bool work_free(dmtz_ctx *c) {  // false: there is none
+    if (!c->work) return false;
     cudaFree(c->work);
     c->work = nullptr;
     c->work_bytes = 0;
+    return true;
+}
+template <class T>
+cudaError_t dalloc(dmtz_ctx *c, T **p, i64 n) {
+    return alloc_retry([&]() { return cudaMalloc((void **)p, sizeof(T) * (size_t)std::max<i64>(n, 1)); },
+                       [&]() {
+                           cudaGetLastError();
+                           return work_free(c);
+                       });
+}
+
+cudaError_t work_take(dmtz_ctx *c, size_t bytes) {
+    if (bytes <= c->work_bytes) return cudaSuccess;
+    work_free(c);
     const cudaError_t e = cudaMalloc((void **)&c->work, bytes);
     if (e == cudaSuccess) c->work_bytes = bytes;
     return e;
 }
 void work_done(dmtz_ctx *c) {
-    if (c->work_bytes <= kWorkKeep) return;
-    cudaFree(c->work);
-    c->work = nullptr;
-    c->work_bytes = 0;
+    if (c->work_bytes > kWorkKeep) work_free(c);
 }
 struct WorkDone {  // gives a large scratch back on every way out
     dmtz_ctx *c;
@@ -1753,7 +1762,7 @@ void free_all(dmtz_ctx *c) {
 }
 
 dmtz_status alloc_field(dmtz_ctx *ctx, DevField &d, i64 V) {
-    CK(dalloc(&d.pv, V)); CK(dalloc(&d.eup, V)); CK(dalloc(&d.fup, V)); CK(dalloc(&d.crit, V)); CK(dalloc(&d.tcode, V));
+    CK(dalloc(ctx, &d.pv, V)); CK(dalloc(ctx, &d.eup, V)); CK(dalloc(ctx, &d.fup, V)); CK(dalloc(ctx, &d.crit, V)); CK(dalloc(ctx, &d.tcode, V));
     return DMTZ_OK;
 }
 
@@ -1772,8 +1781,8 @@ dmtz_status ensure_lists(dmtz_ctx *ctx, const Grid &g) {
         const i64 cap = lean_cap(ctx, cells[k]);
         cudaFree(ctx->list_tmp[k]);
         ctx->list_tmp[k] = nullptr;
-        CK(dalloc(&ctx->lists[k], cap));
-        CK(dalloc(&ctx->list_tmp[k], cap));
+        CK(dalloc(ctx, &ctx->lists[k], cap));
+        CK(dalloc(ctx, &ctx->list_tmp[k], cap));
         ctx->capL[k] = cap;
     }
     return DMTZ_OK;
@@ -1786,22 +1795,23 @@ dmtz_status ensure(dmtz_ctx *ctx, const Grid &g) {
     if (g.V <= ctx->capV && g.E <= ctx->capE && g.F <= ctx->capF && g.T <= ctx->capT && nbr <= ctx->capB)
         return ensure_lists(ctx, g);
     free_all(ctx);
+    work_free(ctx);
     const i64 V = g.V;
-    CK(dalloc(&ctx->f, V)); CK(dalloc(&ctx->g, V));
+    CK(dalloc(ctx, &ctx->f, V)); CK(dalloc(ctx, &ctx->g, V));
     dmtz_status s;
     if ((s = alloc_field(ctx, ctx->P, V)) != DMTZ_OK) return s;
     if ((s = alloc_field(ctx, ctx->Q, V)) != DMTZ_OK) return s;
-    CK(dalloc(&ctx->cnt, V));
-    CK(dalloc(&ctx->reqbits, (V + 31) / 32 + 1));
+    CK(dalloc(ctx, &ctx->cnt, V));
+    CK(dalloc(ctx, &ctx->reqbits, (V + 31) / 32 + 1));
     CK(cudaMemset(ctx->reqbits, 0, sizeof(uint32_t) * (size_t)((V + 31) / 32 + 1)));
-    CK(dalloc(&ctx->reqlist, V));
-    CK(dalloc(&ctx->brick_flags, (nbr + 3) / 4)); CK(dalloc(&ctx->brick_list, nbr));
-    CK(dalloc(&ctx->path_as, 2 * nbr));
+    CK(dalloc(ctx, &ctx->reqlist, V));
+    CK(dalloc(ctx, &ctx->brick_flags, (nbr + 3) / 4)); CK(dalloc(ctx, &ctx->brick_list, nbr));
+    CK(dalloc(ctx, &ctx->path_as, 2 * nbr));
     ctx->path_ds = ctx->path_as + nbr;
-    CK(dalloc(&ctx->brick_n, 8));
+    CK(dalloc(ctx, &ctx->brick_n, 8));
     CK(cudaMemset(ctx->brick_flags, 0, sizeof(uint32_t) * (size_t)((nbr + 3) / 4)));
     ctx->capB = nbr;
-    CK(dalloc(&ctx->counters, 32)); CK(dalloc(&ctx->errword, 1)); CK(dalloc(&ctx->changed, V));
+    CK(dalloc(ctx, &ctx->counters, 32)); CK(dalloc(ctx, &ctx->errword, 1)); CK(dalloc(ctx, &ctx->changed, V));
     ctx->capV = g.V; ctx->capE = g.E; ctx->capF = g.F; ctx->capT = g.T;
     return ensure_lists(ctx, g);
 }
@@ -1815,8 +1825,8 @@ dmtz_status grow_list(dmtz_ctx *ctx, const Grid &g, int k, i64 need) {
     cudaFree(ctx->list_tmp[k]);
     ctx->lists[k] = ctx->list_tmp[k] = nullptr;
     ctx->capL[k] = 0;
-    CK(dalloc(&ctx->lists[k], cap));
-    CK(dalloc(&ctx->list_tmp[k], cap));
+    CK(dalloc(ctx, &ctx->lists[k], cap));
+    CK(dalloc(ctx, &ctx->list_tmp[k], cap));
     ctx->capL[k] = cap;
     return DMTZ_OK;
 }
@@ -2139,7 +2149,7 @@ dmtz_status trace_paths(dmtz_ctx *ctx, const Grid &g) {
             cudaFree(ctx->seg);
             ctx->seg = nullptr;
             ctx->capSeg = 0;
-            CK(dalloc(&ctx->seg, need_seg));
+            CK(dalloc(ctx, &ctx->seg, need_seg));
             ctx->capSeg = need_seg;
         }
         if (need_slot > ctx->capSlot) {
@@ -2148,8 +2158,8 @@ dmtz_status trace_paths(dmtz_ctx *ctx, const Grid &g) {
             ctx->seg_sad = nullptr;
             ctx->seg_res = nullptr;
             ctx->capSlot = 0;
-            CK(dalloc(&ctx->seg_sad, need_slot));
-            CK(dalloc(&ctx->seg_res, need_slot));
+            CK(dalloc(ctx, &ctx->seg_sad, need_slot));
+            CK(dalloc(ctx, &ctx->seg_res, need_slot));
             ctx->capSlot = need_slot;
         }
         CK(cudaMemsetAsync(ctx->counters + 25, 0, 3 * sizeof(unsigned long long), st));  // segments, slots, ticket
@@ -2185,8 +2195,8 @@ dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g, bool trace) {
         cudaFree(ctx->ds_vert);
         ctx->ds_edge = ctx->ds_vert = nullptr;
         ctx->capDS = 0;
-        CK(dalloc(&ctx->ds_edge, (i64)n[0]));
-        CK(dalloc(&ctx->ds_vert, (i64)n[0]));
+        CK(dalloc(ctx, &ctx->ds_edge, (i64)n[0]));
+        CK(dalloc(ctx, &ctx->ds_vert, (i64)n[0]));
         ctx->capDS = (i64)n[0];
     }
     if ((i64)n[1] > ctx->capAS) {
@@ -2194,8 +2204,8 @@ dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g, bool trace) {
         cudaFree(ctx->as_cur);
         ctx->as_tet = ctx->as_cur = nullptr;
         ctx->capAS = 0;
-        CK(dalloc(&ctx->as_tet, (i64)n[1]));
-        CK(dalloc(&ctx->as_cur, (i64)n[1]));
+        CK(dalloc(ctx, &ctx->as_tet, (i64)n[1]));
+        CK(dalloc(ctx, &ctx->as_cur, (i64)n[1]));
         ctx->capAS = (i64)n[1];
     }
     // (of its own: a connectivity check grows the records alone)
@@ -2203,25 +2213,25 @@ dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g, bool trace) {
         cudaFree(ctx->sad2);
         ctx->sad2 = nullptr;
         ctx->capSad2 = 0;
-        CK(dalloc(&ctx->sad2, (i64)n[1]));
+        CK(dalloc(ctx, &ctx->sad2, (i64)n[1]));
         ctx->capSad2 = (i64)n[1];
     }
     // buffers exist even when a count is 0 (kernels take their addresses)
     if (!ctx->ds_edge) {
-        CK(dalloc(&ctx->ds_edge, 1));
-        CK(dalloc(&ctx->ds_vert, 1));
+        CK(dalloc(ctx, &ctx->ds_edge, 1));
+        CK(dalloc(ctx, &ctx->ds_vert, 1));
     }
     if (!ctx->as_tet) {
-        CK(dalloc(&ctx->as_tet, 1));
-        CK(dalloc(&ctx->as_cur, 1));
+        CK(dalloc(ctx, &ctx->as_tet, 1));
+        CK(dalloc(ctx, &ctx->as_cur, 1));
     }
-    if (!ctx->sad2) CK(dalloc(&ctx->sad2, 1));
+    if (!ctx->sad2) CK(dalloc(ctx, &ctx->sad2, 1));
     const i64 nbox = std::max<i64>((i64)n[1], 1);
     if (trace && nbox > ctx->capPB) {
         cudaFree(ctx->path_box);
         ctx->path_box = nullptr;
         ctx->capPB = 0;
-        CK(dalloc(&ctx->path_box, nbox));
+        CK(dalloc(ctx, &ctx->path_box, nbox));
         ctx->capPB = nbox;
     }
     CK(cudaMemsetAsync(ctx->counters + 10, 0, sizeof(unsigned long long), st));
@@ -2233,7 +2243,7 @@ dmtz_status prep_paths(dmtz_ctx *ctx, const Grid &g, bool trace) {
             cudaFree(ctx->sad1);
             ctx->sad1 = nullptr;
             ctx->capSad1 = 0;
-            CK(dalloc(&ctx->sad1, need));
+            CK(dalloc(ctx, &ctx->sad1, need));
             ctx->capSad1 = need;
         }
         CK(cudaMemsetAsync(ctx->counters + 28, 0, sizeof(unsigned long long), st));
@@ -2291,10 +2301,10 @@ dmtz_status ensure_walls(dmtz_ctx *ctx) {
     cudaFree(ctx->wall_sad); cudaFree(ctx->wall_edge); cudaFree(ctx->wall_next[0]); cudaFree(ctx->wall_next[1]);
     ctx->wall_sad = ctx->wall_edge = ctx->wall_next[0] = ctx->wall_next[1] = nullptr;
     ctx->capWall = 0;
-    CK(dalloc(&ctx->wall_sad, need));
-    CK(dalloc(&ctx->wall_edge, need));
-    CK(dalloc(&ctx->wall_next[0], need));
-    CK(dalloc(&ctx->wall_next[1], need));
+    CK(dalloc(ctx, &ctx->wall_sad, need));
+    CK(dalloc(ctx, &ctx->wall_edge, need));
+    CK(dalloc(ctx, &ctx->wall_next[0], need));
+    CK(dalloc(ctx, &ctx->wall_next[1], need));
     ctx->capWall = need;
     return DMTZ_OK;
 }
@@ -2334,7 +2344,7 @@ dmtz_status detect_walls(dmtz_ctx *ctx, const Grid &g, const RuleCtx &rc, i64 &n
             cudaFree(ctx->wall_scratch);
             ctx->wall_scratch = nullptr;
             ctx->capWS = 0;
-            CK(dalloc(&ctx->wall_scratch, chunk * per));
+            CK(dalloc(ctx, &ctx->wall_scratch, chunk * per));
             ctx->capWS = chunk * per;
         }
         unsigned long long *nnext = ctx->counters + 17 + (cur ^ 1);
@@ -2709,7 +2719,7 @@ dmtz_status dmtz_fix_round(dmtz_ctx *ctx, int W, int H, int D, const double *ori
     RuleCtx rc = rule_ctx(ctx, g, bound, edit_type);
     k_fix_cp<<<persistent_grid(), kBlock, 0, ctx->stream>>>(rc, cp_lists(ctx), preserve_saddles);
     double *dd = nullptr;
-    CK(dalloc(&dd, g.V));
+    CK(dalloc(ctx, &dd, g.V));
     const double sentinel = -2000.0 * range;
     std::vector<double> fill((size_t)g.V, sentinel);
     CK(cudaMemcpyAsync(dd, fill.data(), sizeof(double) * (size_t)g.V, cudaMemcpyHostToDevice, ctx->stream));
@@ -2750,8 +2760,8 @@ static dmtz_status path_detect_impl(dmtz_ctx *ctx, int W, int H, int D, const do
             cudaFree(ctx->as_cur);
             ctx->as_tet = ctx->as_cur = nullptr;
             ctx->capAS = 0;
-            CK(dalloc(&ctx->as_tet, (i64)hc[0]));
-            CK(dalloc(&ctx->as_cur, (i64)hc[0]));
+            CK(dalloc(ctx, &ctx->as_tet, (i64)hc[0]));
+            CK(dalloc(ctx, &ctx->as_cur, (i64)hc[0]));
             ctx->capAS = (i64)hc[0];
         }
         if ((i64)hc[1] > ctx->capDS) {
@@ -2759,8 +2769,8 @@ static dmtz_status path_detect_impl(dmtz_ctx *ctx, int W, int H, int D, const do
             cudaFree(ctx->ds_vert);
             ctx->ds_edge = ctx->ds_vert = nullptr;
             ctx->capDS = 0;
-            CK(dalloc(&ctx->ds_edge, (i64)hc[1]));
-            CK(dalloc(&ctx->ds_vert, (i64)hc[1]));
+            CK(dalloc(ctx, &ctx->ds_edge, (i64)hc[1]));
+            CK(dalloc(ctx, &ctx->ds_vert, (i64)hc[1]));
             ctx->capDS = (i64)hc[1];
         }
     }
@@ -3344,7 +3354,7 @@ static dmtz_status features_into(dmtz_ctx *ctx, const Grid &g, double bound, __n
         cudaFree(ctx->mm);
         ctx->mm = nullptr;
         ctx->capMM = 0;
-        CK(dalloc(&ctx->mm, g.V));
+        CK(dalloc(ctx, &ctx->mm, g.V));
         ctx->capMM = g.V;
     }
     cudaStream_t st = ctx->stream;
@@ -3787,15 +3797,15 @@ dmtz_status dmtz_quantize(dmtz_ctx *ctx, int W, int H, int D, const double *orig
         return fail(ctx, DMTZ_ERR_ARG, "rel_eps must be finite and >= 0, noise_frac in [0, 1]");
     CK(cudaSetDevice(ctx->device));
     if (!ctx->counters) {
-        CK(dalloc(&ctx->counters, 32));
-        CK(dalloc(&ctx->errword, 1));
+        CK(dalloc(ctx, &ctx->counters, 32));
+        CK(dalloc(ctx, &ctx->errword, 1));
     }
     cudaStream_t st = ctx->stream;
     const double *fd = orig;
     double *gd = decp;
     double *tmp = nullptr;
     if (!on_device) {  // staging buffers for host fields
-        CK(dalloc(&tmp, 2 * g.V));
+        CK(dalloc(ctx, &tmp, 2 * g.V));
         CK(cudaMemcpyAsync(tmp, orig, sizeof(double) * (size_t)g.V, cudaMemcpyHostToDevice, st));
         fd = tmp;
         gd = tmp + g.V;
@@ -4063,7 +4073,7 @@ dmtz_status dmtz_autotune(dmtz_ctx *ctx, int W, int H, int D, const double *orig
     int bs = 0, bb = 2;
     double *copy = nullptr;  // original, decompressed, corrected
     bool can = std::isfinite(rel) && rel > 0;
-    if (can && dalloc(&copy, 3 * g.V) != cudaSuccess) {  // no room for them: the default shape
+    if (can && dalloc(ctx, &copy, 3 * g.V) != cudaSuccess) {  // no room for them: the default shape
         cudaGetLastError();
         can = false;
     }

@@ -100,7 +100,13 @@ typedef struct {
     int64_t final_walls;        /* wall records left (preserve_connectors = 1) */
 } dmtz_report;
 
-/* Context: owns the device, a stream and all scratch memory.
+/* Context: owns the device, a stream and all scratch memory.  The buffers of the
+ * largest grid so far stay with it (about 125 bytes per vertex after a correction,
+ * see dmtz_set_list_reserve).  dmtz_extract, dmtz_labels, dmtz_separatrix_agreement
+ * and dmtz_link_classes use scratch besides (104, 52, 56 and 1 bytes per vertex; 112 for the
+ * agreement of more than 2^31 / 6 vertices), of which up to 1 GB is kept for the next
+ * such call; it is given back when the buffers grow, when one of the context's
+ * allocations would fail otherwise, and by dmtz_ctx_destroy.
  * Replaces the device globals and cudaMalloc calls of main_3d.cu:43-129,
  * 6466-6714. */
 dmtz_status dmtz_ctx_create(dmtz_ctx **out, int device);
