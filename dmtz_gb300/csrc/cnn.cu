@@ -1628,7 +1628,7 @@ struct dmtz_cnn {
     std::string err;
     float *w = nullptr, *grad = nullptr, *m1 = nullptr, *m2 = nullptr;  // kParams each
     bf16 *wf = nullptr, *wt = nullptr;  // bf16 weights, forward and transposed, per layer at woff[l]
-    float *part = nullptr;              // weight-gradient partials: nsm x all layers, or 2 nsm x one layer (mma.sync)
+    float *part = nullptr;              // weight-gradient partials: nsm x all layers, or 2 nsm x one layer (mma.sync); from the first training pass on
     double *lpart = nullptr, *lres = nullptr;
     float *scale = nullptr;
     i64 step = 0;
@@ -1851,6 +1851,7 @@ dmtz_status pack(dmtz_cnn *net, cudaStream_t st) {
 }
 
 dmtz_status ensure_act(dmtz_cnn *net, i64 V, bool train) {
+    if (train && !net->part) NCK(nalloc(&net->part, net->nsm * kParams));  // (50 MB that inference does without)
     if (V <= net->capV && (!train || net->cap_train)) return DMTZ_OK;
     cudaFree(net->a[0]);
     cudaFree(net->a[1]);
@@ -1967,8 +1968,7 @@ dmtz_status dmtz_cnn_create(dmtz_cnn **out, int device, uint64_t seed) {
     if (cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(DMTZ_ERR_CUDA);
     if (nalloc(&net->w, kParams) || nalloc(&net->grad, kParams) || nalloc(&net->m1, kParams) ||
         nalloc(&net->m2, kParams) || nalloc(&net->wf, kWeights) || nalloc(&net->wt, kWeights) ||
-        nalloc(&net->part, net->nsm * kParams) || nalloc(&net->lpart, 2 * kLossBlocks) ||
-        nalloc(&net->lres, 3) || nalloc(&net->scale, 1))
+        nalloc(&net->lpart, 2 * kLossBlocks) || nalloc(&net->lres, 3) || nalloc(&net->scale, 1))
         return bail(DMTZ_ERR_CUDA);
     net->tc_err = reinterpret_cast<int *>(net->lres + 2);  // behind the loss, so that one copy brings both
     net->lticket = reinterpret_cast<unsigned *>(net->lres + 2) + 1;
