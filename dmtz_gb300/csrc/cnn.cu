@@ -557,13 +557,13 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv_tc(const __grid_consta
 }
 
 // ---------------------------------------- convolution on tcgen05, x-taps folded
-// The same convolution with wider products, marching along x.  A tile is a
-// column: 8 x 16 vertices of the plane across x (axes a and b: y and z, or z
-// and y when that pads fewer rows) are the 128 rows of every product.  The
-// input arrives as slices of constant x (10 x 18 vertices with the halo), each
-// once.  Slice x contributes to the outputs x + 1, x and x - 1 through the
-// taps dx = -1, 0, 1; their weight blocks side by side make one MMA of N =
-// 3 COUT per (dy, dz) offset: 9 x CIN/16 MMAs per slice.  The three
+// The same convolution with wider products, marching along x (or y or z, see
+// make_march).  A tile is a column: 8 x 16 vertices of the plane across x (axes
+// a and b: y and z, or z and y when that pads fewer rows) are the 128 rows of
+// every product.  The input arrives as slices of constant x (10 x 18 vertices
+// with the halo), each once.  Slice x contributes to the outputs x + 1, x and
+// x - 1 through the taps dx = -1, 0, 1; their weight blocks side by side make one
+// MMA of N = 3 COUT per (dy, dz) offset: 9 x CIN/16 MMAs per slice.  The three
 // contributions to an output lie in the same lanes of three successive
 // slices' accumulators, so the epilogue adds them in registers as it goes.
 //
@@ -592,40 +592,50 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv_tc(const __grid_consta
 constexpr int CX_A = 8, CX_B = 16, CX_GA = CX_A + 2, CX_GB = CX_B + 2, CX_NX = 2, CX_ACC = 4, CX_ST = 6;
 constexpr int CX_EPI = 8, CX_THREADS = 96 + 32 * CX_EPI;
 struct March {
-    int W, na, nb;  // extents along x, a, b
-    i64 sa, sb;     // vertex strides of a and b
-    int swapped;    // a = z and b = y
-    int ta, tb;     // a column's outputs along a and b
-    int nta;        // columns along a
-    i64 outputs;    // of all columns
+    int n, na, nb;       // extents along the march, a, b
+    i64 s, sa, sb;       // their vertex strides
+    int t, tp, tq;       // and tap strides: of the march, and of the other axes p before q
+    bool along_x() const { return t == 1; }
+    int swapped;         // a = q and b = p
+    int ta, tb;          // a column's outputs along a and b
+    int nta;             // columns along a
+    i64 outputs;         // of all columns
 };
+inline March march_along(int axis, int W, int H, int D, int ta, int tb) {
+    const int n[3] = {W, H, D}, tap[3] = {1, 3, 9}, p = axis == 0 ? 1 : 0, q = axis == 2 ? 1 : 2;
+    const i64 st[3] = {1, W, (i64)W * H};
+    auto up = [](i64 k, i64 m) { return (k + m - 1) / m * m; };
+    const bool swap = up(n[q], ta) * up(n[p], tb) < up(n[p], ta) * up(n[q], tb);
+    const int a = swap ? q : p, b = swap ? p : q;
+    return March{n[axis], n[a],   n[b],   st[axis], st[a], st[b], tap[axis], tap[p],
+                 tap[q],  swap,   ta,     tb,       (n[a] + ta - 1) / ta,
+                 up(n[a], ta) / ta * (up(n[b], tb) / tb) * n[axis]};
+}
+// Along x, unless fewer than a third of the columns' rows are vertices then (a grid of
+// one or two vertices along y or z, or a few along both) and another axis has fewer
+// slices.  Forward passes along x only, and so: 2000 x 1000 x 1 1.37 and 0.39 ms, 1000 x
+// 2000 x 2 1.36 and 0.54, 20000 x 3 x 3 0.27 and 0.12 (14 x 8 x 2 tiles with halo boxes: 0.84,
+// 0.90 and 0.19); 1000 x 1000 x 3, three eighths: 0.72 (0.88) along x.
 inline March make_march(int W, int H, int D, int ta = CX_A, int tb = CX_B) {
-    auto up = [](i64 n, i64 m) { return (n + m - 1) / m * m; };
-    const bool swap = up(D, ta) * up(H, tb) < up(H, ta) * up(D, tb);
-    March m{};
-    m.W = W;
-    m.na = swap ? D : H;
-    m.nb = swap ? H : D;
-    m.sa = swap ? (i64)W * H : W;
-    m.sb = swap ? W : (i64)W * H;
-    m.swapped = swap;
-    m.ta = ta;
-    m.tb = tb;
-    m.nta = (m.na + ta - 1) / ta;
-    m.outputs = (i64)m.nta * ((m.nb + tb - 1) / tb) * W;
+    March m = march_along(0, W, H, D, ta, tb);
+    if (m.outputs * ta * tb <= 3 * (i64)W * H * D) return m;
+    for (int axis = 1; axis < 3; axis++) {
+        const March o = march_along(axis, W, H, D, ta, tb);
+        if (o.outputs < m.outputs) m = o;
+    }
     return m;
 }
 // the part of a run that lies in one column: outputs [o0, o1) from slices j0..j1
 struct Stretch {
     int a0, b0, o0, o1, j0, j1;
     __device__ __forceinline__ Stretch(const March &m, i64 g, i64 end) {
-        const i64 col = g / m.W;
+        const i64 col = g / m.n;
         a0 = (int)(col % m.nta) * m.ta;
         b0 = (int)(col / m.nta) * m.tb;
-        o0 = (int)(g - col * m.W);
-        o1 = (int)min((i64)m.W, o0 + (end - g));
+        o0 = (int)(g - col * m.n);
+        o1 = (int)min((i64)m.n, o0 + (end - g));
         j0 = max(o0 - 1, 0);
-        j1 = min(o1, m.W - 1);
+        j1 = min(o1, m.n - 1);
     }
 };
 template <int CIN>
@@ -668,7 +678,8 @@ __device__ __forceinline__ void st32(void *p, const Vec8 &r) {
                  "r"(r.v[3]), "r"(r.v[4]), "r"(r.v[5]), "r"(r.v[6]), "r"(r.v[7])
                  : "memory");
 }
-template <int CIN, int COUT, int MODE, bool FLIP>
+// X: the march goes along x (a kernel of its own: with run-time strides 0.6 % of a forward pass)
+template <int CIN, int COUT, int MODE, bool FLIP, bool X>
 __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constant__ CUtensorMap tmap, const March m,
                                                           const bf16 *__restrict__ wt, const float *__restrict__ bias,
                                                           bf16 *out, const bf16 *__restrict__ aux, int *err) {
@@ -719,7 +730,7 @@ __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constan
     if (warp < 2) {  // MMA issuers
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         const uint64_t b0 = smem_desc(wbase, WGRP, 128);
-        const uint32_t dy = (m.swapped ? LINE : ROW) >> 4, dz = (m.swapped ? ROW : LINE) >> 4;
+        const uint32_t dp = (m.swapped ? LINE : ROW) >> 4, dq = (m.swapped ? ROW : LINE) >> 4;
         if (!mbar_wait(wbar, 0u, kConvWaitPolls)) failed = true;
         int c = 0, q = 0;  // copies and slices so far
         for (i64 g = first; g < end && !failed;) {
@@ -745,7 +756,7 @@ __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constan
                             for (int u = 0; u < 9; u++)
 #pragma unroll
                                 for (int kk = 0; kk < KCH / 2; kk++)
-                                    tc_mma(acc, a0 + (u % 3 * dy + u / 3 * dz + kk * 2),
+                                    tc_mma(acc, a0 + (u % 3 * dp + u / 3 * dq + kk * 2),
                                            b0 + (((u * KCH + kk * 2) * WGRP) >> 4), idesc, (u | kk) != 0);
                             tc_commit(mma(q + e));
                         }
@@ -788,13 +799,13 @@ __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constan
         }
         __syncwarp();
     } else {
-        // weights: per offset u = (dy + 1) + 3 (dz + 1) and channel group kc, rows
-        // n = t COUT + c hold tap dx = t - 1 of output channel c (mirrored under FLIP)
+        // weights: per offset u = (dp + 1) + 3 (dq + 1) and channel group kc, rows
+        // n = t COUT + c hold march tap t - 1 of output channel c (mirrored under FLIP)
         unsigned char *ws = smem_raw + (wbase - smem_addr(smem_raw));
         for (int i = tid - 96; i < 9 * KCH * N; i += 32 * CX_EPI) {
             const int u = i / (KCH * N), rem = i - u * (KCH * N), kc = rem / N, n = rem - kc * N;
             const int t = n / COUT, c = n - t * COUT;
-            const int tap = FLIP ? 26 - (t + 3 * u) : t + 3 * u;
+            const int at = X ? t + 3 * u : t * m.t + u % 3 * m.tp + u / 3 * m.tq, tap = FLIP ? 26 - at : at;
             cp16(ws + (u * KCH + kc) * WGRP + n * 16, wt + ((i64)tap * COUT + c) * CIN + kc * 8, 16);
         }
         cp_commit();
@@ -825,7 +836,7 @@ __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constan
             for (int c = 0; c < NC; c++) next[c] = cur[c] = 0.f;
             auto store = [&](int o, const Vec8 &mk) {  // cur is complete: output o
                 if (!row) return;
-                const i64 v = v0 + o;
+                const i64 v = v0 + o * (X ? 1 : m.s);
                 Vec8 pk;
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
@@ -844,7 +855,7 @@ __global__ void __launch_bounds__(CX_THREADS, 1) k_conv_tcx(const __grid_constan
             };
             auto mask = [&](int o) {
                 Vec8 mk{};
-                if (MODE == 2 && row && o >= t.o0 && o < t.o1) mk = ld32(aux + (v0 + o) * COUT + c0);
+                if (MODE == 2 && row && o >= t.o0 && o < t.o1) mk = ld32(aux + (v0 + o * (X ? 1 : m.s)) * COUT + c0);
                 return mk;
             };
             auto slice = [&](int j, const Vec8 &mk) {
@@ -917,7 +928,7 @@ struct OutLayer {
     static constexpr uint32_t ROW = CIN * 2, SLICE = OL_ROWS * ROW, STAGE = OL_NX * SLICE, WBYTES = (CIN / 8) * 32 * 16;
     static constexpr size_t smem = 1024 + (size_t)OL_ST * STAGE + WBYTES + 2 * 9 * OL_ROWS * sizeof(float);
 };
-template <int CIN, int COUT>
+template <int CIN, int COUT, bool X>
 __global__ void __launch_bounds__(OL_THREADS, 2) k_conv_out(const __grid_constant__ CUtensorMap tmap, const March m,
                                                           const bf16 *__restrict__ wt, const float *__restrict__ bias,
                                                           float *__restrict__ out, int *err) {
@@ -955,10 +966,10 @@ __global__ void __launch_bounds__(OL_THREADS, 2) k_conv_out(const __grid_constan
         init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n");
     }
-    // weights: per channel group, row n = 9 (dx + 1) + 3 (db + 1) + (da + 1) is that tap of output channel 0
+    // weights: per channel group, row n = 9 (dm + 1) + 3 (db + 1) + (da + 1) is that tap of output channel 0 (dm: along the march)
     for (int i = tid; i < (CIN / 8) * 32; i += OL_THREADS) {
-        const int kc = i / 32, n = i % 32, dx = n / 9, a = n % 3, b = n / 3 % 3;
-        const int tap = dx + (m.swapped ? 9 * a + 3 * b : 3 * a + 9 * b);
+        const int kc = i / 32, n = i % 32, dm = n / 9, a = n % 3, b = n / 3 % 3;
+        const int tp = X ? 3 : m.tp, tq = X ? 9 : m.tq, tap = dm * (X ? 1 : m.t) + (m.swapped ? tq * a + tp * b : tp * a + tq * b);
         const uint4 v = n < 27 ? *reinterpret_cast<const uint4 *>(wt + (i64)tap * COUT * CIN + kc * 8) : make_uint4(0, 0, 0, 0);
         *reinterpret_cast<uint4 *>(ws + i * 16) = v;
     }
@@ -1054,7 +1065,7 @@ __global__ void __launch_bounds__(OL_THREADS, 2) k_conv_out(const __grid_constan
                     float x = 0.f;
 #pragma unroll
                     for (int u = 0; u < 9; u++) x += sum[buf][u][r + (u % 3 - 1) + 8 * (u / 3 - 1)];
-                    out[v0 + o] = x + b0;
+                    out[v0 + o * (X ? 1 : m.s)] = x + b0;
                 }
                 buf ^= 1;
             };
@@ -1743,10 +1754,10 @@ dmtz_status box_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, int 
     const cuuint32_t box[4] = {8, GX, GY, GZ};
     return encode_map(net, tm, act, 4, dims, strides, box);
 }
-// and for k_conv_tcx's and k_conv_out's slices with their halo: whole vertices, axes (channel, a, b, x)
+// and for k_conv_tcx's and k_conv_out's slices with their halo: whole vertices, axes (channel, a, b, march)
 dmtz_status slice_map(dmtz_cnn *net, CUtensorMap *tm, const bf16 *act, int C, const March &m, int nx) {
-    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)m.na, (cuuint64_t)m.nb, (cuuint64_t)m.W}, row = (cuuint64_t)C * 2;
-    const cuuint64_t strides[3] = {row * m.sa, row * m.sb, row};
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)m.na, (cuuint64_t)m.nb, (cuuint64_t)m.n}, row = (cuuint64_t)C * 2;
+    const cuuint64_t strides[3] = {row * m.sa, row * m.sb, row * m.s};
     const cuuint32_t box[4] = {(cuuint32_t)C, (cuuint32_t)m.ta + 2, (cuuint32_t)m.tb + 2, (cuuint32_t)nx};
     return encode_map(net, tm, act, 4, dims, strides, box, C == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
@@ -1772,14 +1783,14 @@ dmtz_status conv(dmtz_cnn *net, const Dims &d, const bf16 *in, const bf16 *w, co
             March m = make_march(d.W, d.H, d.D, OL_A, OL_B);
             if ((s = slice_map(net, &tm, in, CIN, m, OL_NX)) != DMTZ_OK) return s;
             void *args[] = {&tm, &m, &w, &bias, &out, &err};
-            return launch_persistent(net, k_conv_out<CIN, COUT>, OL_THREADS, OutLayer<CIN>::smem, m.outputs, 2 * net->nsm, nullptr,
-                                     st, args);
+            auto kernel = m.along_x() ? k_conv_out<CIN, COUT, true> : k_conv_out<CIN, COUT, false>;
+            return launch_persistent(net, kernel, OL_THREADS, OutLayer<CIN>::smem, m.outputs, 2 * net->nsm, nullptr, st, args);
         } else {
             March m = make_march(d.W, d.H, d.D);
             if ((s = slice_map(net, &tm, in, CIN, m, CX_NX)) != DMTZ_OK) return s;
             void *args[] = {&tm, &m, &w, &bias, &out, &aux, &err};
-            return launch_persistent(net, k_conv_tcx<CIN, COUT, MODE, FLIP>, CX_THREADS, cx_smem<CIN, COUT>(), m.outputs,
-                                     net->nsm, nullptr, st, args);
+            auto kernel = m.along_x() ? k_conv_tcx<CIN, COUT, MODE, FLIP, true> : k_conv_tcx<CIN, COUT, MODE, FLIP, false>;
+            return launch_persistent(net, kernel, CX_THREADS, cx_smem<CIN, COUT>(), m.outputs, net->nsm, nullptr, st, args);
         }
     }
     if (net->tensor_path) {
