@@ -1494,20 +1494,22 @@ __global__ void k_quantize(i64 V, const double *f, double *g, double fmn, double
 // error (2^-52 relative) is far below the float32 value's; where a
 // reciprocal is not finite and normal the host asks for quotients (EXACT).  With
 // fourteen quotients per vertex 782 us at 160 x 144 x 128; now 206 us.
-constexpr int kFeatX = 32, kFeatY = 8, kFeatZ = 4;
+//
+// Tiles of 32 x 8 x 4, and of 4 x 16 x 16 on grids at most 4 wide in x: 2 x 2000 x 1000
+// 10.2 ms a call and 6.7 (7.9 with a thread per vertex), 4 x 1500 x 800 6.4 and 4.2 (7.7).
 // the seven stencil directions towards larger ids
 __host__ __device__ constexpr int up_dir(int r) { return cxt::dir_by_id(7 + r); }
 __host__ __device__ constexpr int opposite_dir(int d) { return d ^ 1; }
-template <bool EXACT>
+template <int TX, int TY, int TZ, bool EXACT>
 __global__ void __launch_bounds__(kBlock) k_features(Grid g, const double *f, const double *gv, const uint32_t *critP,
                                                     const uint32_t *critQ, double bound, double inv, double inv4,
                                                     __nv_bfloat16 *feat, uint8_t *mm, int ntx, int nty) {
     // box: one layer towards smaller ids in z and y, one to both sides in x
     // (directions with dz or dy = +1 may have dx = -1)
-    constexpr int BX = kFeatX + 2, BY = kFeatY + 1, BZ = kFeatZ + 1, NB = BX * BY * BZ;
+    constexpr int BX = TX + 2, BY = TY + 1, BZ = TZ + 1, NB = BX * BY * BZ;
     __shared__ __nv_bfloat16 slope[7][NB];
-    const int x0 = (int)(blockIdx.x % (unsigned)ntx) * kFeatX, y0 = (int)((blockIdx.x / (unsigned)ntx) % (unsigned)nty) * kFeatY,
-              z0 = (int)(blockIdx.x / ((unsigned)ntx * (unsigned)nty)) * kFeatZ;
+    const int x0 = (int)(blockIdx.x % (unsigned)ntx) * TX, y0 = (int)((blockIdx.x / (unsigned)ntx) % (unsigned)nty) * TY,
+              z0 = (int)(blockIdx.x / ((unsigned)ntx * (unsigned)nty)) * TZ;
     for (int e = threadIdx.x; e < NB; e += kBlock) {
         const int x = x0 - 1 + e % BX, y = y0 - 1 + (e / BX) % BY, z = z0 - 1 + e / (BX * BY);
         const bool in = x >= 0 && y >= 0 && z >= 0 && x < g.W && y < g.H && z < g.D;
@@ -1525,8 +1527,8 @@ __global__ void __launch_bounds__(kBlock) k_features(Grid g, const double *f, co
         });
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < kFeatX * kFeatY * kFeatZ; t += kBlock) {
-        const int lx = t % kFeatX, ly = (t / kFeatX) % kFeatY, lz = t / (kFeatX * kFeatY);
+    for (int t = threadIdx.x; t < TX * TY * TZ; t += kBlock) {
+        const int lx = t % TX, ly = (t / TX) % TY, lz = t / (TX * TY);
         const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
         if (x >= g.W || y >= g.H || z >= g.D) continue;
         const i64 v = x + (i64)y * g.W + (i64)z * g.WH;
@@ -3359,9 +3361,12 @@ static dmtz_status features_into(dmtz_ctx *ctx, const Grid &g, double bound, __n
     }
     cudaStream_t st = ctx->stream;
     const unsigned grid = persistent_grid();
-    const int ntx = (g.W + kFeatX - 1) / kFeatX, nty = (g.H + kFeatY - 1) / kFeatY, ntz = (g.D + kFeatZ - 1) / kFeatZ;
     const double inv = 1.0 / bound, inv4 = 1.0 / (4.0 * bound);
-    auto kern = std::isnormal(inv) && std::isnormal(inv4) ? k_features<false> : k_features<true>;
+    const bool exact = !(std::isnormal(inv) && std::isnormal(inv4)), narrow = g.W <= 4;
+    const int tx = narrow ? 4 : 32, ty = narrow ? 16 : 8, tz = narrow ? 16 : 4;
+    auto kern = narrow ? (exact ? k_features<4, 16, 16, true> : k_features<4, 16, 16, false>)
+                       : (exact ? k_features<32, 8, 4, true> : k_features<32, 8, 4, false>);
+    const int ntx = (g.W + tx - 1) / tx, nty = (g.H + ty - 1) / ty, ntz = (g.D + tz - 1) / tz;
     kern<<<(unsigned)((i64)ntx * nty * ntz), kBlock, 0, st>>>(g, ctx->f, ctx->g, ctx->P.crit, ctx->Q.crit, bound, inv, inv4,
                                                              feat, ctx->mm, ntx, nty);
     k_dilate<<<grid, kBlock, 0, st>>>(g, 0, ctx->mm, active);
