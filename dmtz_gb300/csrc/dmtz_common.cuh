@@ -10,8 +10,9 @@
 //   eup (u32) : 7 x 3 bits, edge -> triangle pairing, coface index + 1
 //   fup (u32) : 12 x 2 bits, triangle -> tetrahedron pairing, coface index + 1
 // The reference's union-valued arrays paired_vertices / _edges / _faces /
-// _tetrahedras are reconstructed from these on demand (pv_ref, pe_ref, pf_ref,
-// pt_ref below); the back-pointer half of every pair is implied.
+// _tetrahedras are reconstructed from these where an id is wanted (k_export;
+// pv_ref, pe_ref and pf_ref of rules.cuh); the back-pointer half of every pair
+// is implied.
 #pragma once
 #include <cstdint>
 #include <cfloat>
@@ -139,10 +140,6 @@ __device__ __forceinline__ bool cell_ok(const Grid &g, int x, int y, int z, int 
 __device__ __forceinline__ void corner_xyz(int c, int &dx, int &dy, int &dz) {
     dx = c & 1; dy = (c >> 1) & 1; dz = (c >> 2) & 1;
 }
-__device__ __forceinline__ int dir_of(int dx, int dy, int dz) {
-    if (dx < -1 || dx > 1 || dy < -1 || dy > 1 || dz < -1 || dz > 1) return -1;
-    return TOPO_DIR_LUT[(dx + 1) + 3 * (dy + 1) + 9 * (dz + 1)];
-}
 // maximum corner offsets of each cell kind (validity test)
 __device__ __forceinline__ void edge_extent(int k, int &mx, int &my, int &mz) {
     int a = TOPO_EDGE_V[k][0] | TOPO_EDGE_V[k][1];
@@ -213,13 +210,7 @@ __device__ __forceinline__ void face_unref(const Grid &g, i64 t, int &x, int &y,
         split3(b, g.dW1H1, g.dW1, z, y, x);
     }
 }
-__device__ __forceinline__ void tet_unref(const Grid &g, i64 t, int &x, int &y, int &z, int &s) {
-    const unsigned long long u = (unsigned long long)t, b = u / 6;
-    s = (int)(u - 6 * b);
-    split3(b, g.dW1H1, g.dW1, z, y, x);
-}
 
-// packed field accessors
 // The kernel launched behind this one (launch_next) may start; and, there: wait
 // until the kernel before is done and its memory visible.  No effect otherwise.
 __device__ __forceinline__ void let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -237,6 +228,7 @@ __device__ __forceinline__ unsigned long long agg_slot(unsigned long long *n) {
     base = __shfl_sync(peers, base, leader);
     return base + (unsigned long long)__popc(peers & ((1u << lane) - 1u));
 }
+// packed field accessors
 __device__ __forceinline__ int eup_get(uint32_t w, int k) { return (w >> (3 * k)) & 7; }
 __device__ __forceinline__ int fup_get(uint32_t w, int s) { return (w >> (2 * s)) & 3; }
 
