@@ -28,6 +28,7 @@
 #include "cnn.cuh"
 #include "dmtz_common.cuh"
 #include "gradient.cuh"
+#include "record_sort.h"
 #include "report_wait.cuh"
 #include "rules.cuh"
 
@@ -182,6 +183,12 @@ __global__ void k_export(Grid g, FieldState s, int32_t *PV, int32_t *PE, int32_t
             PT[tet_ref(g, x, y, z, ts)] = (int32_t)val;
         }
     }
+}
+
+// Reference ids in place of cell codes, in a list for the host.  (Decoded there, a code
+// took several 64-bit divisions.)
+__global__ void __launch_bounds__(kBlock) k_refs(Grid g, i64 *codes, i64 n) {
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) codes[i] = code_ref(g, codes[i]);
 }
 
 // --------------------------------------------------------------- fix rules
@@ -2673,6 +2680,16 @@ static dmtz_status setup_pair(dmtz_ctx *ctx, const Grid &g, const double *orig, 
     return fit_lists(ctx, g, 1, hc);
 }
 
+// the reference ids of a list's first out.size() cells (their codes are gone then)
+static dmtz_status fetch_refs(dmtz_ctx *ctx, const Grid &g, i64 *codes, std::vector<i64> &out) {
+    const i64 n = (i64)out.size();
+    k_refs<<<std::min(grid_for(n), persistent_grid()), kBlock, 0, ctx->stream>>>(g, codes, n);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(out.data(), codes, sizeof(i64) * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    return DMTZ_OK;
+}
+
 dmtz_status dmtz_mismatch(dmtz_ctx *ctx, int W, int H, int D, const double *orig, const double *decp,
                           int64_t counts[4], int32_t *lmin, int32_t *lsad, int32_t *l2sad, int32_t *lmax) {
     Grid g;
@@ -2688,8 +2705,7 @@ dmtz_status dmtz_mismatch(dmtz_ctx *ctx, int W, int H, int D, const double *orig
         counts[k] = (int64_t)hc[k];
         if (!outs[k] || !hc[k]) continue;
         std::vector<i64> tmp(hc[k]);
-        CK(cudaMemcpy(tmp.data(), ctx->lists[k], sizeof(i64) * hc[k], cudaMemcpyDeviceToHost));
-        for (i64 &q : tmp) q = code_ref(g, q);
+        if ((s = fetch_refs(ctx, g, ctx->lists[k], tmp)) != DMTZ_OK) return s;
         std::sort(tmp.begin(), tmp.end());
         for (size_t i = 0; i < tmp.size(); i++) outs[k][i] = (int32_t)tmp[i];
     }
@@ -2778,15 +2794,17 @@ static dmtz_status path_detect_impl(dmtz_ctx *ctx, int W, int H, int D, const do
     }
     counts[0] = (int64_t)hc[0];
     counts[1] = (int64_t)hc[1];
-    // codes to reference ids (the second column of the descending records holds vertices)
+    // (the second column of the descending records holds vertices, not codes)
     auto fetch = [&](i64 *da, i64 *db, unsigned long long n, int32_t *oa, int32_t *ob, bool vert) -> dmtz_status {
         if (!n || !oa) return DMTZ_OK;
         std::vector<i64> a(n), b(n);
-        CK(cudaMemcpy(a.data(), da, sizeof(i64) * n, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(b.data(), db, sizeof(i64) * n, cudaMemcpyDeviceToHost));
+        dmtz_status r = fetch_refs(ctx, g, da, a);
+        if (r == DMTZ_OK && !vert) r = fetch_refs(ctx, g, db, b);
+        if (r != DMTZ_OK) return r;
+        if (vert) CK(cudaMemcpy(b.data(), db, sizeof(i64) * n, cudaMemcpyDeviceToHost));
         std::vector<std::pair<i64, i64>> p(n);
-        for (size_t i = 0; i < n; i++) p[i] = {code_ref(g, a[i]), vert ? b[i] : code_ref(g, b[i])};
-        std::sort(p.begin(), p.end());
+        for (size_t i = 0; i < n; i++) p[i] = {a[i], b[i]};
+        sort_records(p);
         for (size_t i = 0; i < n; i++) {
             oa[i] = (int32_t)p[i].first;
             if (ob) ob[i] = (int32_t)p[i].second;

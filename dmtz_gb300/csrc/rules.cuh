@@ -476,15 +476,11 @@ __host__ __device__ __forceinline__ int cell_kind(i64 code) {
     return b == 0 ? KIND_VERTEX : b < 8 ? KIND_EDGE : b < 20 ? KIND_FACE : KIND_TET;
 }
 // reference id of a cell
-__host__ __device__ __forceinline__ i64 code_ref(const Grid &g, i64 code) {
+__device__ __forceinline__ i64 code_ref(const Grid &g, i64 code) {
     const i64 v = code >> 5;
     const int b = (int)(code & 31);
-#ifdef __CUDA_ARCH__
     int x, y, z;
     decode_v(g, v, x, y, z);
-#else
-    const i64 x = v % g.W, y = (v / g.W) % g.H, z = v / g.WH;
-#endif
     return b == 0 ? v : b < 8 ? edge_ref(g, x, y, z, b - 1) : b < 20 ? face_ref(g, x, y, z, b - 8) : tet_ref(g, x, y, z, b - 20);
 }
 
