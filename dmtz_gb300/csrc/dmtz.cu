@@ -42,10 +42,10 @@ static inline unsigned grid_for(i64 n) { return (unsigned)std::max<i64>(1, (n + 
 // --------------------------------------------------------------- mismatch compaction
 // A kernel launched so starts while the one before it on the stream still runs, up
 // to its own after_previous(); the one before must let it (let_next).  The
-// kernels of a round are short, so their launches show: a host-driven loop over a
-// 64^3 field's extrema takes 12.5 ms so and 13.5 ms without.  Not while a graph is
-// captured: inside a loop graph's conditional nodes such an edge costs more than it
-// hides (noisy 97 x 61 x 75 field: 19.5 ms with, 19.0 without).
+// kernels of a round are short, so their launches show: a host-driven loop over the
+// extrema of a 64^3 Gaussian mixture (uniform noise of 1e-3, seed 1) takes 10.3 ms so
+// and 10.8 ms without.  Not while a graph is captured: inside a loop graph's conditional
+// nodes such an edge costs what it hides (97 x 61 x 75, noise of 1e-2, seed 1: 13.6 ms both).
 template <typename... P, typename... A>
 static void launch_next(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A &&...args) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -89,7 +89,8 @@ struct BrickMarks {
     uint32_t *list;   // packed brick coordinates
     unsigned long long *n;
     int nbx, nby, shx, shy, shz;
-    int lanes;  // per vertex: 8 where the reach spans at most two bricks per axis, else 32 (three)
+    int lanes;   // per vertex: 8 where the reach spans at most two bricks per axis, else 32 (three)
+    i64 sample;  // 0: every updated vertex marks; else about so many of them, blocks of bricks (sampled_marks)
 };
 // Every lane of a warp takes part: lane j of a vertex's lanes has the j-th brick of
 // its reach, so that the marks, and then the list's slots, wait for memory once.
@@ -1141,16 +1142,17 @@ __global__ void __launch_bounds__(kBlock) k_fix_path(const __grid_constant__ Rul
 // The delta is what the reference's buffer holds: get_delta(v), with the
 // buffer's "no request" sentinel -2000*range (a request whose delta is not
 // above the sentinel leaves the buffer unchanged under edit_type 0).
-// Where bricks are marked, a vertex has as many lanes as its reach has bricks
+// Where bricks are marked (mark), a vertex has as many lanes as its reach has bricks
 // (see mark_dirty) and the first of them updates it.
 __device__ __forceinline__ void apply_requests(const RuleCtx &c, double range, int preserve_type, int update, uint8_t *changed,
-                                               double *delta_out, const BrickMarks &B, unsigned block, unsigned blocks) {
+                                               double *delta_out, const BrickMarks &B, bool mark, unsigned block,
+                                               unsigned blocks) {
     const i64 n = min((i64)*c.reqn, c.reqcap);
     const double sentinel = -2000.0 * range;
     const double tiny = 1e-15 * range;
     double *g = const_cast<double *>(c.gv);
     int *cnt = const_cast<int *>(c.cnt);
-    const int lane = threadIdx.x & 31, lanes = B.flags ? B.lanes : 1, per = 32 / lanes, j = lane % lanes;
+    const int lane = threadIdx.x & 31, lanes = mark ? B.lanes : 1, per = 32 / lanes, j = lane % lanes;
     const i64 nw = blockDim.x / 32, step = (i64)blocks * nw * per;
     for (i64 base = ((i64)block * nw + (threadIdx.x >> 5)) * per; base < n; base += step) {
         const i64 i = base + lane / lanes;
@@ -1182,14 +1184,26 @@ __device__ __forceinline__ void apply_requests(const RuleCtx &c, double range, i
                 if (changed) changed[v] = 1;
             }
         }
-        if (B.flags) mark_dirty(c.g, B, req && update, v, j);
+        if (mark) mark_dirty(c.g, B, req && update, v, j);
+    }
+}
+// The blocks of bricks that every n / sample-th request reaches, for a round that re-pairs the
+// whole grid and wants to know how much of it the update reached (see sampled_marks).
+__device__ __forceinline__ void sample_bricks(const RuleCtx &c, const BrickMarks &B) {
+    const i64 n = min((i64)*c.reqn, c.reqcap), every = max(n / B.sample, (i64)1), m = (n + every - 1) / every;
+    const int lane = threadIdx.x & 31, per = 32 / B.lanes, j = lane % B.lanes;
+    const i64 nw = blockDim.x / 32, step = (i64)gridDim.x * nw * per;
+    for (i64 base = ((i64)blockIdx.x * nw + (threadIdx.x >> 5)) * per; base < m; base += step) {
+        const i64 i = base + lane / B.lanes;
+        mark_dirty(c.g, B, i < m, i < m ? c.reqlist[i * every] : 0, j);
     }
 }
 __global__ void __launch_bounds__(kBlock) k_apply(const __grid_constant__ RuleCtx c, double range, int preserve_type, int update,
                                                  uint8_t *changed, double *delta_out, const __grid_constant__ BrickMarks B) {
     let_next();
     after_previous();
-    apply_requests(c, range, preserve_type, update, changed, delta_out, B, blockIdx.x, gridDim.x);
+    if (B.sample) sample_bricks(c, B);
+    apply_requests(c, range, preserve_type, update, changed, delta_out, B, B.flags && !B.sample, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------------------- stall breaker
@@ -1907,10 +1921,10 @@ BrickList all_bricks(const Grid &g, int shape, i64 &nb) {
 // The gradient of the whole grid.  Grids whose bricks fit the GPU in one round
 // (three blocks of k_grad_bricks per SM) take one latency of that kernel: 16^3
 // 6.2 us, against 14.4 us for the march's five pipeline steps; larger ones
-// march (64^3: 25 us, 30 us in bricks; 256^3: 862 us, 1634 us in bricks).
-// Tiles of 32 x 16 columns and one block of 640 threads per SM: with two
-// blocks and 48 registers 935 us at 256^3 and 51 us instead of 43 us at 97 x 61 x
-// 75; 32 x 8 with three blocks 874 and 51 us; 64 x 8 1035 and 58 us.
+// march (64^3: 25 us, 32 us in bricks; 256^3: 823 us, 1656 us in bricks).
+// Tiles of 32 x 16 columns and one block of 640 threads per SM (862 us at 256^3
+// when they were compared, 43 us at 97 x 61 x 75): with two blocks and 48 registers 935
+// and 51 us, 32 x 8 with three blocks 874 and 51, 64 x 8 1035 and 58.
 constexpr int kMarchX = 32, kMarchY = 16, kMarchBlocks = 1;
 bool grad_marches(const dmtz_ctx *ctx, const Grid &g) {
     i64 nb;
@@ -2011,6 +2025,7 @@ BrickMarks brick_marks(const dmtz_ctx *ctx, const Grid &g) {
     B.shy = sh[1];
     B.shz = sh[2];
     B.lanes = std::min(sh[0], std::min(sh[1], sh[2])) >= 2 ? 8 : 32;
+    B.sample = 0;
     return B;
 }
 
@@ -2063,16 +2078,39 @@ void repair_dirty(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint3
 void repair_full(dmtz_ctx *ctx, const Grid &g, const FieldState &s, const uint32_t *crit_o, int want_saddles) {
     run_pairing(ctx, g, s, crit_o, want_saddles);
 }
-// Lists with at least this many cells mean a repair of the whole grid: their
-// updates reach most bricks then, and the march's halo is smaller (256^3 with 189 k
-// listed cells and 131 k bricks: 96 % of the bricks, 1.81 ms by bricks, 0.9 ms
-// by the march, which is even at half of the bricks).  Below 8192 bricks the march's
-// pipeline costs what all bricks do (64^3, 2048 bricks: 29 us either way; 97 x 61
-// x 75, 3952 bricks: 56 and 53 us), so such grids are always repaired by bricks.
+// Lists with at least this many cells, after a round that reached at least as many bricks
+// (before the first: any), mean a repair of the whole grid: the update reaches most bricks
+// then, and the march's halo is smaller (256^3: 0.82 ms by the march, 1.66 by all bricks, even
+// at half of them).  With separatrices, so and never whole, power-law fields with an SZ-like
+// error of 1e-4 of the range: 128^3 (16 k bricks) 1.66 and 1.74 ms, 176^3 (43 k) 3.03 and
+// 3.20, 256^3 (131 k) 6.73 and 7.45; with uniform noise of 1e-2: 7.5 and 8.2, 15.3 and 17.3,
+// 39.9 and 48.2.  The cells alone do not say it: in a Gaussian mixture with uniform noise of 1e-3
+// they crowd where the field is flat, and 600 rounds on its extrema took 63 ms at 104^3 (8.8 k
+// bricks), 87 at 128^3 and 157 at 176^3 by the cells alone, 32, 42 and 74 so.
+// Below 8192 bricks such grids are always repaired by bricks: 64^3 (2048 bricks) within 2 %
+// either way, 96^3 (6912) within 4 %, 7 % slower by bricks for extrema in noise everywhere.
 i64 heavy_cells(const dmtz_ctx *ctx, const Grid &g) {
     i64 nb;
     all_bricks(g, ctx->tune_shape, nb);
     return nb >= 8192 ? nb / 2 : INT64_MAX;
+}
+// The marks of a round that re-pairs the whole grid: up to 4096 blocks of bricks, from twice
+// as many of the requests.  They are listed and cleared as bricks are (a block's coordinates
+// are a brick's, too).  *bricks: how many bricks a block stands for.  (With the bricks of all
+// requests 28 rounds at 256^3 took 22.2 ms, with half as many requests as bricks 20.5; without
+// marks 19.6.)
+BrickMarks sampled_marks(const dmtz_ctx *ctx, const Grid &g, i64 *bricks) {
+    BrickMarks B = brick_marks(ctx, g);
+    i64 nb, blocks;
+    const BrickList bl = all_bricks(g, ctx->tune_shape, nb);
+    for (int k = 0;; k++, B.shx++, B.shy++, B.shz++) {
+        auto up = [&](int n) { return (i64)((n + (1 << k) - 1) >> k); };
+        blocks = up(bl.nbx) * up(bl.nby) * up(bl.nbz);
+        if (blocks <= 4096) break;
+    }
+    B.sample = 2 * blocks;
+    *bricks = nb / blocks;
+    return B;
 }
 
 double key_to_double(unsigned long long k) {
@@ -2883,8 +2921,9 @@ dmtz_status dmtz_wall_detect(dmtz_ctx *ctx, int W, int H, int D, const double *o
 namespace {
 enum { LS_CP = 0, LS_PDF = 1, LS_PCHECK = 2, LS_PFIX = 3, LS_CPF = 4, LS_CPS = 5, LS_DONE = 6, LS_STATES = 6 };
 // bodies of the loop graph's switch: the last one is CPF's or CPS's (a body more costs 50 us to
-// instantiate and destroy, 3 % of a 120 x 89 x 101 field's correction; grids that are ever
-// repaired whole have few rounds, the others many short ones)
+// instantiate and destroy, 3 % of a 120 x 89 x 101 field's correction).  Grids that are ever
+// repaired whole go without the short rounds: 3 % of a 128^3 Gaussian mixture's 236 rounds
+// (uniform noise of 1e-3), nothing where there are few rounds
 constexpr int LS_BODIES = 5;
 __host__ __device__ inline bool is_cp(int state) { return state == LS_CP || state == LS_CPF || state == LS_CPS; }
 struct LoopCtl {
@@ -2895,7 +2934,8 @@ struct LoopCtl {
     long long runs[LS_STATES];  // body executions per state (CPS: rounds)
     long long shorts;           // body executions of CPS
     long long cap[4];           // mismatch list capacities
-    long long heavy;            // listed cells from which a round re-pairs the whole grid
+    long long heavy;            // listed cells, and bricks of the round before, from which a round re-pairs the whole grid
+    long long marked, block;    // bricks that the last round reached (before any: all); in one of sampled_marks' blocks
     int overflow;       // a scan overflowed a list: stop, grow, scan again, resume at `state`
     int last;           // state of the last body run
     int break_stalls;   // stop when a round changed nothing (the host breaks the stall)
@@ -2915,7 +2955,7 @@ __device__ __forceinline__ LoopCtl loop_next(LoopCtl c, const unsigned long long
         for (int k = 0; k < 4; k++) c.cc[k] = (long long)counters[k];
     const long long cells = c.cc[0] + c.cc[1] + c.cc[2] + c.cc[3];
     const bool cp_any = cells > 0;
-    const int cp = cells >= c.heavy ? LS_CPF : cells <= c.few ? LS_CPS : LS_CP;
+    const int cp = cells >= c.heavy && c.marked >= c.heavy ? LS_CPF : cells <= c.few ? LS_CPS : LS_CP;
     int next;
     if (is_cp(st)) {
         c.rounds++;
@@ -3008,6 +3048,7 @@ __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Li
     bool stop = false;
     if (ctl) {
         LoopCtl c = *ctl;
+        if (ends && st != LS_PCHECK) c.marked = st == LS_CPF ? nbrick * c.block : nbrick;
         if (ends) c = loop_next(c, counters);
         c.begun = 1;
         c.ended = c.pending = 0;
@@ -3018,6 +3059,7 @@ __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Li
         if (!stop && (c.state == LS_PDF || c.state == LS_PCHECK)) counters[5] = counters[6] = counters[27] = 0;
     } else {
         for (int k = 0; k < 8; k++) report[k] = counters[k];
+        report[14] = (unsigned long long)nbrick;
         __threadfence_system();
         *reinterpret_cast<volatile unsigned long long *>(report + 8) = seq;
     }
@@ -3035,9 +3077,10 @@ __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Li
 // kernels that it stands for, after its update (report[10]).  In the loop graph
 // (ctl) it is the state CPS and goes on from round to round as k_round_end would.  report: [0..7] the
 // counters as after any round, [9] rounds, [11..13] nanoseconds of fix, update and
-// the rest.  Host-driven loops, 16^3: 2.81 -> 2.47 ms, 64^3 extrema: 10.3 -> 9.7; with 384
-// cells and 64 bricks 2.42 and 9.7, but a batch of eight got 3 % slower.  Graph loop, noisy
-// 97 x 61 x 75 field: 17.3 -> 16.5.
+// the rest, [14] (for few bricks) 0.  Gaussian mixtures with uniform noise, seed 1, without and
+// with it: host-driven loops, 16^3 (1e-2) 3.24 and 2.67 ms, 64^3 extrema (1e-3) 11.0 and 10.3;
+// graph loop, 97 x 61 x 75 (1e-2) 14.05 and 13.56; a batch of eight the same.  With 384 cells and
+// 64 bricks the first two were as fast, but the batch got 3 % slower.
 constexpr unsigned kShortBlocks = 16;
 constexpr i64 kShortCells = 64, kShortBricks = 160, kShortRounds = 256;  // at most that many per launch
 __device__ __forceinline__ void cluster_barrier() {
@@ -3078,7 +3121,7 @@ __global__ void __launch_bounds__((brick_threads<8, 4, 4>()), 2)
         fix_cells(c, CL, preserve_saddles, tab, true, block, blocks, (i64)blocks * (blockDim.x / 32));
         cluster_barrier();
         lap(0);
-        apply_requests(c, range, preserve_type, 1, changed, nullptr, B, block, blocks);
+        apply_requests(c, range, preserve_type, 1, changed, nullptr, B, true, block, blocks);
         cluster_barrier();
         lap(1);
         rounds++;
@@ -3131,6 +3174,7 @@ __global__ void __launch_bounds__((brick_threads<8, 4, 4>()), 2)
             for (int k = 0; k < 8; k++) report[k] = counters[k];
         report[9] = (unsigned long long)rounds;
         report[10] = left;
+        report[14] = 0;  // (few)
         for (int k = 0; k < 3; k++) report[11 + k] = ns[k];
         __threadfence_system();
         *reinterpret_cast<volatile unsigned long long *>(report + 8) = seq;
@@ -3259,6 +3303,7 @@ static dmtz_status build_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx 
     cudaStream_t st = ctx->stream;
     const unsigned pgrid = persistent_grid();
     const CpLists L = cp_lists(ctx);
+    i64 block;
     if (!ctx->loopctl) CK(cudaMalloc(&ctx->loopctl, sizeof(LoopCtl)));
     LoopCtl *dctl = static_cast<LoopCtl *>(ctx->loopctl);
     lg.clear();
@@ -3322,7 +3367,7 @@ static dmtz_status build_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx 
                 if (cp) k_fix_cp<<<pgrid, kBlock, 0, st>>>(rc, L, ps);
                 else k_fix_path<<<pgrid, kBlock, 0, st>>>(rc, PR);
                 launch_next(k_apply, pgrid, kBlock, st, rc, range, pt, 1, ctx->changed, nullptr,
-                                                  state == LS_CPF ? BrickMarks{} : brick_marks(ctx, g));
+                            state == LS_CPF ? sampled_marks(ctx, g, &block) : brick_marks(ctx, g));
                 if (state == LS_CPF) repair_full(ctx, g, Qs, ctx->P.crit, want);
                 else repair_dirty(ctx, g, Qs, ctx->P.crit, want, true);
             }
@@ -3552,12 +3597,14 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     // (the counts stand in pinned memory as soon as the round's end wrote them, some
     // microseconds before a wait for the stream would return; a launch of the round
     // that failed shows here)
+    i64 marked = INT64_MAX;  // bricks of the last round
     auto read_fit = [&](int want_saddles) -> dmtz_status {
         const cudaError_t waited = wait_report(ctx->report + 8, ctx->report_seq, [&]() { return cudaStreamQuery(st); });
         CK(cudaGetLastError());
         CK(waited);
         const volatile unsigned long long *report = ctx->report;
         for (int k = 0; k < 8; k++) hc[k] = report[k];
+        marked = (i64)report[14];
         return fit_lists(ctx, g, want_saddles, hc);
     };
     if ((s = read_counts()) != DMTZ_OK || (s = fit_lists(ctx, g, 1, hc)) != DMTZ_OK) return s;
@@ -3574,6 +3621,8 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
     i64 n_as = 1, n_ds = 1, n_wall = 1;
     ctx->inc_scan = inc;
     const i64 heavy = heavy_cells(ctx, g);
+    i64 block;
+    const BrickMarks whole = sampled_marks(ctx, g, &block);
     i64 rounds = 0;
     int converged = 1;
     if (walls && (s = ensure_walls(ctx)) != DMTZ_OK) return s;
@@ -3590,8 +3639,10 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
         c.break_stalls = opts->break_stalls ? 1 : 0;
         for (int k = 0; k < 4; k++) c.cc[k] = cc[k];
         c.heavy = heavy;
+        c.marked = marked;
+        c.block = block;
         c.few = graph_short_rounds(ctx, g) ? kShortCells : 0;
-        auto cp_state = [&](i64 cells) { return cells >= heavy ? LS_CPF : cells <= c.few ? LS_CPS : LS_CP; };
+        auto cp_state = [&](i64 cells) { return cells >= heavy && marked >= heavy ? LS_CPF : cells <= c.few ? LS_CPS : LS_CP; };
         c.state = cp_any() ? cp_state(cc[0] + cc[1] + cc[2] + cc[3]) : (pvp ? LS_PDF : LS_DONE);
         LoopCtl fin = c;
         if (c.state != LS_DONE) {
@@ -3615,6 +3666,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
                         return s;
                     R.stall_breaks++;
                     if ((s = read_fit(cpst ? (ps == 1) : 1)) != DMTZ_OK) return s;
+                    cur.marked = marked;
                     cur.stalled = 0;
                     for (int k = 0; k < 4; k++) cur.cc[k] = (long long)hc[k];
                     const bool any = hc[0] || hc[1] || hc[2] || hc[3];
@@ -3692,11 +3744,12 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             }
             rounds++;
             R.cp_rounds++;
-            const bool full = cc[0] + cc[1] + cc[2] + cc[3] >= heavy;
+            const bool full = cc[0] + cc[1] + cc[2] + cc[3] >= heavy && marked >= heavy;
             pt_.mark(PH_FIXCP);
             k_fix_cp<<<pgrid, kBlock, 0, st>>>(rc, cp_lists(ctx), ps);
             pt_.mark(PH_APPLY);
-            launch_next(k_apply, pgrid, kBlock, st, rc, range, pt, 1, ctx->changed, nullptr, full ? BrickMarks{} : brick_marks(ctx, g));
+            launch_next(k_apply, pgrid, kBlock, st, rc, range, pt, 1, ctx->changed, nullptr,
+                        full ? whole : brick_marks(ctx, g));
             ctx->launches += 2;
             pt_.mark(PH_PAIR);
             if (full) {  // lists in place: nothing to take back
@@ -3710,7 +3763,9 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
                 host_round_end(ctx, g);
             }
             pt_.stop();
-            if ((s = read_fit(ps == 1)) != DMTZ_OK || (s = stalled()) != DMTZ_OK) return s;
+            if ((s = read_fit(ps == 1)) != DMTZ_OK) return s;
+            if (full) marked *= block;
+            if ((s = stalled()) != DMTZ_OK) return s;
             for (int k = 0; k < 4; k++) cc[k] = (i64)hc[k];
         }
         if (rounds >= max_rounds) {
