@@ -15,9 +15,10 @@
 //            128 rows of a product are a plane across x, which marches (the
 //            default path; see its comment).
 //   k_conv_out  the last layer, of which one channel is needed.
-//   k_conv_tc  all layers with a box of vertices per MMA chain.
+//   k_conv_tc  all layers with a box of vertices per MMA chain (tensor path 1;
+//            slower than the default at every size, there to compare with).
 //   k_conv   the same convolution on mma.sync.m16n8k16 (bf16 in, f32
-//            accumulate).  A block keeps all 27 x out x in weights in shared
+//            accumulate; tensor path 0, as k_conv_tc).  A block keeps all 27 x out x in weights in shared
 //            memory and streams 8x8x4-vertex tiles (+1 halo) through a
 //            cp.async double buffer; operands reach registers by ldmatrix.
 //            The data gradient is the same kernel with transposed weights,
@@ -576,12 +577,11 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv_tc(const __grid_consta
 // Roles: warps 0 and 1 issue the MMAs of every other copy (two slices): the
 // tensor pipe takes a product only when one before it is done, so the 400
 // cycles that a warp spends on waits and commits would be idle, were there no
-// other.  The whole warp walks and one elected lane issues: inside a branch on
-// the lane, the descriptors would be moved to uniform registers one by one,
-// which took longer than the products.  Warp 2 brings the copies (full / empty
-// barriers), warps 3..10 the weights, and then they run the epilogue, half of
-// the channels of a lane quarter each, from four accumulators in turn.  Waits
-// are bounded as in k_conv_tc.
+// other.  The whole warp walks and one elected lane issues: issued inside a
+// branch on the lane, a product took 67 cycles whatever its width.  Warp 2
+// brings the copies (full / empty barriers), warps 3..10 the weights, and then
+// they run the epilogue, half of the channels of a lane quarter each, from four
+// accumulators in turn.  Waits are bounded as in k_conv_tc.
 //
 // Bound by the products: 59 cycles for N = 96, the rate of back-to-back MMAs of
 // that shape, and 47 for N = 48 (and for anything narrower).  161 x 127 x 110,
@@ -1651,7 +1651,7 @@ struct dmtz_cnn {
     int lastW = 0, lastH = 0, lastD = 0, last_train = 0;
     const bf16 *last_feat = nullptr;
     const float *last_out = nullptr;
-    // convolutions on tcgen05 (1, the default) or on mma.sync (0)
+    // convolutions on tcgen05, three taps per product (2, the default) or one (1), or on mma.sync (0)
     int tensor_path = 2;
     unsigned *lticket = nullptr;
     std::map<const void *, int> per_sm;  // blocks of a kernel that an SM holds

@@ -39,7 +39,7 @@
 // reference has them, took 3454 thread instructions per anchor, six stagings
 // of the state between the passes and a separate kernel per pass for the
 // surface anchors; this takes about 1000.  Measured on GB300, a whole
-// gradient: 256^3 3.32 -> 0.86 ms, 120 x 89 x 101 337 -> 72 us, 64^3 25 us,
+// gradient: 256^3 3.32 -> 0.82 ms, 120 x 89 x 101 337 -> 72 us, 64^3 25 us,
 // 16^3 6.2 us.  A repair also covers less: a changed value reaches anchors
 // 2 below to 1 above, where the passes' widest reach was 5 to either side.
 #pragma once

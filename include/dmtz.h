@@ -343,7 +343,10 @@ dmtz_status dmtz_cnn_backward(dmtz_cnn *net, int W, int H, int D, const float *t
  * 2 (the default) = tcgen05.mma with the three x-taps of each (y, z) offset in one product
  * of three times the width (partial sums shifted and added in the epilogue),
  * 0 = the warp-level mma.sync kernels.  Same arithmetic (bf16 products, f32
- * sums); results differ only in the order of the f32 sums. */
+ * sums); results differ only in the order of the f32 sums.  Path 2 was the fastest
+ * at every size measured (forward pass on paths 0, 1 and 2: 256^3 10.5, 5.7 and 1.65 ms,
+ * 16^3 66, 83 and 54 us, 1 x 2000 x 1000 9.9, 5.4 and 0.39 ms); the others are there
+ * to compare with. */
 dmtz_status dmtz_cnn_set_tensor_path(dmtz_cnn *net, int path);
 /* Measurement only: the tensor pipe's rate, in TFLOP/s over all SMs, for
  * back-to-back tcgen05.mma of shape M = 128, N = n (32, 48, 64, 96, 128 or
