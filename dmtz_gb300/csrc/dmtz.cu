@@ -1189,21 +1189,28 @@ __device__ __forceinline__ void apply_requests(const RuleCtx &c, double range, i
 }
 // The blocks of bricks that every n / sample-th request reaches, for a round that re-pairs the
 // whole grid and wants to know how much of it the update reached (see sampled_marks).
-__device__ __forceinline__ void sample_bricks(const RuleCtx &c, const BrickMarks &B) {
+__device__ __forceinline__ void sample_bricks(const RuleCtx &c, const BrickMarks &B, unsigned block, unsigned blocks) {
     const i64 n = min((i64)*c.reqn, c.reqcap), every = max(n / B.sample, (i64)1), m = (n + every - 1) / every;
     const int lane = threadIdx.x & 31, per = 32 / B.lanes, j = lane % B.lanes;
-    const i64 nw = blockDim.x / 32, step = (i64)gridDim.x * nw * per;
-    for (i64 base = ((i64)blockIdx.x * nw + (threadIdx.x >> 5)) * per; base < m; base += step) {
+    const i64 nw = blockDim.x / 32, step = (i64)blocks * nw * per;
+    for (i64 base = ((i64)block * nw + (threadIdx.x >> 5)) * per; base < m; base += step) {
         const i64 i = base + lane / B.lanes;
         mark_dirty(c.g, B, i < m, i < m ? c.reqlist[i * every] : 0, j);
     }
 }
+// SAMPLE: in a round that re-pairs the whole grid; the first blocks sample, beside the others' updates
+constexpr unsigned kSampleBlocks = 64;
+template <bool SAMPLE>
 __global__ void __launch_bounds__(kBlock) k_apply(const __grid_constant__ RuleCtx c, double range, int preserve_type, int update,
                                                  uint8_t *changed, double *delta_out, const __grid_constant__ BrickMarks B) {
     let_next();
     after_previous();
-    if (B.sample) sample_bricks(c, B);
-    apply_requests(c, range, preserve_type, update, changed, delta_out, B, B.flags && !B.sample, blockIdx.x, gridDim.x);
+    constexpr unsigned first = SAMPLE ? kSampleBlocks : 0;
+    if (SAMPLE && blockIdx.x < first) {
+        sample_bricks(c, B, blockIdx.x, first);
+        return;
+    }
+    apply_requests(c, range, preserve_type, update, changed, delta_out, B, !SAMPLE && B.flags, blockIdx.x - first, gridDim.x - first);
 }
 
 // ------------------------------------------------------------- stall breaker
@@ -2097,8 +2104,8 @@ i64 heavy_cells(const dmtz_ctx *ctx, const Grid &g) {
 // The marks of a round that re-pairs the whole grid: up to 4096 blocks of bricks, from twice
 // as many of the requests.  They are listed and cleared as bricks are (a block's coordinates
 // are a brick's, too).  *bricks: how many bricks a block stands for.  (With the bricks of all
-// requests 28 rounds at 256^3 took 22.2 ms, with half as many requests as bricks 20.5; without
-// marks 19.6.)
+// requests 28 rounds at 256^3 took 22.2 ms, with half as many requests as bricks 20.5, so 19.8;
+// without marks 19.7.)
 BrickMarks sampled_marks(const dmtz_ctx *ctx, const Grid &g, i64 *bricks) {
     BrickMarks B = brick_marks(ctx, g);
     i64 nb, blocks;
@@ -2780,7 +2787,7 @@ dmtz_status dmtz_fix_round(dmtz_ctx *ctx, int W, int H, int D, const double *ori
     std::vector<double> fill((size_t)g.V, sentinel);
     CK(cudaMemcpyAsync(dd, fill.data(), sizeof(double) * (size_t)g.V, cudaMemcpyHostToDevice, ctx->stream));
     // report the deltas the rules requested, without updating the field
-    k_apply<<<persistent_grid(), kBlock, 0, ctx->stream>>>(rc, range, 0, 0, nullptr, dd, BrickMarks{});
+    k_apply<false><<<persistent_grid(), kBlock, 0, ctx->stream>>>(rc, range, 0, 0, nullptr, dd, BrickMarks{});
     CK(cudaMemcpyAsync(delta_out, dd, sizeof(double) * (size_t)g.V, cudaMemcpyDeviceToHost, ctx->stream));
     int err = 0;
     CK(cudaMemcpyAsync(&err, ctx->errword, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2926,13 +2933,11 @@ enum { LS_CP = 0, LS_PDF = 1, LS_PCHECK = 2, LS_PFIX = 3, LS_CPF = 4, LS_CPS = 5
 // (uniform noise of 1e-3), nothing where there are few rounds
 constexpr int LS_BODIES = 5;
 __host__ __device__ inline bool is_cp(int state) { return state == LS_CP || state == LS_CPF || state == LS_CPS; }
-struct LoopCtl {
+struct LoopState {
     int state, pvp, converged, pad;
     long long rounds, max_rounds, outer, cp_rounds, path_rounds;
     long long cc[4];
     long long n_as, n_ds;
-    long long runs[LS_STATES];  // body executions per state (CPS: rounds)
-    long long shorts;           // body executions of CPS
     long long cap[4];           // mismatch list capacities
     long long heavy;            // listed cells, and bricks of the round before, from which a round re-pairs the whole grid
     long long marked, block;    // bricks that the last round reached (before any: all); in one of sampled_marks' blocks
@@ -2945,12 +2950,15 @@ struct LoopCtl {
     int pending;        // it left a round's repair to k_grad_bricks
     long long few;      // listed cells up to which rounds are short
 };
+struct LoopCtl : LoopState {
+    long long runs[LS_STATES];  // body executions per state (CPS: rounds)
+    long long shorts;           // body executions of CPS
+};
 }  // namespace
 
 // the state after a body run, from the counters it left
-__device__ __forceinline__ LoopCtl loop_next(LoopCtl c, const unsigned long long *counters) {
+__device__ __forceinline__ LoopState loop_next(LoopState c, const unsigned long long *counters) {
     const int st = c.state;
-    c.runs[st]++;
     if (st != LS_PCHECK)
         for (int k = 0; k < 4; k++) c.cc[k] = (long long)counters[k];
     const long long cells = c.cc[0] + c.cc[1] + c.cc[2] + c.cc[3];
@@ -3047,12 +3055,13 @@ __global__ void __launch_bounds__(kBlock) k_round_end(const __grid_constant__ Li
         }
     bool stop = false;
     if (ctl) {
-        LoopCtl c = *ctl;
+        LoopState c = *ctl;
+        if (ends) ctl->runs[st]++;
         if (ends && st != LS_PCHECK) c.marked = st == LS_CPF ? nbrick * c.block : nbrick;
         if (ends) c = loop_next(c, counters);
         c.begun = 1;
         c.ended = c.pending = 0;
-        *ctl = c;
+        static_cast<LoopState &>(*ctl) = c;
         stop = c.state == LS_DONE || c.overflow || c.stalled;
         cudaGraphSetConditional(hswitch, stop ? (unsigned)LS_BODIES : (unsigned)min(c.state, LS_BODIES - 1));
         cudaGraphSetConditional(hwhile, stop ? 0u : 1u);
@@ -3156,9 +3165,12 @@ __global__ void __launch_bounds__((brick_threads<8, 4, 4>()), 2)
                 T.n[k] = 0;
             }
             *B.n = 0;
-            if (ctl) *ctl = loop_next(*ctl, counters);
-            else if (stop)
+            if (ctl) {
+                ctl->runs[ctl->state]++;
+                static_cast<LoopState &>(*ctl) = loop_next(*ctl, counters);
+            } else if (stop) {
                 for (int k = 0; k < 8; k++) report[k] = counters[k];
+            }
             counters[4] = counters[7] = 0;
         }
         cluster_barrier();
@@ -3366,7 +3378,7 @@ static dmtz_status build_graph_loop(dmtz_ctx *ctx, const Grid &g, const RuleCtx 
                 const int want = cp ? (ps == 1) : 1;
                 if (cp) k_fix_cp<<<pgrid, kBlock, 0, st>>>(rc, L, ps);
                 else k_fix_path<<<pgrid, kBlock, 0, st>>>(rc, PR);
-                launch_next(k_apply, pgrid, kBlock, st, rc, range, pt, 1, ctx->changed, nullptr,
+                launch_next(state == LS_CPF ? k_apply<true> : k_apply<false>, pgrid, kBlock, st, rc, range, pt, 1, ctx->changed, nullptr,
                             state == LS_CPF ? sampled_marks(ctx, g, &block) : brick_marks(ctx, g));
                 if (state == LS_CPF) repair_full(ctx, g, Qs, ctx->P.crit, want);
                 else repair_dirty(ctx, g, Qs, ctx->P.crit, want, true);
@@ -3748,7 +3760,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             pt_.mark(PH_FIXCP);
             k_fix_cp<<<pgrid, kBlock, 0, st>>>(rc, cp_lists(ctx), ps);
             pt_.mark(PH_APPLY);
-            launch_next(k_apply, pgrid, kBlock, st, rc, range, pt, 1, ctx->changed, nullptr,
+            launch_next(full ? k_apply<true> : k_apply<false>, pgrid, kBlock, st, rc, range, pt, 1, ctx->changed, nullptr,
                         full ? whole : brick_marks(ctx, g));
             ctx->launches += 2;
             pt_.mark(PH_PAIR);
@@ -3791,7 +3803,7 @@ static dmtz_status correct_impl(dmtz_ctx *ctx, dmtz_cnn *net, int W, int H, int 
             ctx->launches++;
         }
         pt_.mark(PH_APPLY);
-        launch_next(k_apply, pgrid, kBlock, st, rc, range, pt, 1, ctx->changed, nullptr, brick_marks(ctx, g));
+        launch_next(k_apply<false>, pgrid, kBlock, st, rc, range, pt, 1, ctx->changed, nullptr, brick_marks(ctx, g));
         ctx->launches += 2;
         pt_.mark(PH_PAIR);
         repair_dirty(ctx, g, Qs, ctx->P.crit, 1, true);
