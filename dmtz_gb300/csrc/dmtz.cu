@@ -1143,7 +1143,8 @@ __global__ void __launch_bounds__(kBlock) k_fix_path(const __grid_constant__ Rul
 // buffer's "no request" sentinel -2000*range (a request whose delta is not
 // above the sentinel leaves the buffer unchanged under edit_type 0).
 // Where bricks are marked (mark), a vertex has as many lanes as its reach has bricks
-// (see mark_dirty) and the first of them updates it.
+// (see mark_dirty) and the first of them updates it.  (A flag: `c ? BrickMarks{} : B`, with B a
+// kernel's grid-constant parameter, bound to the reference faulted where c held.)
 __device__ __forceinline__ void apply_requests(const RuleCtx &c, double range, int preserve_type, int update, uint8_t *changed,
                                                double *delta_out, const BrickMarks &B, bool mark, unsigned block,
                                                unsigned blocks) {
